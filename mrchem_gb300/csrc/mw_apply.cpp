@@ -46,6 +46,9 @@ constexpr double TIER_TF32 = 2e3;
 // by at most about 3e-13 b, so items with TIER_FP64 < b / tau <= TIER_DF err by at most 0.03 tau;
 // larger ones, and root-scale items under relative precision, run in FP64.
 constexpr double TIER_DF = 1e11;
+// The fixed-point kernel of the FP64 tier (mw_apply_fx.cu) takes finite inputs; a block norm below
+// this means that every value is finite and its square has not overflowed (false for NaN too).
+constexpr double FX_NORM_MAX = 1e150;
 constexpr int NTIER = 4;  // 0 FP64, 1 FP32, 2 TF32 tensor cores, 3 double-FP32
 constexpr double BOUND_PRUNE = 8.0 * 2.8285;  // (sum_f |in_f|) / |block| <= sqrt(8); 8 output components
 
@@ -125,14 +128,17 @@ struct JobState {
     // have, i.e. of the input nodes at that scale and of the coarser leaves (generated inputs)
     std::vector<double> fmax_lv;
     double fmax_at(int lv) const { return lv < (int)fmax_lv.size() ? fmax_lv[lv] : fmax; }
+    bool fixed_point = true;  // every input norm is finite and far from overflow
     void set_fmax(const Tree &t, int n0) {
         fmax = 0.0;
+        fixed_point = true;
         int nl = 1;
         for (const NodeInfo &ni : t.nodes) nl = std::max(nl, ni.n - n0 + 2);
         std::vector<double> at(nl, 0.0), leaf(nl, 0.0);
         for (int i = 0; i < t.nn(); i++) {
             const int lv = t.nodes[i].n - n0;
             const double v = block_norm8(&t.cn[8 * (size_t)i]);
+            fixed_point = fixed_point && v < FX_NORM_MAX;
             fmax = std::max(fmax, v);
             at[lv] = std::max(at[lv], v);
             if (t.nodes[i].child0 < 0) leaf[lv] = std::max(leaf[lv], v);
@@ -150,6 +156,8 @@ struct JobState {
     GenSet gens;
     double *gbase = nullptr;
     float *gbase32 = nullptr;
+    uint32_t *fx = nullptr;      // the input's and the generated blocks' fixed-point digits (FP64 tier)
+    uint32_t *gbase_fx = nullptr;
     float *gbase_tc = nullptr;  // generated blocks in the tensor-core tier's x-pass layout
     std::vector<double> gcn;
     std::vector<std::vector<Cand>> cand;
@@ -282,7 +290,7 @@ struct DevItems {
 };
 
 int *launch_tier(Ctx &ctx, Arena &arena, LevelItems &li, bool root, bool set, int tier, long long chunk,
-                 mw_stats &st, const DevItems *dv = nullptr, bool split_tc = false) {
+                 mw_stats &st, const DevItems *dv = nullptr, bool split_tc = false, bool fixed_point = false) {
     const int nn = (int)li.nodes;
     const size_t ni = (size_t)li.items;
     if (nn == 0) return nullptr;
@@ -305,7 +313,8 @@ int *launch_tier(Ctx &ctx, Arena &arena, LevelItems &li, bool root, bool set, in
         if (m > CHUNK + CHUNK / 2) nsplit += (m + CHUNK / 2) / CHUNK;
     }
     double *scratch = nsplit ? (double *)arena.alloc(sizeof(double) * (size_t)bs * nsplit) : nullptr;
-    if (scratch && !set) MWG_CUDA(cudaMemsetAsync(scratch, 0, sizeof(double) * (size_t)bs * nsplit, ctx.stream));
+    const bool fx = tier == 0 && fixed_point;  // stores its chunks' partial blocks instead of adding into zeros
+    if (scratch && !set && !fx) MWG_CUDA(cudaMemsetAsync(scratch, 0, sizeof(double) * (size_t)bs * nsplit, ctx.stream));
     long used = 0;
     for (int i = 0; i < nn; i++) {
         const long long b0 = li.begin[i], m = li.begin[i + 1] - b0;
@@ -399,6 +408,8 @@ int *launch_tier(Ctx &ctx, Arena &arena, LevelItems &li, bool root, bool set, in
     } else {
         if (tc)
             k_apply_tc05(ctx.dbasis, L, tier == 1, ctx.stream);
+        else if (fx)
+            k_apply_fx(ctx.dbasis, L, ctx.stream);
         else
             k_apply(ctx.dbasis, L, tier, ctx.nsm, ctx.stream);
     }
@@ -508,7 +519,8 @@ double oper_norm_max(const Oper &op) {
 // its component and block norms (FP64 and FP32), and the jobs' ScreenJob entries, uploaded on the
 // context's current stream.  `idx`: the jobs to set up (all of them, or one job group's when the
 // group's inputs arrive during the apply).
-void screen_setup_inputs(Ctx &ctx, std::vector<ApplyJob> &jobs, const std::vector<int> &idx, DevScreen &ds) {
+void screen_setup_inputs(Ctx &ctx, std::vector<ApplyJob> &jobs, const std::vector<JobState> &js,
+                         const std::vector<int> &idx, DevScreen &ds) {
     std::vector<const Tree *> trees;
     std::unordered_map<const Tree *, int> tix;
     for (int j : idx)
@@ -566,6 +578,7 @@ void screen_setup_inputs(Ctx &ctx, std::vector<ApplyJob> &jobs, const std::vecto
         J.in64 = t.d_coefs;
         J.in32 = t.d_coefs32;
         J.intc = t.d_coefs_tc;
+        J.infx = js[j].fx;
     }
     // read by kernels from the pinned staging: with host inputs these tables go up while the later
     // job groups' input blocks still occupy the copy engines
@@ -585,7 +598,7 @@ void screen_setup_inputs(Ctx &ctx, std::vector<ApplyJob> &jobs, const std::vecto
 // The per-apply part that needs no input data: the levels the GPU screens, the operators' tables,
 // and the ScreenJob array; false when an operator falls outside what the kernels encode (bands
 // above 32767), and the host screens instead.  With `inputs_now` the input tables are built too.
-bool screen_setup(Ctx &ctx, std::vector<ApplyJob> &jobs, DevScreen &ds, bool inputs_now) {
+bool screen_setup(Ctx &ctx, std::vector<ApplyJob> &jobs, const std::vector<JobState> &js, DevScreen &ds, bool inputs_now) {
     const Basis &b = ctx.basis;
     // levels whose translations fit the generation tables' 21-bit fields (deeper levels, about
     // 20 scales below the root, are screened on the host)
@@ -607,7 +620,7 @@ bool screen_setup(Ctx &ctx, std::vector<ApplyJob> &jobs, DevScreen &ds, bool inp
     if (inputs_now) {
         std::vector<int> all(jobs.size());
         for (size_t j = 0; j < jobs.size(); j++) all[j] = (int)j;
-        screen_setup_inputs(ctx, jobs, all, ds);
+        screen_setup_inputs(ctx, jobs, js, all, ds);
     }
     ds.on = true;
     return true;
@@ -640,7 +653,7 @@ constexpr size_t SCREEN_SMEM_MAX = 96 * 1024;  // larger walks (very wide bands)
 // screening does.  The group's stream waits for the item arrays with an event.
 void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobState *> &jp,
                       const std::vector<int> &jglob, int level, int zmax, const TierRule &rule, LevelItems *lt,
-                      DevItems &dv, mw_stats &st, double &t_enum, double &t_gen, double &t_items) {
+                      bool fixed_point, DevItems &dv, mw_stats &st, double &t_enum, double &t_gen, double &t_items) {
     const Basis &b = ctx.basis;
     const int K = b.K, bs = b.bs, bsz = 4 * K * K;
     const double K4 = (double)K * K * K * K;
@@ -806,6 +819,8 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
     P.g64 = (double *)ar.alloc(sizeof(double) * (size_t)bs * ng);
     P.g32 = rule.mixed ? (float *)ar.alloc(sizeof(float) * 2 * (size_t)bs * ng) : nullptr;
     P.gtc = rule.tensor ? (float *)ar.alloc(sizeof(float) * P.tx * ng) : nullptr;
+    P.fx = fixed_point ? fx_words(K) : 0;
+    P.gfx = fixed_point ? (uint32_t *)ar.alloc(sizeof(uint32_t) * P.fx * ng) : nullptr;
     int *hs = (int *)ar.halloc(sizeof(int) * (8 * (size_t)NN + 1));
     {
         StreamSwap fast(ctx, ctx.fast);
@@ -824,6 +839,10 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
             k_screen_gen_norms32(P, ngen, ctx.stream);
             st.launches += 3;
             st.generated += ngen;
+            if (fixed_point) {
+                k_to_fx(P.g64, P.gfx, (size_t)ngen, K, ctx.stream);
+                st.launches++;
+            }
             if (rule.mixed) {
                 k_to_fp32_cube(P.g64, P.g32, (size_t)ngen, K, ctx.stream);
                 st.launches++;
@@ -1041,12 +1060,36 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         if (fixed_grid) max_levels = std::max(max_levels, job.out->max_scale() - b.n0 + 1);
         s.R = 1.0;
     }
+    // The FP64 tier's digits of every distinct input tree, for the length of the call, where that tier
+    // has a large share of the items.  They take 1.8 times the blocks' own space: trees that would not
+    // leave room for them go to the kernel that reads the FP64 blocks.
+    const size_t fxw = fx_words(K);
+    ctx.sarena.reset();
+    auto to_digits = [&](JobState &s) {
+        k_to_fx(s.job->inp->d_coefs, s.fx, (size_t)s.job->inp->nn(), K, ctx.stream);
+        st.launches++;
+    };
+    bool digits = !mixed || near_fp64;
+    if (digits) {
+        std::unordered_map<const Tree *, uint32_t *> have;
+        size_t bytes = 0;
+        for (JobState &s : js)
+            if (have.emplace(s.job->inp, nullptr).second) bytes += sizeof(uint32_t) * fxw * (size_t)s.job->inp->nn();
+        digits = ctx.sarena.room_for(bytes);
+        for (JobState &s : js) {
+            if (!digits) break;
+            uint32_t *&d = have[s.job->inp];
+            const bool made = d != nullptr;
+            if (!made) d = (uint32_t *)ctx.sarena.alloc(sizeof(uint32_t) * fxw * (size_t)s.job->inp->nn());
+            s.fx = d;
+            if (!made && !hin) to_digits(s);
+        }
+    }
     // screening on the GPU (mw_screen.cu) when the context asks for it and the jobs fit its tables
     const TierRule rule{mixed, near_fp64, df_only, dfp, tensor};
     DevScreen ds;
     if (ctx.screening == 1) {
-        ctx.sarena.reset();
-        screen_setup(ctx, jobs, ds, hin == nullptr);
+        screen_setup(ctx, jobs, js, ds, hin == nullptr);
     }
     // fixed grid: per level, the output's nodes at that scale
     auto fixed_level_nodes = [&](JobState &s, int n) {
@@ -1134,8 +1177,9 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                     off += 8 * (size_t)in.nn();
                     js[j].set_fmax(in, b.n0);
                     if (mixed) convert_input(in);
+                    if (digits) to_digits(js[j]);
                 }
-                if (ds.on) screen_setup_inputs(ctx, jobs, G.jobs, ds);
+                if (ds.on) screen_setup_inputs(ctx, jobs, js, G.jobs, ds);
                 MWG_CUDA(cudaEventCreateWithFlags(&G.ev_prep, cudaEventDisableTiming));
                 MWG_CUDA(cudaEventRecord(G.ev_prep, ctx.stream));
             }
@@ -1147,6 +1191,8 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         for (JobState *sp : jp) any |= !sp->work.empty();
         if (!any) return false;
         const bool root = (level == 0);
+        bool fixed_point = digits;
+        for (JobState *sp : jp) fixed_point = fixed_point && sp->fixed_point;
         // thresholds and precision-steering weights
         for (JobState *sp : jp) {
             JobState &s = *sp;
@@ -1161,7 +1207,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         const int zmax = ds.on ? level_zrows(jp, sidx) : 0;
         const bool dscreen = ds.on && level < ds.levels && screen_smem(ds.maxT, zmax) <= SCREEN_SMEM_MAX;
         if (dscreen) {
-            screen_level_gpu(ctx, ar, ds, jp, G.jobs, level, zmax, rule, G.lt, dv, st, st.host_enum_ms,
+            screen_level_gpu(ctx, ar, ds, jp, G.jobs, level, zmax, rule, G.lt, fixed_point, dv, st, st.host_enum_ms,
                              st.host_gen_ms, st.host_items_ms);
         } else {
             // phase A: candidate enumeration (host, all the group's nodes in parallel)
@@ -1231,9 +1277,16 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                         st.launches++;
                     }
                 }
+                uint32_t *firstfx = nullptr;
+                if (fixed_point && total > 0) {
+                    firstfx = (uint32_t *)ar.alloc(sizeof(uint32_t) * fxw * total);
+                    k_to_fx(first, firstfx, total, b.K, ctx.stream);
+                    st.launches++;
+                }
                 for (JobState *sp : jp) {
                     JobState &s = *sp;
                     s.gbase = s.gens.base;
+                    s.gbase_fx = (firstfx && s.gbase) ? firstfx + fxw * (size_t)((s.gbase - first) / bs) : nullptr;
                     s.gcn.swap(s.gens.cn);
                     s.gbase32 = (first32 && s.gbase) ? first32 + 2 * (s.gbase - first) : nullptr;
                     s.gbase_tc = (firsttc && s.gbase) ? firsttc + tc5_x_stride(b.K) * (size_t)((s.gbase - first) / bs) : nullptr;
@@ -1334,7 +1387,10 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                     LevelItems &T = lt[cd.tier];
                     long long &pi = p[cd.tier];
                     if (cd.tier == 0) {
-                        T.in[pi] = cd.gen ? (const void *)(s.gbase + (size_t)cd.src * bs) : (const void *)inp.block(cd.src);
+                        if (fixed_point)
+                            T.in[pi] = cd.gen ? s.gbase_fx + fxw * (size_t)cd.src : s.fx + fxw * (size_t)cd.src;
+                        else
+                            T.in[pi] = cd.gen ? (const void *)(s.gbase + (size_t)cd.src * bs) : (const void *)inp.block(cd.src);
                         T.ax[pi] = op.d_blocks + (size_t)bxi * bsz;
                         T.ay[pi] = op.d_blocks + (size_t)byi * bsz;
                         T.az[pi] = op.d_blocks + (size_t)bzi * bsz;
@@ -1379,7 +1435,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         G.status.clear();
         for (int k = 0; k < NTIER; k++) {
             int *hs = launch_tier(ctx, ar, lt[k], root, false, k, tune.chunk[k], st, dscreen ? &dv : nullptr,
-                                  tensor && k == 1);
+                                  tensor && k == 1, fixed_point);
             if (hs) G.status.push_back({k, hs});
             MWG_CUDA(cudaEventRecord(G.ev[k + 1], ctx.stream));
         }
@@ -2084,6 +2140,17 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
     JobState s;
     s.job = &job;
     for (int i = 0; i < x.nn(); i++) s.fmax = std::max(s.fmax, block_norm8(&x.cn[8 * (size_t)i]));
+    bool fixed_point = true;
+    for (int i = 0; i < y.nn(); i++) fixed_point = fixed_point && block_norm8(&y.cn[8 * (size_t)i]) < FX_NORM_MAX;
+    const size_t fxw = fx_words(b.K);
+    uint32_t *yfx = nullptr;
+    ctx.sarena.reset();
+    fixed_point = fixed_point && ctx.sarena.room_for(sizeof(uint32_t) * fxw * (size_t)y.nn());
+    if (fixed_point) {
+        yfx = (uint32_t *)ctx.sarena.alloc(sizeof(uint32_t) * fxw * (size_t)y.nn());
+        k_to_fx(y.d_coefs, yfx, (size_t)y.nn(), b.K, ctx.stream);
+        st.launches++;
+    }
     LevelItems li;
     const int maxn = y.max_scale();
     for (int n = b.n0; n <= maxn; n++) {
@@ -2153,7 +2220,7 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
                 if (q > 0) li.begin.push_back((long long)q);
                 li.out.push_back(ext.block(it.target));
             }
-            li.in.push_back(y.block(it.o));
+            li.in.push_back(fixed_point ? (const void *)(yfx + fxw * (size_t)it.o) : (const void *)y.block(it.o));
             li.ax.push_back(op.d_blocks + (size_t)op.block_index(it.c->t, sidx, -it.c->lx) * bsz);
             li.ay.push_back(op.d_blocks + (size_t)op.block_index(it.c->t, sidx, -it.c->ly) * bsz);
             li.az.push_back(op.d_blocks + (size_t)op.block_index(it.c->t, sidx, -it.c->lz) * bsz);
@@ -2165,7 +2232,7 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
         st.items += (long long)items.size();
         st.items_fp64 += (long long)items.size();
         st.out_nodes += (long long)li.out.size();
-        launch_tier(ctx, ctx.arena, li, root, true, 0, Ctx::Tuning().chunk[0], st);
+        launch_tier(ctx, ctx.arena, li, root, true, 0, Ctx::Tuning().chunk[0], st, nullptr, false, fixed_point);
         ctx.sync();
         st.levels++;
     }

@@ -161,6 +161,7 @@ struct Arena {
     void *halloc(size_t bytes);
     // call only when the GPU no longer reads anything allocated since the last reset
     void reset();
+    bool room_for(size_t bytes) const;  // held already, or a quarter of the device's free memory
     void release();
 };
 
@@ -198,7 +199,7 @@ struct Ctx {
     // task takes per tier (FP64, FP32, TF32, double-FP32) before a node is split into chunks
     struct Tuning {
         int groups = DEFAULT_GROUPS;
-        long long chunk[4] = {4, 32, 96, 8};
+        long long chunk[4] = {8, 32, 96, 8};
     };
     // settings picked by the autotuner (mw_apply_batch_autotune) per (order K, jobs, precision
     // mode); a batched apply with the same key uses them unless overlap is off (groups == 1)
@@ -348,6 +349,11 @@ inline float tf32_round_host(float x) {
     return r;
 }
 // double-FP32 tier: reads the high and low parts of the same shadows and operator blocks
+// the FP64 tier in 62-bit fixed point (mw_apply_fx.cu): L.in are digit blocks of fx_words(K) words that
+// k_to_fx makes from FP64 blocks with finite values, the operator blocks stay FP64
+void k_apply_fx(const DevBasis &b, const ApplyLaunch &L, cudaStream_t s);
+size_t fx_words(int K);
+void k_to_fx(const double *blocks, uint32_t *out, size_t n, int K, cudaStream_t s);
 void k_apply_df(const DevBasis &b, const ApplyLaunch &L, int nsm, cudaStream_t s);
 void k_norms(const DevBasis &b, double *const *blocks, double *const *cn, int n, cudaStream_t s);
 void k_topdown(const DevBasis &b, const PairTask *tasks, int n, cudaStream_t s);
@@ -440,6 +446,7 @@ struct ScreenJob {  // one job of the apply (device)
     const float *cn32, *bn32;  // the same rounded to FP32
     const double *in64;  // the input's blocks and shadows
     const float *in32, *intc;
+    const uint32_t *infx;  // digits of the fixed-point FP64 tier (fx words per block), or null: FP64 blocks
 };
 struct ScreenNode {  // one output node of the level (device)
     double thr, thr2;      // screening threshold of the walk, and of the items after generation
@@ -483,6 +490,8 @@ struct ScreenLevel {
     double *coef;
     double *g64;                // generated blocks and their shadows
     float *g32, *gtc;
+    uint32_t *gfx;
+    size_t fx;                  // words per block of the fixed-point digits; 0: the FP64 tier reads FP64 blocks
     size_t tx, tb;              // floats per block in the TF32 layouts (input, operator)
 };
 // shared memory of the walk kernels: maxT = most terms of an operator, zmax = most (t, lz) rows of

@@ -650,7 +650,10 @@ __global__ void __launch_bounds__(ST) fill_kernel(ScreenLevel P) {
             const size_t bx = (size_t)(ob + cd.lx), by = (size_t)(ob + cd.ly), bz = (size_t)(ob + cd.lz);
             const size_t src = (size_t)cd.src;
             if (tier == 0) {
-                P.in[dst] = cd.gen ? (const void *)(P.g64 + src * P.bs) : (const void *)(J.in64 + src * P.bs);
+                if (P.fx)
+                    P.in[dst] = cd.gen ? (const void *)(P.gfx + P.fx * src) : (const void *)(J.infx + P.fx * src);
+                else
+                    P.in[dst] = cd.gen ? (const void *)(P.g64 + src * P.bs) : (const void *)(J.in64 + src * P.bs);
                 P.ax[dst] = op.b64 + bx * P.bsz;
                 P.ay[dst] = op.b64 + by * P.bsz;
                 P.az[dst] = op.b64 + bz * P.bsz;

@@ -84,6 +84,14 @@ void Arena::reset() {
     total = 0;
 }
 
+bool Arena::room_for(size_t bytes) const {
+    size_t held = 0, free_b = 0, total_b = 0;
+    for (const auto &c : chunks) held += c.size - c.used;
+    if (bytes <= held) return true;
+    MWG_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    return bytes <= held + free_b / 4;
+}
+
 void Arena::release() {
     for (auto &c : chunks) cudaFree(c.ptr);
     for (auto &c : hchunks) cudaFreeHost(c.ptr);
