@@ -2254,7 +2254,8 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
     // projection onto x's grid: keep x's nodes (their blocks now carry the finer parts)
     copy_grid(res, x);
     arena.reset();
-    combine_on_grid(res, {&ext}, {1.0}, arena, &st);
+    const double one = 1.0;
+    combine_on_grid({&res}, {&ext}, &one, arena, &st);
     ext.free_device();
     arena.reset();
     st.host_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
@@ -2265,7 +2266,7 @@ void add(Tree &out, const std::vector<const Tree *> &trees, const std::vector<do
     auto t_start = std::chrono::steady_clock::now();
     build_grid(out, trees);
     ctx.arena.reset();
-    combine_on_grid(out, trees, coefs, ctx.arena, &st);
+    combine_on_grid({&out}, trees, coefs.data(), ctx.arena, &st);
     ctx.arena.reset();
     st.out_nodes += out.nn();
     st.host_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
@@ -2331,14 +2332,27 @@ void rotate(const std::vector<Tree *> &outs, const std::vector<const Tree *> &in
     grid.ctx = &ctx;
     tree_clear(grid);
     build_grid(grid, ins);
+    // an output given twice holds its last row
     const size_t nj = ins.size();
+    std::vector<Tree *> os;
+    std::vector<double> rows;
     for (size_t i = 0; i < outs.size(); i++) {
-        copy_grid(*outs[i], grid);
-        std::vector<double> row(U + i * nj, U + (i + 1) * nj);
-        ctx.arena.reset();
-        combine_on_grid(*outs[i], ins, row, ctx.arena, &st);
-        st.out_nodes += outs[i]->nn();
+        st.out_nodes += grid.nn();
+        if (std::find(outs.begin() + i + 1, outs.end(), outs[i]) != outs.end()) continue;
+        outs[i]->reserve((size_t)grid.nn());
+        os.push_back(outs[i]);
+        rows.insert(rows.end(), U + i * nj, U + (i + 1) * nj);
     }
+    // the outputs' structure is the grid's; the combination writes every block and norm
+#pragma omp parallel for schedule(dynamic, 1)
+    for (long i = 0; i < (long)os.size(); i++) {
+        os[i]->nodes = grid.nodes;
+        os[i]->map = grid.map;
+        os[i]->nroots = grid.nroots;
+        os[i]->cn.assign(8 * (size_t)grid.nn(), 0.0);
+    }
+    ctx.arena.reset();
+    combine_on_grid(os, ins, rows.data(), ctx.arena, &st);
     grid.free_device();
     ctx.arena.reset();
     st.host_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();

@@ -249,8 +249,12 @@ struct GenTask {
     double *cn;         // 8 norms of the generated block
     uint64_t path;      // 3 bits per step, first step in the lowest bits
     int steps;
-    int pad;
+    int flags;          // GEN_FROM_S, GEN_ONLY_S
 };
+// the ancestor is itself a generated block: its wavelet parts are zero and are not read
+constexpr int GEN_FROM_S = 1;
+// only the block's scaling part is written (the first K^3 values), and no norms
+constexpr int GEN_ONLY_S = 2;
 
 struct ProjFunc {
     int kind;  // 0 gaussian sum, 1 hydrogen
@@ -376,6 +380,21 @@ void k_multiply_values_df(const DevBasis &b, const MulVTask *tasks, int n, int n
 // dst[off[r] ..] = the len[r] doubles at src[r], for n ranges (one download of many small arrays)
 void k_gather_ranges(const double *const *src, const long long *off, const int *len, int n, double *dst,
                      cudaStream_t s);
+// Linear combinations of the same input blocks at the nodes of one grid for several output trees
+// (rotations, sums): per node the input blocks (src[first .. first + count) with their tree's index, bit
+// 31 set when only the scaling part is non-zero and stored), out[o] = sum_k U[o][tree k] src_k, and the
+// outputs' component norms, also written to cn_all[o][node][8].
+struct CombineArgs {
+    const double *const *src;
+    const unsigned *tree;
+    const int *first;          // [n + 1]
+    const double *U;           // nout x nin
+    double *const *out;        // per output: block of node 0
+    double *const *cn;         // per output: norms of node 0
+    double *cn_all;
+    int n, nout, nin, K;
+};
+void k_combine(const CombineArgs &A, cudaStream_t s);
 void k_add(const DevBasis &b, const AddTask *tasks, const double *const *src, const double *coefs, int n, int bs,
            cudaStream_t s);
 void k_to_fp32(const double *in, float *out, size_t n, cudaStream_t s);

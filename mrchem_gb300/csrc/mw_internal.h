@@ -42,8 +42,9 @@ void project_hydrogen(double prec, Tree &t, int n, int l, int m, double Z, const
 
 void copy_grid(Tree &out, const Tree &inp);
 void build_grid(Tree &out, const std::vector<const Tree *> &trees);
-void combine_on_grid(Tree &out, const std::vector<const Tree *> &trees, const std::vector<double> &coefs, Arena &arena,
-                     mw_stats *st);
+std::vector<int> match_nodes(const Tree &grid, const Tree &src);
+void combine_on_grid(const std::vector<Tree *> &outs, const std::vector<const Tree *> &trees, const double *U,
+                     Arena &arena, mw_stats *st);
 void copy_func(Tree &out, const Tree &inp, Arena &arena);
 void crop(Tree &t, double prec, bool abs_prec, Arena &arena);
 double dot(const Tree &a, const Tree &b, Arena &arena);

@@ -223,10 +223,15 @@ __global__ void __launch_bounds__(128) generate_kernel(DevBasis b, const GenTask
     double *t1 = scratch + (size_t)blockIdx.x * per, *t2 = t1 + (size_t)N2 * N2 * K, *sc = t2 + (size_t)N2 * K * K;
     for (int t = blockIdx.x; t < n; t += gridDim.x) {
         const GenTask task = tasks[t];
+        const bool from_s = task.flags & GEN_FROM_S, only_s = task.flags & GEN_ONLY_S;
+        if (from_s) {
+            for (int i = threadIdx.x; i < K3; i += blockDim.x) sc[i] = task.anc[i];
+            __syncthreads();
+        }
         for (int s = 0; s < task.steps; s++) {
             const int c = (int)((task.path >> (3 * s)) & 7);
             const int bx = c & 1, by = (c >> 1) & 1, bz = (c >> 2) & 1;
-            if (s == 0) {
+            if (s == 0 && !from_s) {
                 // from the ancestor's full block (component-major, components cx|cy<<1|cz<<2)
                 for (int i = threadIdx.x; i < N2 * N2 * K; i += blockDim.x) {
                     const int x = i % K, YZ = i / K, Y = YZ % N2, Z = YZ / N2;
@@ -276,6 +281,11 @@ __global__ void __launch_bounds__(128) generate_kernel(DevBasis b, const GenTask
             }
             __syncthreads();
         }
+        if (only_s) {
+            for (int i = threadIdx.x; i < K3; i += blockDim.x) task.out[i] = sc[i];
+            __syncthreads();
+            continue;
+        }
         // the block: component 0 = s, components 1..7 = 0; norms likewise
         double ss = 0.0;
         for (int i = threadIdx.x; i < 8 * K3; i += blockDim.x) {
@@ -312,11 +322,16 @@ __global__ void __launch_bounds__(256) generate_kernel_t(DevBasis b, const GenTa
     __syncthreads();
     for (int t = blockIdx.x; t < n; t += gridDim.x) {
         const GenTask task = tasks[t];
+        const bool from_s = task.flags & GEN_FROM_S, only_s = task.flags & GEN_ONLY_S;
+        if (from_s) {
+            for (int i = threadIdx.x; i < K3; i += blockDim.x) sc[i] = task.anc[i];
+            __syncthreads();
+        }
         for (int s = 0; s < task.steps; s++) {
             const int c = (int)((task.path >> (3 * s)) & 7);
             const double *wx = wt + (c & 1) * K * N2, *wy = wt + ((c >> 1) & 1) * K * N2,
                          *wz = wt + ((c >> 2) & 1) * K * N2;
-            if (s == 0) {
+            if (s == 0 && !from_s) {
                 for (int i = threadIdx.x; i < N2 * N2 * K; i += blockDim.x) {
                     const int x = i % K, YZ = i / K, Y = YZ % N2, Z = YZ / N2;
                     const int cyz = ((Y >= K) ? 2 : 0) | ((Z >= K) ? 4 : 0);
@@ -368,6 +383,11 @@ __global__ void __launch_bounds__(256) generate_kernel_t(DevBasis b, const GenTa
                 }
             }
             __syncthreads();
+        }
+        if (only_s) {
+            for (int i = threadIdx.x; i < K3; i += blockDim.x) task.out[i] = sc[i];
+            __syncthreads();
+            continue;
         }
         double ss = 0.0;
         for (int i = threadIdx.x; i < 8 * K3; i += blockDim.x) {
@@ -804,6 +824,72 @@ __global__ void add_kernel(DevBasis b, const AddTask *tasks, const double *const
     }
 }
 
+// One CTA per node and group of NO outputs; a thread owns elements of the block and keeps its NO sums in
+// registers, so that an input block is read once for NO outputs (add_kernel, one launch per output, read
+// every input again for each).  Bound: the FP64 pipe (1.6 multiply-adds per SM and cycle: NO per element
+// and input) for rotations of many inputs, HBM for sums of a few; the zero wavelet parts of generated
+// blocks are neither stored nor multiplied.  The sums run in input order, as add_kernel's.
+template <int NO>
+__global__ void __launch_bounds__(256) combine_kernel(CombineArgs A) {
+    __shared__ double s_red[8][NO];
+    extern __shared__ double s_u[];  // [input][NO]
+    const int K3 = A.K * A.K * A.K, bs = 8 * K3, o0 = blockIdx.y * NO, no = min(NO, A.nout - o0);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < A.nin * NO; i += blockDim.x) {
+        const int k = i / NO, o = i % NO;
+        s_u[i] = o < no ? A.U[(size_t)(o0 + o) * A.nin + k] : 0.0;
+    }
+    __syncthreads();
+    for (int t = blockIdx.x; t < A.n; t += gridDim.x) {
+        const int f = A.first[t], cnt = A.first[t + 1] - f;
+        for (int c = 0; c < 8; c++) {
+            double sq[NO];
+#pragma unroll
+            for (int o = 0; o < NO; o++) sq[o] = 0.0;
+            for (int i = threadIdx.x; i < K3; i += blockDim.x) {
+                double acc[NO];
+#pragma unroll
+                for (int o = 0; o < NO; o++) acc[o] = 0.0;
+                for (int k = 0; k < cnt; k++) {
+                    const unsigned tr = __ldg(A.tree + f + k);
+                    if (c > 0 && (tr >> 31)) continue;
+                    const double x = __ldg(A.src[f + k] + (size_t)c * K3 + i);
+                    const double *u = s_u + (tr & 0x7fffffffu) * NO;
+#pragma unroll
+                    for (int o = 0; o < NO; o++) acc[o] += u[o] * x;
+                }
+#pragma unroll
+                for (int o = 0; o < NO; o++) {
+                    if (o < no) A.out[o0 + o][(size_t)t * bs + (size_t)c * K3 + i] = acc[o];
+                    sq[o] += acc[o] * acc[o];
+                }
+            }
+#pragma unroll
+            for (int o = 0; o < NO; o++) {
+                for (int s = 16; s > 0; s >>= 1) sq[o] += __shfl_xor_sync(0xffffffffu, sq[o], s);
+                if (lane == 0) s_red[w][o] = sq[o];
+            }
+            __syncthreads();
+            if (threadIdx.x < no) {
+                double s = 0.0;
+                for (int i = 0; i < 8; i++) s += s_red[i][threadIdx.x];
+                s = sqrt(s);
+                A.cn[o0 + threadIdx.x][8 * (size_t)t + c] = s;
+                A.cn_all[((size_t)(o0 + threadIdx.x) * A.n + t) * 8 + c] = s;
+            }
+            __syncthreads();
+        }
+    }
+}
+
+template <int NO>
+void launch_combine(const CombineArgs &A, cudaStream_t s) {
+    const size_t smem = sizeof(double) * (size_t)A.nin * NO;
+    if (smem > 40 * 1024) kernel_smem((const void *)combine_kernel<NO>, (int)smem);
+    combine_kernel<NO><<<dim3(std::min(A.n, 65535), (A.nout + NO - 1) / NO), 256, smem, s>>>(A);
+    MWG_CUDA(cudaGetLastError());
+}
+
 __global__ void to_fp32_kernel(const double *in, float *out, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         out[i] = (float)in[i];
@@ -969,6 +1055,18 @@ void k_add(const DevBasis &b, const AddTask *tasks, const double *const *src, co
     if (n <= 0) return;
     add_kernel<<<grid_for(n), 256, 8 * 256 * sizeof(double), s>>>(b, tasks, src, coefs, n, bs);
     MWG_CUDA(cudaGetLastError());
+}
+
+// outputs per CTA: as many as there are, up to 8 (each input element is then read once for 8 outputs);
+// sums of more inputs than fit in shared memory eight at a time go one output at a time
+void k_combine(const CombineArgs &A, cudaStream_t s) {
+    if (A.n <= 0 || A.nout <= 0) return;
+    if (A.nout >= 5 && A.nin <= 2048)
+        launch_combine<8>(A, s);
+    else if (A.nout >= 2 && A.nin <= 4096)
+        launch_combine<4>(A, s);
+    else
+        launch_combine<1>(A, s);
 }
 
 void k_to_fp32(const double *in, float *out, size_t n, cudaStream_t s) {

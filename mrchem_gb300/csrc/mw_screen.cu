@@ -573,7 +573,7 @@ __global__ void gen_tasks_kernel(ScreenLevel P, GenTask *tasks, int ngen) {
         for (int d = 0; d < 3; d++) c |= (uint64_t)((gi[3 + d] >> sh) & 1) << d;
         tk.path |= c << (3 * s);
     }
-    tk.pad = 0;
+    tk.flags = 0;
     tasks[i] = tk;
 }
 

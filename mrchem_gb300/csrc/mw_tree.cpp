@@ -422,7 +422,7 @@ void generate_all(const std::vector<std::pair<GenSet *, const Tree *>> &sets, Ar
                 for (int d = 0; d < 3; d++) c |= (uint64_t)((k.l[d] >> sh) & 1) << d;
                 tk.path |= c << (3 * s);
             }
-            tk.pad = 0;
+            tk.flags = 0;
         }
         off += (long)gs.keys.size();
     }
@@ -1000,61 +1000,133 @@ void build_grid(Tree &out, const std::vector<const Tree *> &trees) {
     tree_zero(out, before, out.nn() - before);
 }
 
-// out <- linear combination of trees on out's current grid (generated where coarser)
-void combine_on_grid(Tree &out, const std::vector<const Tree *> &trees, const std::vector<double> &coefs, Arena &arena,
-                     mw_stats *st) {
-    Ctx &ctx = *out.ctx;
-    int N = out.nn();
-    std::vector<GenSet> gens(trees.size());
-    std::vector<double *> gbase(trees.size(), nullptr);
-    std::vector<double> gcn;
-    for (size_t k = 0; k < trees.size(); k++) {
-        const Tree &src = *trees[k];
+// The grid's nodes in another tree of the context: the node's index, or -2 - a where the tree ends above
+// it in leaf a.  Parents come before their children in a tree's arrays and siblings are consecutive, so
+// one walk down the grid needs no key lookups.
+std::vector<int> match_nodes(const Tree &grid, const Tree &src) {
+    std::vector<int> m(grid.nn());
+    for (int i = 0; i < grid.nn(); i++) {
+        const int p = grid.nodes[i].parent;
+        if (p < 0) {
+            m[i] = i;  // the roots, in the same order in every tree
+            continue;
+        }
+        const int mp = m[p];
+        if (mp < 0)
+            m[i] = mp;
+        else
+            m[i] = src.nodes[mp].child0 >= 0 ? src.nodes[mp].child0 + (i - grid.nodes[p].child0) : -2 - mp;
+    }
+    return m;
+}
+
+// outs[o] <- sum_k U[o][k] trees[k] on the outputs' common grid.  Blocks missing from an input are
+// generated once for all outputs, one scale step at a time from the block above (only their scaling
+// parts exist), and one launch forms every output.
+void combine_on_grid(const std::vector<Tree *> &outs, const std::vector<const Tree *> &trees, const double *U,
+                     Arena &arena, mw_stats *st) {
+    const Tree &grid = *outs[0];
+    Ctx &ctx = *grid.ctx;
+    const Basis &b = ctx.basis;
+    const int N = grid.nn(), nin = (int)trees.size(), nout = (int)outs.size(), K = b.K, K3 = K * K * K;
+    // generated blocks' zero wavelet parts drop out of the sums only if no coefficient is NaN or infinite
+    bool finite = true;
+    for (size_t i = 0; i < (size_t)nout * nin; i++) finite = finite && std::isfinite(U[i]);
+    std::vector<std::vector<int>> m(nin);
+#pragma omp parallel for schedule(dynamic, 1) if (nin > 1)
+    for (int k = 0; k < nin; k++) m[k] = match_nodes(grid, *trees[k]);
+    // missing blocks: tree k's grid node i is block gen[k][i] of the scratch, made in step `depth`
+    size_t ngen = 0;
+    for (int k = 0; k < nin; k++)
+        for (int i = 0; i < N; i++) ngen += m[k][i] < 0;
+    const size_t gs = finite ? (size_t)K3 : (size_t)b.bs;
+    double *gblk = ngen ? (double *)arena.alloc(sizeof(double) * gs * ngen) : nullptr;
+    double *gcn = ngen && !finite ? (double *)arena.alloc(sizeof(double) * 8 * ngen) : nullptr;
+    std::vector<std::vector<GenTask>> steps;
+    std::vector<std::vector<size_t>> gen(nin);
+    size_t g = 0;
+    for (int k = 0; k < nin; k++) {
+        const Tree &t = *trees[k];
+        gen[k].assign(N, 0);
+        std::vector<int> depth(N, 0);
         for (int i = 0; i < N; i++) {
-            const NodeInfo &nd = out.nodes[i];
-            if (src.find(nd.n, nd.l) >= 0) continue;
-            int a = find_ancestor(src, nd.n, nd.l, nullptr);
-            if (a >= 0) gens[k].request(src, nd.n, nd.l, a);
+            if (m[k][i] >= 0) continue;
+            const int p = grid.nodes[i].parent;
+            depth[i] = depth[p] + 1;
+            gen[k][i] = g;
+            GenTask tk;
+            tk.anc = depth[i] == 1 ? t.block(m[k][p]) : gblk + gs * gen[k][p];
+            tk.out = gblk + gs * g;
+            tk.cn = gcn ? gcn + 8 * g : nullptr;
+            tk.path = (uint64_t)(i - grid.nodes[p].child0);
+            tk.steps = 1;
+            tk.flags = (depth[i] > 1 ? GEN_FROM_S : 0) | (finite ? GEN_ONLY_S : 0);
+            if ((int)steps.size() < depth[i]) steps.resize(depth[i]);
+            steps[depth[i] - 1].push_back(tk);
+            g++;
         }
     }
-    for (size_t k = 0; k < trees.size(); k++) gbase[k] = gens[k].generate(*trees[k], arena, gcn, st);
-    std::vector<AddTask> tasks(N);
     std::vector<const double *> src;
-    std::vector<double> cf;
+    std::vector<unsigned> tree;
+    std::vector<int> first(N + 1, 0);
+    src.reserve((size_t)N * nin);
+    tree.reserve((size_t)N * nin);
     for (int i = 0; i < N; i++) {
-        const NodeInfo &nd = out.nodes[i];
-        tasks[i].out = out.block(i);
-        tasks[i].cn = out.d_cn + (size_t)8 * i;
-        tasks[i].first = (int)src.size();
-        for (size_t k = 0; k < trees.size(); k++) {
-            const Tree &t = *trees[k];
-            int j = t.find(nd.n, nd.l);
-            const double *p = nullptr;
-            if (j >= 0)
-                p = t.block(j);
-            else if (gens[k].slot.count(Key{nd.n, {nd.l[0], nd.l[1], nd.l[2]}}))
-                p = block_at(t, gens[k], gbase[k], nd.n, nd.l);
-            if (!p) continue;
-            src.push_back(p);
-            cf.push_back(coefs[k]);
+        for (int k = 0; k < nin; k++) {
+            const bool made = m[k][i] < 0;
+            src.push_back(made ? gblk + gs * gen[k][i] : trees[k]->block(m[k][i]));
+            tree.push_back((unsigned)k | (made && finite ? 0x80000000u : 0u));
         }
-        tasks[i].count = (int)src.size() - tasks[i].first;
+        first[i + 1] = (int)src.size();
+    }
+    std::vector<double *> ob(nout), oc(nout);
+    for (int o = 0; o < nout; o++) {
+        ob[o] = outs[o]->d_coefs;
+        oc[o] = outs[o]->d_cn;
     }
     Packer pk;
-    pk.add(tasks.data(), tasks.size() * sizeof(AddTask));
     pk.add(src.data(), src.size() * sizeof(double *));
-    pk.add(cf.data(), cf.size() * sizeof(double));
+    pk.add(tree.data(), tree.size() * sizeof(unsigned));
+    pk.add(first.data(), first.size() * sizeof(int));
+    pk.add(U, sizeof(double) * (size_t)nout * nin);
+    pk.add(ob.data(), ob.size() * sizeof(double *));
+    pk.add(oc.data(), oc.size() * sizeof(double *));
+    const int fixed = 6;
+    for (auto &s : steps) pk.add(s.data(), s.size() * sizeof(GenTask));
     pk.ship(ctx, arena);
-    k_add(ctx.dbasis, (const AddTask *)pk.ptr(0), (const double *const *)pk.ptr(1), (const double *)pk.ptr(2), N,
-          ctx.basis.bs, ctx.stream);
-    if (st) st->launches++;
-    MWG_CUDA(cudaMemcpyAsync(out.cn.data(), out.d_cn, sizeof(double) * 8 * N, cudaMemcpyDeviceToHost, ctx.stream));
+    const bool scratch = !(K >= 4 && K <= KMAX);
+    for (size_t d = 0; d < steps.size(); d++) {
+        const int n = (int)steps[d].size(), gg = std::min(n, 4 * std::max(ctx.nsm, 1));
+        double *gscr = scratch ? (double *)arena.alloc(sizeof(double) * generate_scratch_doubles(K) * gg) : nullptr;
+        k_generate(ctx.dbasis, (const GenTask *)pk.ptr(fixed + (int)d), n, gscr, gg, ctx.nsm, ctx.stream);
+    }
+    CombineArgs A;
+    A.src = (const double *const *)pk.ptr(0);
+    A.tree = (const unsigned *)pk.ptr(1);
+    A.first = (const int *)pk.ptr(2);
+    A.U = (const double *)pk.ptr(3);
+    A.out = (double *const *)pk.ptr(4);
+    A.cn = (double *const *)pk.ptr(5);
+    A.cn_all = (double *)arena.alloc(sizeof(double) * 8 * (size_t)N * nout);
+    A.n = N;
+    A.nout = nout;
+    A.nin = nin;
+    A.K = K;
+    k_combine(A, ctx.stream);
+    if (st) {
+        st->launches += 1 + (long long)steps.size();
+        st->generated += (long long)ngen;
+    }
+    double *hcn = (double *)arena.halloc(sizeof(double) * 8 * (size_t)N * nout);
+    MWG_CUDA(cudaMemcpyAsync(hcn, A.cn_all, sizeof(double) * 8 * (size_t)N * nout, cudaMemcpyDeviceToHost, ctx.stream));
     ctx.sync();
+    for (int o = 0; o < nout; o++) std::copy(hcn + 8 * (size_t)N * o, hcn + 8 * (size_t)N * (o + 1), outs[o]->cn.begin());
 }
 
 void copy_func(Tree &out, const Tree &inp, Arena &arena) {
     arena.reset();
-    combine_on_grid(out, {&inp}, {1.0}, arena, nullptr);
+    const double one = 1.0;
+    combine_on_grid({&out}, {&inp}, &one, arena, nullptr);
 }
 
 // remove the children of nodes whose children are all leaves and whose combined
