@@ -181,18 +181,26 @@ void expansion(int kind, double mu, double eps, double rmin, double rmax, double
     }
 }
 
-double expansion_error(int kind, double mu, const std::vector<double> &c, const std::vector<double> &a, double rmin,
-                       double rmax) {
-    double err = 0.0;
+// Whether the expansion's error relative to 1/r is at most eps at 4001 log-spaced r.  A step that is too
+// coarse is off over wide ranges of r, so every 32nd point comes first and most rejected steps end there.
+bool expansion_fits(int kind, double mu, const std::vector<double> &c, const std::vector<double> &a, double rmin,
+                    double rmax, double eps) {
     const int N = 4000;
-#pragma omp parallel for reduction(max : err) schedule(static)
-    for (int i = 0; i <= N; i++) {
+    auto error_at = [&](int i) {
         double r = rmin * std::pow(rmax / rmin, (double)i / N), v = 0.0;
-        for (size_t t = 0; t < c.size(); t++) v += c[t] * std::exp(-a[t] * r * r);
+        for (size_t t = 0; t < c.size(); t++) {
+            const double e = a[t] * r * r;
+            if (e < 746.0) v += c[t] * std::exp(-e);  // exp(-746) is zero
+        }
         double ex = kind == 1 ? std::exp(-mu * r) / r : 1.0 / r;
-        err = std::max(err, std::fabs(v - ex) * r);
-    }
-    return err;
+        return std::fabs(v - ex) * r;
+    };
+    for (int i = 0; i <= N; i += 32)
+        if (!(error_at(i) <= eps)) return false;
+    double err = 0.0;
+#pragma omp parallel for reduction(max : err) schedule(static)
+    for (int i = 0; i <= N; i++) err = std::max(err, error_at(i));
+    return err <= eps;
 }
 
 // Legendre expansion of the scaling-function cross-correlations
@@ -252,7 +260,7 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
         double h = M_PI * M_PI / (2.0 * std::log(1.0 / op->eps));
         for (int it = 0; it < 60; it++) {
             expansion(op->kind, op->mu, op->eps, op->rmin, op->rmax, h, op->c, op->a);
-            if (expansion_error(op->kind, op->mu, op->c, op->a, op->rmin, op->rmax) <= op->eps) break;
+            if (expansion_fits(op->kind, op->mu, op->c, op->a, op->rmin, op->rmax, op->eps)) break;
             h *= 0.93;
         }
         op->T = (int)op->c.size();
@@ -286,20 +294,24 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
     int *d_band = nullptr;
     OpBuildTask *d_tasks = nullptr;
     OpBlockJob *d_jobs = nullptr;
-    MWG_CUDA(cudaMalloc(&d_cc, sizeof(double) * cc.coef.size()));
-    MWG_CUDA(cudaMalloc(&d_q, sizeof(double) * 2 * 16));
-    MWG_CUDA(cudaMalloc(&d_tasks, sizeof(OpBuildTask) * ntask));
-    MWG_CUDA(cudaMalloc(&d_nrm, sizeof(double) * nrm_total));
-    MWG_CUDA(cudaMalloc(&d_band, sizeof(int) * ntask));
-    MWG_CUDA(cudaMalloc(&d_peak, sizeof(double) * ntask));
-    MWG_CUDA(cudaMalloc(&d_head, sizeof(double) * ntask * 4 * OP_NRM_HEAD));
+    // scratch from the stream-ordered pool, which keeps it for the next construction (MRChem builds an
+    // operator per orbital and iteration)
+    double *d_keep = nullptr;
+    MWG_CUDA(cudaMallocAsync(&d_cc, sizeof(double) * cc.coef.size(), st));
+    MWG_CUDA(cudaMallocAsync(&d_q, sizeof(double) * 2 * 16, st));
+    MWG_CUDA(cudaMallocAsync(&d_tasks, sizeof(OpBuildTask) * ntask, st));
+    MWG_CUDA(cudaMallocAsync(&d_nrm, sizeof(double) * nrm_total, st));
+    MWG_CUDA(cudaMallocAsync(&d_band, sizeof(int) * ntask, st));
+    MWG_CUDA(cudaMallocAsync(&d_peak, sizeof(double) * ntask, st));
+    MWG_CUDA(cudaMallocAsync(&d_head, sizeof(double) * ntask * 4 * OP_NRM_HEAD, st));
+    MWG_CUDA(cudaMallocAsync(&d_keep, sizeof(double) * OP_KEEP * (size_t)ntask * bsz, st));
     double q[32];
     std::copy(cc.gx, cc.gx + 16, q);
     std::copy(cc.gw, cc.gw + 16, q + 16);
     MWG_CUDA(cudaMemcpyAsync(d_cc, cc.coef.data(), sizeof(double) * cc.coef.size(), cudaMemcpyHostToDevice, st));
     MWG_CUDA(cudaMemcpyAsync(d_q, q, sizeof(q), cudaMemcpyHostToDevice, st));
     MWG_CUDA(cudaMemcpyAsync(d_tasks, tasks.data(), sizeof(OpBuildTask) * ntask, cudaMemcpyHostToDevice, st));
-    k_op_band(K, cx.dbasis.W, d_cc, d_q, d_q + 16, d_tasks, ntask, d_nrm, d_head, d_band, d_peak, st);
+    k_op_band(K, cx.dbasis.W, d_cc, d_q, d_q + 16, d_tasks, ntask, d_nrm, d_head, d_band, d_peak, d_keep, cx.nsm, st);
     std::vector<int> walked(ntask);
     std::vector<double> peak(ntask), head((size_t)ntask * 4 * OP_NRM_HEAD);
     MWG_CUDA(cudaMemcpyAsync(walked.data(), d_band, sizeof(int) * ntask, cudaMemcpyDeviceToHost, st));
@@ -388,9 +400,9 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
         }
     }
     if (!jobs.empty()) {
-        MWG_CUDA(cudaMalloc(&d_jobs, sizeof(OpBlockJob) * jobs.size()));
+        MWG_CUDA(cudaMallocAsync(&d_jobs, sizeof(OpBlockJob) * jobs.size(), st));
         MWG_CUDA(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(OpBlockJob) * jobs.size(), cudaMemcpyHostToDevice, st));
-        k_op_blocks(K, cx.dbasis.W, d_cc, d_q, d_q + 16, d_tasks, d_jobs, (int)jobs.size(), st);
+        k_op_blocks(K, cx.dbasis.W, d_cc, d_q, d_q + 16, d_tasks, d_jobs, (int)jobs.size(), d_keep, st);
     }
     // device copies for the reduced tiers: FP32 high part then low part per block (FP32 and
     // double-FP32 tiers), and the tensor-core tier's B operand (mw_tc05_layout.h)
@@ -405,10 +417,10 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
         k_op_convert(op->d_blocks, op->d_blocks32, tc ? op->d_blocks_tc : nullptr, op->d_blocks_tc2, nb,
                      K, tc5_n(K), 2 * tc5_ks(K), st);
     }
-    MWG_CUDA(cudaStreamSynchronize(st));
     for (void *pp : {(void *)d_cc, (void *)d_q, (void *)d_tasks, (void *)d_nrm, (void *)d_band, (void *)d_peak,
-                     (void *)d_jobs, (void *)d_head})
-        if (pp) cudaFree(pp);
+                     (void *)d_jobs, (void *)d_head, (void *)d_keep})
+        if (pp) cudaFreeAsync(pp, st);
+    MWG_CUDA(cudaStreamSynchronize(st));
 }
 
 void Oper::free_device() {

@@ -409,12 +409,12 @@ struct OpBlockJob {  // one block pair NS(+l), NS(-l) of a task, at blocks + (of
     long off;
     double *blocks;           // the operator's FP64 blocks
 };
-size_t op_build_smem();
-constexpr int OP_NRM_HEAD = 64;  // translations per task whose norms phase 1 also writes compactly
+constexpr int OP_NRM_HEAD = 16;  // translations per task whose norms phase 1 also writes compactly
+constexpr int OP_KEEP = 3;       // translations per task whose blocks phase 1 keeps for phase 2
 void k_op_band(int K, const double *W, const double *cc, const double *gx, const double *gw, const OpBuildTask *tasks,
-               int ntask, double *nrm, double *head, int *band, double *peak, cudaStream_t s);
+               int ntask, double *nrm, double *head, int *band, double *peak, double *keep, int nsm, cudaStream_t s);
 void k_op_blocks(int K, const double *W, const double *cc, const double *gx, const double *gw, const OpBuildTask *tasks,
-                 const OpBlockJob *jobs, int njob, cudaStream_t s);
+                 const OpBlockJob *jobs, int njob, const double *keep, cudaStream_t s);
 void k_op_convert(const double *blocks, float *b32, float *btc, float *btc2, long nblocks, int K, int NB, int groups,
                   cudaStream_t s);
 // FP32 shadow of whole blocks in cube order cube[Z][Y][X] (X = cx*K + ix): per block a high cube

@@ -8,12 +8,13 @@
 //   G[p] = int_0^1 P_p(2z-1) exp(-beta (z + m)^2) dz
 // by composite 16-point Gauss-Legendre quadrature, as the host construction does (mw_basis.cpp).
 //
-// Phase 1 (one CTA per (term, scale)) walks l = 0, 1, ... and keeps only the four sub-block
-// norms of each NS(l), stopping where the host construction stops: the band follows from them.
-// Phase 2 (one CTA per (term, scale, l) inside the band) recomputes the block, zeroes the
-// sub-blocks the host marked, and writes NS(l) and NS(-l) = NS(l)^T at their final places.
-// All arithmetic is FP64; the quadrature points of a moment are spread over the CTA's threads
-// and their partial sums added in a fixed order, so the blocks are reproducible.
+// Phase 1 walks l = 0, 1, ... of every (term, scale), writes the four sub-block norms of each NS(l) and
+// stops where the host construction stops: the band follows from them.  It keeps the blocks of the first
+// translations.  Phase 2 (one CTA per (term, scale, l) inside the band) zeroes the sub-blocks the host
+// marked, and writes NS(l) and NS(-l) = NS(l)^T at their final places.  All arithmetic is FP64 in a fixed
+// order, so the blocks are reproducible.
+#include <algorithm>
+
 #include "mw_host.h"
 
 namespace mwg {
@@ -22,146 +23,188 @@ namespace {
 
 constexpr int OB_THREADS = 128;
 constexpr int OB_QPTS = 16;
+constexpr int OB_UNIT = 8 * OB_QPTS;  // points of the 8 panels of a kernel wide against [0, 1]
 
+// Shared memory of one CTA, K known at compile time (K = 10: 45 KB, five CTAs per SM).
+template <int K>
 struct ObShared {
-    double G[2][2 * KMAX + 2];              // moments of +m and -m
-    double red[OB_THREADS][2 * KMAX + 2];   // partial sums of the threads
-    double tm1[KMAX * KMAX], t0[KMAX * KMAX], tp1[KMAX * KMAX];
-    double M[4 * KMAX * KMAX], T1[4 * KMAX * KMAX], ns[4 * KMAX * KMAX];
+    static constexpr int N2 = 2 * K;
+    double P[OB_UNIT][N2 + 1];  // P_p(2z-1) at the points of 8 panels on [0, 1]; an odd pitch
+    double W[N2 * N2];
+    double G[4][N2];            // moments
+    double tm1[K * K], t0[K * K], tp1[K * K];
+    double T1[N2 * N2], ns[N2 * N2];
     double nrm[4];
     double gx[OB_QPTS], gw[OB_QPTS];
 };
 
-// G[p] = int_0^1 P_p(2z-1) exp(-beta (z + l)^2) dz, p < np, into S.G[slot] (all threads call)
-__device__ void ob_moments(double beta, double l, int np, int slot, ObShared &S) {
-    const int tid = threadIdx.x;
-    double acc[2 * KMAX + 2];
+// P_0..P_{2K-1} at t by the three-term recurrence
+template <int N2>
+__device__ __forceinline__ void ob_legendre(double t, double (&P)[N2]) {
+    P[0] = 1.0;
+    P[1] = t;
 #pragma unroll
-    for (int p = 0; p < 2 * KMAX + 2; p++) acc[p] = 0.0;
+    for (int j = 1; j + 1 < N2; j++) P[j + 1] = ((2.0 * j + 1.0) / (j + 1.0)) * t * P[j] - (j / (j + 1.0)) * P[j - 1];
+}
+
+// One warp: S.G[slot][p] = int_0^1 P_p(2z-1) exp(-beta (z + l)^2) dz.  The lanes share the points out and
+// their partial sums are added by butterflies, a fixed order.  A kernel wide enough for 8 panels on all of
+// [0, 1] takes its Legendre values from the table.
+template <int K>
+__device__ void ob_moments(double beta, double l, int slot, ObShared<K> &S) {
+    constexpr int N2 = 2 * K;
+    const int lane = threadIdx.x & 31;
+    double acc[N2];
+#pragma unroll
+    for (int p = 0; p < N2; p++) acc[p] = 0.0;
     const double c0 = -l, w = 1.0 / sqrt(beta);
     const double lo = fmax(0.0, c0 - 12.0 * w), hi = fmin(1.0, c0 + 12.0 * w);
     if (lo < hi) {
         const double pw = fmin(0.125, 0.5 * w);
         const int npc = (int)ceil((hi - lo) / pw);
         const double step = (hi - lo) / npc;
-        for (int i = tid; i < npc * OB_QPTS; i += blockDim.x) {
+        const bool unit = npc == 8 && lo == 0.0 && hi == 1.0;
+        for (int i = lane; i < npc * OB_QPTS; i += 32) {
             const int k = i / OB_QPTS, q = i - k * OB_QPTS;
             const double z = (lo + k * step) + step * S.gx[q], e = beta * (z + l) * (z + l);
             if (e > 745.0) continue;
             const double g = step * S.gw[q] * exp(-e);
-            const double t = 2.0 * z - 1.0;
-            double pm = 1.0, pc = t;
-            acc[0] += g;
-            acc[1] += g * t;
+            if (unit) {
 #pragma unroll
-            for (int j = 1; j + 1 < 2 * KMAX + 2; j++) {  // P_{j+1} by the three-term recurrence
-                if (j + 1 >= np) break;
-                const double pn = ((2.0 * j + 1.0) * t * pc - j * pm) / (j + 1.0);
-                acc[j + 1] += g * pn;
-                pm = pc;
-                pc = pn;
+                for (int p = 0; p < N2; p++) acc[p] += g * S.P[i][p];
+            } else {
+                double P[N2];
+                ob_legendre<N2>(2.0 * z - 1.0, P);
+#pragma unroll
+                for (int p = 0; p < N2; p++) acc[p] += g * P[p];
             }
         }
     }
 #pragma unroll
-    for (int p = 0; p < 2 * KMAX + 2; p++)
-        if (p < np) S.red[tid][p] = acc[p];
-    __syncthreads();
-    if (tid < np) {
-        double s = 0.0;
-        for (int r = 0; r < (int)blockDim.x; r++) s += S.red[r][tid];
-        S.G[slot][tid] = s;
+    for (int p = 0; p < N2; p++) {
+        for (int o = 16; o > 0; o >>= 1) acc[p] += __shfl_xor_sync(0xffffffffu, acc[p], o);
+        if (lane == 0) S.G[slot][p] = acc[p];
     }
-    __syncthreads();
 }
 
-// out = tau(m) (K x K), all threads call
-__device__ void ob_tau(int K, double beta, double pref, int m, const double *cc, ObShared &S, double *out) {
-    const int K2 = 2 * K;
-    ob_moments(beta, (double)m, K2, 0, S);
-    ob_moments(beta, (double)(-m), K2, 1, S);
-    for (int e = threadIdx.x; e < K * K; e += blockDim.x) {
+// out = tau(m) (K x K) from the moments of +m (slot gp) and -m (slot gm); tau(-m) is its transpose
+template <int K>
+__device__ __forceinline__ void ob_tau(double pref, const double *cc, const ObShared<K> &S, int gp, int gm, double *out) {
+    constexpr int N2 = 2 * K;
+    for (int e = threadIdx.x; e < K * K; e += OB_THREADS) {
         const int i = e / K, j = e - i * K;
-        const double *aij = cc + (size_t)(i * K + j) * K2, *aji = cc + (size_t)(j * K + i) * K2;
+        const double *aij = cc + (size_t)(i * K + j) * N2, *aji = cc + (size_t)(j * K + i) * N2;
         double v = 0.0;
-        for (int p = 0; p < K2; p++) v += aij[p] * S.G[0][p] + aji[p] * S.G[1][p];
+#pragma unroll
+        for (int p = 0; p < N2; p++) v += __ldg(aij + p) * S.G[gp][p] + __ldg(aji + p) * S.G[gm][p];
         out[e] = pref * v;
     }
-    __syncthreads();
 }
 
 // S.ns = W [[t0, tm1], [tp1, t0]] W^T and its four sub-block norms, all threads call
-__device__ void ob_ns(int K, const double *W, ObShared &S) {
-    const int K2 = 2 * K, KK2 = K2 * K2;
-    for (int e = threadIdx.x; e < KK2; e += blockDim.x) {
-        const int r = e / K2, c = e - r * K2, i = r % K, j = c % K;
-        const double *src = r < K ? (c < K ? S.t0 : S.tm1) : (c < K ? S.tp1 : S.t0);
-        S.M[e] = src[i * K + j];
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < KK2; e += blockDim.x) {
-        const int r = e / K2, c = e - r * K2;
+template <int K>
+__device__ void ob_ns(ObShared<K> &S) {
+    constexpr int N2 = 2 * K;
+    for (int e = threadIdx.x; e < N2 * N2; e += OB_THREADS) {
+        const int r = e / N2, c = e - r * N2, j = c % K;
+        const double *up = c < K ? S.t0 : S.tm1, *dn = c < K ? S.tp1 : S.t0;
         double v = 0.0;
-        for (int k = 0; k < K2; k++) v += W[r * K2 + k] * S.M[k * K2 + c];
+#pragma unroll
+        for (int k = 0; k < K; k++) v += S.W[r * N2 + k] * up[k * K + j];
+#pragma unroll
+        for (int k = 0; k < K; k++) v += S.W[r * N2 + K + k] * dn[k * K + j];
         S.T1[e] = v;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < KK2; e += blockDim.x) {
-        const int r = e / K2, c = e - r * K2;
+    for (int e = threadIdx.x; e < N2 * N2; e += OB_THREADS) {
+        const int r = e / N2, c = e - r * N2;
         double v = 0.0;
-        for (int k = 0; k < K2; k++) v += S.T1[r * K2 + k] * W[c * K2 + k];
+#pragma unroll
+        for (int k = 0; k < N2; k++) v += S.T1[r * N2 + k] * S.W[c * N2 + k];
         S.ns[e] = v;
     }
     __syncthreads();
-    if (threadIdx.x < 4) {
-        const int g = threadIdx.x >> 1, f = threadIdx.x & 1;
+    {  // a warp per sub-block
+        const int q = threadIdx.x >> 5, lane = threadIdx.x & 31, g = q >> 1, f = q & 1;
         double s = 0.0;
-        for (int i = 0; i < K; i++)
-            for (int j = 0; j < K; j++) {
-                const double v = S.ns[(g * K + i) * K2 + f * K + j];
-                s += v * v;
-            }
-        S.nrm[threadIdx.x] = sqrt(s);
+        for (int e = lane; e < K * K; e += 32) {
+            const double v = S.ns[(g * K + e / K) * N2 + f * K + e % K];
+            s += v * v;
+        }
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) S.nrm[q] = sqrt(s);
     }
     __syncthreads();
 }
 
-__device__ void ob_setup(const double *gx, const double *gw, ObShared &S) {
+template <int K>
+__device__ void ob_setup(const double *W, const double *gx, const double *gw, ObShared<K> &S) {
+    constexpr int N2 = 2 * K;
     if (threadIdx.x < OB_QPTS) {
         S.gx[threadIdx.x] = gx[threadIdx.x];
         S.gw[threadIdx.x] = gw[threadIdx.x];
     }
+    for (int e = threadIdx.x; e < N2 * N2; e += OB_THREADS) S.W[e] = W[e];
+    __syncthreads();
+    for (int i = threadIdx.x; i < OB_UNIT; i += OB_THREADS) {
+        double P[N2];
+        ob_legendre<N2>(2.0 * (0.125 * (i / OB_QPTS) + 0.125 * S.gx[i % OB_QPTS]) - 1.0, P);
+        for (int p = 0; p < N2; p++) S.P[i][p] = P[p];
+    }
     __syncthreads();
 }
 
-// phase 1: per task the sub-block norms of NS(0..L) and L, where the walk stops
-__global__ void __launch_bounds__(OB_THREADS) op_band_kernel(int K, const double *W, const double *cc, const double *gx,
+// tau(2l-1), tau(2l), tau(2l+1) of block l; `next`: tau(2l-1) is the last block's tau(2l+1).  A warp per
+// moment: at l = 0 those of 0, 1 and -1, else of +-2l and +-(2l+1) (and, not `next`, +-(2l-1)).
+template <int K>
+__device__ void ob_taus(const OpBuildTask &T, int l, bool next, const double *cc, ObShared<K> &S) {
+    const int q = threadIdx.x >> 5;
+    if (l > 0) {
+        if (next) {
+            for (int e = threadIdx.x; e < K * K; e += OB_THREADS) S.tm1[e] = S.tp1[e];
+        } else {
+            if (q < 2) ob_moments<K>(T.beta, q ? 1.0 - 2.0 * l : 2.0 * l - 1.0, q, S);
+            __syncthreads();
+            ob_tau<K>(T.pref, cc, S, 0, 1, S.tm1);
+            __syncthreads();
+        }
+    }
+    const int m = 2 * l + (q >> 1);  // warps: 2l, -2l, 2l+1, -(2l+1)
+    if (m > 0 || q == 0) ob_moments<K>(T.beta, q & 1 ? -(double)m : (double)m, q, S);
+    __syncthreads();
+    ob_tau<K>(T.pref, cc, S, 0, l > 0 ? 1 : 0, S.t0);
+    ob_tau<K>(T.pref, cc, S, 2, 3, S.tp1);
+    if (l == 0) ob_tau<K>(T.pref, cc, S, 3, 2, S.tm1);
+    __syncthreads();
+}
+
+// Phase 1: per task the sub-block norms of NS(0..L) and L, where the walk stops; the blocks themselves for
+// l < OP_KEEP, which most walks do not pass.  Persistent CTAs.  Bound: the FP64 pipe (per block 2 (2K)^3
+// multiply-adds for W tau W^T, 8 K^3 for the two taus, and per moment 128 points of an exponential and 2K
+// multiply-adds); one warp per moment, the Legendre table and the butterfly sums leave little else.
+template <int K>
+__global__ void __launch_bounds__(OB_THREADS) op_band_kernel(const double *W, const double *cc, const double *gx,
                                                              const double *gw, const OpBuildTask *tasks, int ntask,
-                                                             double *nrm, double *head, int *band, double *peak) {
+                                                             double *nrm, double *head, int *band, double *peak,
+                                                             double *keep) {
     extern __shared__ __align__(16) unsigned char ob_smem[];
-    ObShared &S = *reinterpret_cast<ObShared *>(ob_smem);
-    ob_setup(gx, gw, S);
+    ObShared<K> &S = *reinterpret_cast<ObShared<K> *>(ob_smem);
+    ob_setup<K>(W, gx, gw, S);
     for (int t = blockIdx.x; t < ntask; t += gridDim.x) {
         const OpBuildTask T = tasks[t];
         double *tn = nrm + T.nrm_off;
         double pk = 0.0;
         int L = -1;
         for (int l = 0; l <= T.cap; l++) {
-            if (l == 0) {
-                ob_tau(K, T.beta, T.pref, -1, cc, S, S.tm1);
-                ob_tau(K, T.beta, T.pref, 0, cc, S, S.t0);
-            } else {
-                // tau(2l-1) is the previous step's tau(2l+1)
-                for (int e = threadIdx.x; e < K * K; e += blockDim.x) S.tm1[e] = S.tp1[e];
-                __syncthreads();
-                ob_tau(K, T.beta, T.pref, 2 * l, cc, S, S.t0);
-            }
-            ob_tau(K, T.beta, T.pref, 2 * l + 1, cc, S, S.tp1);
-            ob_ns(K, W, S);
+            ob_taus<K>(T, l, true, cc, S);
+            ob_ns<K>(S);
             if (threadIdx.x < 4) {
                 tn[4 * l + threadIdx.x] = S.nrm[threadIdx.x];
                 if (l < OP_NRM_HEAD) head[((size_t)t * OP_NRM_HEAD + l) * 4 + threadIdx.x] = S.nrm[threadIdx.x];
             }
+            if (l < OP_KEEP)
+                for (int e = threadIdx.x; e < 4 * K * K; e += OB_THREADS)
+                    keep[((size_t)t * OP_KEEP + l) * 4 * K * K + e] = S.ns[e];
             L = l;
             bool stop = false;
             if (!T.root) {
@@ -183,32 +226,38 @@ __global__ void __launch_bounds__(OB_THREADS) op_band_kernel(int K, const double
     }
 }
 
-// phase 2: block l of task `task` (one CTA per (task, l) pair); zero: 4 bits, sub-blocks to zero
-__global__ void __launch_bounds__(OB_THREADS) op_block_kernel(int K, const double *W, const double *cc, const double *gx,
+// Phase 2: block l of task `task` (one CTA per (task, l) pair), kept by phase 1 or, from OP_KEEP on, computed
+// again; zero: 4 bits, sub-blocks to zero.
+template <int K>
+__global__ void __launch_bounds__(OB_THREADS) op_block_kernel(const double *W, const double *cc, const double *gx,
                                                               const double *gw, const OpBuildTask *tasks,
-                                                              const OpBlockJob *jobs, int njob) {
+                                                              const OpBlockJob *jobs, int njob, const double *keep) {
     extern __shared__ __align__(16) unsigned char ob_smem[];
-    ObShared &S = *reinterpret_cast<ObShared *>(ob_smem);
-    ob_setup(gx, gw, S);
-    const int K2 = 2 * K, bsz = K2 * K2;
+    ObShared<K> &S = *reinterpret_cast<ObShared<K> *>(ob_smem);
+    constexpr int N2 = 2 * K, bsz = N2 * N2;
+    bool set = false;
     for (int q = blockIdx.x; q < njob; q += gridDim.x) {
         const OpBlockJob J = jobs[q];
-        const OpBuildTask T = tasks[J.task];
         const int l = J.l;
-        ob_tau(K, T.beta, T.pref, 2 * l - 1, cc, S, S.tm1);
-        ob_tau(K, T.beta, T.pref, 2 * l, cc, S, S.t0);
-        ob_tau(K, T.beta, T.pref, 2 * l + 1, cc, S, S.tp1);
-        ob_ns(K, W, S);
-        double *pos = J.blocks + (size_t)(J.off + J.band + l) * bsz;
-        double *neg = J.blocks + (size_t)(J.off + J.band - l) * bsz;
-        for (int e = threadIdx.x; e < bsz; e += blockDim.x) {
-            const int r = e / K2, c = e - r * K2;
-            const int g = r / K, f = c / K;
-            const double v = (J.zero >> (2 * g + f)) & 1 ? 0.0 : S.ns[e];
-            pos[e] = v;
-            if (l > 0) neg[c * K2 + r] = v;  // NS(-l) = NS(l)^T
+        __syncthreads();
+        if (l < OP_KEEP) {
+            const double *k = keep + ((size_t)J.task * OP_KEEP + l) * bsz;
+            for (int e = threadIdx.x; e < bsz; e += OB_THREADS) S.ns[e] = k[e];
+        } else {
+            if (!set) ob_setup<K>(W, gx, gw, S);
+            set = true;
+            ob_taus<K>(tasks[J.task], l, false, cc, S);
+            ob_ns<K>(S);
         }
         __syncthreads();
+        double *pos = J.blocks + (size_t)(J.off + J.band + l) * bsz;
+        double *neg = J.blocks + (size_t)(J.off + J.band - l) * bsz;
+        for (int e = threadIdx.x; e < bsz; e += OB_THREADS) {
+            const int r = e / N2, c = e - r * N2, g = r / K, f = c / K;
+            pos[e] = (J.zero >> (2 * g + f)) & 1 ? 0.0 : S.ns[e];
+            // NS(-l) = NS(l)^T, written in its own order
+            if (l > 0) neg[e] = (J.zero >> (2 * f + g)) & 1 ? 0.0 : S.ns[c * N2 + r];
+        }
     }
 }
 
@@ -260,24 +309,58 @@ __global__ void op_convert_kernel(const double *blocks, float *b32, float *btc, 
 
 }  // namespace
 
-size_t op_build_smem() { return sizeof(ObShared); }
+namespace {
 
-void k_op_band(int K, const double *W, const double *cc, const double *gx, const double *gw, const OpBuildTask *tasks,
-               int ntask, double *nrm, double *head, int *band, double *peak, cudaStream_t s) {
-    if (ntask <= 0) return;
-    const int smem = (int)sizeof(ObShared);
-    MWG_CUDA(cudaFuncSetAttribute(op_band_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    op_band_kernel<<<ntask, OB_THREADS, smem, s>>>(K, W, cc, gx, gw, tasks, ntask, nrm, head, band, peak);
+template <int K>
+void launch_band(const double *W, const double *cc, const double *gx, const double *gw, const OpBuildTask *tasks,
+                 int ntask, double *nrm, double *head, int *band, double *peak, double *keep, int nsm, cudaStream_t s) {
+    const int smem = (int)sizeof(ObShared<K>);
+    kernel_smem((const void *)op_band_kernel<K>, smem);
+    const int per = std::max(1, kernel_ctas_per_sm((const void *)op_band_kernel<K>, OB_THREADS, smem));
+    op_band_kernel<K><<<std::min(ntask, per * std::max(nsm, 1)), OB_THREADS, smem, s>>>(W, cc, gx, gw, tasks, ntask, nrm,
+                                                                                     head, band, peak, keep);
     MWG_CUDA(cudaGetLastError());
 }
 
-void k_op_blocks(int K, const double *W, const double *cc, const double *gx, const double *gw, const OpBuildTask *tasks,
-                 const OpBlockJob *jobs, int njob, cudaStream_t s) {
-    if (njob <= 0) return;
-    const int smem = (int)sizeof(ObShared);
-    MWG_CUDA(cudaFuncSetAttribute(op_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    op_block_kernel<<<njob < 65535 ? njob : 65535, OB_THREADS, smem, s>>>(K, W, cc, gx, gw, tasks, jobs, njob);
+template <int K>
+void launch_blocks(const double *W, const double *cc, const double *gx, const double *gw, const OpBuildTask *tasks,
+                   const OpBlockJob *jobs, int njob, const double *keep, cudaStream_t s) {
+    const int smem = (int)sizeof(ObShared<K>);
+    kernel_smem((const void *)op_block_kernel<K>, smem);
+    op_block_kernel<K><<<std::min(njob, 65535), OB_THREADS, smem, s>>>(W, cc, gx, gw, tasks, jobs, njob, keep);
     MWG_CUDA(cudaGetLastError());
+}
+
+}  // namespace
+
+void k_op_band(int K, const double *W, const double *cc, const double *gx, const double *gw, const OpBuildTask *tasks,
+               int ntask, double *nrm, double *head, int *band, double *peak, double *keep, int nsm, cudaStream_t s) {
+    if (ntask <= 0) return;
+    switch (K) {
+        case 4: launch_band<4>(W, cc, gx, gw, tasks, ntask, nrm, head, band, peak, keep, nsm, s); break;
+        case 5: launch_band<5>(W, cc, gx, gw, tasks, ntask, nrm, head, band, peak, keep, nsm, s); break;
+        case 6: launch_band<6>(W, cc, gx, gw, tasks, ntask, nrm, head, band, peak, keep, nsm, s); break;
+        case 7: launch_band<7>(W, cc, gx, gw, tasks, ntask, nrm, head, band, peak, keep, nsm, s); break;
+        case 8: launch_band<8>(W, cc, gx, gw, tasks, ntask, nrm, head, band, peak, keep, nsm, s); break;
+        case 9: launch_band<9>(W, cc, gx, gw, tasks, ntask, nrm, head, band, peak, keep, nsm, s); break;
+        case 10: launch_band<10>(W, cc, gx, gw, tasks, ntask, nrm, head, band, peak, keep, nsm, s); break;
+        default: throw Error(MW_ERR_ARG, "no operator kernel for this order");
+    }
+}
+
+void k_op_blocks(int K, const double *W, const double *cc, const double *gx, const double *gw, const OpBuildTask *tasks,
+                 const OpBlockJob *jobs, int njob, const double *keep, cudaStream_t s) {
+    if (njob <= 0) return;
+    switch (K) {
+        case 4: launch_blocks<4>(W, cc, gx, gw, tasks, jobs, njob, keep, s); break;
+        case 5: launch_blocks<5>(W, cc, gx, gw, tasks, jobs, njob, keep, s); break;
+        case 6: launch_blocks<6>(W, cc, gx, gw, tasks, jobs, njob, keep, s); break;
+        case 7: launch_blocks<7>(W, cc, gx, gw, tasks, jobs, njob, keep, s); break;
+        case 8: launch_blocks<8>(W, cc, gx, gw, tasks, jobs, njob, keep, s); break;
+        case 9: launch_blocks<9>(W, cc, gx, gw, tasks, jobs, njob, keep, s); break;
+        case 10: launch_blocks<10>(W, cc, gx, gw, tasks, jobs, njob, keep, s); break;
+        default: throw Error(MW_ERR_ARG, "no operator kernel for this order");
+    }
 }
 
 void k_op_convert(const double *blocks, float *b32, float *btc, float *btc2, long nblocks, int K, int NB, int groups,
