@@ -35,7 +35,7 @@ ORDER, PREC = 9, 1e-6
 # tier launch of two mixed steps of the first 8 orbitals of the batch with the caches left warm
 # (--cache-control none), divided by those launches' items; summarised with its command in
 # profiles/dram_traffic_tiers_k10.md and re-captured whenever a tier kernel changes
-DRAM_PER_ITEM = {"fp32": 2.45e3, "tf32": 0.43e3, "df32": 4.55e3}
+DRAM_PER_ITEM = {"fp32": 2.45e3, "tf32": 0.43e3}
 NORB = 16
 METRIC = "Helmholtz-apply nodes/s: batched mixed vs plain FP64 GPU at 1e-6 rel. error"
 
@@ -652,7 +652,6 @@ def run(args):
     mra.set_screening("host")
     host_scr_ms, st_hs = timed("mixed", 3)
     mra.set_screening("gpu")
-    fp64_tf = mra.probe_fma_peak(True)
     fp32_tf = mra.probe_fma_peak(False)
     tf32_tf = mra.probe_mma_peak("tc05")          # tcgen05 TF32, M128 N256 K8: the device's dense rate
     tf32_n32_tf = mra.probe_mma_peak("tc05_n32")  # the same at the tier's own MMA shape, N = 32
@@ -710,8 +709,13 @@ def run(args):
     fma_src = "probed FMA throughput of this GPU (mw_probe_fma_peak); MEASURED_PEAKS.json holds no FP64/FP32 figure"
     mma_src = ("probed dense tcgen05.mma TF32 throughput of this GPU at M128 N256 K8 (mw_probe_mma_peak kind 2); "
                "MEASURED_PEAKS.json holds no TF32 figure")
+    # the fixed-point kernel's multiply-add takes 48.6 products of mma.sync (per 8 columns two row tiles x 38
+    # products of 16 x 8 x 16, for 8 x 20 x 20 multiply-adds), which runs 960 of them per SM and cycle, 7.5
+    # times the FP32 pipe's 128
+    fx_tf = fp32_tf * (960.0 / 128.0) / 48.6
+    fx_src = fma_src + "; FP32 rate times 7.5 for mma.sync's FP16 products, divided by 48.6 products per multiply-add"
     roofs = {
-        "fp64": roof("fp64", st_ser["kernel_ms_fp64"], fp64_tf, "apply_kernel<double,10>", "fp64-pipe", fma_src),
+        "fp64": roof("fp64", st_ser["kernel_ms_fp64"], fx_tf, "apply_fx_kernel<10>", "tensor (62-bit fixed point)", fx_src),
         # the FP32-accuracy tier of the mixed step runs on the tensor cores as split TF32: per tile
         # and k-step A_hi * [B_hi B_lo] (width 64) and A_lo * B_hi (width 32), the issued work of
         # three N = 32 MMAs (hi*hi, hi*lo, lo*hi), 3 x the TF32 tier's
@@ -719,11 +723,7 @@ def run(args):
                      mma_src, tc_mult=3),
         "tf32": roof("tf32", st_ser["kernel_ms_tf32"], tf32_tf, "apply_tc05_kernel<10,0>", "tensor", mma_src,
                      tc_mult=1),
-        # a double-FP32 multiply-add costs about 12 FP32 instructions in this kernel: its ceiling is the
-        # FP32 FMA rate / 12 (multiply-adds), i.e. peak flops = FP32 FMA flops / 12
-        "df32": roof("df32", st_ser["kernel_ms_df"], fp32_tf / 12.0, "apply_df_kernel<10>",
-                     "fp32-pipe (double-FP32)", fma_src + "; divided by 12 FP32 instructions per double-FP32 "
-                     "multiply-add"),
+        "df32": roof("df32", st_ser["kernel_ms_df"], fx_tf, "apply_fx_kernel<10>", "tensor (62-bit fixed point)", fx_src),
     }
     for t in ("tf32", "fp32"):
         roofs[t]["peak_tc05_n32"] = tf32_n32_tf

@@ -42,14 +42,14 @@ constexpr double TIER_FP64 = 2e6;
 // small weight of the large root boxes, so many items just under it would add up to more than
 // prec relative to a small output.
 constexpr double TIER_TF32 = 2e3;
-// An item in double-FP32 (values as unevaluated FP32 pairs, error-free products and sums) is off
-// by at most about 3e-13 b, so items with TIER_FP64 < b / tau <= TIER_DF err by at most 0.03 tau;
-// larger ones, and root-scale items under relative precision, run in FP64.
+// Tier 3 (the double-FP32 tier's name and place in the counters; the fixed-point kernel runs its items,
+// within 1e-15 b) takes TIER_FP64 < b / tau <= TIER_DF; larger ones, and root-scale items under relative
+// precision, count as FP64 and run in the same kernel.
 constexpr double TIER_DF = 1e11;
 // The fixed-point kernel of the FP64 tier (mw_apply_fx.cu) takes finite inputs; a block norm below
 // this means that every value is finite and its square has not overflowed (false for NaN too).
 constexpr double FX_NORM_MAX = 1e150;
-constexpr int NTIER = 4;  // 0 FP64, 1 FP32, 2 TF32 tensor cores, 3 double-FP32
+constexpr int NTIER = 4;  // 0 FP64, 1 FP32, 2 TF32 tensor cores, 3 large bounds (double-FP32 or better)
 constexpr double BOUND_PRUNE = 8.0 * 2.8285;  // (sum_f |in_f|) / |block| <= sqrt(8); 8 output components
 
 double split_thr(double prec, double R, int n) { return prec * R * std::pow(2.0, -0.5 * (n + 1)); }
@@ -287,6 +287,9 @@ struct DevItems {
     const void **in = nullptr, **ax = nullptr, **ay = nullptr, **az = nullptr;
     double *coef = nullptr;
     long long base[NTIER] = {0, 0, 0, 0};
+    const double *g64 = nullptr;  // the level's generated blocks and the place of their digits
+    uint32_t *gfx = nullptr;
+    size_t ngen = 0;
 };
 
 int *launch_tier(Ctx &ctx, Arena &arena, LevelItems &li, bool root, bool set, int tier, long long chunk,
@@ -298,9 +301,9 @@ int *launch_tier(Ctx &ctx, Arena &arena, LevelItems &li, bool root, bool set, in
     // writes a partial block; the CTA that ends a node's last chunk sums its partials in chunk
     // order (mw_chunks.cuh).
     // The split depends only on the tier and the node's own item count, so results do not depend
-    // on which nodes share the launch.  CHUNK (Ctx::Tuning; by default 4, 32, 96 and 8 items) is
-    // about half a millisecond of one CTA's work: an item costs ~200 us (FP64), ~20 us (FP32),
-    // ~3 us (TF32) and ~70 us (double-FP32).
+    // on which nodes share the launch.  CHUNK (Ctx::Tuning; by default 8, 32, 96 and 8 items) is
+    // two to six tenths of a millisecond of one CTA's work at order 9: an item costs ~22 us (fixed point),
+    // ~20 us (FP32) and ~3 us (TF32).
     const long long CHUNK = chunk > 0 ? chunk : 1;
     const int bs = ctx.basis.bs;
     std::vector<double *> vout;
@@ -313,7 +316,7 @@ int *launch_tier(Ctx &ctx, Arena &arena, LevelItems &li, bool root, bool set, in
         if (m > CHUNK + CHUNK / 2) nsplit += (m + CHUNK / 2) / CHUNK;
     }
     double *scratch = nsplit ? (double *)arena.alloc(sizeof(double) * (size_t)bs * nsplit) : nullptr;
-    const bool fx = tier == 0 && fixed_point;  // stores its chunks' partial blocks instead of adding into zeros
+    const bool fx = (tier == 0 || tier == 3) && fixed_point;  // stores its chunks' partial blocks instead of adding into zeros
     if (scratch && !set && !fx) MWG_CUDA(cudaMemsetAsync(scratch, 0, sizeof(double) * (size_t)bs * nsplit, ctx.stream));
     long used = 0;
     for (int i = 0; i < nn; i++) {
@@ -403,16 +406,12 @@ int *launch_tier(Ctx &ctx, Arena &arena, LevelItems &li, bool root, bool set, in
     // tier 1 in the tensor-core modes: the split-TF32 tcgen05 kernel (FP32 accuracy); else the
     // FP32 CUDA-core kernel
     const bool tc = tier == 2 || (tier == 1 && split_tc);
-    if (tier == 3) {
-        k_apply_df(ctx.dbasis, L, ctx.nsm, ctx.stream);
-    } else {
-        if (tc)
-            k_apply_tc05(ctx.dbasis, L, tier == 1, ctx.stream);
-        else if (fx)
-            k_apply_fx(ctx.dbasis, L, ctx.stream);
-        else
-            k_apply(ctx.dbasis, L, tier, ctx.nsm, ctx.stream);
-    }
+    if (tc)
+        k_apply_tc05(ctx.dbasis, L, tier == 1, ctx.stream);
+    else if (fx)
+        k_apply_fx(ctx.dbasis, L, ctx.stream);
+    else
+        k_apply(ctx.dbasis, L, tier == 1, ctx.nsm, ctx.stream);
     // the status word (the tensor-core kernels wait for bulk copies with a bound) and the row count
     hs = (int *)arena.halloc(2 * sizeof(int));
     hs[0] = hs[1] = 0;
@@ -441,14 +440,14 @@ struct DevScreen {
     cudaEvent_t ev_counts = nullptr;  // the write pass's per-node tier counts have reached the host
 };
 
-// layout of Oper::d_screen: int band[TS], int off[TS] | double amax[TS], xmax[TS], c[T], norms[4 nb]
+// layout of Oper::d_screen: int band[TS], off[TS], first[TS] | double amax[TS], xmax[TS], c[T], norms[4 nb]
 // | float amax32[TS], xmax32[TS], norms32[4 nb]   (TS = T * S, nb = blocks)
 struct OperScreenLayout {
     size_t TS, nb, ib, db, fb;
     explicit OperScreenLayout(const Oper &op) {
         TS = (size_t)op.T * op.S;
         nb = (size_t)std::max<long>(op.nblocks, 1);
-        ib = ((2 * TS * sizeof(int)) + 255) & ~size_t(255);
+        ib = ((3 * TS * sizeof(int)) + 255) & ~size_t(255);
         db = ((sizeof(double) * (2 * TS + (size_t)op.T + 4 * nb)) + 255) & ~size_t(255);
         fb = sizeof(float) * (2 * TS + 4 * nb);
     }
@@ -468,6 +467,7 @@ bool oper_screen_tables(Oper &op) {
     for (size_t i = 0; i < TS; i++) {
         iv[i] = op.band[i];
         iv[TS + i] = (int)op.off[i];
+        iv[2 * TS + i] = op.fx_first[i];
         dd[i] = op.amax[i];
         dd[TS + i] = op.xmax[i];
         ff[i] = (float)op.amax[i];
@@ -492,6 +492,7 @@ ScreenOp oper_screen_view(const Oper &op) {
     ScreenOp so;
     so.band = iv;
     so.off = iv + TS;
+    so.first = iv + 2 * TS;
     so.amax = dd;
     so.xmax = dd + TS;
     so.c = dd + 2 * TS;
@@ -507,6 +508,31 @@ ScreenOp oper_screen_view(const Oper &op) {
     so.S = op.S;
     return so;
 }
+
+// The digits of the operators' blocks at one scale (the fixed-point kernel's operands): room in the arena
+// for every distinct operator, which make() fills.  Block (t, l) is fx_first[t][s] + band + l.
+struct FxLevelOps {
+    std::unordered_map<const Oper *, uint32_t *> base;
+    std::vector<FxOpJob> jobs;
+    size_t words = 0, zoff = 0;
+    int s = 0;
+    bool add(Oper &op, Arena &ar) {
+        if (base.count(&op)) return true;
+        if (!oper_screen_tables(op)) return false;
+        const int n = op.fx_count[s];
+        uint32_t *b = (uint32_t *)ar.alloc(sizeof(uint32_t) * words * (size_t)std::max(n, 1));
+        base.emplace(&op, b);
+        jobs.push_back(FxOpJob{oper_screen_view(op), b, s, n});
+        return true;
+    }
+    const uint32_t *block(const Oper &op, int t, int l) const {
+        return base.at(&op) + words * (size_t)(op.fx_first[t * op.S + s] + op.band[t * op.S + s] + l);
+    }
+    void make(Ctx &ctx, mw_stats &st) const {
+        k_op_to_fx(jobs.data(), jobs.size(), ctx.basis.K, ctx.stream);
+        st.launches++;
+    }
+};
 
 // the largest sub-block norm of an operator (the FP32 estimates need it well inside FP32's range)
 double oper_norm_max(const Oper &op) {
@@ -653,7 +679,7 @@ constexpr size_t SCREEN_SMEM_MAX = 96 * 1024;  // larger walks (very wide bands)
 // screening does.  The group's stream waits for the item arrays with an event.
 void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobState *> &jp,
                       const std::vector<int> &jglob, int level, int zmax, const TierRule &rule, LevelItems *lt,
-                      bool fixed_point, DevItems &dv, mw_stats &st, double &t_enum, double &t_gen, double &t_items) {
+                      const FxLevelOps *fxops, DevItems &dv, mw_stats &st, double &t_enum, double &t_gen, double &t_items) {
     const Basis &b = ctx.basis;
     const int K = b.K, bs = b.bs, bsz = 4 * K * K;
     const double K4 = (double)K * K * K * K;
@@ -819,15 +845,27 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
     P.g64 = (double *)ar.alloc(sizeof(double) * (size_t)bs * ng);
     P.g32 = rule.mixed ? (float *)ar.alloc(sizeof(float) * 2 * (size_t)bs * ng) : nullptr;
     P.gtc = rule.tensor ? (float *)ar.alloc(sizeof(float) * P.tx * ng) : nullptr;
-    P.fx = fixed_point ? fx_words(K) : 0;
-    P.gfx = fixed_point ? (uint32_t *)ar.alloc(sizeof(uint32_t) * P.fx * ng) : nullptr;
+    P.fx = fxops ? fx_words(K) : 0;
+    P.gfx = fxops ? (uint32_t *)ar.alloc(sizeof(uint32_t) * P.fx * ng) : nullptr;
+    dv.g64 = P.g64;
+    dv.gfx = P.gfx;
+    dv.ngen = fxops ? (size_t)ngen : 0;
+    std::vector<const uint32_t *> fxop;  // per job of the apply its operator's digits
+    if (fxops) {
+        P.fxo = fxops->words;
+        P.fxz = fxops->zoff;
+        fxop.resize(*std::max_element(jglob.begin(), jglob.end()) + 1, nullptr);
+        for (size_t j = 0; j < jp.size(); j++) fxop[jglob[j]] = fxops->base.at(jp[j]->job->op);
+    }
     int *hs = (int *)ar.halloc(sizeof(int) * (8 * (size_t)NN + 1));
     {
         StreamSwap fast(ctx, ctx.fast);
         Packer pk;
         pk.add(coff.data(), sizeof(long long) * NN);
+        pk.add(fxop.data(), sizeof(uint32_t *) * fxop.size());
         pk.ship(ctx, ar);
         P.cand_off = (const long long *)pk.ptr(0);
+        P.fxop = (const uint32_t *const *)pk.ptr(1);
         if (ngen > 0) {
             GenTask *tasks = (GenTask *)ar.alloc(sizeof(GenTask) * (size_t)ngen);
             k_screen_gen_tasks(P, tasks, ngen, ctx.stream);
@@ -839,10 +877,6 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
             k_screen_gen_norms32(P, ngen, ctx.stream);
             st.launches += 3;
             st.generated += ngen;
-            if (fixed_point) {
-                k_to_fx(P.g64, P.gfx, (size_t)ngen, K, ctx.stream);
-                st.launches++;
-            }
             if (rule.mixed) {
                 k_to_fp32_cube(P.g64, P.g32, (size_t)ngen, K, ctx.stream);
                 st.launches++;
@@ -1060,31 +1094,43 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         if (fixed_grid) max_levels = std::max(max_levels, job.out->max_scale() - b.n0 + 1);
         s.R = 1.0;
     }
-    // The FP64 tier's digits of every distinct input tree, for the length of the call, where that tier
-    // has a large share of the items.  They take 1.8 times the blocks' own space: trees that would not
-    // leave room for them go to the kernel that reads the FP64 blocks.
+    // The digits of every distinct input tree (the FP64 and double-FP32 tiers' fixed-point kernel), for the
+    // length of the call.  They take 1.8 times the blocks' own space: trees that would not leave room for
+    // them go to the kernel that reads the FP64 blocks.
     const size_t fxw = fx_words(K);
     ctx.sarena.reset();
-    auto to_digits = [&](JobState &s) {
-        k_to_fx(s.job->inp->d_coefs, s.fx, (size_t)s.job->inp->nn(), K, ctx.stream);
-        st.launches++;
-    };
-    bool digits = !mixed || near_fp64;
-    if (digits) {
-        std::unordered_map<const Tree *, uint32_t *> have;
+    bool digits = true;
+    std::unordered_map<const Tree *, uint32_t *> tree_fx;
+    {
         size_t bytes = 0;
         for (JobState &s : js)
-            if (have.emplace(s.job->inp, nullptr).second) bytes += sizeof(uint32_t) * fxw * (size_t)s.job->inp->nn();
+            if (tree_fx.emplace(s.job->inp, nullptr).second) bytes += sizeof(uint32_t) * fxw * (size_t)s.job->inp->nn();
         digits = ctx.sarena.room_for(bytes);
         for (JobState &s : js) {
             if (!digits) break;
-            uint32_t *&d = have[s.job->inp];
-            const bool made = d != nullptr;
-            if (!made) d = (uint32_t *)ctx.sarena.alloc(sizeof(uint32_t) * fxw * (size_t)s.job->inp->nn());
+            uint32_t *&d = tree_fx[s.job->inp];
+            if (!d) d = (uint32_t *)ctx.sarena.alloc(sizeof(uint32_t) * fxw * (size_t)s.job->inp->nn());
             s.fx = d;
-            if (!made && !hin) to_digits(s);
         }
     }
+    auto to_digits = [&](const std::vector<int> &which) {  // of these jobs' trees, each once
+        std::vector<FxBlocks> sets;
+        std::unordered_map<const Tree *, int> seen;
+        for (int j : which) {
+            const Tree *t = js[j].job->inp;
+            if (seen.emplace(t, 0).second) sets.push_back(FxBlocks{t->d_coefs, js[j].fx, (size_t)t->nn()});
+        }
+        k_to_fx(sets.data(), sets.size(), K, ctx.stream);
+        st.launches++;
+    };
+    if (digits && !hin) {
+        std::vector<int> all(js.size());
+        for (size_t j = 0; j < js.size(); j++) all[j] = (int)j;
+        to_digits(all);
+    }
+    // the operators' digits of a level: beside its screening where most items need them, else once it is
+    // known that any does
+    const bool ops_first = !mixed || near_fp64 || df_only;
     // screening on the GPU (mw_screen.cu) when the context asks for it and the jobs fit its tables
     const TierRule rule{mixed, near_fp64, df_only, dfp, tensor};
     DevScreen ds;
@@ -1177,8 +1223,8 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                     off += 8 * (size_t)in.nn();
                     js[j].set_fmax(in, b.n0);
                     if (mixed) convert_input(in);
-                    if (digits) to_digits(js[j]);
                 }
+                if (digits) to_digits(G.jobs);
                 if (ds.on) screen_setup_inputs(ctx, jobs, js, G.jobs, ds);
                 MWG_CUDA(cudaEventCreateWithFlags(&G.ev_prep, cudaEventDisableTiming));
                 MWG_CUDA(cudaEventRecord(G.ev_prep, ctx.stream));
@@ -1193,6 +1239,12 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         const bool root = (level == 0);
         bool fixed_point = digits;
         for (JobState *sp : jp) fixed_point = fixed_point && sp->fixed_point;
+        FxLevelOps fxops;
+        fxops.words = fx_op_words(K);
+        fxops.zoff = fx_op_z(K);
+        fxops.s = sidx;
+        for (JobState *sp : jp) fixed_point = fixed_point && fxops.add(*sp->job->op, ar);
+        if (fixed_point && ops_first) fxops.make(ctx, st);
         // thresholds and precision-steering weights
         for (JobState *sp : jp) {
             JobState &s = *sp;
@@ -1207,7 +1259,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         const int zmax = ds.on ? level_zrows(jp, sidx) : 0;
         const bool dscreen = ds.on && level < ds.levels && screen_smem(ds.maxT, zmax) <= SCREEN_SMEM_MAX;
         if (dscreen) {
-            screen_level_gpu(ctx, ar, ds, jp, G.jobs, level, zmax, rule, G.lt, fixed_point, dv, st, st.host_enum_ms,
+            screen_level_gpu(ctx, ar, ds, jp, G.jobs, level, zmax, rule, G.lt, fixed_point ? &fxops : nullptr, dv, st, st.host_enum_ms,
                              st.host_gen_ms, st.host_items_ms);
         } else {
             // phase A: candidate enumeration (host, all the group's nodes in parallel)
@@ -1278,11 +1330,10 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                     }
                 }
                 uint32_t *firstfx = nullptr;
-                if (fixed_point && total > 0) {
-                    firstfx = (uint32_t *)ar.alloc(sizeof(uint32_t) * fxw * total);
-                    k_to_fx(first, firstfx, total, b.K, ctx.stream);
-                    st.launches++;
-                }
+                if (fixed_point && total > 0) firstfx = (uint32_t *)ar.alloc(sizeof(uint32_t) * fxw * total);
+                dv.g64 = first;
+                dv.gfx = firstfx;
+                dv.ngen = total;
                 for (JobState *sp : jp) {
                     JobState &s = *sp;
                     s.gbase = s.gens.base;
@@ -1386,14 +1437,18 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                          bzi = op.block_index(cd.t, sidx, cd.lz);
                     LevelItems &T = lt[cd.tier];
                     long long &pi = p[cd.tier];
-                    if (cd.tier == 0) {
-                        if (fixed_point)
+                    if (cd.tier == 0 || cd.tier == 3) {
+                        if (fixed_point) {
                             T.in[pi] = cd.gen ? s.gbase_fx + fxw * (size_t)cd.src : s.fx + fxw * (size_t)cd.src;
-                        else
+                            T.ax[pi] = fxops.block(op, cd.t, cd.lx);
+                            T.ay[pi] = fxops.block(op, cd.t, cd.ly);
+                            T.az[pi] = fxops.block(op, cd.t, cd.lz) + fxops.zoff;
+                        } else {
                             T.in[pi] = cd.gen ? (const void *)(s.gbase + (size_t)cd.src * bs) : (const void *)inp.block(cd.src);
-                        T.ax[pi] = op.d_blocks + (size_t)bxi * bsz;
-                        T.ay[pi] = op.d_blocks + (size_t)byi * bsz;
-                        T.az[pi] = op.d_blocks + (size_t)bzi * bsz;
+                            T.ax[pi] = op.d_blocks + (size_t)bxi * bsz;
+                            T.ay[pi] = op.d_blocks + (size_t)byi * bsz;
+                            T.az[pi] = op.d_blocks + (size_t)bzi * bsz;
+                        }
                     } else if (cd.tier == 2 || (cd.tier == 1 && tensor)) {
                         // the tensor-core tiers read their own operand layouts (mw_tc05_layout.h)
                         const size_t tx = tc5_x_stride(b.K), tb = tc5_b_stride(b.K);
@@ -1433,6 +1488,14 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         const auto tD = std::chrono::steady_clock::now();
         MWG_CUDA(cudaEventRecord(G.ev[0], ctx.stream));
         G.status.clear();
+        if (fixed_point && lt[0].items + lt[3].items > 0) {
+            if (!ops_first) fxops.make(ctx, st);
+            if (dv.ngen > 0) {
+                const FxBlocks gen{dv.g64, dv.gfx, dv.ngen};
+                k_to_fx(&gen, 1, K, ctx.stream);
+                st.launches++;
+            }
+        }
         for (int k = 0; k < NTIER; k++) {
             int *hs = launch_tier(ctx, ar, lt[k], root, false, k, tune.chunk[k], st, dscreen ? &dv : nullptr,
                                   tensor && k == 1, fixed_point);
@@ -2145,10 +2208,11 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
     const size_t fxw = fx_words(b.K);
     uint32_t *yfx = nullptr;
     ctx.sarena.reset();
-    fixed_point = fixed_point && ctx.sarena.room_for(sizeof(uint32_t) * fxw * (size_t)y.nn());
+    fixed_point = fixed_point && oper_screen_tables(op) && ctx.sarena.room_for(sizeof(uint32_t) * fxw * (size_t)y.nn());
     if (fixed_point) {
         yfx = (uint32_t *)ctx.sarena.alloc(sizeof(uint32_t) * fxw * (size_t)y.nn());
-        k_to_fx(y.d_coefs, yfx, (size_t)y.nn(), b.K, ctx.stream);
+        const FxBlocks ys{y.d_coefs, yfx, (size_t)y.nn()};
+        k_to_fx(&ys, 1, b.K, ctx.stream);
         st.launches++;
     }
     LevelItems li;
@@ -2212,6 +2276,11 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
             }
         }
         std::stable_sort(items.begin(), items.end(), [](const TItem &a, const TItem &b2) { return a.target < b2.target; });
+        FxLevelOps fxops;
+        fxops.words = fx_op_words(b.K);
+        fxops.zoff = fx_op_z(b.K);
+        fxops.s = sidx;
+        if (fixed_point) fxops.add(op, arena);
         li = LevelItems();
         li.begin.assign(1, 0);
         for (size_t q = 0; q < items.size(); q++) {
@@ -2221,9 +2290,14 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
                 li.out.push_back(ext.block(it.target));
             }
             li.in.push_back(fixed_point ? (const void *)(yfx + fxw * (size_t)it.o) : (const void *)y.block(it.o));
-            li.ax.push_back(op.d_blocks + (size_t)op.block_index(it.c->t, sidx, -it.c->lx) * bsz);
-            li.ay.push_back(op.d_blocks + (size_t)op.block_index(it.c->t, sidx, -it.c->ly) * bsz);
-            li.az.push_back(op.d_blocks + (size_t)op.block_index(it.c->t, sidx, -it.c->lz) * bsz);
+            const int l[3] = {-it.c->lx, -it.c->ly, -it.c->lz};
+            const void *a[3];
+            for (int d = 0; d < 3; d++)
+                a[d] = fixed_point ? (const void *)(fxops.block(op, it.c->t, l[d]) + (d == 2 ? fxops.zoff : 0))
+                                   : (const void *)(op.d_blocks + (size_t)op.block_index(it.c->t, sidx, l[d]) * bsz);
+            li.ax.push_back(a[0]);
+            li.ay.push_back(a[1]);
+            li.az.push_back(a[2]);
             li.coef.push_back(op.c[it.c->t]);
         }
         if (!items.empty()) li.begin.push_back((long long)items.size());
@@ -2232,6 +2306,7 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
         st.items += (long long)items.size();
         st.items_fp64 += (long long)items.size();
         st.out_nodes += (long long)li.out.size();
+        if (fixed_point && !items.empty()) fxops.make(ctx, st);
         launch_tier(ctx, ctx.arena, li, root, true, 0, Ctx::Tuning().chunk[0], st, nullptr, false, fixed_point);
         ctx.sync();
         st.levels++;

@@ -8,22 +8,30 @@
 // the rounding of a pass's result to 62 bits are below 2^-58 of (row 1-norm) x (column maximum), less
 // than FP64's own rounding of the same sums.
 //
-// Why mma.sync and not tcgen05: its accumulator fragment of one pass, once cut into digits, is the B
-// fragment of the next (rows X' and columns Y of the x pass are columns X' and contraction index Y
-// of the y pass), so the x and y passes run in a warp's registers.  With tcgen05 every intermediate
-// would cross TMEM, registers and shared memory in 2-byte pieces; at these sizes that costs more
-// than the tensor time it saves.  Bound: the mma.sync pipe (960 multiply-adds per SM and cycle, 600
-// with the remainders of K = 9, 10), with the integer work of the digits close behind.
+// Why mma.sync and not tcgen05: an item needs ten accumulators (one per weight, two for the widest)
+// and its digits cut anew before each pass, and that integer work takes about as long as the tensor
+// pipe at mma.sync's rate (960 multiply-adds per SM and cycle, measured; 24 of 46 thousand SM cycles
+// per item at 2K = 20).  mma.sync's accumulator fragments turn into 62-bit numbers in the registers that
+// hold them; through TMEM every one of the ten would be read back by a second instruction stream.
+// Bound: issue slots, half of them for the digits (35 instructions per pair of numbers), then the pipe.
 //
-// Layout (one CTA per task, one warp per Z plane, for K > 8 per pair of planes):
-//   x pass  T1[X'][Y, Z] = sum_X Ax[X'][X] in[X][Y, Z]     the warp's planes; data columns (Y, Z)
-//   y pass  T2[Y'][X', Z] = sum_Y Ay[Y'][Y] T1[Y][X', Z]   the warp's planes; data columns X'
-//   z pass  out[Z'][Y', X'] += sum_Z c Az[Z'][Z] T2[Z]     columns (Y', X') shared out among the warps
-// T2 crosses the CTA through shared memory as digits, two Z to a word.  Rows of items as in
-// apply_kernel: a row's x passes add up, its y and z passes run once.  Below the root scale the
-// scaling-scaling path is left out exactly: u (wavelet-in-x part) comes from extra operator rows in
-// the x pass's second row tile, and the (Y' < K, X' < K) columns of the z pass take a second operand
-// whose Z < K part avoids that path.
+// Layout (one CTA per task, 7 to 16 warps that share out the column tiles of every pass):
+//   x pass  T[Z][Y][X'] = sum_X Ax[X'][X] in[X][Y, Z]    input digits read as they lie in memory
+//   y pass  T[Z][Y'][X'] = sum_Y Ay[Y'][Y] T[Z][Y][X']   in place: a warp owns its columns (X', Z)
+//   z pass  out[Z'][Y', X'] += sum_Z c Az[Z'][Z] T[Z]    columns (Y', X')
+// T is int64 in shared memory (64 KB at 2K = 20), its row pitches 2 modulo 4 so that the rows 2t apart of
+// one operand fall into distinct banks.  Digits are made where they serve many times: an input block's
+// once per call, an operator block's once per level (op_to_fx_kernel; the z pass's with its term's
+// coefficient), both laid out as mma.sync operands, the operators' copied to shared memory by cp.async one
+// pass ahead.  Rows of items as in apply_kernel: a row's x passes add up, its y and z passes run once.
+// Below the root scale the scaling-scaling path is left out exactly: u (wavelet-in-x part) comes from extra
+// operator rows in the x pass's second row tile, and the (Y' < K, X' < K) columns of the z pass take a
+// second operand whose Z < K part avoids that path.
+//
+// Measured on a full chip, ns per item without and with this kernel (apply_kernel's FP64 pipe first):
+// 2K = 20: 653, 147;  2K = 18: 444, 133;  2K = 16: 256, 46;  2K = 12: 91, 33.  With T in registers and the
+// operators' digits made per item 2K = 20 took 172 and 2K = 12 36.  Tier 3 of the 16-orbital Helmholtz batch
+// (22 thousand items, alone on the chip): 5.3 ms with their digits, 6.9 ms with the double-FP32 kernel it had.
 //
 // K > 8: the contraction index is 16 + (2K - 16).  The remainder's digit pairs are folded: one MMA
 // carries four digit pairs of the same weight in its 16 k slots, 10 MMAs instead of 28.
@@ -45,44 +53,46 @@ namespace mwg {
 
 namespace {
 
-constexpr int pitch_for(int cols) {  // columns padded so that four rows of eight words hit distinct banks
-    int p = (cols + 7) / 8 * 8;
-    while (p % 32 != 8 && p % 32 != 24) p += 8;
-    return p;
+constexpr int fx_pitch(int n) {  // n or a little more, 2 modulo 4: int64 rows 2t apart hit distinct banks
+    while (n % 4 != 2) n++;
+    return n;
 }
+// warps of a CTA: a divisor of the column tiles' number (50, 41, 32, 25, 18, 13, 8) with little left over, at
+// most 16 (128 registers)
+constexpr int fx_warps(int K) { return K == 10 ? 16 : K == 9 ? 14 : K == 8 ? 16 : K == 7 ? 13 : K == 6 ? 9 : K == 5 ? 7 : 8; }
 
 template <int K>
 struct FxGeo {
     static constexpr int N2 = 2 * K, NC = N2 * N2, K2 = K * K, K3 = K2 * K;
     static constexpr bool BIG = N2 > 16;              // contraction remainder and a second row tile
-    static constexpr int PL = BIG ? 2 : 1;            // Z planes of a warp
-    static constexpr int WARPS = N2 / PL, THREADS = 32 * WARPS;
-    static constexpr int MINB = K == 4 ? 2 : 1;       // CTAs per SM that the registers are cut for
-    static constexpr int UT = BIG ? 2 : 1;            // column tiles that have u
-    static constexpr int RP = BIG ? 2 : 1;            // operator rows of a block per lane group of a warp (fx_rows)
-    static constexpr int NT = (NC + 7) / 8;           // column tiles of the z pass
+    static constexpr int WARPS = fx_warps(K), THREADS = 32 * WARPS;
+    static constexpr int MINB = K <= 6 ? 2 : 1;       // CTAs per SM that the registers are cut for
+    // column tiles of the x pass: Y = 0..7, 8..15 of every plane Z; K > 8: Y >= 16 of two planes together
+    static constexpr int CT = N2 > 8 ? 2 : 1, GRP = BIG ? K : N2, TL = BIG ? 5 : CT, NTIN = GRP * TL;
+    static constexpr int NT = (NC + 7) / 8;           // column tiles of the y and z passes
     static constexpr int NTX = (K2 + 7) / 8;          // ... of which take the second operand
     static constexpr int TPW = (NT + WARPS - 1) / WARPS;
-    static constexpr int KE = (K + 1) / 2;            // Z pairs of the second operand
-    static constexpr int P = pitch_for(NC), PE = pitch_for(K2);
+    static constexpr int YT = BIG ? 2 : 1;            // row tiles of the y and z passes
+    // T[Z][Y][X'] and u[Z][Y][X'] (Z, Y, X' < K), 62-bit numbers
+    static constexpr int PX = fx_pitch(N2), PZ = fx_pitch(N2 * PX), UX = fx_pitch(K), UZ = fx_pitch(K * UX);
     static constexpr int MAINW = 7 * 128;             // words of a row tile's digits (512 B per digit)
     static constexpr int TILEW = MAINW + (BIG ? 10 * 128 : 0);
-    static constexpr int YT = BIG ? 2 : 1;            // row tiles of the y and z passes
-    static constexpr int W_T2 = 7 * K * P, W_EX = 7 * KE * PE;
-    static constexpr int O_EX = W_T2, O_X = O_EX + W_EX, O_Y = O_X + 4 * TILEW, O_Z = O_Y + YT * TILEW,
-                         O_U = O_Z + YT * TILEW, WORDS = O_U + 2 * (PL * UT * 2) * THREADS;
-    static_assert(W_T2 % 4 == 0 && W_EX % 4 == 0 && TILEW % 4 == 0, "16-byte aligned operator digits");
+    static constexpr int O_U = 2 * N2 * PZ, O_X = O_U + 2 * K * UZ + (2 * K * UZ) % 4, O_Y = O_X + 4 * TILEW,
+                         O_Z = O_Y + YT * TILEW, WORDS = O_Z + YT * TILEW;
     static constexpr size_t SMEM = 4 * (size_t)WORDS;
-    // input digits of a block: per warp and column tile (Y = 0..7, 8..15 of each plane; K > 8: 16.. of both)
-    // the lanes' operands as 16-byte groups and one 8-byte group, then per warp the scale's exponent
-    static constexpr int CT = N2 > 8 ? 2 : 1, TL = BIG ? 5 : CT, WB = BIG ? 18 : 14;
-    static constexpr int IN_EXP = WARPS * TL * WB * 32, IN_WORDS = IN_EXP + 16;
+    // input digits of a block: per column tile the lanes' operands as 16-byte groups and one 8-byte group, then
+    // the tiles' exponents
+    static constexpr int WB = BIG ? 18 : 14, IN_EXP = NTIN * WB * 32, IN_WORDS = IN_EXP + (NTIN + 7) / 8 * 4;
+    // operator digits of a block: row tiles 0 and 1 (1 with u's rows) and the rows' exponents; then those of
+    // the block times its term's coefficient (the z pass's operand)
+    static constexpr int X_EXP = 2 * TILEW, Z_OFF = X_EXP + 16, Z_EXP = YT * TILEW, OP_WORDS = Z_OFF + Z_EXP + 16;
+    static_assert(O_U % 4 == 0 && O_X % 4 == 0 && TILEW % 4 == 0 && IN_WORDS % 4 == 0, "16-byte aligned copies");
 };
 
 constexpr float FX_MAGIC = 12582912.0f;  // 1.5 * 2^23
 constexpr int FX_MAGIC_BITS = 0x4B400000;
-constexpr int FX_SEG = 64;           // items whose pointers a CTA holds at a time
-constexpr int FX_NONE = -1000000;  // exponent of a zero row or column
+constexpr int FX_SEG = 32;           // items whose pointers and exponents a CTA holds at a time
+constexpr int FX_NONE = -20000;      // exponent of a zero row or block
 
 // accumulator of digit pair (i, d - i): weights 0..3 have one, 4..6 two
 __device__ constexpr int fx_slot(int d, int i) { return d < 4 ? d : 4 + 2 * (d - 4) + ((i >= 2 && i <= 4) ? 1 : 0); }
@@ -210,16 +220,21 @@ __device__ __forceinline__ long long fx_from_double(double x, int efmax) {
     return ef == 0 ? 0 : (hi < 0 ? -f : f);
 }
 
+template <int K>
+struct FxRows {
+    static constexpr int N = FxGeo<K>::BIG ? 2 : 1;
+};
+
 // A 2K x 2K operator block's elements as a set of K warps holds them (unit = 0..K-1 the warp's place in
 // the set): lane k of a row's lane group has element k of that row.  A warp takes two rows side by side
 // where they fit (2K <= 16), else two one after the other.
 template <int K>
-__device__ __forceinline__ void fx_rows(double (&a)[FxGeo<K>::RP], const double *blk, int unit, int lane) {
+__device__ __forceinline__ void fx_rows(double (&a)[FxRows<K>::N], const double *blk, int unit, int lane) {
     using G = FxGeo<K>;
     constexpr int LW = G::BIG ? 32 : 16;
     const int k = lane % LW;
 #pragma unroll
-    for (int i = 0; i < G::RP; i++) {
+    for (int i = 0; i < FxRows<K>::N; i++) {
         const int r = G::BIG ? unit + i * K : 2 * unit + lane / LW;
         a[i] = k < G::N2 ? __ldg(blk + r * G::N2 + k) : 0.0;
     }
@@ -229,14 +244,14 @@ __device__ __forceinline__ void fx_rows(double (&a)[FxGeo<K>::RP], const double 
 // rows 4..; with U also u's rows, the wavelet columns of rows r < K: row 8 + r, or r - 8 for r >= 8, when
 // K > 8, else row r), and the rows' exponents e: sum_k |a| <= 2^e.
 template <int K, bool U>
-__device__ __forceinline__ void fx_put(const double (&rows)[FxGeo<K>::RP], double cf, int unit, int lane, uint32_t *d0,
-                                       uint32_t *d1, int *exps) {
+__device__ __forceinline__ void fx_put(const double (&rows)[FxRows<K>::N], double cf, int unit, int lane, uint32_t *d0,
+                                       uint32_t *d1, short *exps) {
     using G = FxGeo<K>;
     constexpr int LW = G::BIG ? 32 : 16;
     const int k = lane % LW;
     const unsigned mask = G::BIG ? 0xffffffffu : (lane < 16 ? 0xffffu : 0xffff0000u);
 #pragma unroll
-    for (int it = 0; it < G::RP; it++) {
+    for (int it = 0; it < FxRows<K>::N; it++) {
         const int r = G::BIG ? unit + it * K : 2 * unit + lane / LW;
         const double a = rows[it] * cf;
         const int hi = __double2hiint(a), lo = __double2loint(a);
@@ -253,7 +268,7 @@ __device__ __forceinline__ void fx_put(const double (&rows)[FxGeo<K>::RP], doubl
         if (hi < 0) f = -f;
         uint32_t q[7];
         fx_digits(f, 0, q);
-        if (k == 0) exps[r] = e;
+        if (k == 0) exps[r] = (short)e;
         if (k >= G::N2) continue;
 #pragma unroll
         for (int u = 0; u < (U ? 2 : 1); u++) {
@@ -286,33 +301,102 @@ __device__ __forceinline__ void fx_put(const double (&rows)[FxGeo<K>::RP], doubl
     }
 }
 
-// The digits of input blocks as the x pass's column operands (FxGeo::IN_WORDS words per block): an input
-// block serves a hundred items and more, so they are made once per apply.  One CTA per block, its warps
-// as in the apply.
+// kernel arguments by value: nothing to upload
+struct FxOpJobs {
+    static constexpr int MAX = 16;
+    FxOpJob job[MAX];
+};
+struct FxSets {
+    static constexpr int MAX = 16;
+    const double *in[MAX];
+    uint32_t *out[MAX];
+    long long first[MAX + 1];  // blocks of the sets before
+    int n;
+};
+
+// Operator blocks' digits (FxGeo::OP_WORDS words per block), the blocks of one scale of the grid's y-th
+// operator.  One CTA of K warps per block: the row tiles are put together in shared memory and leave in
+// 16-byte pieces.
 template <int K>
-__global__ void __launch_bounds__(FxGeo<K>::THREADS) to_fx_kernel(const double *blocks, uint32_t *out, int nblocks) {
+__global__ void __launch_bounds__(32 * K) op_to_fx_kernel(__grid_constant__ const FxOpJobs jobs) {
+    using G = FxGeo<K>;
+    extern __shared__ __align__(16) uint32_t fsm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const FxOpJob &J = jobs.job[blockIdx.y];
+    for (int b = blockIdx.x; b < J.n; b += gridDim.x) {
+        int t = 0, hi = J.op.T;  // the last term whose first block is at most b
+        while (hi - t > 1) {
+            const int m = (t + hi) / 2;
+            if (J.op.first[m * J.op.S + J.s] <= b)
+                t = m;
+            else
+                hi = m;
+        }
+        const int ts = t * J.op.S + J.s;
+        const double *block = J.op.b64 + (size_t)(J.op.off[ts] + b - J.op.first[ts]) * G::NC;
+        uint32_t *out = J.out + (size_t)b * G::OP_WORDS;
+        double rows[FxRows<K>::N];
+        fx_rows<K>(rows, block, warp, lane);
+        for (int i = threadIdx.x; i < G::OP_WORDS; i += 32 * K) {
+            const bool exps = (i >= G::X_EXP && i < G::Z_OFF) || i >= G::Z_OFF + G::Z_EXP;
+            fsm[i] = exps ? 0x10001u * (uint32_t)(FX_NONE & 0xffff) : 0u;  // rows that there are not
+        }
+        __syncthreads();
+        fx_put<K, true>(rows, 1.0, warp, lane, fsm, fsm + G::TILEW, reinterpret_cast<short *>(fsm + G::X_EXP));
+        uint32_t *z = fsm + G::Z_OFF;
+        fx_put<K, false>(rows, J.op.c[t], warp, lane, z, z + G::TILEW, reinterpret_cast<short *>(z + G::Z_EXP));
+        __syncthreads();
+        for (int i = threadIdx.x; i < G::OP_WORDS / 4; i += 32 * K)
+            reinterpret_cast<uint4 *>(out)[i] = reinterpret_cast<const uint4 *>(fsm)[i];
+        __syncthreads();
+    }
+}
+
+// plane Z and row Y of column n of the x pass's tile ti of plane group gr
+template <int K>
+__device__ __forceinline__ void fx_in_column(int gr, int ti, int n, int &Y, int &Z) {
+    using G = FxGeo<K>;
+    if (G::BIG && ti == 4) {
+        Y = 16 + (n & 3);
+        Z = 2 * gr + (n >> 2);
+    } else {
+        Y = 8 * (ti % G::CT) + n;
+        Z = G::BIG ? 2 * gr + ti / G::CT : gr;
+    }
+}
+
+// The digits of input blocks as the x pass's column operands (FxGeo::IN_WORDS words per block), one scale
+// per column tile (16-bit exponents), for the blocks of several trees at once.  One CTA per block, a warp
+// per tile.
+template <int K>
+__global__ void __launch_bounds__(FxGeo<K>::THREADS) to_fx_kernel(__grid_constant__ const FxSets S) {
     using G = FxGeo<K>;
     constexpr int N2 = G::N2, K2 = G::K2, K3 = G::K3;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3, Z0 = G::PL * warp;
-    for (int b = blockIdx.x; b < nblocks; b += gridDim.x) {
-        const double *in = blocks + (size_t)b * 8 * K3;
-        uint32_t *o = out + (size_t)b * G::IN_WORDS;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    for (long long b = blockIdx.x; b < S.first[S.n]; b += gridDim.x) {
+        int k = 0;
+        while (b >= S.first[k + 1]) k++;
+        const double *in = S.in[k] + (size_t)(b - S.first[k]) * 8 * K3;
+        uint32_t *o = S.out[k] + (size_t)(b - S.first[k]) * G::IN_WORDS;
         int ef = 0;
-        for (int i = lane; i < G::PL * G::NC; i += 32) {
-            const int zi = i >= G::NC, q = i - zi * G::NC, c = q / K2, Z = Z0 + zi, cz = Z >= K;
-            ef = max(ef, (__double2hiint(in[(size_t)(4 * cz + c) * K3 + (Z - cz * K) * K2 + (q - c * K2)]) >> 20) & 0x7ff);
-        }
-        ef = __reduce_max_sync(0xffffffffu, ef);
-        if (lane == 0) o[G::IN_EXP + warp] = (uint32_t)(ef == 0 ? FX_NONE : ef - 1022);
         auto at = [&](int X, int Y, int Z) -> long long {
             if (X >= N2 || Y >= N2) return 0;
             const int cx = X >= K, cy = Y >= K, cz = Z >= K;
             return fx_from_double(
                 in[(size_t)(cx + 2 * cy + 4 * cz) * K3 + (Z - cz * K) * K2 + (Y - cy * K) * K + (X - cx * K)], ef);
         };
-        for (int ti = 0; ti < G::TL; ti++) {
-            const bool rest = ti == G::PL * G::CT;  // K > 8: Y >= 16 of both planes
-            const int zi = rest ? g >> 2 : ti / G::CT, Y = rest ? 16 + (g & 3) : 8 * (ti % G::CT) + g, Z = Z0 + zi;
+        auto field = [&](int X, int Y, int Z) -> int {
+            if (X >= N2 || Y >= N2) return 0;
+            const int cx = X >= K, cy = Y >= K, cz = Z >= K;
+            return (__double2hiint(in[(size_t)(cx + 2 * cy + 4 * cz) * K3 + (Z - cz * K) * K2 + (Y - cy * K) * K + (X - cx * K)]) >> 20) & 0x7ff;
+        };
+        for (int tile = warp; tile < G::NTIN; tile += G::WARPS) {
+            int Y, Z;
+            fx_in_column<K>(tile / G::TL, tile % G::TL, g, Y, Z);
+            ef = 0;
+            for (int X = t; X < N2; X += 4) ef = max(ef, field(X, Y, Z));
+            ef = __reduce_max_sync(0xffffffffu, ef);
+            if (lane == 0) reinterpret_cast<short *>(o + G::IN_EXP)[tile] = (short)(ef == 0 ? FX_NONE : ef - 1022);
             uint32_t w[G::WB];
             uint32_t q[7];
             fx_digits(at(2 * t, Y, Z), at(2 * t + 1, Y, Z), q);
@@ -331,7 +415,7 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS) to_fx_kernel(const double *
                 w[16] = B.s56;
                 w[17] = B.s4;
             }
-            uint32_t *d = o + (warp * G::TL + ti) * G::WB * 32;
+            uint32_t *d = o + (size_t)tile * G::WB * 32;
 #pragma unroll
             for (int v = 0; v < G::WB / 4; v++)
                 reinterpret_cast<uint4 *>(d)[v * 32 + lane] = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
@@ -340,23 +424,21 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS) to_fx_kernel(const double *
     }
 }
 
-// one lane's operand of column tile ti of a warp's planes
+// one lane's operand of an x-pass tile
 template <int K>
-__device__ __forceinline__ void fx_load(FxB &B, const uint32_t *blk, int warp, int ti, int lane) {
+__device__ __forceinline__ void fx_load(FxB &B, const uint32_t *blk, int tile, int lane) {
     using G = FxGeo<K>;
-    const uint32_t *d = blk + (warp * G::TL + ti) * G::WB * 32;
+    const uint32_t *d = blk + tile * G::WB * 32;
+    // volatile: the loads stay where they are written, ahead of a barrier or of the tile before
     uint32_t w[G::WB];
 #pragma unroll
-    for (int v = 0; v < G::WB / 4; v++) {
-        const uint4 x = __ldg(reinterpret_cast<const uint4 *>(d) + v * 32 + lane);
-        w[4 * v] = x.x;
-        w[4 * v + 1] = x.y;
-        w[4 * v + 2] = x.z;
-        w[4 * v + 3] = x.w;
-    }
-    const uint2 y = __ldg(reinterpret_cast<const uint2 *>(d + (G::WB / 4) * 128) + lane);
-    w[G::WB - 2] = y.x;
-    w[G::WB - 1] = y.y;
+    for (int v = 0; v < G::WB / 4; v++)
+        asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(w[4 * v]), "=r"(w[4 * v + 1]), "=r"(w[4 * v + 2]), "=r"(w[4 * v + 3])
+                     : "l"(reinterpret_cast<const uint4 *>(d) + v * 32 + lane));
+    asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];"
+                 : "=r"(w[G::WB - 2]), "=r"(w[G::WB - 1])
+                 : "l"(reinterpret_cast<const uint2 *>(d + (G::WB / 4) * 128) + lane));
 #pragma unroll
     for (int s = 0; s < 7; s++) {
         B.m[s][0] = w[2 * s];
@@ -370,32 +452,67 @@ __device__ __forceinline__ void fx_load(FxB &B, const uint32_t *blk, int warp, i
     }
 }
 
+// One lane's operand of a y- or z-pass tile: p(k) is the column's k-th value, zero for k >= 2K.
+template <int K, typename F>
+__device__ __forceinline__ void fx_operand(FxB &B, int t, F p) {
+    using G = FxGeo<K>;
+    uint32_t q[7];
+    fx_digits(p(2 * t), p(2 * t + 1), q);
+#pragma unroll
+    for (int s = 0; s < 7; s++) B.m[s][0] = q[s];
+    if constexpr (G::N2 > 8) {
+        fx_digits(p(2 * t + 8), p(2 * t + 9), q);
+#pragma unroll
+        for (int s = 0; s < 7; s++) B.m[s][1] = q[s];
+    } else {
+#pragma unroll
+        for (int s = 0; s < 7; s++) B.m[s][1] = 0u;
+    }
+    if constexpr (G::BIG) {
+        const int k = 16 + 2 * (t & 1);
+        fx_digits(p(k), p(k + 1), q);
+        B.fold(q, t >= 2);
+    }
+}
+
+// column c of the y pass (a = Z) or z pass (a = Y'): the scaling columns (a < K, X' < K) first
+template <int K>
+__device__ __forceinline__ void fx_column(int c, int &a, int &x) {
+    constexpr int K2 = K * K;
+    const int q = c / K2, r = c - q * K2, i = r / K;
+    a = (q >> 1) * K + i;
+    x = (q & 1) * K + r - i * K;
+}
+
+__device__ __forceinline__ void fx_copy(uint32_t *dst, const uint32_t *src, int words) {
+    for (int i = 4 * threadIdx.x; i < words; i += 4 * blockDim.x)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + i)),
+                     "l"(src + i)
+                     : "memory");
+}
+
+// every copy issued so far has landed, for all threads of the CTA
+__device__ __forceinline__ void fx_landed() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+}
+
 template <int K>
 __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_kernel(ApplyLaunch L) {
     using G = FxGeo<K>;
-    constexpr int N2 = G::N2, K2 = G::K2, K3 = G::K3;
+    constexpr int N2 = G::N2, K2 = G::K2, K3 = G::K3, PX = G::PX, PZ = G::PZ, UX = G::UX, UZ = G::UZ;
     constexpr bool BIG = G::BIG;
-    constexpr int YT = G::CT;              // column tiles of Y < 16 (K > 8: one more of Y >= 16 for both planes)
-    constexpr int UT = G::UT, PL = G::PL;
-    constexpr int RA = BIG ? 6 : 4;        // results of a thread per column tile
+    constexpr int RA = BIG ? 6 : 4;  // results of a thread per column tile
     extern __shared__ __align__(16) uint32_t fsm[];
-    uint32_t *s_t2 = fsm, *s_ex = fsm + G::O_EX;
-    long long *s_u = reinterpret_cast<long long *>(fsm + G::O_U) + threadIdx.x;  // u: a thread's own values
-    __shared__ int s_node, s_redf;
-    __shared__ int s_exx[2][32], s_exy[2][32], s_exz[2][32], s_e1[2][32];  // row exponents; T1's column exponents
-    __shared__ const uint32_t *s_pi[FX_SEG];
-    __shared__ const double *s_px[FX_SEG], *s_py[FX_SEG], *s_pz[FX_SEG];
-    __shared__ double s_cf[FX_SEG];
+    long long *s_t = reinterpret_cast<long long *>(fsm), *s_u = reinterpret_cast<long long *>(fsm + G::O_U);
+    __shared__ int s_node, s_redf, s_e1[2][32];  // s_e1: T1's column exponents
+    __shared__ const uint32_t *s_pi[FX_SEG], *s_px[FX_SEG], *s_py[FX_SEG], *s_pz[FX_SEG];
+    __shared__ short s_ein[FX_SEG][(G::NTIN + 7) / 8 * 8];  // column exponents, per x-pass tile
+    __shared__ short s_exx[FX_SEG][32], s_exy[FX_SEG][32], s_exz[FX_SEG][32];  // row exponents
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const bool root = L.root != 0;
-    const int Z0 = PL * warp;  // this warp's planes Z0 (and Z0 + 1)
-    const bool ux[2] = {!root && Z0 < K, PL > 1 && !root && Z0 + 1 < K};  // the planes that have u
-    // operator digits: sets of K warps; with twice as many warps the second set takes A_y and A_z
-    const int unit = BIG || warp < K ? warp : warp - K;
-    const bool put_x = BIG || warp < K, put_yz = BIG || warp >= K;
-
-    for (int i = G::O_X + tid; i < G::WORDS; i += G::THREADS) fsm[i] = 0u;  // unused operator rows and columns
-    if (tid < 64) (&s_exx[0][0])[tid] = (&s_exy[0][0])[tid] = (&s_exz[0][0])[tid] = FX_NONE;
+    // the rows of this lane's results: g, 8 + g and, in the second row tile, 12 + g (g >= 4) or u's 8 + g
+    const int x2 = g >= 4 ? 12 + g : 8 + g;
 
     while (true) {
         __syncthreads();
@@ -405,295 +522,209 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
         const int w = s_node;
         if (w >= L.nnodes) break;
         const long long b0 = L.begin[w], b1 = L.end[w];
-        // node accumulator: per column tile (8 nt + 2t, + 1) rows Z' = g, 8 + g, 12 + g (g >= 4), each
-        // tile of a thread in units of 2^(ea - 62).  Indexed in a rolled loop, so it lives in local
-        // memory between the z passes and leaves the registers to T1.
+        // node accumulator: per column tile of this warp (columns 8 nt + 2t, + 1) rows Z' = g, 8 + g, 12 + g
+        // (g >= 4), each tile of a thread in units of 2^(ea - 62).  Indexed in a rolled loop, so it lives in
+        // local memory between the z passes.
         long long acc[G::TPW][RA];
         int ea[G::TPW];
 #pragma unroll 1
         for (int q = 0; q < G::TPW; q++) {
-            ea[q] = 2 * FX_NONE;
+            ea[q] = -1000000;
             for (int r = 0; r < RA; r++) acc[q][r] = 0;
         }
-        int nrows = 0, par = 0, xb = 0, zb = 0;
-        const double *lastz = nullptr;
+        int nrows = 0, par = 0;
         for (long long sb = b0; sb < b1; sb += FX_SEG) {
             const int ni = (int)min((long long)FX_SEG, b1 - sb);
             if (sb != b0) __syncthreads();
             for (int i = tid; i < ni; i += G::THREADS) {
                 s_pi[i] = reinterpret_cast<const uint32_t *>(L.in[sb + i]);
-                s_px[i] = reinterpret_cast<const double *>(L.ax[sb + i]);
-                s_py[i] = reinterpret_cast<const double *>(L.ay[sb + i]);
-                s_pz[i] = reinterpret_cast<const double *>(L.az[sb + i]);
-                s_cf[i] = L.coef[sb + i];
+                s_px[i] = reinterpret_cast<const uint32_t *>(L.ax[sb + i]);
+                s_py[i] = reinterpret_cast<const uint32_t *>(L.ay[sb + i]);
+                s_pz[i] = reinterpret_cast<const uint32_t *>(L.az[sb + i]);
             }
             __syncthreads();
-            double rx[G::RP], ry[G::RP], rz[G::RP];  // operator elements on their way
-            if (put_x) fx_rows<K>(rx, s_px[0], unit, lane);
-            if (put_yz) fx_rows<K>(ry, s_py[0], unit, lane);
+            fx_copy(fsm + G::O_X, s_px[0], 2 * G::TILEW);
+            fx_copy(fsm + G::O_Y, s_py[0], G::YT * G::TILEW);
+            for (int i = tid; i < 32 * ni; i += G::THREADS) {
+                const int j = i >> 5, r = i & 31;
+                s_exx[j][r] = reinterpret_cast<const short *>(s_px[j] + G::X_EXP)[r];
+                s_exy[j][r] = reinterpret_cast<const short *>(s_py[j] + G::X_EXP)[r];
+                s_exz[j][r] = reinterpret_cast<const short *>(s_pz[j] + G::Z_EXP)[r];
+            }
+            for (int i = tid; i < ni * G::NTIN; i += G::THREADS) {
+                const int j = i / G::NTIN, r = i - j * G::NTIN;
+                s_ein[j][r] = reinterpret_cast<const short *>(s_pi[j] + G::IN_EXP)[r];
+            }
+            const uint32_t *lastz = nullptr;
             for (int j0 = 0; j0 < ni;) {
                 int j1 = j0 + 1;  // the row: items of one term, ly and lz
                 while (j1 < ni && s_py[j1] == s_py[j0] && s_pz[j1] == s_pz[j0]) j1++;
                 const int hb = 32 - __clz(j1 - j0 - 1);  // head room of the row's sum, bits
-                const bool single = j1 == j0 + 1, newz = s_pz[j0] != lastz;  // rows of one term and lz share A_z
-                if (put_yz) fx_put<K, false>(ry, 1.0, unit, lane, fsm + G::O_Y, fsm + G::O_Y + G::TILEW, s_exy[par]);
-                // T1: [plane][Y tile][register]; cm, cs: the tile Y >= 16 of both planes (K > 8)
-                long long tm[PL][YT][4], ts[2][2][2], cm[4], cs[2];
-                int et0 = FX_NONE, et1 = FX_NONE, et2 = FX_NONE;  // exponents of rows X' = g, 8 + g, 12 + g (u: 8 + g)
+                const bool single = j1 == j0 + 1;
+                int h0 = 5 * FX_NONE, h1 = h0, h2 = h0;  // largest exponents of T1's rows X' = g, 8 + g, x2
                 for (int j = j0; j < j1; j++) {
-                    const bool first = j == j0;
+                    const bool first = j == j0, last = j + 1 == j1;
                     const uint32_t *in = s_pi[j];
                     FxB B, Bn;
-                    fx_load<K>(Bn, in, warp, 0, lane);
-                    const int ein = (int)__ldg(in + G::IN_EXP + warp);
-                    uint32_t *fx0 = fsm + G::O_X + xb * 2 * G::TILEW, *fx1 = fx0 + G::TILEW;
-                    if (put_x) fx_put<K, true>(rx, 1.0, unit, lane, fx0, fx1, s_exx[xb]);
-                    __syncthreads();
-                    if (put_x && j + 1 < ni) fx_rows<K>(rx, s_px[j + 1], unit, lane);
-                    if (put_yz && first && newz) fx_rows<K>(rz, s_pz[j0], unit, lane);
-                    const int ex0 = ein + s_exx[xb][g], ex1 = ein + s_exx[xb][8 + g],
-                              ex2 = ein + s_exx[xb][g >= 4 ? 12 + g : 8 + g];
-                    // sums of the row's items at a common exponent (hb bits of head room)
-                    const int n0 = max(et0, ex0 + hb), n1 = max(et1, ex1 + hb), n2 = max(et2, ex2 + hb);
-                    if (!first && __any_sync(0xffffffffu, n0 > et0 || n1 > et1 || n2 > et2)) {
-                        // a larger scale than the row's so far: its sums move there
-#pragma unroll
-                        for (int zi = 0; zi < PL; zi++)
-#pragma unroll
-                            for (int tl = 0; tl < YT; tl++) {
-#pragma unroll
-                                for (int r = 0; r < 4; r++) tm[zi][tl][r] = fx_shift(tm[zi][tl][r], r < 2 ? n0 - et0 : n1 - et1);
-#pragma unroll
-                                for (int r = 0; r < 2; r++) {
-                                    if constexpr (BIG) ts[zi][tl][r] = fx_shift(ts[zi][tl][r], n2 - et2);
-                                    if (tl < UT && ux[zi]) {
-                                        long long *u = s_u + ((zi * UT + tl) * 2 + r) * G::THREADS;
-                                        *u = fx_shift(*u, n0 - et0);
-                                    }
-                                }
-                            }
-                        if constexpr (BIG) {
-#pragma unroll
-                            for (int r = 0; r < 4; r++) cm[r] = fx_shift(cm[r], r < 2 ? n0 - et0 : n1 - et1);
-#pragma unroll
-                            for (int r = 0; r < 2; r++) cs[r] = fx_shift(cs[r], n2 - et2);
+                    if (warp < G::NTIN) fx_load<K>(Bn, in, warp, lane);
+                    fx_landed();  // A_x (and A_y); the z pass has read T
+                    if (first) {
+                        if (s_pz[j0] != lastz) {  // rows of one term and lz share A_z
+                            lastz = s_pz[j0];
+                            fx_copy(fsm + G::O_Z, lastz, G::YT * G::TILEW);
                         }
                     }
-                    // several items: every result moves right by at least the head room, rounded
-                    const int m0 = min(n0 - ex0 - 1, 62), m1 = min(n1 - ex1 - 1, 62), m2 = min(n2 - ex2 - 1, 62);
-                    auto add = [&](long long s, long long v, int m) -> long long {
-                        if (single) return v;
-                        v = ((v >> m) + 1) >> 1;
-                        return first ? v : s + v;
-                    };
-                    float D[10][4];
-#pragma unroll
-                    for (int zi = 0; zi < PL; zi++) {
-#pragma unroll
-                        for (int tl = 0; tl < YT; tl++) {
-                            B = Bn;  // the next tile's operand comes from L2 behind this one's products
-                            if (zi * YT + tl + 1 < G::TL) fx_load<K>(Bn, in, warp, zi * YT + tl + 1, lane);
-                            fx_tile<BIG>(D, fx0, B, lane);
-#pragma unroll
-                            for (int r = 0; r < 4; r++)
-                                tm[zi][tl][r] = add(tm[zi][tl][r], fx_value(D, r), r < 2 ? m0 : m1);
-                            if (BIG || (tl == 0 && ux[zi])) {
-                                fx_tile<BIG>(D, fx1, B, lane);
-#pragma unroll
-                                for (int r = 0; r < 2; r++) {
-                                    if constexpr (BIG) ts[zi][tl][r] = add(ts[zi][tl][r], fx_value(D, r), m2);
-                                    if (ux[zi]) {
-                                        long long *u = s_u + ((zi * UT + (BIG ? tl : 0)) * 2 + r) * G::THREADS;
-                                        *u = add(*u, fx_value(D, (BIG ? 2 : 0) + r), m0);
-                                    }
-                                }
+                    const int exg = s_exx[j][g], exh = s_exx[j][8 + g], exq = s_exx[j][x2];
+                    const uint32_t *fx0 = fsm + G::O_X + (j & 1) * 2 * G::TILEW, *fx1 = fx0 + G::TILEW;
+                    if (j + 1 < ni) fx_copy(fsm + G::O_X + ((j + 1) & 1) * 2 * G::TILEW, s_px[j + 1], 2 * G::TILEW);
+#pragma unroll 1
+                    for (int tile = warp; tile < G::NTIN; tile += G::WARPS) {
+                        B = Bn;  // the next tile's operand comes from L2 behind this one's products
+                        if (tile + G::WARPS < G::NTIN) fx_load<K>(Bn, in, tile + G::WARPS, lane);
+                        const int gr = tile / G::TL, ti = tile - gr * G::TL;
+                        // the row's sums at the tile's largest exponents, with head room; of several items every
+                        // result moves right by at least that, rounded
+                        const int ej = s_ein[j][tile];
+                        int et0 = ej + exg, et1 = ej + exh, et2 = ej + exq, m0 = 0, m1 = 0, m2 = 0;
+                        if (!single) {
+                            const int f0 = et0, f1 = et1, f2 = et2;
+                            for (int i = j0; i < j1; i++) {
+                                const int e = s_ein[i][tile];
+                                et0 = max(et0, e + s_exx[i][g]);
+                                et1 = max(et1, e + s_exx[i][8 + g]);
+                                if (BIG) et2 = max(et2, e + s_exx[i][x2]);
                             }
+                            et0 += hb;
+                            et1 += hb;
+                            et2 += hb;
+                            m0 = min(et0 - f0 - 1, 62), m1 = min(et1 - f1 - 1, 62), m2 = min(et2 - f2 - 1, 62);
                         }
-                    }
-                    if constexpr (BIG) {
-                        B = Bn;
+                        unsigned long long o0 = 0, o1 = 0, o2 = 0;
+                        auto add = [&](long long *s, long long v, int m, unsigned long long &o) {
+                            if (!single) {
+                                v = ((v >> m) + 1) >> 1;
+                                if (!first) v += *s;
+                            }
+                            *s = v;
+                            o |= (unsigned long long)(v ^ (v >> 63));
+                        };
+                        int Y, Z;  // of column 2t; column 2t + 1 is Y + 1
+                        fx_in_column<K>(gr, ti, 2 * t, Y, Z);
+                        long long *T = s_t + Z * PZ + Y * PX, *u = s_u + Z * UZ + Y * UX;
+                        float D[10][4];
                         fx_tile<BIG>(D, fx0, B, lane);
 #pragma unroll
-                        for (int r = 0; r < 4; r++) cm[r] = add(cm[r], fx_value(D, r), r < 2 ? m0 : m1);
-                        fx_tile<BIG>(D, fx1, B, lane);
+                        for (int r = 0; r < 4; r++)
+                            if (g + 8 * (r >> 1) < N2 && Y + (r & 1) < N2)
+                                add(T + (r & 1) * PX + g + 8 * (r >> 1), fx_value(D, r), r < 2 ? m0 : m1, r < 2 ? o0 : o1);
+                        const bool has_u = !root && Z < K && Y < K;
+                        if constexpr (BIG) {
+                            fx_tile<BIG>(D, fx1, B, lane);
 #pragma unroll
-                        for (int r = 0; r < 2; r++) cs[r] = add(cs[r], fx_value(D, r), m2);
-                    }
-                    et0 = n0;
-                    et1 = n1;
-                    et2 = n2;
-                    xb ^= 1;
-                }
-                // T1's columns to the largest magnitude over the CTA's planes
-                {
-                    auto mag = [](long long v) { return (unsigned long long)(v ^ (v >> 63)); };
-                    unsigned long long o0 = 0, o1 = 0, o2 = 0;
-#pragma unroll
-                    for (int zi = 0; zi < PL; zi++)
-#pragma unroll
-                        for (int tl = 0; tl < YT; tl++) {
-                            o0 |= mag(tm[zi][tl][0]) | mag(tm[zi][tl][1]);
-                            o1 |= mag(tm[zi][tl][2]) | mag(tm[zi][tl][3]);
-                            if constexpr (BIG) o2 |= mag(ts[zi][tl][0]) | mag(ts[zi][tl][1]);
-                            if (tl < UT && ux[zi]) {
-                                const long long *u = s_u + (zi * UT + tl) * 2 * G::THREADS;
-                                o0 |= mag(u[0]) | mag(u[G::THREADS]);
+                            for (int r = 0; r < 2; r++) {
+                                if (g >= 4 && 12 + g < N2 && Y + r < N2) add(T + r * PX + 12 + g, fx_value(D, r), m2, o2);
+                                if (g < 2 && 8 + g < K && has_u && Y + r < K) add(u + r * UX + 8 + g, fx_value(D, r), m2, o2);
+                                if (has_u && Y + r < K) add(u + r * UX + g, fx_value(D, 2 + r), m0, o0);
                             }
+                        } else if (!root && ti == 0 && gr < K) {
+                            fx_tile<BIG>(D, fx1, B, lane);
+#pragma unroll
+                            for (int r = 0; r < 2; r++)
+                                if (g < K && Y + r < K) add(u + r * UX + g, fx_value(D, r), m0, o0);
                         }
-                    if constexpr (BIG) {
-                        o0 |= mag(cm[0]) | mag(cm[1]);
-                        o1 |= mag(cm[2]) | mag(cm[3]);
-                        o2 |= mag(cs[0]) | mag(cs[1]);
+                        if (last) {  // |v| < 2^(64 - clz)
+                            if (o0) h0 = max(h0, et0 + 2 - __clzll(o0));
+                            if (o1) h1 = max(h1, et1 + 2 - __clzll(o1));
+                            if (o2) h2 = max(h2, et2 + 2 - __clzll(o2));
+                        }
                     }
-                    auto post = [&](unsigned long long o, int e, int X) {
-                        o |= __shfl_xor_sync(0xffffffffu, o, 1);
-                        o |= __shfl_xor_sync(0xffffffffu, o, 2);
-                        if (t == 0 && o != 0 && X < N2) atomicMax(&s_e1[par][X], e + 2 - __clzll(o));  // |v| < 2^(64 - clz)
+                }
+                // T1's columns X' to their largest magnitude
+                {
+                    auto post = [&](int e, int X) {
+                        e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
+                        e = max(e, __shfl_xor_sync(0xffffffffu, e, 2));
+                        if (t == 0 && e > FX_NONE) atomicMax(&s_e1[par][X], e);
                     };
-                    post(o0, et0, g);
-                    if (N2 > 8) post(o1, et1, 8 + g);
-                    if constexpr (BIG) post(o2, et2, g >= 4 ? 12 + g : 8 + (g & 1));
+                    post(h0, g);
+                    if (N2 > 8) post(h1, 8 + g);
+                    if constexpr (BIG) post(h2, x2);
                 }
-                __syncthreads();
-                if (newz) {
-                    lastz = s_pz[j0];
-                    zb ^= 1;
-                    if (put_yz) fx_put<K, false>(rz, s_cf[j0], unit, lane, fsm + G::O_Z, fsm + G::O_Z + G::TILEW, s_exz[zb]);
-                }
-                if (put_yz && j1 < ni) fx_rows<K>(ry, s_py[j1], unit, lane);
+                fx_landed();
                 if (tid < 32) s_e1[par ^ 1][tid] = FX_NONE;
-                // y pass, one column tile of X' at a time; results to shared memory as digits
-                {
-                    const FxShift d0(s_e1[par][g] - et0), d1(N2 > 8 ? s_e1[par][8 + g] - et1 : 0),
-                        d2(BIG ? s_e1[par][g >= 4 ? 12 + g : 8 + (g & 1)] - et2 : 0);
-                    const uint32_t *fy0 = fsm + G::O_Y, *fy1 = fy0 + G::TILEW;
-                    // columns X' of tile kind 0: 0..7, 1: 8..15, 2: 16..19 (n >= 4) and u's 8, 9 (n < 2), 3: u's 0..7
-                    auto run = [&](auto kind_c) {
-                        constexpr int kind = decltype(kind_c)::value;
-                        const FxShift &dk = kind == 1 ? d1 : (kind == 2 ? d2 : d0);
-                        [[maybe_unused]] uint32_t wr[7];
-                        if constexpr (BIG) {  // the remainder Y >= 16: lanes t < 2 hold plane 0, t >= 2 plane 1
-                            const bool u8 = kind == 2 && g < 4;
-                            const long long c0 = kind == 1 || u8 ? cm[2] : (kind == 2 ? cs[0] : cm[0]),
-                                            c1 = kind == 1 || u8 ? cm[3] : (kind == 2 ? cs[1] : cm[1]);
-                            const FxShift &dr = u8 ? d1 : dk;
-                            fx_digits(dr(c0), dr(c1), wr);
+                // y pass in place: a warp reads its 8 columns (Z, X') whole before it writes them
+                const uint32_t *fy0 = fsm + G::O_Y, *fy1 = fy0 + G::TILEW;
+#pragma unroll 1
+                for (int tile = warp; tile < G::NT; tile += G::WARPS) {
+                    const int c = 8 * tile + g;
+                    int Z, X;
+                    fx_column<K>(min(c, G::NC - 1), Z, X);
+                    // T1's exponents by the x-pass tiles that Y = 0..7, 8..15 and 16.. came from
+                    const int gr = BIG ? Z >> 1 : Z, it = gr * G::TL + (BIG ? (Z & 1) * G::CT : 0);
+                    int e0 = 5 * FX_NONE, e1 = e0, e2 = e0;
+                    for (int i = j0; i < j1; i++) {
+                        const int ex = s_exx[i][X] + hb;
+                        e0 = max(e0, s_ein[i][it] + ex);
+                        if (N2 > 8) e1 = max(e1, s_ein[i][it + 1] + ex);
+                        if (BIG) e2 = max(e2, s_ein[i][gr * G::TL + 4] + ex);
+                    }
+                    const int ee = s_e1[par][X];
+                    const FxShift sh0(ee - e0), sh1(ee - e1), sh2(ee - e2);
+                    auto sh = [&](long long v, int Y) { return Y < 8 ? sh0(v) : (Y < 16 ? sh1(v) : sh2(v)); };
+                    const long long *T = s_t + Z * PZ + X, *u = s_u + Z * UZ + X;
+                    int Zr[2], Xr[2];  // of the results' columns 2t, 2t + 1
+#pragma unroll
+                    for (int b = 0; b < 2; b++) fx_column<K>(min(8 * tile + 2 * t + b, G::NC - 1), Zr[b], Xr[b]);
+                    FxB B;
+                    float D[10][4];
+                    if (!root && tile < G::NTX) {  // scaling columns: u where Y < K
+                        const bool in = c < K2;
+                        fx_operand<K>(B, t, [&](int Y) -> long long {
+                            return !in || Y >= N2 ? 0 : sh(Y < K ? u[Y * UX] : T[Y * PX], Y);
+                        });
+                        fx_tile<BIG>(D, fy0, B, lane);
+                        __syncwarp();
+#pragma unroll
+                        for (int r = 0; r < 4; r++) {
+                            const int Yq = g + 8 * (r >> 1), b = r & 1;
+                            if (Yq < K && 8 * tile + 2 * t + b < K2) s_u[Zr[b] * UZ + Yq * UX + Xr[b]] = fx_value(D, r);
                         }
+                    }
+                    const bool in = c < G::NC;
+                    fx_operand<K>(B, t, [&](int Y) -> long long { return !in || Y >= N2 ? 0 : sh(T[Y * PX], Y); });
+                    fx_tile<BIG>(D, fy0, B, lane);
+                    __syncwarp();
 #pragma unroll
-                        for (int zi = 0; zi < PL; zi++) {
-                            if (kind == 3 && !ux[zi]) continue;
-                            const int Z = Z0 + zi;
-                            FxB B;
-                            uint32_t q[7];
-                            long long p0, p1, p2 = 0, p3 = 0;  // Y = 2t, 2t + 1, 2t + 8, 2t + 9
-                            if constexpr (kind == 0) {
-                                p0 = tm[zi][0][0], p1 = tm[zi][0][1];
-                                if constexpr (N2 > 8) p2 = tm[zi][YT - 1][0], p3 = tm[zi][YT - 1][1];
-                            } else if constexpr (kind == 1) {
-                                p0 = tm[zi][0][2], p1 = tm[zi][0][3];
-                                p2 = tm[zi][YT - 1][2], p3 = tm[zi][YT - 1][3];
-                            } else if constexpr (kind == 2) {
-                                p0 = ts[zi][0][0], p1 = ts[zi][0][1];
-                                p2 = g >= 4 || 8 + 2 * t < K ? ts[zi][1][0] : tm[zi][YT - 1][2];
-                                p3 = g >= 4 || 9 + 2 * t < K ? ts[zi][1][1] : tm[zi][YT - 1][3];
-                            } else {
-                                const long long *u = s_u + zi * UT * 2 * G::THREADS;
-                                p0 = 2 * t < K ? u[0] : tm[zi][0][0];
-                                p1 = 2 * t + 1 < K ? u[G::THREADS] : tm[zi][0][1];
-                                if constexpr (N2 > 8) {
-                                    p2 = BIG && 8 + 2 * t < K ? u[2 * (UT - 1) * G::THREADS] : tm[zi][YT - 1][0];
-                                    p3 = BIG && 9 + 2 * t < K ? u[(2 * (UT - 1) + 1) * G::THREADS] : tm[zi][YT - 1][1];
-                                }
-                            }
-                            fx_digits(dk(p0), dk(p1), q);
+                    for (int r = 0; r < 4; r++) {
+                        const int Yq = g + 8 * (r >> 1), b = r & 1;
+                        if (Yq < N2 && 8 * tile + 2 * t + b < G::NC) s_t[Zr[b] * PZ + Yq * PX + Xr[b]] = fx_value(D, r);
+                    }
+                    if constexpr (BIG) {
+                        fx_tile<BIG>(D, fy1, B, lane);
 #pragma unroll
-                            for (int s = 0; s < 7; s++) B.m[s][0] = q[s];
-                            if constexpr (N2 > 8) fx_digits(dk(p2), dk(p3), q);
-#pragma unroll
-                            for (int s = 0; s < 7; s++) B.m[s][1] = N2 > 8 ? q[s] : 0u;
-                            if constexpr (BIG) {
-                                const int src = 4 * g + (t & 1) + 2 * zi;
-#pragma unroll
-                                for (int s = 0; s < 7; s++) q[s] = __shfl_sync(0xffffffffu, wr[s], src);
-                                B.fold(q, t >= 2);
-                            }
-                            // results of one row of Y' for columns n = 2t, 2t + 1: digit halves into the words of
-                            // the plane's Z pair
-                            auto put = [&](long long v0, long long v1, int Yq) {
-                                fx_digits(v0, v1, q);
-                                const int n = 2 * t;
-                                const bool ext = kind == 3 || (kind == 2 && n < 2);
-#pragma unroll
-                                for (int b = 0; b < 2; b++) {
-                                    const int nb = n + b;
-                                    const int Xq = kind == 0 || kind == 3 ? nb : (kind == 1 || nb < 2 ? 8 + nb : (nb >= 4 ? 12 + nb : N2));
-                                    unsigned short *o;
-                                    int step;
-                                    if (ext) {
-                                        if (!ux[zi] || Yq >= K || Xq >= K) continue;
-                                        o = reinterpret_cast<unsigned short *>(s_ex + (Z >> 1) * G::PE + Yq * K + Xq) + (Z & 1);
-                                        step = 2 * G::KE * G::PE;
-                                    } else {
-                                        if (Yq >= N2 || Xq >= N2) continue;
-                                        const int hy = Yq >= K, hx = Xq >= K;
-                                        o = reinterpret_cast<unsigned short *>(
-                                                s_t2 + (Z >> 1) * G::P + (2 * hy + hx) * K2 + (Yq - hy * K) * K + (Xq - hx * K)) + (Z & 1);
-                                        step = 2 * K * G::P;
-                                    }
-#pragma unroll
-                                    for (int s = 0; s < 7; s++) o[s * step] = (unsigned short)(b ? q[s] >> 16 : q[s]);
-                                }
-                            };
-                            float D[10][4];
-                            fx_tile<BIG>(D, fy0, B, lane);
-                            put(fx_value(D, 0), fx_value(D, 1), g);
-                            if constexpr (N2 > 8) put(fx_value(D, 2), fx_value(D, 3), 8 + g);
-                            if constexpr (BIG && kind != 3) {
-                                fx_tile<BIG>(D, fy1, B, lane);
-                                put(fx_value(D, 0), fx_value(D, 1), g >= 4 ? 12 + g : N2);
-                            }
-                        }
-                    };
-                    run(std::integral_constant<int, 0>());
-                    if constexpr (N2 > 8) run(std::integral_constant<int, 1>());
-                    if constexpr (BIG) run(std::integral_constant<int, 2>());
-                    if (ux[0]) run(std::integral_constant<int, 3>());
+                        for (int b = 0; b < 2; b++)
+                            if (g >= 4 && 12 + g < N2 && 8 * tile + 2 * t + b < G::NC)
+                                s_t[Zr[b] * PZ + (12 + g) * PX + Xr[b]] = fx_value(D, b);
+                    }
                 }
-                __syncthreads();
+                fx_landed();  // T2 (and A_z)
+                if (j1 < ni) fx_copy(fsm + G::O_Y, s_py[j1], G::YT * G::TILEW);
                 // z pass over this warp's column tiles
                 const uint32_t *fz0 = fsm + G::O_Z, *fz1 = fz0 + G::TILEW;
-                const int ez0 = s_exz[zb][g], ez1 = s_exz[zb][8 + g], ez2 = s_exz[zb][g >= 4 ? 12 + g : 31];
+                const int ez0 = s_exz[j0][g], ez1 = s_exz[j0][8 + g], ez2 = g >= 4 && BIG ? s_exz[j0][12 + g] : FX_NONE;
 #pragma unroll 1
                 for (int q = 0; q < G::TPW; q++) {
                     const int nt = warp + q * G::WARPS;
                     if (nt >= G::NT) continue;
-                    // word of Z pair zp, digit s, column 8 nt + g; second operand: Z < K from s_ex
-                    auto word = [&](int s, int zp, bool second) -> uint32_t {
-                        if (zp >= K) return 0u;
-                        const int c = 8 * nt + g;
-                        if (!second || zp >= G::KE) return s_t2[(s * K + zp) * G::P + c];
-                        uint32_t e = s_ex[(s * G::KE + zp) * G::PE + c];
-                        if ((K & 1) && zp == G::KE - 1) e = __byte_perm(e, s_t2[(s * K + zp) * G::P + c], 0x7610);
-                        return e;
-                    };
-                    auto operand = [&](FxB &B, bool second) {
-#pragma unroll
-                        for (int s = 0; s < 7; s++) {
-                            B.m[s][0] = word(s, t, second);
-                            B.m[s][1] = word(s, t + 4, second);
-                        }
-                        if constexpr (BIG) {
-                            const int zp = 8 + (t & 1), h = t >> 1;
-                            B.s01 = word(h, zp, second);
-                            B.s23 = word(2 + h, zp, second);
-                            B.s56 = word(5 + h, zp, second);
-                            B.s4 = h ? 0u : word(4, zp, second);
-                        }
-                    };
+                    const int c = 8 * nt + g;
+                    int Yc, X;
+                    fx_column<K>(min(c, G::NC - 1), Yc, X);
+                    const long long *T = s_t + Yc * PX + X, *u = s_u + Yc * UX + X;
                     FxB B;
                     float D[10][4];
                     long long v[RA];
-                    operand(B, false);
+                    const bool in = c < G::NC;
+                    fx_operand<K>(B, t, [&](int Z) -> long long { return !in || Z >= N2 ? 0 : T[Z * PZ]; });
                     fx_tile<BIG>(D, fz0, B, lane);
 #pragma unroll
                     for (int r = 0; r < 4; r++) v[r] = fx_value(D, r);
@@ -702,20 +733,20 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
 #pragma unroll
                         for (int r = 0; r < 2; r++) v[4 + r] = fx_value(D, r);
                     }
-                    if (!root && nt < G::NTX) {
-                        operand(B, true);
+                    if (!root && nt < G::NTX) {  // scaling columns: the path without scaling-scaling where Z < K
+                        const bool ins = c < K2;
+                        fx_operand<K>(B, t, [&](int Z) -> long long { return !ins || Z >= N2 ? 0 : Z < K ? u[Z * UZ] : T[Z * PZ]; });
                         fx_tile<BIG>(D, fz0, B, lane);
 #pragma unroll
-                        for (int r = 0; r < 4; r++) {
-                            const int Zq = r < 2 ? g : 8 + g;
-                            if (8 * nt + 2 * t + (r & 1) < K2 && Zq < K) v[r] = fx_value(D, r);
-                        }
+                        for (int r = 0; r < 4; r++)
+                            if (8 * nt + 2 * t + (r & 1) < K2 && g + 8 * (r >> 1) < K) v[r] = fx_value(D, r);
                     }
                     int ec[2];
 #pragma unroll
                     for (int b = 0; b < 2; b++) {
-                        const int c = min(8 * nt + 2 * t + b, G::NC - 1), hq = c / K2, rq = c - hq * K2, yq = rq / K;
-                        ec[b] = s_e1[par][(hq & 1) * K + rq - yq * K] + s_exy[par][(hq >> 1) * K + yq];
+                        int Yr, Xr;
+                        fx_column<K>(min(8 * nt + 2 * t + b, G::NC - 1), Yr, Xr);
+                        ec[b] = s_e1[par][Xr] + s_exy[j0][Yr];
                     }
                     int e[RA];
 #pragma unroll
@@ -779,8 +810,17 @@ void launch_fx(const ApplyLaunch &L, cudaStream_t s) {
 }
 
 template <int K>
-void launch_to_fx(const double *blocks, uint32_t *out, size_t n, cudaStream_t s) {
-    to_fx_kernel<K><<<(int)std::min<size_t>(n, 65535), FxGeo<K>::THREADS, 0, s>>>(blocks, out, (int)n);
+void launch_to_fx(const FxSets &S, cudaStream_t s) {
+    const int grid = (int)std::min<long long>(S.first[S.n], 65535);
+    to_fx_kernel<K><<<grid, FxGeo<K>::THREADS, 0, s>>>(S);
+    MWG_CUDA(cudaGetLastError());
+}
+
+template <int K>
+void launch_op_to_fx(const FxOpJobs &jobs, int njobs, int most, cudaStream_t s) {
+    const size_t smem = 4 * (size_t)FxGeo<K>::OP_WORDS;
+    kernel_smem((const void *)op_to_fx_kernel<K>, (int)smem);
+    op_to_fx_kernel<K><<<dim3(most, njobs), 32 * K, smem, s>>>(jobs);
     MWG_CUDA(cudaGetLastError());
 }
 
@@ -799,17 +839,63 @@ size_t fx_words(int K) {
     }
 }
 
-void k_to_fx(const double *blocks, uint32_t *out, size_t n, int K, cudaStream_t s) {
-    if (n == 0) return;
+size_t fx_op_words(int K) {
     switch (K) {
-        case 4: launch_to_fx<4>(blocks, out, n, s); break;
-        case 5: launch_to_fx<5>(blocks, out, n, s); break;
-        case 6: launch_to_fx<6>(blocks, out, n, s); break;
-        case 7: launch_to_fx<7>(blocks, out, n, s); break;
-        case 8: launch_to_fx<8>(blocks, out, n, s); break;
-        case 9: launch_to_fx<9>(blocks, out, n, s); break;
-        case 10: launch_to_fx<10>(blocks, out, n, s); break;
+        case 4: return FxGeo<4>::OP_WORDS;
+        case 5: return FxGeo<5>::OP_WORDS;
+        case 6: return FxGeo<6>::OP_WORDS;
+        case 7: return FxGeo<7>::OP_WORDS;
+        case 8: return FxGeo<8>::OP_WORDS;
+        case 9: return FxGeo<9>::OP_WORDS;
+        case 10: return FxGeo<10>::OP_WORDS;
         default: throw Error(MW_ERR_ARG, "no fixed-point apply kernel for this order");
+    }
+}
+
+size_t fx_op_z(int K) { return 2 * (7 * 128 + (K > 8 ? 10 * 128 : 0)) + 16; }  // FxGeo::Z_OFF
+
+void k_op_to_fx(const FxOpJob *jobs, size_t n, int K, cudaStream_t s) {
+    for (size_t at = 0; at < n; at += FxOpJobs::MAX) {
+        FxOpJobs J{};
+        int m = 0, most = 0;
+        for (; m < FxOpJobs::MAX && at + m < n; m++) {
+            J.job[m] = jobs[at + m];
+            most = std::max(most, J.job[m].n);
+        }
+        if (most == 0) continue;
+        switch (K) {
+            case 4: launch_op_to_fx<4>(J, m, most, s); break;
+            case 5: launch_op_to_fx<5>(J, m, most, s); break;
+            case 6: launch_op_to_fx<6>(J, m, most, s); break;
+            case 7: launch_op_to_fx<7>(J, m, most, s); break;
+            case 8: launch_op_to_fx<8>(J, m, most, s); break;
+            case 9: launch_op_to_fx<9>(J, m, most, s); break;
+            case 10: launch_op_to_fx<10>(J, m, most, s); break;
+            default: throw Error(MW_ERR_ARG, "no fixed-point apply kernel for this order");
+        }
+    }
+}
+
+void k_to_fx(const FxBlocks *sets, size_t n, int K, cudaStream_t s) {
+    for (size_t at = 0; at < n; at += FxSets::MAX) {
+        FxSets S{};
+        for (; S.n < FxSets::MAX && at + S.n < n; S.n++) {
+            const FxBlocks &b = sets[at + S.n];
+            S.in[S.n] = b.in;
+            S.out[S.n] = b.out;
+            S.first[S.n + 1] = S.first[S.n] + (long long)b.n;
+        }
+        if (S.first[S.n] == 0) continue;
+        switch (K) {
+            case 4: launch_to_fx<4>(S, s); break;
+            case 5: launch_to_fx<5>(S, s); break;
+            case 6: launch_to_fx<6>(S, s); break;
+            case 7: launch_to_fx<7>(S, s); break;
+            case 8: launch_to_fx<8>(S, s); break;
+            case 9: launch_to_fx<9>(S, s); break;
+            case 10: launch_to_fx<10>(S, s); break;
+            default: throw Error(MW_ERR_ARG, "no fixed-point apply kernel for this order");
+        }
     }
 }
 

@@ -370,6 +370,13 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
             op.off[i] = op.nblocks;
             if (op.band[i] >= 0) op.nblocks += 2 * op.band[i] + 1;
         }
+        op.fx_first.assign(nt, 0);
+        op.fx_count.assign(op.S, 0);
+        for (int s = 0; s < op.S; s++)
+            for (int t = 0; t < op.T; t++) {
+                op.fx_first[t * op.S + s] = op.fx_count[s];
+                if (op.band[t * op.S + s] >= 0) op.fx_count[s] += 2 * op.band[t * op.S + s] + 1;
+            }
         op.norms.assign((size_t)std::max<long>(op.nblocks, 1) * 4, 0.0);
         op.amax.assign(nt, 0.0);
         op.xmax.assign(nt, 0.0);
@@ -404,8 +411,8 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
         MWG_CUDA(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(OpBlockJob) * jobs.size(), cudaMemcpyHostToDevice, st));
         k_op_blocks(K, cx.dbasis.W, d_cc, d_q, d_q + 16, d_tasks, d_jobs, (int)jobs.size(), d_keep, st);
     }
-    // device copies for the reduced tiers: FP32 high part then low part per block (FP32 and
-    // double-FP32 tiers), and the tensor-core tier's B operand (mw_tc05_layout.h)
+    // device copies for the reduced tiers: FP32 high part then low part per block (FP32
+    // tier), and the tensor-core tier's B operand (mw_tc05_layout.h)
     const bool tc = K >= 4 && K <= KMAX;
     for (Oper *op : ops) {
         const long nb = std::max<long>(op->nblocks, 1);

@@ -138,6 +138,7 @@ struct Oper {
     // the screening tables on the device (bands, block offsets, sub-block norms, amax, xmax, term
     // coefficients), uploaded by the first apply that screens on the GPU (mw_screen.cu)
     void *d_screen = nullptr;
+    std::vector<int> fx_first, fx_count;  // per (term, scale) the blocks of the terms before; per scale all blocks
     void free_device();
     const double *norm(int t, int s, int l) const { return &norms[(size_t)(off[t * S + s] + l + band[t * S + s]) * 4]; }
     long block_index(int t, int s, int l) const { return off[t * S + s] + l + band[t * S + s]; }
@@ -352,13 +353,17 @@ inline float tf32_round_host(float x) {
     std::memcpy(&r, &u, 4);
     return r;
 }
-// double-FP32 tier: reads the high and low parts of the same shadows and operator blocks
-// the FP64 tier in 62-bit fixed point (mw_apply_fx.cu): L.in are digit blocks of fx_words(K) words that
-// k_to_fx makes from FP64 blocks with finite values, the operator blocks stay FP64
+// the FP64 tier and tier 3 in 62-bit fixed point (mw_apply_fx.cu): L.in are digit blocks of fx_words(K)
+// words that k_to_fx makes from FP64 blocks with finite values, L.ax, ay and az operator digits
+// (k_op_to_fx; az those with the term's coefficient)
 void k_apply_fx(const DevBasis &b, const ApplyLaunch &L, cudaStream_t s);
 size_t fx_words(int K);
-void k_to_fx(const double *blocks, uint32_t *out, size_t n, int K, cudaStream_t s);
-void k_apply_df(const DevBasis &b, const ApplyLaunch &L, int nsm, cudaStream_t s);
+struct FxBlocks {  // n consecutive blocks
+    const double *in;
+    uint32_t *out;
+    size_t n;
+};
+void k_to_fx(const FxBlocks *sets, size_t n, int K, cudaStream_t s);
 void k_norms(const DevBasis &b, double *const *blocks, double *const *cn, int n, cudaStream_t s);
 void k_topdown(const DevBasis &b, const PairTask *tasks, int n, cudaStream_t s);
 void k_compress(const DevBasis &b, const PairTask *tasks, double *const *cn, int n, cudaStream_t s);
@@ -447,6 +452,7 @@ constexpr int HASH_EMPTY = (int)0x80000000;  // n of an empty slot of an input t
 
 struct ScreenOp {  // one operator's tables (device)
     const int *band, *off;             // [T*S]: band L(t, n), block index of l = -L
+    const int *first;                  // [T*S]: blocks at the scale of the terms before t
     const double *norms;               // 4 sub-block norms per block
     const float *norms32;              // the same rounded to FP32 (the fast path's estimates)
     const double *amax, *xmax, *c;     // [T*S], [T*S], [T]
@@ -455,6 +461,16 @@ struct ScreenOp {  // one operator's tables (device)
     const float *b32, *btc, *btc2;
     int T, S;
 };
+struct FxOpJob {  // the blocks of one scale of an operator, n of them, and the place of their digits
+    ScreenOp op;
+    uint32_t *out;
+    int s, n;
+};
+// an operator block's digits: fx_op_words(K) words, those of the z pass's operand (the block times its
+// term's coefficient) from word fx_op_z(K) on
+size_t fx_op_words(int K);
+size_t fx_op_z(int K);
+void k_op_to_fx(const FxOpJob *jobs, size_t n, int K, cudaStream_t s);
 struct ScreenJob {  // one job of the apply (device)
     ScreenOp op;
     const int4 *hkey;  // the input tree's hash table: key (n, l) per slot, n = HASH_EMPTY when free
@@ -510,6 +526,8 @@ struct ScreenLevel {
     double *g64;                // generated blocks and their shadows
     float *g32, *gtc;
     uint32_t *gfx;
+    const uint32_t *const *fxop;  // per job its operator's digits at this scale
+    size_t fxo, fxz;            // words per operator block, and the place of the z pass's operand in it
     size_t fx;                  // words per block of the fixed-point digits; 0: the FP64 tier reads FP64 blocks
     size_t tx, tb;              // floats per block in the TF32 layouts (input, operator)
 };

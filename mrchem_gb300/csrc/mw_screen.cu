@@ -649,14 +649,20 @@ __global__ void __launch_bounds__(ST) fill_kernel(ScreenLevel P) {
             const long ob = (long)op.off[cd.t * S + s] + op.band[cd.t * S + s];
             const size_t bx = (size_t)(ob + cd.lx), by = (size_t)(ob + cd.ly), bz = (size_t)(ob + cd.lz);
             const size_t src = (size_t)cd.src;
-            if (tier == 0) {
-                if (P.fx)
+            if (tier == 0 || tier == 3) {  // the same kernel, or for both the FP64 one
+                if (P.fx) {
+                    const uint32_t *b = P.fxop[nd.job] + P.fxo * (size_t)(op.first[cd.t * S + s] + op.band[cd.t * S + s]);
+                    const long o = (long)P.fxo;
                     P.in[dst] = cd.gen ? (const void *)(P.gfx + P.fx * src) : (const void *)(J.infx + P.fx * src);
-                else
+                    P.ax[dst] = b + o * cd.lx;
+                    P.ay[dst] = b + o * cd.ly;
+                    P.az[dst] = b + o * cd.lz + P.fxz;
+                } else {
                     P.in[dst] = cd.gen ? (const void *)(P.g64 + src * P.bs) : (const void *)(J.in64 + src * P.bs);
-                P.ax[dst] = op.b64 + bx * P.bsz;
-                P.ay[dst] = op.b64 + by * P.bsz;
-                P.az[dst] = op.b64 + bz * P.bsz;
+                    P.ax[dst] = op.b64 + bx * P.bsz;
+                    P.ay[dst] = op.b64 + by * P.bsz;
+                    P.az[dst] = op.b64 + bz * P.bsz;
+                }
             } else if (tier == 2 || (tier == 1 && P.tensor)) {
                 // the tensor-core tiers (TF32, and split-TF32 for tier 1 in the tensor modes)
                 P.in[dst] = cd.gen ? (const void *)(P.gtc + P.tx * src) : (const void *)(J.intc + P.tx * src);

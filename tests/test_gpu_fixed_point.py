@@ -72,3 +72,23 @@ def test_values_outside_the_kernels_range_take_the_fp64_kernel(engine, order, va
     engine.apply(prec, V, engine.PoissonOperator(mra, prec), g, max_iter=0)
     v = V.download()[1]
     assert not np.isfinite(v).all() if not np.isfinite(value) else np.abs(v).max() > 1e190
+
+
+@pytest.mark.parametrize("precision", ["fp64", "df"])
+def test_batch_of_more_operators_and_trees_than_one_launch_takes(engine, precision):
+    # 66 trees and operators over at most four groups: more than the 16 that one launch of the digit kernels
+    # takes.  The items of a node are the same as alone, only grouped otherwise: FP64 rounding of sums.
+    prec, n = 1e-2, 66
+    mra = engine.MultiResolutionAnalysis(3)
+    fs = [engine.project(prec, engine.FunctionTree(mra), [(1.0, 2.0 + 0.1 * i, (0.02 * i - 0.5, 0.1, -0.2), (0, 0, 0))])
+          for i in range(n)]
+    Hs = [engine.HelmholtzOperator(mra, 0.5 + 0.02 * i, prec) for i in range(n)]
+    many = [engine.FunctionTree(mra) for _ in range(n)]
+    st = engine.apply_batch([prec] * n, many, Hs, fs, precision=precision)
+    # "df" leaves the root scale's items, among others, to the FP64 tier
+    assert st["items_df"] + st["items_fp64"] == st["items"] and (st["items_df"] > 0) == (precision == "df")
+    for f, H, v in zip(fs, Hs, many):
+        one = engine.FunctionTree(mra)
+        engine.apply(prec, one, H, f, precision=precision)
+        (k1, c1, _), (k2, c2, _) = v.download(), one.download()
+        assert np.array_equal(k1, k2) and rel_l2(c1, c2) <= 2e-14
