@@ -670,7 +670,7 @@ int level_zrows(const std::vector<JobState *> &jp, int sidx) {
     }
     return zmax;
 }
-constexpr size_t SCREEN_SMEM_MAX = 96 * 1024;  // larger walks (very wide bands) are screened on the host
+constexpr size_t SCREEN_SMEM_MAX = 136 * 1024;  // larger walks (very wide bands) are screened on the host
 
 // One level of a job group screened on the GPU (mw_screen.cu).  The walk, the generation of
 // missing inputs, the exact screening, the tiers and the item arrays run on the high-priority

@@ -14,7 +14,7 @@
 //   gen_tasks_kernel  the generation tasks of the registered positions;
 //   screen_kernel<1>  the same walk after generation: generated inputs are screened again with
 //                     their own norms, every item gets its tier, and the items are written in
-//                     walk order (block-wide prefix sums per round of rows);
+//                     walk order (block-wide prefix sums per round of candidates);
 //   tier_offsets_kernel  per tier and node the first item (prefix sums in node order);
 //   fill_kernel       the tier kernels' item arrays (input block, three operator blocks,
 //                     coefficient), each tier's items in node order.
@@ -29,7 +29,9 @@ namespace mwg {
 
 namespace {
 
-constexpr int ST = 128;  // threads per CTA
+constexpr int ST = 256, FT = 128;  // threads per CTA of the walks and of the fill
+constexpr int RB = 2 * ST;          // (t, lz, ly) rows whose candidates are walked at a time
+constexpr int TAB = 2048;             // positions of a node whose inputs are kept
 
 // products and sums as the host's -ffp-contract=off code rounds them (no fused multiply-adds)
 __device__ __forceinline__ double M(double a, double b) { return __dmul_rn(a, b); }
@@ -136,7 +138,7 @@ __device__ int gen_find(const ScreenLevel &P, const ScreenNode &nd, const int *p
 }
 
 // exclusive prefix sum over the CTA (every thread calls it); *total gets the CTA's sum
-template <typename U>
+template <typename U, int NT = ST>
 __device__ U block_scan(U v, U *wsum, U *total) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     U x = v;
@@ -149,7 +151,7 @@ __device__ U block_scan(U v, U *wsum, U *total) {
     __syncthreads();
     U before = 0, all = 0;
 #pragma unroll
-    for (int i = 0; i < ST / 32; i++) {
+    for (int i = 0; i < NT / 32; i++) {
         if (i < w) before += wsum[i];
         all += wsum[i];
     }
@@ -198,31 +200,29 @@ struct Row {  // the operator norms of one (t, lz, ly) row: FP64 for exact decis
     const float *ny32, *nz32;
 };
 
-// One candidate of the walk.  Returns true when it survives the first screen (the host's phase A:
-// real inputs with their exact bound, missing ones with their leaf ancestor's block norm as the
-// scaling norm); src / gen / an describe it.  The FP32 estimate decides where it is clear of the
-// threshold, the host's FP64 arithmetic elsewhere, so the result is the host's.
-__device__ bool candidate(const ScreenLevel &P, const ScreenJob &J, const ScreenNode &nd, const int *p,
-                          const double *nx, const float *nx32, const Row &rw, int &src, int &gen, int &an) {
-    for (int d = 0; d < 3; d++)
-        if (p[d] < P.lo[d] || p[d] >= P.hi[d]) return false;
+// The input of an in-world position: the input tree's node there (gen = 0), or its leaf ancestor, of scale
+// an, for a missing one (gen = 1).  As one number: the node, IN_GEN; or -1 (unreachable: the roots cover
+// the world).
+enum : int { IN_GEN = 1 << 30, IN_SEEN = 1 << 29, IN_NODE = IN_SEEN - 1 };
+__device__ int locate(const ScreenLevel &P, const ScreenJob &J, const int *p, int &an) {
+    an = P.n;
     const int i = hash_find(J, P.n, p[0], p[1], p[2]);
-    if (i >= 0) {
-        src = i;
-        gen = 0;
-        an = P.n;
-    } else {
-        int a = -1, al[3] = {p[0], p[1], p[2]};
-        an = P.n;
-        while (a < 0 && an > P.n0) {
-            an--;
-            for (int d = 0; d < 3; d++) al[d] = floordiv2_d(al[d]);
-            a = hash_find(J, an, al[0], al[1], al[2]);
-        }
-        if (a < 0) return false;  // unreachable: the roots cover the world
-        src = a;
-        gen = 1;
+    if (i >= 0) return i;
+    int a = -1, al[3] = {p[0], p[1], p[2]};
+    while (a < 0 && an > P.n0) {
+        an--;
+        for (int d = 0; d < 3; d++) al[d] = floordiv2_d(al[d]);
+        a = hash_find(J, an, al[0], al[1], al[2]);
     }
+    return a < 0 ? -1 : (a | IN_GEN);
+}
+
+// True when a candidate survives the first screen (the host's phase A: real inputs with their exact
+// bound, missing ones with their leaf ancestor's block norm as the scaling norm).  The FP32 estimate
+// decides where it is clear of the threshold, the host's FP64 arithmetic elsewhere, so the result is the
+// host's.
+__device__ bool first_screen(const ScreenLevel &P, const ScreenJob &J, const ScreenNode &nd, int src, bool gen,
+                             const double *nx, const float *nx32, const Row &rw) {
     if (P.root) return true;
     if (nd.flags & 4) {
         const float b32 = gen ? scaling_bound_f(nx32, rw.ny32, rw.nz32, J.bn32[src], false)
@@ -235,29 +235,16 @@ __device__ bool candidate(const ScreenLevel &P, const ScreenJob &J, const Screen
     return !(bd < nd.thr);
 }
 
-// An item after generation: a candidate that survives the first screen and the host's phase C
-// (the exact bound, with a generated block's own norms, against thr2), and its tier.
+// A candidate that survived the first screen, after generation: the host's phase C (the exact bound, with a
+// generated block's own norms, against thr2), and its tier.
 struct Item {
     int src, gen, tier;
     const double *cn;
 };
-__device__ bool final_item(const ScreenLevel &P, const ScreenJob &J, const ScreenNode &nd, const int *p, int lx,
-                           int ly, int lz, const double *nx, const float *nx32, const Row &rw, Item &it) {
-    int an;
-    if (!candidate(P, J, nd, p, nx, nx32, rw, it.src, it.gen, an)) return false;
-    const float *cn32;
-    if (!it.gen) {
-        it.cn = J.cn + 8 * (size_t)it.src;
-        cn32 = J.cn32 + 8 * (size_t)it.src;
-    } else {
-        it.src = gen_find(P, nd, p);
-        if (it.src < 0) {  // unreachable after a count pass without overflow
-            atomicExch(P.overflow, 2);
-            return false;
-        }
-        it.cn = P.gcn + 8 * (size_t)it.src;
-        cn32 = P.gcn32 + 8 * (size_t)it.src;
-    }
+__device__ bool final_item(const ScreenLevel &P, const ScreenJob &J, const ScreenNode &nd, int lx, int ly, int lz,
+                           const double *nx, const float *nx32, const Row &rw, Item &it) {
+    it.cn = (it.gen ? P.gcn : J.cn) + 8 * (size_t)it.src;
+    const float *cn32 = (it.gen ? P.gcn32 : J.cn32) + 8 * (size_t)it.src;
     const bool root = P.root != 0, fast = (nd.flags & 4) != 0;
     const float b32 = fast ? item_bound_f(nx32, rw.ny32, rw.nz32, cn32, root) : 0.0f;
     double bd = 0.0;
@@ -315,18 +302,32 @@ __device__ __forceinline__ int last_le(const int *pre, int n, int r) {
 
 // One CTA per output node.  The walk prunes as the host does (mw_apply.cpp enumerate_node), level
 // by level so that FP64 work is spent only on what survives: whole terms, then (t, lz) rows, then
-// (t, lz, ly) rows, each with the host's expression; the surviving rows are compacted in walk
-// order in shared memory, and every thread then walks the lx of one (t, lz, ly) row.
+// (t, lz, ly) rows, each with the host's expression; the survivors are compacted in walk order in shared
+// memory, and then every thread takes one (t, lz, ly, lx) at a time.
 // PASS 0: count the first screen's survivors per node and register missing inputs.
 // PASS 1: screen generated inputs with their own norms, choose tiers, write the items in walk order.
+//
+// Bound: latency.  A candidate is a chain of dependent loads (hash slots of the position and of its
+// ancestors, then norms), and a level has tens to hundreds of nodes, one CTA each.  So candidates, not rows,
+// go to the threads, and a position's input, which does not depend on the term, is looked up once per
+// node and kept in a table in shared memory: one entry per (position modulo TAB) of the box of the live
+// terms' translations, written as one 64-bit word with its position, so that threads may race for it.  Bands
+// are 6 (order 9) to some 250 (order 3) boxes wide; the survivors of a node touch a few hundred positions, and
+// 4096 entries are no faster than 2048 (36 and 34 us of PASS 1 below, the applies alike).
+// Measured per launch, 5 Helmholtz applies of order 6, one thread per row before: PASS 0 92 -> 24 us, PASS 1
+// 107 -> 36 us; one FP64 Poisson apply of order 7: 43 -> 20 us and 58 -> 31 us.
 template <int PASS>
 __global__ void __launch_bounds__(ST) screen_kernel(ScreenLevel P, int maxT, int zmax) {
-    extern __shared__ int sm[];
-    int *zpre = sm;                // [maxT + 1]: first z row of each term (live terms only)
-    int *zlist = sm + maxT + 1;    // [zmax]: live z rows, t << 16 | (lz + L)
+    extern __shared__ __align__(16) unsigned long long sm[];
+    volatile unsigned long long *tab = sm;  // [TAB]: inputs by position, (position + 1) << 32 | input
+    volatile unsigned long long *slot = sm + TAB;  // [TAB], PASS 1: generated blocks by position
+    int2 *rows = (int2 *)(sm + (1 + PASS) * TAB);  // [RB]: live rows, (t << 16 | (lz + L), ly)
+    int *xpre = (int *)(rows + RB);  // [RB + 1]: first candidate of each
+    int *zpre = xpre + RB + 1;     // [maxT + 1]: first z row of each term (live terms only)
+    int *zlist = zpre + maxT + 1;  // [zmax]: live z rows, t << 16 | (lz + L)
     int *ypre = zlist + zmax;      // [zmax + 1]: first y row of each live z row
-    __shared__ unsigned wsum[ST / 32];
-    __shared__ int s_cnt[8];
+    __shared__ unsigned long long wsum[ST / 32];
+    __shared__ int s_cnt[8], s_band;
     const int q = blockIdx.x, tid = threadIdx.x;
     const ScreenNode nd = P.nodes[q];
     const ScreenJob &J = P.jobs[nd.job];
@@ -344,38 +345,53 @@ __global__ void __launch_bounds__(ST) screen_kernel(ScreenLevel P, int maxT, int
         wlo[d] = nd.l[d] - P.hi[d] + 1;
         whi[d] = nd.l[d] - P.lo[d];
     }
+    if (tid < 8) s_cnt[tid] = 0;
+    if (tid == 0) s_band = -1;
+    __syncthreads();
     // terms
-    for (int t = tid; t < T; t += ST) {
-        const int L = op.band[t * S + s];
-        bool live = L >= 0 && !skip;
-        if (live && !P.root) {
-            if (fast) {
-                const float X = op.xmax32[t * S + s], Am = op.amax32[t * S + s];
-                live = !(nd.fm32 * (3.0f * X * Am * Am) < nd.prune32);
-            } else {
-                const double X = op.xmax[t * S + s], Am = op.amax[t * S + s];
-                live = !(M(M(M(M(fm, 3.0), X), Am), Am) < thr);
+    int Z = 0, band = -1;
+    for (int t0 = 0; t0 < T; t0 += ST) {
+        const int t = t0 + tid;
+        int c = 0;
+        if (t < T) {
+            const int L = op.band[t * S + s];
+            bool live = L >= 0 && !skip;
+            if (live && !P.root) {
+                if (fast) {
+                    const float X = op.xmax32[t * S + s], Am = op.amax32[t * S + s];
+                    live = !(nd.fm32 * (3.0f * X * Am * Am) < nd.prune32);
+                } else {
+                    const double X = op.xmax[t * S + s], Am = op.amax[t * S + s];
+                    live = !(M(M(M(M(fm, 3.0), X), Am), Am) < thr);
+                }
+            }
+            // rows only where every direction has an in-world translation
+            int n = 1;
+            for (int d = 0; d < 3; d++) n = min(n, min(L, whi[d]) - max(-L, wlo[d]) + 1);
+            if (live && n > 0) {
+                c = min(L, whi[2]) - max(-L, wlo[2]) + 1;
+                band = max(band, L);
             }
         }
-        // rows only where every direction has an in-world translation
-        int rows = 1;
-        for (int d = 0; d < 3; d++) rows = min(rows, min(L, whi[d]) - max(-L, wlo[d]) + 1);
-        zpre[t] = (live && rows > 0) ? min(L, whi[2]) - max(-L, wlo[2]) + 1 : 0;
+        unsigned total;
+        const unsigned pre = block_scan<unsigned>((unsigned)c, (unsigned *)wsum, &total);
+        if (t < T) zpre[t] = Z + (int)pre;
+        Z += (int)total;
     }
-    if (tid < 8) s_cnt[tid] = 0;
+    if (tid == 0) zpre[T] = Z;
+    if (band >= 0) atomicMax(&s_band, band);
     __syncthreads();
-    if (tid == 0) {
-        int acc = 0;
-        for (int t = 0; t < T; t++) {
-            const int c = zpre[t];
-            zpre[t] = acc;
-            acc += c;
-        }
-        zpre[T] = acc;
+    // the box of the live terms' translations
+    int t0[3], tn[3];
+    long long boxed = 1;
+    for (int d = 0; d < 3; d++) {
+        t0[d] = max(-s_band, wlo[d]);
+        tn[d] = max(min(s_band, whi[d]) - t0[d] + 1, 0);
+        boxed = min(boxed * tn[d], 1ll << 31);
     }
-    __syncthreads();
+    const bool keep = boxed < (1ll << 31);  // a position in the box is 31 bits
+    for (int i = tid; i < (1 + PASS) * TAB; i += ST) tab[i] = 0ull;
     // z rows of the live terms
-    const int Z = zpre[T];
     int nzr = 0;
     for (int z0 = 0; z0 < Z; z0 += ST) {
         const int z = z0 + tid;
@@ -405,7 +421,7 @@ __global__ void __launch_bounds__(ST) screen_kernel(ScreenLevel P, int maxT, int
             packed = (t << 16) | (lz + L);
         }
         unsigned total;
-        const unsigned pos = block_scan<unsigned>(live, wsum, &total);
+        const unsigned pos = block_scan<unsigned>(live, (unsigned *)wsum, &total);
         if (live) {
             zlist[nzr + pos] = packed;
             ypre[nzr + pos] = min(L, whi[1]) - max(-L, wlo[1]) + 1;  // >= 1: the term has rows
@@ -419,134 +435,149 @@ __global__ void __launch_bounds__(ST) screen_kernel(ScreenLevel P, int maxT, int
         const int i = i0 + tid;
         const unsigned v = i < nzr ? (unsigned)ypre[i] : 0u;
         unsigned total;
-        const unsigned pre = block_scan<unsigned>(v, wsum, &total);
+        const unsigned pre = block_scan<unsigned>(v, (unsigned *)wsum, &total);
         if (i < nzr) ypre[i] = ytot + (int)pre;
         ytot += (int)total;
     }
     if (tid == 0) ypre[nzr] = ytot;
     __syncthreads();
-    // (t, lz, ly) rows: the y test, then the walk over lx
+    // (t, lz, ly) rows: the y test, then the live rows' lx, RB rows at a time
     int mine = 0;           // PASS 0: this thread's survivors
-    long long written = 0;  // PASS 1: items written by earlier rounds
+    long long written = 0;  // PASS 1: items written so far
     const long long base = PASS ? P.cand_off[q] : 0;
-    for (int r0 = 0; r0 < ytot; r0 += ST) {
-        const int r = r0 + tid;
-        int t = 0, L = -1, lz = 0, ly = 0;
-        bool live = false;
-        Row rw{nullptr, nullptr, nullptr, nullptr};
-        long ob = 0;
-        if (r < ytot) {
-            const int i = last_le(ypre, nzr, r);
-            const int packed = zlist[i];
-            t = packed >> 16;
-            L = op.band[t * S + s];
-            lz = (packed & 0xffff) - L;
-            ly = max(-L, wlo[1]) + r - ypre[i];
-            ob = (long)op.off[t * S + s] + L;
-            rw.nz = op.norms + 4 * (size_t)(ob + lz);
-            rw.ny = op.norms + 4 * (size_t)(ob + ly);
-            rw.nz32 = op.norms32 + 4 * (size_t)(ob + lz);
-            rw.ny32 = op.norms32 + 4 * (size_t)(ob + ly);
-            live = true;
-            if (!P.root) {
-                if (fast) {
-                    const float *nz = rw.nz32, *ny = rw.ny32;
-                    const float X = op.xmax32[t * S + s], Am = op.amax32[t * S + s];
-                    const float az = fmaxf(fmaxf(nz[0], nz[1]), fmaxf(nz[2], nz[3]));
-                    const float xz = fmaxf(nz[1], fmaxf(nz[2], nz[3]));
-                    const float ay = fmaxf(fmaxf(ny[0], ny[1]), fmaxf(ny[2], ny[3]));
-                    const float xy = fmaxf(ny[1], fmaxf(ny[2], ny[3]));
-                    live = !(nd.fm32 * (xz * ay * Am + az * xy * Am + az * ay * X) < nd.prune32);
-                } else {
-                    const double *nz = rw.nz, *ny = rw.ny;
-                    const double X = op.xmax[t * S + s], Am = op.amax[t * S + s];
-                    const double az = dmax(dmax(nz[0], nz[1]), dmax(nz[2], nz[3]));
-                    const double xz = dmax(nz[1], dmax(nz[2], nz[3]));
-                    const double ay = dmax(dmax(ny[0], ny[1]), dmax(ny[2], ny[3]));
-                    const double xy = dmax(ny[1], dmax(ny[2], ny[3]));
-                    live = !(M(fm, A(A(M(M(xz, ay), Am), M(M(az, xy), Am)), M(M(az, ay), X))) < thr);
-                }
-            }
-        }
-        if (PASS == 0) {
-            if (live) {
-                for (int lx = max(-L, wlo[0]); lx <= min(L, whi[0]); lx++) {
-                    const int p[3] = {nd.l[0] - lx, nd.l[1] - ly, nd.l[2] - lz};
-                    int src, gen, an;
-                    if (!candidate(P, J, nd, p, op.norms + 4 * (size_t)(ob + lx), op.norms32 + 4 * (size_t)(ob + lx), rw,
-                                   src, gen, an))
-                        continue;
-                    mine++;
-                    if (gen) gen_insert(P, nd, p, src, an);
-                }
-            }
-        } else {
-            // two walks of the row: screen and count its items, then write them at their place in
-            // walk order.  Rows of at most 32 translations keep the first walk's survivors and tiers
-            // in bit masks, so that the second walk only looks the inputs up again
-            int c = 0;
-            const int xlo = max(-L, wlo[0]), xhi = min(L, whi[0]);
-            const bool keep = xhi - xlo < 32;
-            unsigned surv = 0u;
-            unsigned long long tiers = 0ull;
-            if (live)
-                for (int lx = xlo; lx <= xhi; lx++) {
-                    const int p[3] = {nd.l[0] - lx, nd.l[1] - ly, nd.l[2] - lz};
-                    const double *nx = op.norms + 4 * (size_t)(ob + lx);
-                    Item it;
-                    if (!final_item(P, J, nd, p, lx, ly, lz, nx, op.norms32 + 4 * (size_t)(ob + lx), rw, it)) continue;
-                    c++;
-                    if (keep) {
-                        surv |= 1u << (lx - xlo);
-                        tiers |= (unsigned long long)it.tier << (2 * (lx - xlo));
+    for (int r0 = 0; r0 < ytot;) {
+        int nrow = 0, nx = 0;
+        for (; r0 < ytot && nrow + ST <= RB; r0 += ST) {
+            const int r = r0 + tid;
+            bool live = false;
+            int packed = 0, ly = 0, len = 0;
+            if (r < ytot) {
+                const int i = last_le(ypre, nzr, r);
+                packed = zlist[i];
+                const int t = packed >> 16, L = op.band[t * S + s];
+                ly = max(-L, wlo[1]) + r - ypre[i];
+                len = min(L, whi[0]) - max(-L, wlo[0]) + 1;
+                live = true;
+                if (!P.root) {
+                    const size_t ob = 4 * (size_t)op.off[t * S + s];
+                    const size_t oz = ob + 4 * (size_t)(packed & 0xffff), oy = ob + 4 * (size_t)(L + ly);
+                    if (fast) {
+                        const float *nz = op.norms32 + oz, *ny = op.norms32 + oy;
+                        const float X = op.xmax32[t * S + s], Am = op.amax32[t * S + s];
+                        const float az = fmaxf(fmaxf(nz[0], nz[1]), fmaxf(nz[2], nz[3]));
+                        const float xz = fmaxf(nz[1], fmaxf(nz[2], nz[3]));
+                        const float ay = fmaxf(fmaxf(ny[0], ny[1]), fmaxf(ny[2], ny[3]));
+                        const float xy = fmaxf(ny[1], fmaxf(ny[2], ny[3]));
+                        live = !(nd.fm32 * (xz * ay * Am + az * xy * Am + az * ay * X) < nd.prune32);
+                    } else {
+                        const double *nz = op.norms + oz, *ny = op.norms + oy;
+                        const double X = op.xmax[t * S + s], Am = op.amax[t * S + s];
+                        const double az = dmax(dmax(nz[0], nz[1]), dmax(nz[2], nz[3]));
+                        const double xz = dmax(nz[1], dmax(nz[2], nz[3]));
+                        const double ay = dmax(dmax(ny[0], ny[1]), dmax(ny[2], ny[3]));
+                        const double xy = dmax(ny[1], dmax(ny[2], ny[3]));
+                        live = !(M(fm, A(A(M(M(xz, ay), Am), M(M(az, xy), Am)), M(M(az, ay), X))) < thr);
                     }
-                    atomicAdd(&s_cnt[it.tier], 1);
-                    atomicAdd(&s_cnt[4 + it.tier], item_pairs_d(nx, rw.ny, rw.nz, it.cn, P.root != 0));
                 }
-            unsigned total;
-            const int pos = (int)block_scan<unsigned>((unsigned)c, wsum, &total);
-            if (live && c > 0) {
-                int k = 0;
-                auto put = [&](int lx, int src, int gen, int tier) {
-                    ScreenCand &cd = P.cand[base + written + pos + k];
-                    cd.src = src;
+            }
+            unsigned long long total;
+            const unsigned long long pre =
+                block_scan<unsigned long long>(live ? (1ull << 32) + (unsigned)len : 0ull, wsum, &total);
+            if (live) {
+                const int at = nrow + (int)(pre >> 32);
+                rows[at] = make_int2(packed, ly);
+                xpre[at] = nx + (int)(unsigned)pre;
+            }
+            nrow += (int)(total >> 32);
+            nx += (int)(unsigned)total;
+        }
+        __syncthreads();
+        for (int x0 = 0; x0 < nx; x0 += ST) {
+            const int x = x0 + tid;
+            bool pass = false;
+            Item it;
+            int t = 0, lx = 0, ly = 0, lz = 0, pairs = 0;
+            if (x < nx) {
+                const int i = last_le(xpre, nrow, x);
+                const int2 row = rows[i];
+                t = row.x >> 16;
+                const int L = op.band[t * S + s];
+                lz = (row.x & 0xffff) - L;
+                ly = row.y;
+                lx = max(-L, wlo[0]) + x - xpre[i];
+                const long ob = (long)op.off[t * S + s] + L;
+                const Row rw{op.norms + 4 * (size_t)(ob + ly), op.norms + 4 * (size_t)(ob + lz),
+                             op.norms32 + 4 * (size_t)(ob + ly), op.norms32 + 4 * (size_t)(ob + lz)};
+                const double *nxd = op.norms + 4 * (size_t)(ob + lx);
+                const float *nxf = op.norms32 + 4 * (size_t)(ob + lx);
+                const int p[3] = {nd.l[0] - lx, nd.l[1] - ly, nd.l[2] - lz};
+                const unsigned c = keep ? ((lz - t0[2]) * tn[1] + ly - t0[1]) * tn[0] + lx - t0[0] : 0;
+                const unsigned long long tag = (unsigned long long)(c + 1) << 32, known = tab[c % TAB];
+                int an = -1, in = (int)(unsigned)known;
+                if (!keep || (known ^ tag) >> 32) {
+                    in = locate(P, J, p, an);
+                    if (keep) tab[c % TAB] = tag | (unsigned)in;
+                }
+                it.src = in & IN_NODE;
+                it.gen = (in & IN_GEN) != 0;
+                pass = in >= 0 && first_screen(P, J, nd, it.src, it.gen, nxd, nxf, rw);
+                if (PASS == 0) {
+                    mine += pass;
+                    if (pass && it.gen && !(in & IN_SEEN)) {
+                        if (an < 0) locate(P, J, p, an);  // known from the table
+                        gen_insert(P, nd, p, it.src, an);
+                        if (keep) tab[c % TAB] = tag | (unsigned)(in | IN_SEEN);
+                    }
+                } else if (pass) {
+                    if (it.gen) {
+                        const unsigned long long kg = slot[c % TAB];
+                        int g = (int)(unsigned)kg;
+                        if (!keep || (kg ^ tag) >> 32) {
+                            g = gen_find(P, nd, p);
+                            if (keep) slot[c % TAB] = tag | (unsigned)g;
+                        }
+                        it.src = g;
+                        if (g < 0) {  // unreachable after a count pass without overflow
+                            atomicExch(P.overflow, 2);
+                            pass = false;
+                        }
+                    }
+                    if (pass) pass = final_item(P, J, nd, lx, ly, lz, nxd, nxf, rw, it);
+                    if (pass) pairs = item_pairs_d(nxd, rw.ny, rw.nz, it.cn, P.root != 0);
+                }
+            }
+            if (PASS == 1) {
+                unsigned total;
+                const int pos = (int)block_scan<unsigned>(pass ? 1u : 0u, (unsigned *)wsum, &total);
+                if (total == 0) continue;
+                for (int k = 0; k < 4; k++) {
+                    const bool mine_k = pass && it.tier == k;
+                    const unsigned m = __ballot_sync(0xffffffffu, mine_k);
+                    if (!m) continue;
+                    const int sum = __reduce_add_sync(0xffffffffu, mine_k ? pairs : 0);
+                    if ((tid & 31) == 0) {
+                        atomicAdd(&s_cnt[k], __popc(m));
+                        atomicAdd(&s_cnt[4 + k], sum);
+                    }
+                }
+                if (pass) {
+                    ScreenCand &cd = P.cand[base + written + pos];
+                    cd.src = it.src;
                     cd.lx = (short)lx;
                     cd.ly = (short)ly;
                     cd.lz = (short)lz;
-                    cd.tier = (unsigned char)tier;
-                    cd.gen = (unsigned char)gen;
+                    cd.tier = (unsigned char)it.tier;
+                    cd.gen = (unsigned char)it.gen;
                     cd.t = t;
-                    k++;
-                };
-                if (keep) {
-                    for (unsigned m = surv; m; m &= m - 1) {
-                        const int bit = __ffs(m) - 1, lx = xlo + bit;
-                        const int p[3] = {nd.l[0] - lx, nd.l[1] - ly, nd.l[2] - lz};
-                        // the input as final_item found it: a node of the input tree, or a generated slot
-                        int src = hash_find(J, P.n, p[0], p[1], p[2]), gen = 0;
-                        if (src < 0) {
-                            src = gen_find(P, nd, p);
-                            gen = 1;
-                        }
-                        put(lx, src, gen, (int)((tiers >> (2 * bit)) & 3ull));
-                    }
-                } else {
-                    for (int lx = xlo; lx <= xhi; lx++) {
-                        const int p[3] = {nd.l[0] - lx, nd.l[1] - ly, nd.l[2] - lz};
-                        Item it;
-                        if (!final_item(P, J, nd, p, lx, ly, lz, op.norms + 4 * (size_t)(ob + lx),
-                                        op.norms32 + 4 * (size_t)(ob + lx), rw, it))
-                            continue;
-                        put(lx, it.src, it.gen, it.tier);
-                    }
                 }
+                written += total;
             }
-            written += total;
         }
+        __syncthreads();  // before the next rows take the lists' place
     }
     if (PASS == 0) {
         unsigned total;
-        block_scan<unsigned>((unsigned)mine, wsum, &total);
+        block_scan<unsigned>((unsigned)mine, (unsigned *)wsum, &total);
         if (tid == 0) P.cnt[q] = (int)total;
     } else {
         __syncthreads();
@@ -619,8 +650,8 @@ __global__ void __launch_bounds__(1024) tier_offsets_kernel(ScreenLevel P) {
 }
 
 // the tier kernels' item arrays: each node's items of a tier at its first item, in walk order
-__global__ void __launch_bounds__(ST) fill_kernel(ScreenLevel P) {
-    __shared__ unsigned wsum[ST / 32];
+__global__ void __launch_bounds__(FT) fill_kernel(ScreenLevel P) {
+    __shared__ unsigned wsum[FT / 32];
     __shared__ long long s_run[4];
     const int q = blockIdx.x, tid = threadIdx.x;
     const ScreenNode &nd = P.nodes[q];
@@ -632,7 +663,7 @@ __global__ void __launch_bounds__(ST) fill_kernel(ScreenLevel P) {
     const long long c0 = P.cand_off[q];
     if (tid < 4) s_run[tid] = P.tier_off[4 * (size_t)q + tid];
     __syncthreads();
-    for (int i0 = 0; i0 < m; i0 += ST) {
+    for (int i0 = 0; i0 < m; i0 += FT) {
         const int i = i0 + tid;
         int tier = 0;
         unsigned onehot = 0;
@@ -640,10 +671,10 @@ __global__ void __launch_bounds__(ST) fill_kernel(ScreenLevel P) {
         if (i < m) {
             cd = P.cand[c0 + i];
             tier = cd.tier;
-            onehot = 1u << (8 * tier);  // at most ST = 128 items of a tier per round: 8 bits each
+            onehot = 1u << (8 * tier);  // at most FT = 128 items of a tier per round: 8 bits each
         }
         unsigned total;
-        const unsigned pre = block_scan<unsigned>(onehot, wsum, &total);
+        const unsigned pre = block_scan<unsigned, FT>(onehot, wsum, &total);
         if (i < m) {
             const long long dst = s_run[tier] + ((pre >> (8 * tier)) & 255);
             const long ob = (long)op.off[cd.t * S + s] + op.band[cd.t * S + s];
@@ -686,12 +717,16 @@ __global__ void __launch_bounds__(ST) fill_kernel(ScreenLevel P) {
 
 }  // namespace
 
-size_t screen_smem(int maxT, int zmax) { return sizeof(int) * ((size_t)maxT + 2 + 2 * (size_t)zmax); }
+static size_t walk_smem(int maxT, int zmax, int pass) {
+    return sizeof(long long) * (1 + pass) * (size_t)TAB + sizeof(int) * (3 * RB + 1 + (size_t)maxT + 2 + 2 * (size_t)zmax);
+}
+
+size_t screen_smem(int maxT, int zmax) { return walk_smem(maxT, zmax, 1); }
 
 void k_screen_count(const ScreenLevel &P, int maxT, int zmax, cudaStream_t s) {
     if (P.nn <= 0) return;
-    const size_t sm = screen_smem(maxT, zmax);
-    if (sm > 48 * 1024) kernel_smem((const void *)screen_kernel<0>, (int)sm);
+    const size_t sm = walk_smem(maxT, zmax, 0);
+    if (sm > 40 * 1024) kernel_smem((const void *)screen_kernel<0>, (int)sm);
     screen_kernel<0><<<P.nn, ST, sm, s>>>(P, maxT, zmax);
 }
 
@@ -707,15 +742,15 @@ void k_screen_gen_norms32(const ScreenLevel &P, int ngen, cudaStream_t s) {
 
 void k_screen_write(const ScreenLevel &P, int maxT, int zmax, cudaStream_t s) {
     if (P.nn <= 0) return;
-    const size_t sm = screen_smem(maxT, zmax);
-    if (sm > 48 * 1024) kernel_smem((const void *)screen_kernel<1>, (int)sm);
+    const size_t sm = walk_smem(maxT, zmax, 1);
+    if (sm > 40 * 1024) kernel_smem((const void *)screen_kernel<1>, (int)sm);
     screen_kernel<1><<<P.nn, ST, sm, s>>>(P, maxT, zmax);
     tier_offsets_kernel<<<1, 1024, 0, s>>>(P);
 }
 
 void k_screen_fill(const ScreenLevel &P, cudaStream_t s) {
     if (P.nn <= 0) return;
-    fill_kernel<<<P.nn, ST, 0, s>>>(P);
+    fill_kernel<<<P.nn, FT, 0, s>>>(P);
 }
 
 }  // namespace mwg

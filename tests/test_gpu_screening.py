@@ -189,3 +189,25 @@ def test_generation_tables_grow(engine, monkeypatch):
     res = both(engine, mra, run)
     check_identical(res)
     assert res[1][1]["screen_regrows"] > 0 and res[1][1]["generated"] > 0
+
+
+@pytest.mark.parametrize("order", [3, 9])
+def test_wide_and_narrow_bands(engine, order):
+    # the walk keeps 2048 positions of a node's box of translations: at order 3 the bands span the whole
+    # world, 16^3 positions four scales down, so that positions take over each other's entries; order 9's
+    # box holds 13^3 at most
+    prec = 1e-4
+    mra = engine.MultiResolutionAnalysis(order)
+    f = engine.project(prec, engine.FunctionTree(mra), [(30.0, 40.0, (0.3, -0.2, 0.1), (0, 0, 0))])
+    P = engine.PoissonOperator(mra, prec)
+    band = max(P.band(t, 3) for t in range(P.nterms))
+    assert band >= 15 if order == 3 else band <= 6
+
+    def run():
+        V = engine.FunctionTree(mra)
+        engine.apply(prec, V, P, f, precision="mixed")
+        return [V]
+
+    res = both(engine, mra, run)
+    check_identical(res)
+    assert res[1][1]["levels"] >= 4
