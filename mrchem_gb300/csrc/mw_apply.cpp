@@ -534,6 +534,58 @@ struct FxLevelOps {
     }
 };
 
+// Two-scale transforms of parents and their children in the fixed-point kernel: an item whose three operator
+// blocks are W^T (down: the parents' reconstructions are added to their children's scaling parts) or W (up: the
+// parents' blocks are computed from their children's scaling parts; no norms).  The digits of up to FX_PAIRS
+// blocks at a time (59 MB at 2K = 20) take `fx`.  topdown_kernel and compress_kernel hold a node's 3 (2K)^4
+// multiply-adds on one SM's FP64 pipe (1.6 per cycle), 91 us at 2K = 16 however few nodes a scale has; the
+// digits (7 us) and the fixed-point kernel (20 us) take a third of that, and one norms launch serves all
+// scales.  FP64 Poisson apply of order 7: 4.49 -> 3.90 ms.  The mixed modes keep the double-FP32 kernels of
+// mw_post_df.cu (26 us).
+constexpr size_t FX_PAIRS = 512;
+void fx_pairs(Ctx &ctx, Arena &ar, const std::vector<PairTask> &all, bool up, uint32_t *fx, mw_stats &st) {
+    const int K = ctx.basis.K;
+    const size_t fxw = fx_words(K), opw = fx_op_words(K), k3 = (size_t)K * K * K;
+    for (size_t at = 0; at < all.size(); at += FX_PAIRS) {
+        const size_t n = std::min(FX_PAIRS, all.size() - at);
+        const PairTask *tasks = all.data() + at;
+        const uint32_t *w = ctx.d_wfx + (up ? 0 : opw);
+        std::vector<double *> out(n);
+        std::vector<long long> begin(n + 1);
+        std::vector<const void *> in(n), a(n, w), az(n, w + fx_op_z(K));
+        for (size_t i = 0; i < n; i++) {
+            out[i] = up ? tasks[i].parent : tasks[i].child0;
+            in[i] = fx + fxw * i;
+            begin[i + 1] = (long long)i + 1;
+        }
+        const int zero = 0;
+        Packer pk;
+        pk.add(tasks, n * sizeof(PairTask));
+        pk.add(out.data(), n * sizeof(double *));
+        pk.add(begin.data(), (n + 1) * sizeof(long long));
+        pk.add(in.data(), n * sizeof(void *));
+        pk.add(a.data(), n * sizeof(void *));
+        pk.add(az.data(), n * sizeof(void *));
+        pk.add(&zero, sizeof zero);
+        pk.ship(ctx, ar);
+        k_pairs_to_fx((const PairTask *)pk.ptr(0), up, fx, n, K, ctx.stream);
+        ApplyLaunch L{};
+        L.nnodes = (int)n;
+        L.root = 1;
+        L.set = up ? 1 : 0;
+        L.cstride = up ? k3 : 8 * k3;
+        L.out = (double *const *)pk.ptr(1);
+        L.begin = (const long long *)pk.ptr(2);
+        L.end = L.begin + 1;
+        L.in = (const void *const *)pk.ptr(3);
+        L.ax = L.ay = (const void *const *)pk.ptr(4);
+        L.az = (const void *const *)pk.ptr(5);
+        L.counter = (int *)pk.ptr(6);
+        k_apply_fx(ctx.dbasis, L, ctx.stream);
+        st.launches += 2;
+    }
+}
+
 // the largest sub-block norm of an operator (the FP32 estimates need it well inside FP32's range)
 double oper_norm_max(const Oper &op) {
     double m = 0.0;
@@ -1588,6 +1640,13 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
     auto post_process = [&](const std::vector<JobState *> &jset, Arena &ar) {
         int maxn = b.n0;
         for (JobState *sp : jset) maxn = std::max(maxn, sp->job->out->max_scale());
+        bool fx = !mixed && digits;
+        size_t most = 0;
+        for (JobState *sp : jset) {
+            fx = fx && sp->fixed_point;
+            most += (size_t)sp->job->out->nn() / 8;
+        }
+        uint32_t *fxbuf = fx && most ? (uint32_t *)ar.alloc(sizeof(uint32_t) * fxw * std::min(most, FX_PAIRS)) : nullptr;
         for (int n = b.n0; n < maxn; n++) {
             std::vector<PairTask> tasks;
             for (JobState *sp : jset) {
@@ -1597,6 +1656,10 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                         tasks.push_back({out.block(i), out.block(out.nodes[i].child0)});
             }
             if (tasks.empty()) continue;
+            if (fx) {
+                fx_pairs(ctx, ar, tasks, false, fxbuf, st);
+                continue;
+            }
             Packer pk;
             pk.add(tasks.data(), tasks.size() * sizeof(PairTask));
             pk.ship(ctx, ar);
@@ -1618,6 +1681,10 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                     }
             }
             if (tasks.empty()) continue;
+            if (fx) {
+                fx_pairs(ctx, ar, tasks, true, fxbuf, st);
+                continue;
+            }
             Packer pk;
             pk.add(tasks.data(), tasks.size() * sizeof(PairTask));
             pk.add(cnp.data(), cnp.size() * sizeof(double *));
@@ -1630,12 +1697,12 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                            ctx.stream);
             st.launches++;
         }
-        // leaf norms after the top-down pass
+        // leaf norms after the top-down pass; the fixed-point compression leaves the parents' to this launch too
         std::vector<double *> bl, cnp;
         for (JobState *sp : jset) {
             Tree &out = *sp->job->out;
             for (int i = 0; i < out.nn(); i++)
-                if (out.nodes[i].child0 < 0) {
+                if (fx || out.nodes[i].child0 < 0) {
                     bl.push_back(out.block(i));
                     cnp.push_back(out.d_cn + (size_t)8 * i);
                 }
@@ -1749,12 +1816,40 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
 }
 
 // ------------------------------------------------------------------ multiply
+void make_transform_digits(Ctx &ctx) {
+    // two operators of one block each, with their tables in front of the digits
+    const int K = ctx.basis.K;
+    const size_t opw = fx_op_words(K);
+    const struct { double c; int zero[2]; } head = {1.0, {0, 0}};
+    MWG_CUDA(cudaMalloc(&ctx.d_wfx, sizeof(uint32_t) * 2 * opw + sizeof head));
+    char *dh = (char *)(ctx.d_wfx + 2 * opw);
+    MWG_CUDA(cudaMemcpy(dh, &head, sizeof head, cudaMemcpyHostToDevice));
+    FxOpJob jobs[2];
+    for (int i = 0; i < 2; i++) {
+        ScreenOp op{};
+        op.c = (const double *)dh;
+        op.off = op.first = (const int *)(dh + sizeof(double));
+        op.b64 = i ? ctx.dbasis.WT : ctx.dbasis.W;
+        op.T = op.S = 1;
+        jobs[i] = FxOpJob{op, ctx.d_wfx + opw * i, 0, 1};
+    }
+    k_op_to_fx(jobs, 2, K, ctx.stream);
+    MWG_CUDA(cudaStreamSynchronize(ctx.stream));
+}
+
 // bottom-up compression of several trees, one launch per scale
-void compress_batch(const std::vector<Tree *> &trees, Arena &arena, mw_stats *st, bool df) {
+void compress_batch(const std::vector<Tree *> &trees, Arena &arena, mw_stats *st, bool df, bool fx) {
     if (trees.empty()) return;
     Ctx &ctx = *trees[0]->ctx;
     int maxn = ctx.basis.n0;
     for (Tree *t : trees) maxn = std::max(maxn, t->max_scale());
+    // fixed point: the parents' norms in one launch at the end
+    std::vector<double *> pbl, pcn;
+    mw_stats fst{};
+    size_t most = 0;
+    for (Tree *t : trees) most += (size_t)t->nn() / 8;
+    uint32_t *fxbuf =
+        fx && most ? (uint32_t *)arena.alloc(sizeof(uint32_t) * fx_words(ctx.basis.K) * std::min(most, FX_PAIRS)) : nullptr;
     for (int n = maxn - 1; n >= ctx.basis.n0; n--) {
         std::vector<PairTask> tasks;
         std::vector<double *> cnp;
@@ -1765,6 +1860,12 @@ void compress_batch(const std::vector<Tree *> &trees, Arena &arena, mw_stats *st
                     cnp.push_back(t->d_cn + (size_t)8 * i);
                 }
         if (tasks.empty()) continue;
+        if (fx) {
+            fx_pairs(ctx, arena, tasks, true, fxbuf, fst);
+            pcn.insert(pcn.end(), cnp.begin(), cnp.end());
+            for (const PairTask &p : tasks) pbl.push_back(p.parent);
+            continue;
+        }
         Packer pk;
         pk.add(tasks.data(), tasks.size() * sizeof(PairTask));
         pk.add(cnp.data(), cnp.size() * sizeof(double *));
@@ -1776,6 +1877,14 @@ void compress_batch(const std::vector<Tree *> &trees, Arena &arena, mw_stats *st
             k_compress(ctx.dbasis, (const PairTask *)pk.ptr(0), (double *const *)pk.ptr(1), (int)tasks.size(),
                        ctx.stream);
         if (st) st->launches++;
+    }
+    if (!pbl.empty()) {
+        Packer pk;
+        pk.add(pbl.data(), pbl.size() * sizeof(double *));
+        pk.add(pcn.data(), pcn.size() * sizeof(double *));
+        pk.ship(ctx, arena);
+        k_norms(ctx.dbasis, (double *const *)pk.ptr(0), (double *const *)pk.ptr(1), (int)pbl.size(), ctx.stream);
+        if (st) st->launches += fst.launches + 1;
     }
     // every tree's norms in one download (gathered on the device into pinned memory)
     std::vector<const double *> gsrc;
@@ -2313,19 +2422,24 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
     }
     // the forward's post-processing: top-down sum over scales, bottom-up compression
     arena.reset();
+    uint32_t *fxbuf = fixed_point ? (uint32_t *)arena.alloc(sizeof(uint32_t) * fxw * std::min((size_t)ext.nn() / 8 + 1, FX_PAIRS)) : nullptr;
     for (int n = b.n0; n < ext.max_scale(); n++) {
         std::vector<PairTask> tasks;
         for (int i = 0; i < ext.nn(); i++)
             if (ext.nodes[i].n == n && ext.nodes[i].child0 >= 0)
                 tasks.push_back({ext.block(i), ext.block(ext.nodes[i].child0)});
         if (tasks.empty()) continue;
+        if (fixed_point) {
+            fx_pairs(ctx, arena, tasks, false, fxbuf, st);
+            continue;
+        }
         Packer pk;
         pk.add(tasks.data(), tasks.size() * sizeof(PairTask));
         pk.ship(ctx, arena);
         k_topdown(ctx.dbasis, (const PairTask *)pk.ptr(0), (int)tasks.size(), ctx.stream);
         st.launches++;
     }
-    compress_batch({&ext}, arena, &st);
+    compress_batch({&ext}, arena, &st, false, fixed_point);
     // projection onto x's grid: keep x's nodes (their blocks now carry the finer parts)
     copy_grid(res, x);
     arena.reset();

@@ -312,6 +312,8 @@ struct FxSets {
     uint32_t *out[MAX];
     long long first[MAX + 1];  // blocks of the sets before
     int n;
+    const PairTask *pairs;  // or (n = 1): pairs' parents, or the cubes of their children's scaling parts (up)
+    int up;
 };
 
 // Operator blocks' digits (FxGeo::OP_WORDS words per block), the blocks of one scale of the grid's y-th
@@ -373,22 +375,24 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS) to_fx_kernel(__grid_constan
     using G = FxGeo<K>;
     constexpr int N2 = G::N2, K2 = G::K2, K3 = G::K3;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const size_t cs = (size_t)(S.pairs && S.up ? 8 : 1) * K3;  // distance of a block's components
     for (long long b = blockIdx.x; b < S.first[S.n]; b += gridDim.x) {
         int k = 0;
         while (b >= S.first[k + 1]) k++;
-        const double *in = S.in[k] + (size_t)(b - S.first[k]) * 8 * K3;
+        const double *in = S.pairs ? (S.up ? S.pairs[b].child0 : S.pairs[b].parent)
+                                   : S.in[k] + (size_t)(b - S.first[k]) * 8 * K3;
         uint32_t *o = S.out[k] + (size_t)(b - S.first[k]) * G::IN_WORDS;
         int ef = 0;
         auto at = [&](int X, int Y, int Z) -> long long {
             if (X >= N2 || Y >= N2) return 0;
             const int cx = X >= K, cy = Y >= K, cz = Z >= K;
             return fx_from_double(
-                in[(size_t)(cx + 2 * cy + 4 * cz) * K3 + (Z - cz * K) * K2 + (Y - cy * K) * K + (X - cx * K)], ef);
+                in[(cx + 2 * cy + 4 * cz) * cs + (Z - cz * K) * K2 + (Y - cy * K) * K + (X - cx * K)], ef);
         };
         auto field = [&](int X, int Y, int Z) -> int {
             if (X >= N2 || Y >= N2) return 0;
             const int cx = X >= K, cy = Y >= K, cz = Z >= K;
-            return (__double2hiint(in[(size_t)(cx + 2 * cy + 4 * cz) * K3 + (Z - cz * K) * K2 + (Y - cy * K) * K + (X - cx * K)]) >> 20) & 0x7ff;
+            return (__double2hiint(in[(cx + 2 * cy + 4 * cz) * cs + (Z - cz * K) * K2 + (Y - cy * K) * K + (X - cx * K)]) >> 20) & 0x7ff;
         };
         for (int tile = warp; tile < G::NTIN; tile += G::WARPS) {
             int Y, Z;
@@ -779,6 +783,7 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
         // a chunk's partial block is this task's alone; a whole node's block takes other tiers' sums too
         const bool set = L.set || (L.red_of && L.red_of[w] >= 0);
         double *out = L.out[w];
+        const size_t cs = L.cstride ? L.cstride : (size_t)K3;
 #pragma unroll 1
         for (int q = 0; q < G::TPW; q++) {
             const int nt = warp + q * G::WARPS;
@@ -789,7 +794,7 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
                 if (c >= G::NC || Zq >= N2) continue;
                 const int hq = c / K2, hz = Zq >= K;
                 const double v = fx_to_double(acc[q][r], ea[q] - 62);
-                double *o = out + (hq + 4 * hz) * K3 + (Zq - hz * K) * K2 + (c - hq * K2);
+                double *o = out + (hq + 4 * hz) * cs + (Zq - hz * K) * K2 + (c - hq * K2);
                 *o = set ? v : *o + v;
             }
         }
@@ -876,6 +881,20 @@ void k_op_to_fx(const FxOpJob *jobs, size_t n, int K, cudaStream_t s) {
     }
 }
 
+static void to_fx(const FxSets &S, int K, cudaStream_t s) {
+    if (S.first[S.n] == 0) return;
+    switch (K) {
+        case 4: launch_to_fx<4>(S, s); break;
+        case 5: launch_to_fx<5>(S, s); break;
+        case 6: launch_to_fx<6>(S, s); break;
+        case 7: launch_to_fx<7>(S, s); break;
+        case 8: launch_to_fx<8>(S, s); break;
+        case 9: launch_to_fx<9>(S, s); break;
+        case 10: launch_to_fx<10>(S, s); break;
+        default: throw Error(MW_ERR_ARG, "no fixed-point apply kernel for this order");
+    }
+}
+
 void k_to_fx(const FxBlocks *sets, size_t n, int K, cudaStream_t s) {
     for (size_t at = 0; at < n; at += FxSets::MAX) {
         FxSets S{};
@@ -885,18 +904,18 @@ void k_to_fx(const FxBlocks *sets, size_t n, int K, cudaStream_t s) {
             S.out[S.n] = b.out;
             S.first[S.n + 1] = S.first[S.n] + (long long)b.n;
         }
-        if (S.first[S.n] == 0) continue;
-        switch (K) {
-            case 4: launch_to_fx<4>(S, s); break;
-            case 5: launch_to_fx<5>(S, s); break;
-            case 6: launch_to_fx<6>(S, s); break;
-            case 7: launch_to_fx<7>(S, s); break;
-            case 8: launch_to_fx<8>(S, s); break;
-            case 9: launch_to_fx<9>(S, s); break;
-            case 10: launch_to_fx<10>(S, s); break;
-            default: throw Error(MW_ERR_ARG, "no fixed-point apply kernel for this order");
-        }
+        to_fx(S, K, s);
     }
+}
+
+void k_pairs_to_fx(const PairTask *pairs, bool up, uint32_t *out, size_t n, int K, cudaStream_t s) {
+    FxSets S{};
+    S.n = 1;
+    S.out[0] = out;
+    S.first[1] = (long long)n;
+    S.pairs = pairs;
+    S.up = up ? 1 : 0;
+    to_fx(S, K, s);
 }
 
 void k_apply_fx(const DevBasis &b, const ApplyLaunch &L, cudaStream_t s) {

@@ -101,6 +101,7 @@ int mw_ctx_create(int device, int root_scale, const int corner[3], const int box
         c->ctx.dbasis = mwg::DevBasis{K, basis, d, d + K2 * K2, d + 2 * K2 * K2, d + 2 * K2 * K2 + K * K,
                                       d + 2 * K2 * K2 + 2 * K * K, d + 2 * K2 * K2 + 2 * K * K + K,
                                       d + 2 * K2 * K2 + 2 * K * K + 2 * K};
+        mwg::make_transform_digits(c->ctx);
         // tree growth allocates from the device's stream-ordered pool (Tree::reserve); the pool keeps
         // what is returned to it instead of handing it back to the driver at every synchronisation
         cudaMemPool_t pool = nullptr;
@@ -139,6 +140,7 @@ static void ctx_free(mw_ctx c) {
     for (auto &xa : c->ctx.xarena) xa.release();
     if (c->ctx.h_pinned) cudaFreeHost(c->ctx.h_pinned);
     if (c->ctx.d_basis) cudaFree(c->ctx.d_basis);
+    if (c->ctx.d_wfx) cudaFree(c->ctx.d_wfx);
     cudaStreamDestroy(c->ctx.stream);
     for (auto &xs : c->ctx.xstream)
         if (xs) cudaStreamDestroy(xs);

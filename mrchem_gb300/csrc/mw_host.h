@@ -172,6 +172,7 @@ struct Ctx {
     Basis basis;
     DevBasis dbasis{};
     double *d_basis = nullptr;
+    uint32_t *d_wfx = nullptr;  // operator digits of W and of its transpose (two-scale transforms in fixed point)
     std::string err;
     mw_stats last{};
     int nsm = 0;
@@ -293,6 +294,7 @@ struct ApplyLaunch {
     const void *const *ay;
     const void *const *az;
     const double *coef;           // per item
+    size_t cstride = 0;           // distance of an output block's components (0: K^3; fixed-point kernel only)
     int *counter;                 // dynamic node counter (persistent grid); zero at launch
     int *status;                  // 0, or non-zero when a bounded wait of the launch ran out (TF32 tier)
     int *rows = nullptr;          // rows processed (y and z passes run), summed over the launch's tasks
@@ -364,6 +366,8 @@ struct FxBlocks {  // n consecutive blocks
     size_t n;
 };
 void k_to_fx(const FxBlocks *sets, size_t n, int K, cudaStream_t s);
+// digits of n pairs' parent blocks, or (up) of the cubes of their children's scaling parts
+void k_pairs_to_fx(const PairTask *pairs, bool up, uint32_t *out, size_t n, int K, cudaStream_t s);
 void k_norms(const DevBasis &b, double *const *blocks, double *const *cn, int n, cudaStream_t s);
 void k_topdown(const DevBasis &b, const PairTask *tasks, int n, cudaStream_t s);
 void k_compress(const DevBasis &b, const PairTask *tasks, double *const *cn, int n, cudaStream_t s);

@@ -112,8 +112,11 @@ double dot_noalloc(const Tree &a, const Tree &b);
 void noalloc_setup(int device);
 void tree_save(Tree &t, const char *path);
 void tree_load(Tree &t, const char *path);
-// bottom-up compression of several trees, one launch per scale; df: double-FP32 transforms
-void compress_batch(const std::vector<Tree *> &trees, Arena &arena, mw_stats *st, bool df = false);
+// the digits of W and its transpose (Ctx::d_wfx)
+void make_transform_digits(Ctx &ctx);
+// bottom-up compression of several trees, one launch per scale; df: double-FP32 transforms,
+// fx: fixed-point ones (every value finite and below 1e150)
+void compress_batch(const std::vector<Tree *> &trees, Arena &arena, mw_stats *st, bool df = false, bool fx = false);
 void add(Tree &out, const std::vector<const Tree *> &trees, const std::vector<double> &coefs, mw_stats &st);
 
 }  // namespace mwg

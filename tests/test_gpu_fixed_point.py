@@ -92,3 +92,24 @@ def test_batch_of_more_operators_and_trees_than_one_launch_takes(engine, precisi
         engine.apply(prec, one, H, f, precision=precision)
         (k1, c1, _), (k2, c2, _) = v.download(), one.download()
         assert np.array_equal(k1, k2) and rel_l2(c1, c2) <= 2e-14
+
+
+def test_transforms_of_more_pairs_than_one_slice(engine):
+    # the two-scale transforms after an FP64 apply take 512 parents of a scale at a time: 320 trees over four
+    # groups with eight parents at each of several scales.  Against each apply alone, as above.
+    prec, n = 1e-2, 320
+    mra = engine.MultiResolutionAnalysis(3)
+    H = engine.HelmholtzOperator(mra, 1.0, prec)
+    fs = [engine.project(prec, engine.FunctionTree(mra), [(1.0, 2.0 + 0.01 * i, (0.005 * i - 0.5, 0.1, -0.2), (0, 0, 0))])
+          for i in range(n)]
+    many = [engine.FunctionTree(mra) for _ in range(n)]
+    engine.apply_batch([prec] * n, many, [H] * n, fs)
+    finest = [np.bincount(v.download()[0][:, 0] + 32).max() // 8 for v in many[:n // 4]]
+    assert sum(finest) > 512
+    for f, v in list(zip(fs, many))[::13]:
+        one = engine.FunctionTree(mra)
+        engine.apply(prec, one, H, f)
+        (k1, c1, l1), (k2, c2, l2) = v.download(), one.download()
+        assert np.array_equal(k1, k2) and np.array_equal(l1, l2) and rel_l2(c1, c2) <= 2e-14
+        # the norms that come with the blocks
+        assert abs(v.norm() - one.norm()) <= 2e-14 * one.norm()
