@@ -586,6 +586,14 @@ void fx_pairs(Ctx &ctx, Arena &ar, const std::vector<PairTask> &all, bool up, ui
     }
 }
 
+void ensure_fast(Ctx &ctx) {  // the generation's and screening's high-priority stream
+    if (ctx.fast) return;
+    int least = 0, greatest = 0;
+    MWG_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    MWG_CUDA(cudaStreamCreateWithPriority(&ctx.fast, cudaStreamNonBlocking, greatest));
+    MWG_CUDA(cudaEventCreateWithFlags(&ctx.fast_done, cudaEventDisableTiming));
+}
+
 // the largest sub-block norm of an operator (the FP32 estimates need it well inside FP32's range)
 double oper_norm_max(const Oper &op) {
     double m = 0.0;
@@ -1196,12 +1204,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
             if (s.job->out->nodes[i].n == n) s.work.push_back(i);
     };
 
-    if (!ctx.fast) {
-        int least = 0, greatest = 0;
-        MWG_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        MWG_CUDA(cudaStreamCreateWithPriority(&ctx.fast, cudaStreamNonBlocking, greatest));
-        MWG_CUDA(cudaEventCreateWithFlags(&ctx.fast_done, cudaEventDisableTiming));
-    }
+    ensure_fast(ctx);
     cudaEvent_t ev_start = nullptr;
     std::vector<cudaEvent_t> ev_end(ngroups, nullptr);
     // the generation stream and groups 1.. start after everything queued on the context's stream
@@ -2324,27 +2327,39 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
         k_to_fx(&ys, 1, b.K, ctx.stream);
         st.launches++;
     }
-    LevelItems li;
     const int maxn = y.max_scale();
+    // The host prepares a scale's items while the GPU runs the scale before: two arenas in turn, each free
+    // again when its scale's launches have ended; generation on the high-priority stream.
+    ensure_fast(ctx);
+    struct Event {
+        cudaEvent_t e = nullptr;
+        Event() { MWG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)); }
+        ~Event() { cudaEventDestroy(e); }
+    } ready, done[2];
+    MWG_CUDA(cudaEventRecord(ready.e, ctx.stream));
+    MWG_CUDA(cudaStreamWaitEvent(ctx.fast, ready.e, 0));
+    for (Event &e : done) MWG_CUDA(cudaEventRecord(e.e, ctx.stream));
+    const std::vector<int> in_ext = match_nodes(x, ext);  // ext starts as x's grid
+    int turn = 0;
     for (int n = b.n0; n <= maxn; n++) {
         const int sidx = n - b.n0;
         const bool root = (n == b.n0);
-        arena.reset();
         s.work.clear();
         for (int i = 0; i < y.nn(); i++)
             if (y.nodes[i].n == n) s.work.push_back(i);
         if (s.work.empty()) continue;
-        s.wgt.assign(s.work.size(), 1.0);
-        s.cand.assign(s.work.size(), {});
+        const long nw = (long)s.work.size();
+        s.wgt.assign(nw, 1.0);
+        s.cand.assign(nw, {});
         const double thr = root ? 0.0 : SCREEN_FAC * split_thr(prec, 1.0, n);
 #pragma omp parallel
         {
             LookupCache cache;
 #pragma omp for schedule(dynamic, 4)
-            for (long w = 0; w < (long)s.work.size(); w++) enumerate_node(s, (int)w, sidx, root, thr, cache);
+            for (long w = 0; w < nw; w++) enumerate_node(s, (int)w, sidx, root, thr, cache);
         }
         s.gens.clear();
-        for (size_t w = 0; w < s.work.size(); w++) {
+        for (long w = 0; w < nw; w++) {
             const NodeInfo &o = y.nodes[s.work[w]];
             for (Cand &c : s.cand[w]) {
                 if (!c.gen) continue;
@@ -2352,74 +2367,115 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
                 c.src = s.gens.request(x, n, p, c.src);
             }
         }
-        generate_all({{&s.gens, &x}}, arena, &st);
-        // surviving items, each with its input position; grow the result grid to hold every position
-        struct TItem {
-            int target, o;
-            const Cand *c;
-        };
-        std::vector<TItem> items;
-        for (size_t w = 0; w < s.work.size(); w++) {
-            const NodeInfo &o = y.nodes[s.work[w]];
-            for (const Cand &c : s.cand[w]) {
+        Arena &ar = turn ? ctx.xarena[0] : arena;
+        MWG_CUDA(cudaEventSynchronize(done[turn].e));
+        ar.reset();
+        {
+            StreamSwap fast(ctx, ctx.fast);
+            generate_all({{&s.gens, &x}}, ar, &st);
+            ctx.sync();
+        }
+        // the surviving items of every node of y, and the generated positions that any of them has
+        std::vector<std::vector<int>> keep(nw);
+        std::vector<char> wanted(s.gens.keys.size(), 0);
+        std::vector<double> pairs(nw, 0.0);
+#pragma omp parallel for schedule(dynamic, 4)
+        for (long w = 0; w < nw; w++)
+            for (int q = 0; q < (int)s.cand[w].size(); q++) {
+                const Cand &c = s.cand[w][q];
                 const double *cn = c.gen ? &s.gens.cn[8 * (size_t)c.src] : &x.cn[8 * (size_t)c.src];
                 const double *nx = op.norm(c.t, sidx, c.lx), *ny = op.norm(c.t, sidx, c.ly),
                              *nz = op.norm(c.t, sidx, c.lz);
                 if (!root && item_bound(nx, ny, nz, cn, root) < thr) continue;
-                int p[3] = {o.l[0] - c.lx, o.l[1] - c.ly, o.l[2] - c.lz};
-                int t = ext.find(n, p);
-                while (t < 0) {  // split the deepest existing ancestor until the position exists
-                    int an = n, al[3] = {p[0], p[1], p[2]}, a = -1;
-                    while (a < 0) {
-                        an--;
-                        for (int d = 0; d < 3; d++) al[d] = floordiv2(al[d]);
-                        a = ext.find(an, al);
-                    }
-                    int first = ext.nn();
-                    ext.split(a);
-                    tree_zero(ext, first, 8);
-                    t = ext.find(n, p);
+                keep[w].push_back(q);
+                pairs[w] += item_pairs(nx, ny, nz, cn, root);
+                if (c.gen) {
+#pragma omp atomic write
+                    wanted[c.src] = 1;
                 }
-                items.push_back({t, s.work[w], &c});
-                st.flops += 6.0 * K4 * item_pairs(nx, ny, nz, cn, root);
             }
+        // grow the result grid to hold every position
+        std::vector<int> gen_in_ext(s.gens.keys.size(), -1);
+        for (size_t g = 0; g < s.gens.keys.size(); g++) {
+            if (!wanted[g]) continue;
+            const int *p = s.gens.keys[g].l;
+            int t = ext.find(n, p);
+            while (t < 0) {  // split the deepest existing ancestor until the position exists
+                int an = n, al[3] = {p[0], p[1], p[2]}, a = -1;
+                while (a < 0) {
+                    an--;
+                    for (int d = 0; d < 3; d++) al[d] = floordiv2(al[d]);
+                    a = ext.find(an, al);
+                }
+                int first = ext.nn();
+                ext.split(a);
+                tree_zero(ext, first, 8);
+                t = ext.find(n, p);
+            }
+            gen_in_ext[g] = t;
         }
-        std::stable_sort(items.begin(), items.end(), [](const TItem &a, const TItem &b2) { return a.target < b2.target; });
+        // the items grouped by position (in the order of the positions in ext; a position's items in the order
+        // of y's nodes and of their walks)
+        auto target = [&](const Cand &c) { return c.gen ? gen_in_ext[c.src] : in_ext[c.src]; };
+        std::vector<long long> at(ext.nn() + 1, 0);
+        std::vector<std::vector<long long>> place(nw);
+        for (long w = 0; w < nw; w++) {
+            st.flops += 6.0 * K4 * pairs[w];
+            for (int q : keep[w]) at[target(s.cand[w][q]) + 1]++;
+        }
+        LevelItems li;
+        li.begin.assign(1, 0);
+        for (int t = 0; t < ext.nn(); t++) {
+            if (at[t + 1] > 0) {
+                li.out.push_back(ext.block(t));
+                li.begin.push_back(at[t] + at[t + 1]);
+            }
+            at[t + 1] += at[t];
+        }
+        const long long items = at[ext.nn()];
+        for (long w = 0; w < nw; w++) {
+            place[w].reserve(keep[w].size());
+            for (int q : keep[w]) place[w].push_back(at[target(s.cand[w][q])]++);
+        }
         FxLevelOps fxops;
         fxops.words = fx_op_words(b.K);
         fxops.zoff = fx_op_z(b.K);
         fxops.s = sidx;
-        if (fixed_point) fxops.add(op, arena);
-        li = LevelItems();
-        li.begin.assign(1, 0);
-        for (size_t q = 0; q < items.size(); q++) {
-            const TItem &it = items[q];
-            if (q == 0 || it.target != items[q - 1].target) {
-                if (q > 0) li.begin.push_back((long long)q);
-                li.out.push_back(ext.block(it.target));
+        if (fixed_point) fxops.add(op, ar);
+        li.in.resize(items);
+        li.ax.resize(items);
+        li.ay.resize(items);
+        li.az.resize(items);
+        li.coef.resize(items);
+#pragma omp parallel for schedule(dynamic, 4)
+        for (long w = 0; w < nw; w++)
+            for (size_t j = 0; j < keep[w].size(); j++) {
+                const Cand &c = s.cand[w][keep[w][j]];
+                const long long q = place[w][j];
+                const int l[3] = {-c.lx, -c.ly, -c.lz};
+                const void *a[3];
+                for (int d = 0; d < 3; d++)
+                    a[d] = fixed_point ? (const void *)(fxops.block(op, c.t, l[d]) + (d == 2 ? fxops.zoff : 0))
+                                       : (const void *)(op.d_blocks + (size_t)op.block_index(c.t, sidx, l[d]) * bsz);
+                li.in[q] = fixed_point ? (const void *)(yfx + fxw * (size_t)s.work[w]) : (const void *)y.block(s.work[w]);
+                li.ax[q] = a[0];
+                li.ay[q] = a[1];
+                li.az[q] = a[2];
+                li.coef[q] = op.c[c.t];
             }
-            li.in.push_back(fixed_point ? (const void *)(yfx + fxw * (size_t)it.o) : (const void *)y.block(it.o));
-            const int l[3] = {-it.c->lx, -it.c->ly, -it.c->lz};
-            const void *a[3];
-            for (int d = 0; d < 3; d++)
-                a[d] = fixed_point ? (const void *)(fxops.block(op, it.c->t, l[d]) + (d == 2 ? fxops.zoff : 0))
-                                   : (const void *)(op.d_blocks + (size_t)op.block_index(it.c->t, sidx, l[d]) * bsz);
-            li.ax.push_back(a[0]);
-            li.ay.push_back(a[1]);
-            li.az.push_back(a[2]);
-            li.coef.push_back(op.c[it.c->t]);
-        }
-        if (!items.empty()) li.begin.push_back((long long)items.size());
         li.nodes = (long)li.out.size();
-        li.items = (long long)items.size();
-        st.items += (long long)items.size();
-        st.items_fp64 += (long long)items.size();
+        li.items = items;
+        st.items += items;
+        st.items_fp64 += items;
         st.out_nodes += (long long)li.out.size();
-        if (fixed_point && !items.empty()) fxops.make(ctx, st);
-        launch_tier(ctx, ctx.arena, li, root, true, 0, Ctx::Tuning().chunk[0], st, nullptr, false, fixed_point);
-        ctx.sync();
+        if (fixed_point && items > 0) fxops.make(ctx, st);
+        launch_tier(ctx, ar, li, root, true, 0, Ctx::Tuning().chunk[0], st, nullptr, false, fixed_point);
+        MWG_CUDA(cudaEventRecord(done[turn].e, ctx.stream));
+        turn ^= 1;
         st.levels++;
     }
+    ctx.sync();
+    ctx.xarena[0].reset();
     // the forward's post-processing: top-down sum over scales, bottom-up compression
     arena.reset();
     uint32_t *fxbuf = fixed_point ? (uint32_t *)arena.alloc(sizeof(uint32_t) * fxw * std::min((size_t)ext.nn() / 8 + 1, FX_PAIRS)) : nullptr;
