@@ -2414,11 +2414,13 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
             }
             gen_in_ext[g] = t;
         }
-        // the items grouped by position (in the order of the positions in ext; a position's items in the order
-        // of y's nodes and of their walks)
+        // the items grouped by position, a position's in walk order: its rows of one term, ly and lz then share
+        // their y and z passes (in the order of y's nodes every item was a row of its own)
+        struct Item {
+            int w, q;
+        };
         auto target = [&](const Cand &c) { return c.gen ? gen_in_ext[c.src] : in_ext[c.src]; };
         std::vector<long long> at(ext.nn() + 1, 0);
-        std::vector<std::vector<long long>> place(nw);
         for (long w = 0; w < nw; w++) {
             st.flops += 6.0 * K4 * pairs[w];
             for (int q : keep[w]) at[target(s.cand[w][q]) + 1]++;
@@ -2433,10 +2435,9 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
             at[t + 1] += at[t];
         }
         const long long items = at[ext.nn()];
-        for (long w = 0; w < nw; w++) {
-            place[w].reserve(keep[w].size());
-            for (int q : keep[w]) place[w].push_back(at[target(s.cand[w][q])]++);
-        }
+        std::vector<Item> order(items);
+        for (long w = 0; w < nw; w++)
+            for (int q : keep[w]) order[at[target(s.cand[w][q])]++] = Item{(int)w, q};
         FxLevelOps fxops;
         fxops.words = fx_op_words(b.K);
         fxops.zoff = fx_op_z(b.K);
@@ -2448,10 +2449,14 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
         li.az.resize(items);
         li.coef.resize(items);
 #pragma omp parallel for schedule(dynamic, 4)
-        for (long w = 0; w < nw; w++)
-            for (size_t j = 0; j < keep[w].size(); j++) {
-                const Cand &c = s.cand[w][keep[w][j]];
-                const long long q = place[w][j];
+        for (size_t t = 0; t < li.out.size(); t++) {
+            std::sort(order.begin() + li.begin[t], order.begin() + li.begin[t + 1], [&](const Item &a, const Item &b2) {
+                const Cand &ca = s.cand[a.w][a.q], &cb = s.cand[b2.w][b2.q];
+                return std::tie(ca.t, ca.lz, ca.ly, ca.lx) < std::tie(cb.t, cb.lz, cb.ly, cb.lx);
+            });
+            for (long long q = li.begin[t]; q < li.begin[t + 1]; q++) {
+                const int w = order[q].w;
+                const Cand &c = s.cand[w][order[q].q];
                 const int l[3] = {-c.lx, -c.ly, -c.lz};
                 const void *a[3];
                 for (int d = 0; d < 3; d++)
@@ -2463,6 +2468,7 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
                 li.az[q] = a[2];
                 li.coef[q] = op.c[c.t];
             }
+        }
         li.nodes = (long)li.out.size();
         li.items = items;
         st.items += items;

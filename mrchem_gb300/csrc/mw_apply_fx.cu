@@ -72,20 +72,23 @@ struct FxGeo {
     static constexpr int NT = (NC + 7) / 8;           // column tiles of the y and z passes
     static constexpr int NTX = (K2 + 7) / 8;          // ... of which take the second operand
     static constexpr int TPW = (NT + WARPS - 1) / WARPS;
-    static constexpr int YT = BIG ? 2 : 1;            // row tiles of the y and z passes
     // T[Z][Y][X'] and u[Z][Y][X'] (Z, Y, X' < K), 62-bit numbers
     static constexpr int PX = fx_pitch(N2), PZ = fx_pitch(N2 * PX), UX = fx_pitch(K), UZ = fx_pitch(K * UX);
     static constexpr int MAINW = 7 * 128;             // words of a row tile's digits (512 B per digit)
     static constexpr int TILEW = MAINW + (BIG ? 10 * 128 : 0);
-    static constexpr int O_U = 2 * N2 * PZ, O_X = O_U + 2 * K * UZ + (2 * K * UZ) % 4, O_Y = O_X + 4 * TILEW,
-                         O_Z = O_Y + YT * TILEW, WORDS = O_Z + YT * TILEW;
+    static constexpr int STACKW = BIG ? 14 * 128 : 0;  // words of the stacked rows 16.. (fx_stack)
+    // an operator in the x pass: row tile 1 (u's rows and 16..), row tile 0, the stack; in the others without tile 1
+    static constexpr int YW = TILEW + STACKW, XW = TILEW + YW;
+    static constexpr int O_U = 2 * N2 * PZ, O_X = O_U + 2 * K * UZ + (2 * K * UZ) % 4, O_Y = O_X + 2 * XW,
+                         O_Z = O_Y + YW, WORDS = O_Z + YW;
     static constexpr size_t SMEM = 4 * (size_t)WORDS;
     // input digits of a block: per column tile the lanes' operands as 16-byte groups and one 8-byte group, then
     // the tiles' exponents
     static constexpr int WB = BIG ? 18 : 14, IN_EXP = NTIN * WB * 32, IN_WORDS = IN_EXP + (NTIN + 7) / 8 * 4;
-    // operator digits of a block: row tiles 0 and 1 (1 with u's rows) and the rows' exponents; then those of
-    // the block times its term's coefficient (the z pass's operand)
-    static constexpr int X_EXP = 2 * TILEW, Z_OFF = X_EXP + 16, Z_EXP = YT * TILEW, OP_WORDS = Z_OFF + Z_EXP + 16;
+    // operator digits of a block: the x pass's (the y pass's from X_Y on) and the rows' exponents; then those
+    // of the block times its term's coefficient (the z pass's)
+    static constexpr int X_Y = TILEW, X_EXP = XW, Z_OFF = X_EXP + 16, Z_EXP = YW, OP_WORDS = Z_OFF + Z_EXP + 16;
+    static_assert(Z_OFF == (BIG ? 2 * (7 + 10) + 14 : 2 * 7) * 128 + 16, "the same for all K of a kind");
     static_assert(O_U % 4 == 0 && O_X % 4 == 0 && TILEW % 4 == 0 && IN_WORDS % 4 == 0, "16-byte aligned copies");
 };
 
@@ -167,6 +170,34 @@ __device__ __forceinline__ long long fx_value(const float (&D)[10][4], int r) {
     return (long long)((unsigned long long)v + ((unsigned long long)((h << 5) - (M * 513u << 5)) << 32));
 }
 
+// Rows 16.. of an operator, four at most, would fill a quarter of a row tile of their own: instead row 4a + r
+// of these tiles holds row 16 + r for the weight d = a (D[0]) or 4 + a (D[1], D[2]), with the digit d - j that
+// goes with the data's digit j.  Eleven products and three of the folded remainder in place of 38, and
+// three accumulators in place of ten.  The weights 4..6 are split over D[1] and D[2]: at most 64 x 2^16 in each.
+__device__ __forceinline__ void fx_stack(float (&D)[3][4], const uint32_t *frag, const FxB &B, int lane) {
+    const uint4 *f = reinterpret_cast<const uint4 *>(frag) + lane;
+    fx_mma(D[0], f[11 * 32], B.s01, B.s23, true);
+    fx_mma(D[1], f[13 * 32], B.s4, B.s56, true);
+    fx_mma(D[2], f[12 * 32], B.s01, B.s23, true);
+#pragma unroll
+    for (int j = 0; j < 7; j++) {
+        if (j < 4) fx_mma(D[0], f[j * 32], B.m[j][0], B.m[j][1], false);
+        fx_mma(D[j >= 2 && j <= 4 ? 2 : 1], f[(4 + j) * 32], B.m[j][0], B.m[j][1], false);
+    }
+}
+
+// row 16 + (g & 3), column 2t + b, in every lane: this lane's weights (a = g >> 2 and a + 2) and its partner's
+__device__ __forceinline__ long long fx_stack_value(const float (&D)[3][4], int b, int g) {
+    const int n0 = __float_as_int(D[0][b]) - FX_MAGIC_BITS, n2 = __float_as_int(D[0][2 + b]) - FX_MAGIC_BITS;
+    const int p0 = (int)(__float_as_uint(D[1][b]) + __float_as_uint(D[2][b]) - 2u * FX_MAGIC_BITS);
+    const int p2 = (int)(__float_as_uint(D[1][2 + b]) + __float_as_uint(D[2][2 + b]) + (128u - 2u * FX_MAGIC_BITS));
+    const unsigned long long q = ((unsigned long long)(long long)n0 << 18) + (unsigned long long)(long long)n2;
+    const unsigned long long c = (unsigned long long)(long long)p0;
+    unsigned long long v = (g & 4) ? (q << 19) + (c << 1) : (q << 28) + (c << 10);
+    v += (unsigned long long)(long long)(p2 >> 8);
+    return (long long)(v + __shfl_xor_sync(0xffffffffu, v, 16));
+}
+
 // the seven digits of two 62-bit numbers as FP16 pairs (a in the low half)
 __device__ __forceinline__ void fx_digits(long long a, long long b, uint32_t (&w)[7]) {
     constexpr unsigned long long BIAS = 256ull * (((1ull << 63) - 1) / 511ull);  // 256 in every digit
@@ -240,12 +271,12 @@ __device__ __forceinline__ void fx_rows(double (&a)[FxRows<K>::N], const double 
     }
 }
 
-// These rows times cf into the digit fragments of the row tiles at d0 (rows 0..15) and d1 (rows 16.. as
-// rows 4..; with U also u's rows, the wavelet columns of rows r < K: row 8 + r, or r - 8 for r >= 8, when
-// K > 8, else row r), and the rows' exponents e: sum_k |a| <= 2^e.
+// These rows times cf into the digit fragments of row tile 0 at d0 (rows 0..15), of the stack at st (rows
+// 16..; fx_stack) and with U of row tile 1 at d1 (rows 16.. as rows 4.., and u's rows, the wavelet columns of rows
+// r < K: row 8 + r, or r - 8 for r >= 8, when K > 8, else row r), and the rows' exponents e: sum_k |a| <= 2^e.
 template <int K, bool U>
 __device__ __forceinline__ void fx_put(const double (&rows)[FxRows<K>::N], double cf, int unit, int lane, uint32_t *d0,
-                                       uint32_t *d1, short *exps) {
+                                       uint32_t *d1, uint32_t *st, short *exps) {
     using G = FxGeo<K>;
     constexpr int LW = G::BIG ? 32 : 16;
     const int k = lane % LW;
@@ -270,8 +301,28 @@ __device__ __forceinline__ void fx_put(const double (&rows)[FxRows<K>::N], doubl
         fx_digits(f, 0, q);
         if (k == 0) exps[r] = (short)e;
         if (k >= G::N2) continue;
+        if constexpr (G::BIG) {
+            if (r >= 16) {
+                __half *base = reinterpret_cast<__half *>(st);
+                auto put = [&](int tile, int a, int ks, int i) {  // digit i in row 4a + r - 16, slot ks
+                    const int R = 4 * a + r - 16;
+                    base[tile * 256 + ((R & 7) * 4 + ((ks & 7) >> 1)) * 8 + ((R >> 3) + 2 * (ks >> 3)) * 2 + (ks & 1)] =
+                        __ushort_as_half((unsigned short)q[i]);
+                };
+#pragma unroll
+                for (int d = 0; d < 7; d++)  // its weight
+#pragma unroll
+                    for (int j = 0; j <= d; j++) {  // the data's digit
+                        if (k < 16)
+                            put((d < 4 ? 0 : 4) + j, d & 3, k, d - j);
+                        else
+                            put(d < 4 ? 11 : j < 4 ? 12 : 13, d & 3, 4 * (j < 4 ? j : j == 4 ? 0 : j - 3) + k - 16, d - j);
+                    }
+            }
+        }
 #pragma unroll
         for (int u = 0; u < (U ? 2 : 1); u++) {
+            if (!U && r >= 16) continue;
             const bool second = u || r >= 16;
             const int rr = u ? (G::BIG ? (r < 8 ? 8 + r : r - 8) : r) : (r >= 16 ? r - 12 : r);
             if (u && (r >= K || k < K)) continue;
@@ -344,9 +395,10 @@ __global__ void __launch_bounds__(32 * K) op_to_fx_kernel(__grid_constant__ cons
             fsm[i] = exps ? 0x10001u * (uint32_t)(FX_NONE & 0xffff) : 0u;  // rows that there are not
         }
         __syncthreads();
-        fx_put<K, true>(rows, 1.0, warp, lane, fsm, fsm + G::TILEW, reinterpret_cast<short *>(fsm + G::X_EXP));
+        fx_put<K, true>(rows, 1.0, warp, lane, fsm + G::X_Y, fsm, fsm + G::X_Y + G::TILEW,
+                        reinterpret_cast<short *>(fsm + G::X_EXP));
         uint32_t *z = fsm + G::Z_OFF;
-        fx_put<K, false>(rows, J.op.c[t], warp, lane, z, z + G::TILEW, reinterpret_cast<short *>(z + G::Z_EXP));
+        fx_put<K, false>(rows, J.op.c[t], warp, lane, z, nullptr, z + G::TILEW, reinterpret_cast<short *>(z + G::Z_EXP));
         __syncthreads();
         for (int i = threadIdx.x; i < G::OP_WORDS / 4; i += 32 * K)
             reinterpret_cast<uint4 *>(out)[i] = reinterpret_cast<const uint4 *>(fsm)[i];
@@ -547,8 +599,8 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
                 s_pz[i] = reinterpret_cast<const uint32_t *>(L.az[sb + i]);
             }
             __syncthreads();
-            fx_copy(fsm + G::O_X, s_px[0], 2 * G::TILEW);
-            fx_copy(fsm + G::O_Y, s_py[0], G::YT * G::TILEW);
+            fx_copy(fsm + G::O_X, s_px[0], G::XW);
+            fx_copy(fsm + G::O_Y, s_py[0] + G::X_Y, G::YW);
             for (int i = tid; i < 32 * ni; i += G::THREADS) {
                 const int j = i >> 5, r = i & 31;
                 s_exx[j][r] = reinterpret_cast<const short *>(s_px[j] + G::X_EXP)[r];
@@ -575,12 +627,12 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
                     if (first) {
                         if (s_pz[j0] != lastz) {  // rows of one term and lz share A_z
                             lastz = s_pz[j0];
-                            fx_copy(fsm + G::O_Z, lastz, G::YT * G::TILEW);
+                            fx_copy(fsm + G::O_Z, lastz, G::YW);
                         }
                     }
                     const int exg = s_exx[j][g], exh = s_exx[j][8 + g], exq = s_exx[j][x2];
-                    const uint32_t *fx0 = fsm + G::O_X + (j & 1) * 2 * G::TILEW, *fx1 = fx0 + G::TILEW;
-                    if (j + 1 < ni) fx_copy(fsm + G::O_X + ((j + 1) & 1) * 2 * G::TILEW, s_px[j + 1], 2 * G::TILEW);
+                    const uint32_t *fx1 = fsm + G::O_X + (j & 1) * G::XW, *fx0 = fx1 + G::X_Y, *fxs = fx0 + G::TILEW;
+                    if (j + 1 < ni) fx_copy(fsm + G::O_X + ((j + 1) & 1) * G::XW, s_px[j + 1], G::XW);
 #pragma unroll 1
                     for (int tile = warp; tile < G::NTIN; tile += G::WARPS) {
                         B = Bn;  // the next tile's operand comes from L2 behind this one's products
@@ -622,7 +674,15 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
                             if (g + 8 * (r >> 1) < N2 && Y + (r & 1) < N2)
                                 add(T + (r & 1) * PX + g + 8 * (r >> 1), fx_value(D, r), r < 2 ? m0 : m1, r < 2 ? o0 : o1);
                         const bool has_u = !root && Z < K && Y < K;
-                        if constexpr (BIG) {
+                        if (BIG && (root || ti == 4 || 2 * gr + ti / 2 >= K)) {  // no column with u (the warp's tile as a whole)
+                            float E[3][4];
+                            fx_stack(E, fxs, B, lane);
+#pragma unroll
+                            for (int r = 0; r < 2; r++) {
+                                const long long v = fx_stack_value(E, r, g);
+                                if (g >= 4 && 12 + g < N2 && Y + r < N2) add(T + r * PX + 12 + g, v, m2, o2);
+                            }
+                        } else if constexpr (BIG) {
                             fx_tile<BIG>(D, fx1, B, lane);
 #pragma unroll
                             for (int r = 0; r < 2; r++) {
@@ -657,7 +717,7 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
                 fx_landed();
                 if (tid < 32) s_e1[par ^ 1][tid] = FX_NONE;
                 // y pass in place: a warp reads its 8 columns (Z, X') whole before it writes them
-                const uint32_t *fy0 = fsm + G::O_Y, *fy1 = fy0 + G::TILEW;
+                const uint32_t *fy0 = fsm + G::O_Y, *fys = fy0 + G::TILEW;
 #pragma unroll 1
                 for (int tile = warp; tile < G::NT; tile += G::WARPS) {
                     const int c = 8 * tile + g;
@@ -704,17 +764,20 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
                         if (Yq < N2 && 8 * tile + 2 * t + b < G::NC) s_t[Zr[b] * PZ + Yq * PX + Xr[b]] = fx_value(D, r);
                     }
                     if constexpr (BIG) {
-                        fx_tile<BIG>(D, fy1, B, lane);
+                        float E[3][4];
+                        fx_stack(E, fys, B, lane);
 #pragma unroll
-                        for (int b = 0; b < 2; b++)
+                        for (int b = 0; b < 2; b++) {
+                            const long long v = fx_stack_value(E, b, g);
                             if (g >= 4 && 12 + g < N2 && 8 * tile + 2 * t + b < G::NC)
-                                s_t[Zr[b] * PZ + (12 + g) * PX + Xr[b]] = fx_value(D, b);
+                                s_t[Zr[b] * PZ + (12 + g) * PX + Xr[b]] = v;
+                        }
                     }
                 }
                 fx_landed();  // T2 (and A_z)
-                if (j1 < ni) fx_copy(fsm + G::O_Y, s_py[j1], G::YT * G::TILEW);
+                if (j1 < ni) fx_copy(fsm + G::O_Y, s_py[j1] + G::X_Y, G::YW);
                 // z pass over this warp's column tiles
-                const uint32_t *fz0 = fsm + G::O_Z, *fz1 = fz0 + G::TILEW;
+                const uint32_t *fz0 = fsm + G::O_Z, *fzs = fz0 + G::TILEW;
                 const int ez0 = s_exz[j0][g], ez1 = s_exz[j0][8 + g], ez2 = g >= 4 && BIG ? s_exz[j0][12 + g] : FX_NONE;
 #pragma unroll 1
                 for (int q = 0; q < G::TPW; q++) {
@@ -733,9 +796,10 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
 #pragma unroll
                     for (int r = 0; r < 4; r++) v[r] = fx_value(D, r);
                     if constexpr (BIG) {
-                        fx_tile<BIG>(D, fz1, B, lane);
+                        float E[3][4];
+                        fx_stack(E, fzs, B, lane);
 #pragma unroll
-                        for (int r = 0; r < 2; r++) v[4 + r] = fx_value(D, r);
+                        for (int r = 0; r < 2; r++) v[4 + r] = fx_stack_value(E, r, g);
                     }
                     if (!root && nt < G::NTX) {  // scaling columns: the path without scaling-scaling where Z < K
                         const bool ins = c < K2;
@@ -857,7 +921,7 @@ size_t fx_op_words(int K) {
     }
 }
 
-size_t fx_op_z(int K) { return 2 * (7 * 128 + (K > 8 ? 10 * 128 : 0)) + 16; }  // FxGeo::Z_OFF
+size_t fx_op_z(int K) { return K > 8 ? FxGeo<10>::Z_OFF : FxGeo<8>::Z_OFF; }
 
 void k_op_to_fx(const FxOpJob *jobs, size_t n, int K, cudaStream_t s) {
     for (size_t at = 0; at < n; at += FxOpJobs::MAX) {
