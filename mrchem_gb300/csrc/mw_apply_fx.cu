@@ -10,10 +10,11 @@
 //
 // Why mma.sync and not tcgen05: an item needs ten accumulators (one per weight, two for the widest)
 // and its digits cut anew before each pass, and that integer work takes about as long as the tensor
-// pipe at mma.sync's rate (960 multiply-adds per SM and cycle, measured; 24 of 46 thousand SM cycles
+// pipe at mma.sync's rate (960 multiply-adds per SM and cycle, measured; 20 of 42 thousand SM cycles
 // per item at 2K = 20).  mma.sync's accumulator fragments turn into 62-bit numbers in the registers that
 // hold them; through TMEM every one of the ten would be read back by a second instruction stream.
-// Bound: issue slots, half of them for the digits (35 instructions per pair of numbers), then the pipe.
+// Bound: latency.  The products' pipe and the issue slots are each busy less than half of the time at four warps
+// per scheduler (registers); the warps wait for fixed-latency results, barriers and the pipe in turn.
 //
 // Layout (one CTA per task, 7 to 16 warps that share out the column tiles of every pass):
 //   x pass  T[Z][Y][X'] = sum_X Ax[X'][X] in[X][Y, Z]    input digits read as they lie in memory
@@ -28,10 +29,11 @@
 // operator rows in the x pass's second row tile, and the (Y' < K, X' < K) columns of the z pass take a
 // second operand whose Z < K part avoids that path.
 //
-// Measured on a full chip, ns per item without and with this kernel (apply_kernel's FP64 pipe first):
-// 2K = 20: 653, 147;  2K = 18: 444, 133;  2K = 16: 256, 46;  2K = 12: 91, 33.  With T in registers and the
-// operators' digits made per item 2K = 20 took 172 and 2K = 12 36.  Tier 3 of the 16-orbital Helmholtz batch
-// (22 thousand items, alone on the chip): 5.3 ms with their digits, 6.9 ms with the double-FP32 kernel it had.
+// Measured on a full chip, ns per item, apply_kernel's FP64 pipe first and then this kernel:
+// 2K = 20: 653, 134;  2K = 18: 444, 119;  2K = 16: 256, 40;  2K = 12: 91, 33.  With T in registers and the
+// operators' digits made per item 2K = 20 took 172 and 2K = 12 36; with a row tile of their own for rows
+// 16.. 2K = 20 took 147 and 2K = 18 133.  Tier 3 of the 16-orbital Helmholtz batch (22 thousand items, alone
+// on the chip): 5.3 ms with their digits, 6.9 ms with the double-FP32 kernel it had.
 //
 // K > 8: the contraction index is 16 + (2K - 16).  The remainder's digit pairs are folded: one MMA
 // carries four digit pairs of the same weight in its 16 k slots, 10 MMAs instead of 28.
@@ -58,15 +60,17 @@ constexpr int fx_pitch(int n) {  // n or a little more, 2 modulo 4: int64 rows 2
     return n;
 }
 // warps of a CTA: a divisor of the column tiles' number (50, 41, 32, 25, 18, 13, 8) with little left over, at
-// most 16 (128 registers)
-constexpr int fx_warps(int K) { return K == 10 ? 16 : K == 9 ? 14 : K == 8 ? 16 : K == 7 ? 13 : K == 6 ? 9 : K == 5 ? 7 : 8; }
+// most 16 (128 registers).  Two CTAs of 8 at 2K = 16: one's products run during the other's barriers (40 ns per item on a
+// full chip against 46 with one of 16; the FP64 Poisson apply alike).  Not at 2K = 18, 20, where shared memory
+// holds one CTA; 17 warps at 2K = 20 (no nearly empty last round) spill: 146 ns against 134.
+constexpr int fx_warps(int K) { return K == 10 ? 16 : K == 9 ? 14 : K == 8 ? 8 : K == 7 ? 13 : K == 6 ? 9 : K == 5 ? 7 : 8; }
 
 template <int K>
 struct FxGeo {
     static constexpr int N2 = 2 * K, NC = N2 * N2, K2 = K * K, K3 = K2 * K;
     static constexpr bool BIG = N2 > 16;              // contraction remainder and a second row tile
     static constexpr int WARPS = fx_warps(K), THREADS = 32 * WARPS;
-    static constexpr int MINB = K <= 6 ? 2 : 1;       // CTAs per SM that the registers are cut for
+    static constexpr int MINB = K == 8 || K <= 6 ? 2 : 1;  // CTAs per SM that the registers are cut for
     // column tiles of the x pass: Y = 0..7, 8..15 of every plane Z; K > 8: Y >= 16 of two planes together
     static constexpr int CT = N2 > 8 ? 2 : 1, GRP = BIG ? K : N2, TL = BIG ? 5 : CT, NTIN = GRP * TL;
     static constexpr int NT = (NC + 7) / 8;           // column tiles of the y and z passes
