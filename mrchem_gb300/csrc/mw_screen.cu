@@ -613,40 +613,40 @@ __global__ void gen_norms32_kernel(ScreenLevel P, int n) {
     if (i < n) P.gcn32[i] = (float)P.gcn[i];
 }
 
-// per tier: the nodes' first items (prefix sums in node order), the tiers one after the other
+// per tier: the nodes' first items (prefix sums in node order), the tiers one after the other.  All four
+// tiers' sums go through the rounds together (one tier after the other took 8.4 us for a few dozen nodes).
 __global__ void __launch_bounds__(1024) tier_offsets_kernel(ScreenLevel P) {
-    __shared__ long long wpart[32];
-    __shared__ long long s_base;
+    __shared__ long long wpart[32][4];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
-    if (tid == 0) s_base = 0;
-    __syncthreads();
-    for (int k = 0; k < 4; k++) {
-        long long run = s_base;
-        for (int q0 = 0; q0 < P.nn; q0 += blockDim.x) {
-            const int q = q0 + tid;
-            const long long v = q < P.nn ? P.tcnt[8 * (size_t)q + k] : 0;
-            long long x = v;
-            for (int o = 1; o < 32; o <<= 1) {
-                const long long y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
+    long long run[4] = {0, 0, 0, 0};
+    for (int q0 = 0; q0 < P.nn; q0 += blockDim.x) {
+        const int q = q0 + tid;
+        long long v[4], x[4];
+        for (int k = 0; k < 4; k++) x[k] = v[k] = q < P.nn ? P.tcnt[8 * (size_t)q + k] : 0;
+        for (int o = 1; o < 32; o <<= 1)
+            for (int k = 0; k < 4; k++) {
+                const long long y = __shfl_up_sync(0xffffffffu, x[k], o);
+                if (lane >= o) x[k] += y;
             }
-            if (lane == 31) wpart[w] = x;
-            __syncthreads();
+        if (lane == 31)
+            for (int k = 0; k < 4; k++) wpart[w][k] = x[k];
+        __syncthreads();
+        for (int k = 0; k < 4; k++) {
             long long before = 0, all = 0;
             for (int i = 0; i < nw; i++) {
-                if (i < w) before += wpart[i];
-                all += wpart[i];
+                if (i < w) before += wpart[i][k];
+                all += wpart[i][k];
             }
-            if (q < P.nn) P.tier_off[4 * (size_t)q + k] = run + x - v + before;
-            run += all;
-            __syncthreads();
-        }
-        if (tid == 0) {
-            P.tier_tot[k] = run - s_base;
-            s_base = run;
+            if (q < P.nn) P.tier_off[4 * (size_t)q + k] = run[k] + x[k] - v[k] + before;
+            run[k] += all;
         }
         __syncthreads();
     }
+    // the tiers' totals, known to all threads: the tiers' places
+    long long base[4] = {0, run[0], run[0] + run[1], run[0] + run[1] + run[2]};
+    if (tid < 4) P.tier_tot[tid] = run[tid];
+    for (int q = tid; q < P.nn; q += blockDim.x)
+        for (int k = 1; k < 4; k++) P.tier_off[4 * (size_t)q + k] += base[k];
 }
 
 // the tier kernels' item arrays: each node's items of a tier at its first item, in walk order
@@ -745,7 +745,7 @@ void k_screen_write(const ScreenLevel &P, int maxT, int zmax, cudaStream_t s) {
     const size_t sm = walk_smem(maxT, zmax, 1);
     if (sm > 40 * 1024) kernel_smem((const void *)screen_kernel<1>, (int)sm);
     screen_kernel<1><<<P.nn, ST, sm, s>>>(P, maxT, zmax);
-    tier_offsets_kernel<<<1, 1024, 0, s>>>(P);
+    tier_offsets_kernel<<<1, P.nn <= 128 ? 128 : P.nn <= 512 ? 512 : 1024, 0, s>>>(P);
 }
 
 void k_screen_fill(const ScreenLevel &P, cudaStream_t s) {
