@@ -96,25 +96,29 @@ __device__ void store_block(double *g, const double *cube, int K) {
     for (int gi = threadIdx.x; gi < n; gi += blockDim.x) g[gi] = cube[cube_of_block(gi, K)];
 }
 
-// 8 component norms of a block in global memory; deterministic fixed-order reduction
-// the 8 component norms of a block: per thread strided sums of squares, a butterfly sum per warp,
-// then the warps' sums in warp order (blockDim a multiple of 32; red holds 8 x warps doubles)
-__device__ void block_norms(const double *g, double *cn, int K, double *red) {
-    const int K3 = K * K * K, nt = blockDim.x, nw = nt >> 5, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int c = 0; c < 8; c++) {
-        double s = 0.0;
-        for (int i = threadIdx.x; i < K3; i += nt) {
-            const double v = g[c * K3 + i];
-            s += v * v;
+// The 8 component norms of a block in global memory, in a fixed order: a warp per component, strided sums of
+// squares with eight loads in flight and a butterfly sum (blockDim a multiple of 32).  Bound: latency.  All
+// threads on one component after another, and their warps' sums through shared memory, took 14.5 us a launch
+// at 2K = 16, this 6.6 us.
+__device__ void block_norms(const double *g, double *cn, int K) {
+    const int K3 = K * K * K, nw = blockDim.x >> 5, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int c = w; c < 8; c += nw) {
+        double s0 = 0.0, s1 = 0.0;
+        int i = lane;
+        for (; i + 224 < K3; i += 256) {
+            double v[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[j] = g[c * K3 + i + 32 * j];
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+                s0 += v[j] * v[j];
+                s1 += v[j + 1] * v[j + 1];
+            }
         }
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) red[c * nw + w] = s;
-    }
-    __syncthreads();
-    if (threadIdx.x < 8) {
-        double s = 0.0;
-        for (int i = 0; i < nw; i++) s += red[threadIdx.x * nw + i];
-        cn[threadIdx.x] = sqrt(s);
+        for (; i < K3; i += 32) s0 += g[c * K3 + i] * g[c * K3 + i];
+        s0 += s1;
+        for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+        if (lane == 0) cn[c] = sqrt(s0);
     }
     __syncthreads();
 }
@@ -178,7 +182,7 @@ __device__ double func_eval(const ProjFunc &f, double x, double y, double z) {
 __global__ void project_kernel(DevBasis b, ProjFunc f, const ProjTask *tasks, int n) {
     extern __shared__ double sm[];
     int K = b.K, N2 = 2 * K, C = N2 * N2 * N2;
-    double *cube = sm, *tmp = sm + C, *red = sm + 2 * C;
+    double *cube = sm, *tmp = sm + C;
     for (int t = blockIdx.x; t < n; t += gridDim.x) {
         ProjTask task = tasks[t];
         if (task.zero) {
@@ -203,7 +207,7 @@ __global__ void project_kernel(DevBasis b, ProjFunc f, const ProjTask *tasks, in
         cube_transform(cube, tmp, b.W, K);
         store_block(task.out, cube, K);
         __syncthreads();
-        block_norms(task.out, task.cn, K, red);
+        block_norms(task.out, task.cn, K);
     }
 }
 
@@ -769,8 +773,7 @@ void launch_apply_k(int K, const ApplyLaunch &L, int nsm, cudaStream_t s) {
 
 // ----------------------------------------------------------------- post-processing
 __global__ void norms_kernel(DevBasis b, double *const *blocks, double *const *cn, int n) {
-    extern __shared__ double sm[];
-    for (int t = blockIdx.x; t < n; t += gridDim.x) block_norms(blocks[t], cn[t], b.K, sm);
+    for (int t = blockIdx.x; t < n; t += gridDim.x) block_norms(blocks[t], cn[t], b.K);
 }
 
 __global__ void topdown_kernel(DevBasis b, const PairTask *tasks, int n) {
@@ -794,7 +797,7 @@ __global__ void topdown_kernel(DevBasis b, const PairTask *tasks, int n) {
 __global__ void compress_kernel(DevBasis b, const PairTask *tasks, double *const *cn, int n) {
     extern __shared__ double sm[];
     int K = b.K, N2 = 2 * K, C = N2 * N2 * N2, K3 = K * K * K;
-    double *cube = sm, *tmp = sm + C, *red = sm + 2 * C;
+    double *cube = sm, *tmp = sm + C;
     for (int t = blockIdx.x; t < n; t += gridDim.x) {
         PairTask task = tasks[t];
         for (int gi = threadIdx.x; gi < 8 * K3; gi += blockDim.x) {
@@ -805,13 +808,12 @@ __global__ void compress_kernel(DevBasis b, const PairTask *tasks, double *const
         cube_transform(cube, tmp, b.W, K);
         store_block(task.parent, cube, K);
         __syncthreads();
-        block_norms(task.parent, cn[t], K, red);
+        block_norms(task.parent, cn[t], K);
     }
 }
 
 __global__ void add_kernel(DevBasis b, const AddTask *tasks, const double *const *src, const double *coefs, int n,
                            int bs) {
-    extern __shared__ double sm[];
     for (int t = blockIdx.x; t < n; t += gridDim.x) {
         AddTask task = tasks[t];
         for (int i = threadIdx.x; i < bs; i += blockDim.x) {
@@ -820,7 +822,7 @@ __global__ void add_kernel(DevBasis b, const AddTask *tasks, const double *const
             task.out[i] = s;
         }
         __syncthreads();
-        block_norms(task.out, task.cn, b.K, sm);
+        block_norms(task.out, task.cn, b.K);
     }
 }
 
@@ -915,18 +917,39 @@ __global__ void scale_kernel(double *x, size_t n, double c) {
         x[i] *= c;
 }
 
-__global__ void dot_kernel(const double *const *a, const double *const *bb, const int *start, int n, int bs,
-                           double *partial) {
-    extern __shared__ double sm[];
+// <a|b> of node pairs from element `start` on; the pointers and the partial sums may be pinned host memory.
+// Bound: latency (a K = 8 node takes 1.2 us of an SM's FP64 pipe).  With a serial sum over 256 threads'
+// shares a launch over some 200 nodes of 2K = 16 took 21 us, with shuffles 8.8 us; one overlap, with its pairs found
+// by a joint walk in place of hash lookups and no copies, 50 -> 20 us.
+__global__ void __launch_bounds__(256) dot_kernel(const double *const *a, const double *const *bb, const int *start, int n,
+                                                  int bs, double *partial) {
+    __shared__ double s_w[8];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int t = blockIdx.x; t < n; t += gridDim.x) {
         const double *x = a[t], *y = bb[t];
-        double s = 0.0;
-        for (int i = start[t] + threadIdx.x; i < bs; i += blockDim.x) s += x[i] * y[i];
-        sm[threadIdx.x] = s;
+        double s0 = 0.0, s1 = 0.0;
+        int i = start[t] + threadIdx.x;
+        for (; i + 768 < bs; i += 1024) {
+            double u[4], v[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                u[j] = x[i + 256 * j];
+                v[j] = y[i + 256 * j];
+            }
+            s0 += u[0] * v[0];
+            s1 += u[1] * v[1];
+            s0 += u[2] * v[2];
+            s1 += u[3] * v[3];
+        }
+        for (; i < bs; i += 256) s0 += x[i] * y[i];
+        s0 += s1;
+        for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+        if (lane == 0) s_w[w] = s0;
         __syncthreads();
         if (threadIdx.x == 0) {
             double tot = 0.0;
-            for (int i = 0; i < (int)blockDim.x; i++) tot += sm[i];
+#pragma unroll
+            for (int k = 0; k < 8; k++) tot += s_w[k];
             partial[t] = tot;
         }
         __syncthreads();
@@ -981,7 +1004,7 @@ size_t cube_bytes(int K) { return sizeof(double) * 8 * K * K * K; }
 
 void k_project(const DevBasis &b, const ProjFunc &f, const ProjTask *tasks, int n, cudaStream_t s) {
     if (n <= 0) return;
-    size_t smem = 2 * cube_bytes(b.K) + 8 * 256 * sizeof(double);
+    size_t smem = 2 * cube_bytes(b.K);
     MWG_CUDA(cudaFuncSetAttribute(project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     project_kernel<<<grid_for(n), 256, smem, s>>>(b, f, tasks, n);
     MWG_CUDA(cudaGetLastError());
@@ -1013,7 +1036,7 @@ void k_apply(const DevBasis &b, const ApplyLaunch &L, int fp32, int nsm, cudaStr
 
 void k_norms(const DevBasis &b, double *const *blocks, double *const *cn, int n, cudaStream_t s) {
     if (n <= 0) return;
-    norms_kernel<<<grid_for(n), 256, 8 * 256 * sizeof(double), s>>>(b, blocks, cn, n);
+    norms_kernel<<<grid_for(n), 256, 0, s>>>(b, blocks, cn, n);
     MWG_CUDA(cudaGetLastError());
 }
 
@@ -1027,7 +1050,7 @@ void k_topdown(const DevBasis &b, const PairTask *tasks, int n, cudaStream_t s) 
 
 void k_compress(const DevBasis &b, const PairTask *tasks, double *const *cn, int n, cudaStream_t s) {
     if (n <= 0) return;
-    size_t smem = 2 * cube_bytes(b.K) + 8 * 256 * sizeof(double);
+    size_t smem = 2 * cube_bytes(b.K);
     kernel_smem((const void *)compress_kernel, (int)smem);
     compress_kernel<<<grid_for(n), 256, smem, s>>>(b, tasks, cn, n);
     MWG_CUDA(cudaGetLastError());
@@ -1053,7 +1076,7 @@ void k_gather_ranges(const double *const *src, const long long *off, const int *
 void k_add(const DevBasis &b, const AddTask *tasks, const double *const *src, const double *coefs, int n, int bs,
            cudaStream_t s) {
     if (n <= 0) return;
-    add_kernel<<<grid_for(n), 256, 8 * 256 * sizeof(double), s>>>(b, tasks, src, coefs, n, bs);
+    add_kernel<<<grid_for(n), 256, 0, s>>>(b, tasks, src, coefs, n, bs);
     MWG_CUDA(cudaGetLastError());
 }
 
@@ -1128,7 +1151,7 @@ void k_scale(double *x, size_t n, double c, cudaStream_t s) {
 void k_dot(const double *const *a, const double *const *b, const int *start, int n, int bs, double *partial,
            cudaStream_t s) {
     if (n <= 0) return;
-    dot_kernel<<<grid_for(n), 256, 256 * sizeof(double), s>>>(a, b, start, n, bs, partial);
+    dot_kernel<<<grid_for(n), 256, 0, s>>>(a, b, start, n, bs, partial);
     MWG_CUDA(cudaGetLastError());
 }
 

@@ -1200,32 +1200,27 @@ void crop(Tree &t, double prec, bool abs_prec, Arena &arena) {
 double dot(const Tree &a, const Tree &b, Arena &arena) {
     Ctx &ctx = *a.ctx;
     int K3 = ctx.basis.K * ctx.basis.K * ctx.basis.K;
-    std::vector<const double *> pa, pb;
-    std::vector<int> start;
-    for (int i = 0; i < a.nn(); i++) {
-        const NodeInfo &nd = a.nodes[i];
-        int j = b.find(nd.n, nd.l);
-        if (j < 0) continue;
-        pa.push_back(a.block(i));
-        pb.push_back(b.block(j));
-        start.push_back(nd.n == ctx.basis.n0 ? 0 : K3);
-    }
-    int n = (int)pa.size();
-    if (n == 0) return 0.0;
+    // the pairs and the partial sums lie in pinned memory, which the kernel reads and writes in place: a
+    // call is one launch and one wait
+    const std::vector<int> m = match_nodes(a, b);
     arena.reset();
-    Packer pk;
-    pk.add(pa.data(), n * sizeof(double *));
-    pk.add(pb.data(), n * sizeof(double *));
-    pk.add(start.data(), n * sizeof(int));
-    pk.ship(ctx, arena);
-    double *part = (double *)arena.alloc(sizeof(double) * n);
-    k_dot((const double *const *)pk.ptr(0), (const double *const *)pk.ptr(1), (const int *)pk.ptr(2), n, ctx.basis.bs,
-          part, ctx.stream);
-    std::vector<double> h(n);
-    MWG_CUDA(cudaMemcpyAsync(h.data(), part, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx.stream));
+    const size_t most = m.size();
+    const double **pa = (const double **)arena.halloc(3 * sizeof(double *) * most + sizeof(int) * most);
+    const double **pb = pa + most;
+    double *part = (double *)(pb + most);
+    int *start = (int *)(part + most);
+    int n = 0;
+    for (int i = 0; i < a.nn(); i++) {
+        if (m[i] < 0) continue;
+        pa[n] = a.block(i);
+        pb[n] = b.block(m[i]);
+        start[n++] = a.nodes[i].n == ctx.basis.n0 ? 0 : K3;
+    }
+    if (n == 0) return 0.0;
+    k_dot(pa, pb, start, n, ctx.basis.bs, part, ctx.stream);
     ctx.sync();
     double s = 0.0;
-    for (double v : h) s += v;
+    for (int t = 0; t < n; t++) s += part[t];
     return s;
 }
 
