@@ -440,49 +440,6 @@ struct DevScreen {
     cudaEvent_t ev_counts = nullptr;  // the write pass's per-node tier counts have reached the host
 };
 
-// layout of Oper::d_screen: int band[TS], off[TS], first[TS] | double amax[TS], xmax[TS], c[T], norms[4 nb]
-// | float amax32[TS], xmax32[TS], norms32[4 nb]   (TS = T * S, nb = blocks)
-struct OperScreenLayout {
-    size_t TS, nb, ib, db, fb;
-    explicit OperScreenLayout(const Oper &op) {
-        TS = (size_t)op.T * op.S;
-        nb = (size_t)std::max<long>(op.nblocks, 1);
-        ib = ((3 * TS * sizeof(int)) + 255) & ~size_t(255);
-        db = ((sizeof(double) * (2 * TS + (size_t)op.T + 4 * nb)) + 255) & ~size_t(255);
-        fb = sizeof(float) * (2 * TS + 4 * nb);
-    }
-};
-
-bool oper_screen_tables(Oper &op) {
-    if (op.d_screen) return true;
-    const OperScreenLayout ly(op);
-    const size_t TS = ly.TS;
-    for (size_t i = 0; i < TS; i++)
-        if (op.band[i] > 32767 || op.off[i] > 0x3fffffffL) return false;
-    if (op.nblocks > 0x3fffffffL) return false;
-    std::vector<char> h(ly.ib + ly.db + ly.fb, 0);
-    int *iv = (int *)h.data();
-    double *dd = (double *)(h.data() + ly.ib);
-    float *ff = (float *)(h.data() + ly.ib + ly.db);
-    for (size_t i = 0; i < TS; i++) {
-        iv[i] = op.band[i];
-        iv[TS + i] = (int)op.off[i];
-        iv[2 * TS + i] = op.fx_first[i];
-        dd[i] = op.amax[i];
-        dd[TS + i] = op.xmax[i];
-        ff[i] = (float)op.amax[i];
-        ff[TS + i] = (float)op.xmax[i];
-    }
-    for (int t = 0; t < op.T; t++) dd[2 * TS + t] = op.c[t];
-    for (size_t i = 0; i < op.norms.size(); i++) {
-        dd[2 * TS + op.T + i] = op.norms[i];
-        ff[2 * TS + i] = (float)op.norms[i];
-    }
-    MWG_CUDA(cudaMalloc(&op.d_screen, h.size()));
-    MWG_CUDA(cudaMemcpy(op.d_screen, h.data(), h.size(), cudaMemcpyHostToDevice));
-    return true;
-}
-
 ScreenOp oper_screen_view(const Oper &op) {
     const OperScreenLayout ly(op);
     const size_t TS = ly.TS;
@@ -518,7 +475,7 @@ struct FxLevelOps {
     int s = 0;
     bool add(Oper &op, Arena &ar) {
         if (base.count(&op)) return true;
-        if (!oper_screen_tables(op)) return false;
+        if (!op.d_screen) return false;
         const int n = op.fx_count[s];
         uint32_t *b = (uint32_t *)ar.alloc(sizeof(uint32_t) * words * (size_t)std::max(n, 1));
         base.emplace(&op, b);
@@ -696,7 +653,7 @@ bool screen_setup(Ctx &ctx, std::vector<ApplyJob> &jobs, const std::vector<JobSt
         ds.levels++;
     }
     for (ApplyJob &job : jobs)
-        if (!oper_screen_tables(*job.op)) return false;
+        if (!job.op->d_screen) return false;
     for (ApplyJob &job : jobs) {
         ds.op_max.push_back(oper_norm_max(*job.op));
         ds.maxT = std::max(ds.maxT, job.op->T);
@@ -2320,7 +2277,7 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
     const size_t fxw = fx_words(b.K);
     uint32_t *yfx = nullptr;
     ctx.sarena.reset();
-    fixed_point = fixed_point && oper_screen_tables(op) && ctx.sarena.room_for(sizeof(uint32_t) * fxw * (size_t)y.nn());
+    fixed_point = fixed_point && op.d_screen && ctx.sarena.room_for(sizeof(uint32_t) * fxw * (size_t)y.nn());
     if (fixed_point) {
         yfx = (uint32_t *)ctx.sarena.alloc(sizeof(uint32_t) * fxw * (size_t)y.nn());
         const FxBlocks ys{y.d_coefs, yfx, (size_t)y.nn()};

@@ -272,7 +272,10 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
     std::vector<int> base(ops.size() + 1, 0);
     for (size_t o = 0; o < ops.size(); o++) base[o + 1] = base[o] + ops[o]->T * ops[o]->S;
     const int ntask = base.back();
-    std::vector<OpBuildTask> tasks(ntask);
+    // what goes to and comes from the device lies in the context's pinned memory
+    Arena &arena = cx.arena;
+    arena.reset();
+    OpBuildTask *tasks = (OpBuildTask *)arena.halloc(sizeof(OpBuildTask) * (size_t)ntask);
     long nrm_total = 0;
     for (size_t o = 0; o < ops.size(); o++) {
         const Oper &op = *ops[o];
@@ -310,26 +313,25 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
     std::copy(cc.gw, cc.gw + 16, q + 16);
     MWG_CUDA(cudaMemcpyAsync(d_cc, cc.coef.data(), sizeof(double) * cc.coef.size(), cudaMemcpyHostToDevice, st));
     MWG_CUDA(cudaMemcpyAsync(d_q, q, sizeof(q), cudaMemcpyHostToDevice, st));
-    MWG_CUDA(cudaMemcpyAsync(d_tasks, tasks.data(), sizeof(OpBuildTask) * ntask, cudaMemcpyHostToDevice, st));
+    MWG_CUDA(cudaMemcpyAsync(d_tasks, tasks, sizeof(OpBuildTask) * ntask, cudaMemcpyHostToDevice, st));
     k_op_band(K, cx.dbasis.W, d_cc, d_q, d_q + 16, d_tasks, ntask, d_nrm, d_head, d_band, d_peak, d_keep, cx.nsm, st);
-    std::vector<int> walked(ntask);
-    std::vector<double> peak(ntask), head((size_t)ntask * 4 * OP_NRM_HEAD);
-    MWG_CUDA(cudaMemcpyAsync(walked.data(), d_band, sizeof(int) * ntask, cudaMemcpyDeviceToHost, st));
-    MWG_CUDA(cudaMemcpyAsync(peak.data(), d_peak, sizeof(double) * ntask, cudaMemcpyDeviceToHost, st));
-    MWG_CUDA(cudaMemcpyAsync(head.data(), d_head, sizeof(double) * head.size(), cudaMemcpyDeviceToHost, st));
+    int *walked = (int *)arena.halloc(sizeof(int) * (size_t)ntask);
+    double *peak = (double *)arena.halloc(sizeof(double) * (size_t)ntask);
+    double *head = (double *)arena.halloc(sizeof(double) * (size_t)ntask * 4 * OP_NRM_HEAD);
+    MWG_CUDA(cudaMemcpyAsync(walked, d_band, sizeof(int) * ntask, cudaMemcpyDeviceToHost, st));
+    MWG_CUDA(cudaMemcpyAsync(peak, d_peak, sizeof(double) * ntask, cudaMemcpyDeviceToHost, st));
+    MWG_CUDA(cudaMemcpyAsync(head, d_head, sizeof(double) * (size_t)ntask * 4 * OP_NRM_HEAD, cudaMemcpyDeviceToHost, st));
     MWG_CUDA(cudaStreamSynchronize(st));
     // the walked norms: the first OP_NRM_HEAD translations of every task came in one copy, longer
     // walks are fetched one by one
-    std::vector<std::vector<double>> pnr(ntask);
+    std::vector<double *> pnr(ntask);
     bool fetch = false;
     for (int i = 0; i < ntask; i++) {
-        pnr[i].resize(4 * (size_t)(walked[i] + 1));
-        if (walked[i] < OP_NRM_HEAD) {
-            std::copy(&head[(size_t)i * 4 * OP_NRM_HEAD], &head[(size_t)i * 4 * OP_NRM_HEAD] + pnr[i].size(),
-                      pnr[i].begin());
-        } else {
-            MWG_CUDA(cudaMemcpyAsync(pnr[i].data(), d_nrm + tasks[i].nrm_off, sizeof(double) * pnr[i].size(),
-                                     cudaMemcpyDeviceToHost, st));
+        pnr[i] = head + (size_t)i * 4 * OP_NRM_HEAD;
+        if (walked[i] >= OP_NRM_HEAD) {
+            const size_t bytes = sizeof(double) * 4 * (size_t)(walked[i] + 1);
+            pnr[i] = (double *)arena.halloc(bytes);
+            MWG_CUDA(cudaMemcpyAsync(pnr[i], d_nrm + tasks[i].nrm_off, bytes, cudaMemcpyDeviceToHost, st));
             fetch = true;
         }
     }
@@ -337,17 +339,20 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
     // per operator: band cut (sub-blocks below NS_CLEAN x the (t, n) peak are zeroed, and a term
     // with no scaling-wavelet, wavelet-scaling or wavelet-wavelet sub-block left is inactive at
     // n), block offsets, host norm tables, device allocations and phase 2 jobs
-    std::vector<OpBlockJob> jobs;
+    std::vector<std::vector<std::vector<int>>> zero(ops.size());
+    std::vector<long> first_job(ops.size() + 1, 0);
+#pragma omp parallel for schedule(dynamic, 1) if (ops.size() > 1)
     for (size_t o = 0; o < ops.size(); o++) {
         Oper &op = *ops[o];
         const int nt = op.T * op.S;
         op.band.assign(nt, -1);
         op.off.assign(nt, 0);
-        std::vector<std::vector<int>> zero(nt);
+        zero[o].resize(nt);
+        long njob = 0;
         for (int i = 0; i < nt; i++) {
             const int g0 = base[o] + i;
             int L = walked[g0];
-            zero[i].assign(L + 1, 0);
+            zero[o][i].assign(L + 1, 0);
             if (!tasks[g0].root) {
                 bool active = false;
                 for (int l = 0; l <= L; l++)
@@ -356,7 +361,7 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
                             double &v = pnr[g0][4 * l + 2 * g + f];
                             if (v < NS_CLEAN * peak[g0]) {
                                 v = 0.0;
-                                zero[i][l] |= 1 << (2 * g + f);
+                                zero[o][i][l] |= 1 << (2 * g + f);
                             } else if (g + f > 0) {
                                 active = true;
                             }
@@ -364,7 +369,9 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
                 if (!active) L = -1;
             }
             op.band[i] = L;
+            njob += L + 1;
         }
+        first_job[o + 1] = njob;
         op.nblocks = 0;
         for (int i = 0; i < nt; i++) {
             op.off[i] = op.nblocks;
@@ -380,9 +387,6 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
         op.norms.assign((size_t)std::max<long>(op.nblocks, 1) * 4, 0.0);
         op.amax.assign(nt, 0.0);
         op.xmax.assign(nt, 0.0);
-        const size_t nel = (size_t)std::max<long>(op.nblocks, 1) * bsz;
-        MWG_CUDA(cudaMalloc(&op.d_blocks, sizeof(double) * nel));
-        MWG_CUDA(cudaMemsetAsync(op.d_blocks, 0, sizeof(double) * nel, st));
         for (int i = 0; i < nt; i++) {
             const int L = op.band[i];
             if (L < 0) continue;
@@ -403,23 +407,80 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
                     if (k > 0) op.xmax[i] = std::max(op.xmax[i], dn[k]);
                 }
             }
-            for (int l = 0; l <= L; l++) jobs.push_back(OpBlockJob{g0, l, L, zero[i][l], op.off[i], op.d_blocks});
         }
     }
-    if (!jobs.empty()) {
-        MWG_CUDA(cudaMallocAsync(&d_jobs, sizeof(OpBlockJob) * jobs.size(), st));
-        MWG_CUDA(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(OpBlockJob) * jobs.size(), cudaMemcpyHostToDevice, st));
-        k_op_blocks(K, cx.dbasis.W, d_cc, d_q, d_q + 16, d_tasks, d_jobs, (int)jobs.size(), d_keep, st);
+    for (size_t o = 0; o < ops.size(); o++) {
+        first_job[o + 1] += first_job[o];
+        const size_t nel = (size_t)std::max<long>(ops[o]->nblocks, 1) * bsz;
+        // the operators' own memory, from the same pool (a device allocation per array took half of a
+        // batch's construction and release)
+        MWG_CUDA(cudaMallocAsync(&ops[o]->d_blocks, sizeof(double) * nel, st));
+        if (ops[o]->nblocks == 0) MWG_CUDA(cudaMemsetAsync(ops[o]->d_blocks, 0, sizeof(double) * nel, st));
+    }
+    const size_t njobs = (size_t)first_job.back();
+    if (njobs > 0) {
+        OpBlockJob *jobs = (OpBlockJob *)arena.halloc(sizeof(OpBlockJob) * njobs);
+#pragma omp parallel for schedule(dynamic, 1) if (ops.size() > 1)
+        for (size_t o = 0; o < ops.size(); o++) {
+            const Oper &op = *ops[o];
+            OpBlockJob *j = jobs + first_job[o];
+            for (int i = 0; i < op.T * op.S; i++)
+                for (int l = 0; l <= op.band[i]; l++)
+                    *j++ = OpBlockJob{base[o] + i, l, op.band[i], zero[o][i][l], op.off[i], op.d_blocks};
+        }
+        MWG_CUDA(cudaMallocAsync(&d_jobs, sizeof(OpBlockJob) * njobs, st));
+        MWG_CUDA(cudaMemcpyAsync(d_jobs, jobs, sizeof(OpBlockJob) * njobs, cudaMemcpyHostToDevice, st));
+        k_op_blocks(K, cx.dbasis.W, d_cc, d_q, d_q + 16, d_tasks, d_jobs, (int)njobs, d_keep, st);
+    }
+    // the screening's tables (not for bands or block numbers beyond its fields: screened on the host)
+    std::vector<char *> stage(ops.size(), nullptr);
+    for (size_t o = 0; o < ops.size(); o++) {
+        Oper &op = *ops[o];
+        bool fits = op.nblocks <= 0x3fffffffL;
+        for (size_t i = 0; i < op.band.size(); i++) fits = fits && op.band[i] <= 32767 && op.off[i] <= 0x3fffffffL;
+        if (!fits) continue;
+        const OperScreenLayout ly(op);
+        stage[o] = (char *)arena.halloc(ly.ib + ly.db + ly.fb);
+        MWG_CUDA(cudaMallocAsync(&op.d_screen, ly.ib + ly.db + ly.fb, st));
+    }
+#pragma omp parallel for schedule(dynamic, 1) if (ops.size() > 1)
+    for (size_t o = 0; o < ops.size(); o++) {
+        if (!stage[o]) continue;
+        const Oper &op = *ops[o];
+        const OperScreenLayout ly(op);
+        const size_t TS = ly.TS;
+        int *iv = (int *)stage[o];
+        double *dd = (double *)(stage[o] + ly.ib);
+        float *ff = (float *)(stage[o] + ly.ib + ly.db);
+        for (size_t i = 0; i < TS; i++) {
+            iv[i] = op.band[i];
+            iv[TS + i] = (int)op.off[i];
+            iv[2 * TS + i] = op.fx_first[i];
+            dd[i] = op.amax[i];
+            dd[TS + i] = op.xmax[i];
+            ff[i] = (float)op.amax[i];
+            ff[TS + i] = (float)op.xmax[i];
+        }
+        for (int t = 0; t < op.T; t++) dd[2 * TS + t] = op.c[t];
+        for (size_t i = 0; i < op.norms.size(); i++) {
+            dd[2 * TS + op.T + i] = op.norms[i];
+            ff[2 * TS + i] = (float)op.norms[i];
+        }
+    }
+    for (size_t o = 0; o < ops.size(); o++) {
+        if (!stage[o]) continue;
+        const OperScreenLayout ly(*ops[o]);
+        MWG_CUDA(cudaMemcpyAsync(ops[o]->d_screen, stage[o], ly.ib + ly.db + ly.fb, cudaMemcpyHostToDevice, st));
     }
     // device copies for the reduced tiers: FP32 high part then low part per block (FP32
     // tier), and the tensor-core tier's B operand (mw_tc05_layout.h)
     const bool tc = K >= 4 && K <= KMAX;
     for (Oper *op : ops) {
         const long nb = std::max<long>(op->nblocks, 1);
-        MWG_CUDA(cudaMalloc(&op->d_blocks32, sizeof(float) * 2 * (size_t)nb * bsz));
+        MWG_CUDA(cudaMallocAsync(&op->d_blocks32, sizeof(float) * 2 * (size_t)nb * bsz, st));
         if (tc) {
-            MWG_CUDA(cudaMalloc(&op->d_blocks_tc, sizeof(float) * tc5_b_stride(K) * (size_t)nb));
-            if (tc5_split_wide(K)) MWG_CUDA(cudaMalloc(&op->d_blocks_tc2, sizeof(float) * tc5_b_stride(K) * (size_t)nb));
+            MWG_CUDA(cudaMallocAsync(&op->d_blocks_tc, sizeof(float) * tc5_b_stride(K) * (size_t)nb, st));
+            if (tc5_split_wide(K)) MWG_CUDA(cudaMallocAsync(&op->d_blocks_tc2, sizeof(float) * tc5_b_stride(K) * (size_t)nb, st));
         }
         k_op_convert(op->d_blocks, op->d_blocks32, tc ? op->d_blocks_tc : nullptr, op->d_blocks_tc2, nb,
                      K, tc5_n(K), 2 * tc5_ks(K), st);
@@ -428,14 +489,13 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
                      (void *)d_jobs, (void *)d_head, (void *)d_keep})
         if (pp) cudaFreeAsync(pp, st);
     MWG_CUDA(cudaStreamSynchronize(st));
+    arena.reset();
 }
 
+// stream-ordered: calls on a context have ended on all of its streams when they return
 void Oper::free_device() {
-    if (d_blocks) cudaFree(d_blocks);
-    if (d_blocks32) cudaFree(d_blocks32);
-    if (d_blocks_tc) cudaFree(d_blocks_tc);
-    if (d_blocks_tc2) cudaFree(d_blocks_tc2);
-    if (d_screen) cudaFree(d_screen);
+    for (void *p : {(void *)d_blocks, (void *)d_blocks32, (void *)d_blocks_tc, (void *)d_blocks_tc2, d_screen})
+        if (p) cudaFreeAsync(p, ctx->stream);
     d_blocks = nullptr;
     d_blocks32 = nullptr;
     d_blocks_tc = nullptr;

@@ -144,6 +144,19 @@ struct Oper {
     long block_index(int t, int s, int l) const { return off[t * S + s] + l + band[t * S + s]; }
     void build(const Basis &b);  // build_operators({this}, b)
 };
+
+// layout of Oper::d_screen: int band[TS], off[TS], first[TS] | double amax[TS], xmax[TS], c[T], norms[4 nb]
+// | float amax32[TS], xmax32[TS], norms32[4 nb]   (TS = T * S, nb = blocks)
+struct OperScreenLayout {
+    size_t TS, nb, ib, db, fb;
+    explicit OperScreenLayout(const Oper &op) {
+        TS = (size_t)op.T * op.S;
+        nb = (size_t)std::max<long>(op.nblocks, 1);
+        ib = ((3 * TS * sizeof(int)) + 255) & ~size_t(255);
+        db = ((sizeof(double) * (2 * TS + (size_t)op.T + 4 * nb)) + 255) & ~size_t(255);
+        fb = sizeof(float) * (2 * TS + 4 * nb);
+    }
+};
 // several operators of one context at once (mw_basis.cpp)
 void build_operators(const std::vector<Oper *> &ops, const Basis &b);
 

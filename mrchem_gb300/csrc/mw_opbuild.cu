@@ -31,7 +31,8 @@ struct ObShared {
     static constexpr int N2 = 2 * K;
     double P[OB_UNIT][N2 + 1];  // P_p(2z-1) at the points of 8 panels on [0, 1]; an odd pitch
     double W[N2 * N2];
-    double G[4][N2];            // moments
+    double G[3][N2];            // moments of 2l-1, 2l, 2l+1
+    double H[4][N2];            // two moments, each in halves
     double tm1[K * K], t0[K * K], tp1[K * K];
     double T1[N2 * N2], ns[N2 * N2];
     double nrm[4];
@@ -47,11 +48,12 @@ __device__ __forceinline__ void ob_legendre(double t, double (&P)[N2]) {
     for (int j = 1; j + 1 < N2; j++) P[j + 1] = ((2.0 * j + 1.0) / (j + 1.0)) * t * P[j] - (j / (j + 1.0)) * P[j - 1];
 }
 
-// One warp: S.G[slot][p] = int_0^1 P_p(2z-1) exp(-beta (z + l)^2) dz.  The lanes share the points out and
-// their partial sums are added by butterflies, a fixed order.  A kernel wide enough for 8 panels on all of
-// [0, 1] takes its Legendre values from the table.
+// One warp: half the points' share of G_m[p] = int_0^1 P_p(2z-1) exp(-beta (z + m)^2) dz, to S.H[slot].  The
+// lanes share the points out; their partial sums are added by a fixed order of exchanges, after each of
+// which a lane keeps half of the values, so that lane p ends with the sum for p.  A kernel wide enough for 8
+// panels on all of [0, 1] takes its Legendre values from the table.
 template <int K>
-__device__ void ob_moments(double beta, double l, int slot, ObShared<K> &S) {
+__device__ void ob_moments(double beta, double l, int half, int slot, ObShared<K> &S) {
     constexpr int N2 = 2 * K;
     const int lane = threadIdx.x & 31;
     double acc[N2];
@@ -64,7 +66,7 @@ __device__ void ob_moments(double beta, double l, int slot, ObShared<K> &S) {
         const int npc = (int)ceil((hi - lo) / pw);
         const double step = (hi - lo) / npc;
         const bool unit = npc == 8 && lo == 0.0 && hi == 1.0;
-        for (int i = lane; i < npc * OB_QPTS; i += 32) {
+        for (int i = 32 * half + lane; i < npc * OB_QPTS; i += 64) {
             const int k = i / OB_QPTS, q = i - k * OB_QPTS;
             const double z = (lo + k * step) + step * S.gx[q], e = beta * (z + l) * (z + l);
             if (e > 745.0) continue;
@@ -81,23 +83,50 @@ __device__ void ob_moments(double beta, double l, int slot, ObShared<K> &S) {
         }
     }
 #pragma unroll
-    for (int p = 0; p < N2; p++) {
-        for (int o = 16; o > 0; o >>= 1) acc[p] += __shfl_xor_sync(0xffffffffu, acc[p], o);
-        if (lane == 0) S.G[slot][p] = acc[p];
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int j = 0; j < o; j++) {
+            if (j >= N2) continue;
+            const double high = j + o < N2 ? acc[(j + o) % N2] : 0.0;
+            const double got = __shfl_xor_sync(0xffffffffu, up ? acc[j] : high, o);
+            acc[j] = (up ? high : acc[j]) + got;
+        }
     }
+    if (lane < N2) S.H[slot][lane] = acc[0];
 }
 
-// out = tau(m) (K x K) from the moments of +m (slot gp) and -m (slot gm); tau(-m) is its transpose
+// All threads: S.G[1] = G_m and S.G[2] = G_{m+1}, S.G[0] = the last S.G[2].  Two warps per moment.
 template <int K>
-__device__ __forceinline__ void ob_tau(double pref, const double *cc, const ObShared<K> &S, int gp, int gm, double *out) {
+__device__ void ob_pair(double beta, int m, ObShared<K> &S) {
+    const int q = threadIdx.x >> 5, p = threadIdx.x;
+    ob_moments<K>(beta, (double)(m + (q >> 1)), q & 1, q, S);
+    __syncthreads();
+    if (p < 2 * K) {
+        S.G[0][p] = S.G[2][p];
+        S.G[1][p] = S.H[0][p] + S.H[1][p];
+        S.G[2][p] = S.H[2][p] + S.H[3][p];
+    }
+    __syncthreads();
+}
+
+// out = tau(m) (K x K) from the moments of m and -m, each as it is or (odd) its mirror image: with z -> 1 - z,
+// G_{-m}[p] = (-1)^p G_{m-1}[p]
+template <int K>
+__device__ __forceinline__ void ob_tau(double pref, const double *cc, const double *gp, bool odd_p, const double *gm,
+                                       bool odd_m, double *out) {
     constexpr int N2 = 2 * K;
     for (int e = threadIdx.x; e < K * K; e += OB_THREADS) {
         const int i = e / K, j = e - i * K;
         const double *aij = cc + (size_t)(i * K + j) * N2, *aji = cc + (size_t)(j * K + i) * N2;
-        double v = 0.0;
+        double even = 0.0, up = 0.0, um = 0.0;  // even p, odd p of both
 #pragma unroll
-        for (int p = 0; p < N2; p++) v += __ldg(aij + p) * S.G[gp][p] + __ldg(aji + p) * S.G[gm][p];
-        out[e] = pref * v;
+        for (int p = 0; p < N2; p += 2) {
+            even += __ldg(aij + p) * gp[p] + __ldg(aji + p) * gm[p];
+            up += __ldg(aij + p + 1) * gp[p + 1];
+            um += __ldg(aji + p + 1) * gm[p + 1];
+        }
+        out[e] = pref * (even + ((odd_p ? -up : up) + (odd_m ? -um : um)));
     }
 }
 
@@ -154,34 +183,32 @@ __device__ void ob_setup(const double *W, const double *gx, const double *gw, Ob
     __syncthreads();
 }
 
-// tau(2l-1), tau(2l), tau(2l+1) of block l; `next`: tau(2l-1) is the last block's tau(2l+1).  A warp per
-// moment: at l = 0 those of 0, 1 and -1, else of +-2l and +-(2l+1) (and, not `next`, +-(2l-1)).
+// tau(2l-1), tau(2l), tau(2l+1) of block l; `next`: the last block was l - 1, whose tau(2l+1) and moment are
+// this one's tau(2l-1) and G_{2l-1}.  Two moments per block: those of -2l and -(2l+1) are the mirror images of
+// G_{2l-1} and G_{2l}.
 template <int K>
 __device__ void ob_taus(const OpBuildTask &T, int l, bool next, const double *cc, ObShared<K> &S) {
-    const int q = threadIdx.x >> 5;
     if (l > 0) {
         if (next) {
             for (int e = threadIdx.x; e < K * K; e += OB_THREADS) S.tm1[e] = S.tp1[e];
         } else {
-            if (q < 2) ob_moments<K>(T.beta, q ? 1.0 - 2.0 * l : 2.0 * l - 1.0, q, S);
-            __syncthreads();
-            ob_tau<K>(T.pref, cc, S, 0, 1, S.tm1);
+            ob_pair<K>(T.beta, 2 * l - 2, S);
+            ob_tau<K>(T.pref, cc, S.G[2], false, S.G[1], true, S.tm1);
             __syncthreads();
         }
     }
-    const int m = 2 * l + (q >> 1);  // warps: 2l, -2l, 2l+1, -(2l+1)
-    if (m > 0 || q == 0) ob_moments<K>(T.beta, q & 1 ? -(double)m : (double)m, q, S);
-    __syncthreads();
-    ob_tau<K>(T.pref, cc, S, 0, l > 0 ? 1 : 0, S.t0);
-    ob_tau<K>(T.pref, cc, S, 2, 3, S.tp1);
-    if (l == 0) ob_tau<K>(T.pref, cc, S, 3, 2, S.tm1);
+    ob_pair<K>(T.beta, 2 * l, S);
+    ob_tau<K>(T.pref, cc, S.G[1], false, l > 0 ? S.G[0] : S.G[1], l > 0, S.t0);
+    ob_tau<K>(T.pref, cc, S.G[2], false, S.G[1], true, S.tp1);
+    if (l == 0) ob_tau<K>(T.pref, cc, S.G[1], true, S.G[2], false, S.tm1);
     __syncthreads();
 }
 
 // Phase 1: per task the sub-block norms of NS(0..L) and L, where the walk stops; the blocks themselves for
 // l < OP_KEEP, which most walks do not pass.  Persistent CTAs.  Bound: the FP64 pipe (per block 2 (2K)^3
-// multiply-adds for W tau W^T, 8 K^3 for the two taus, and per moment 128 points of an exponential and 2K
-// multiply-adds); one warp per moment, the Legendre table and the butterfly sums leave little else.
+// multiply-adds for W tau W^T, 8 K^3 for the two taus, and two moments of at most 128 points with an exponential
+// and 2K multiply-adds each).  8 Helmholtz operators of order 9: 3.8 ms; 5.4 ms with the moments of negative
+// translations computed too and every lane adding every partial sum.
 template <int K>
 __global__ void __launch_bounds__(OB_THREADS) op_band_kernel(const double *W, const double *cc, const double *gx,
                                                              const double *gw, const OpBuildTask *tasks, int ntask,
