@@ -5,6 +5,7 @@
 // is staged as the (2K)^3 "cube" cube[Z][Y][X] with X = cx*K + ix, so a
 // multiwavelet transform or a non-standard-form operator application is three
 // 2K x 2K matrix passes, one per dimension.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -310,115 +311,169 @@ __global__ void __launch_bounds__(128) generate_kernel(DevBasis b, const GenTask
     }
 }
 
-// The same generation with K known at compile time: the filter matrix and the three
-// intermediates in shared memory (56 KB at K = 10, four CTAs per SM), the loops unrolled.  The
-// sums run in the same order as in generate_kernel, so the blocks and norms are identical.
+// The same generation with K known at compile time.  Bound: the FP64 pipe (14 K^4 multiply-adds for the step
+// out of a full block, 3 K^4 for each further one), so a task is shared out over a cluster of (K + 1) / 2 CTAs:
+// contracting Z first makes every pass of a CTA work for its own two output planes z alone.  A further step
+// reads all planes of the step before from the other CTAs' shared memory (two buffers in turn, one cluster
+// barrier per step).  The norm's partial sums are added in rank order.  From two tasks per SM on one CTA
+// takes a task whole, with the same operations in the same order.  Measured at K = 10, some 100 tasks a launch:
+// 71 us with a CTA each, 51 us with clusters (28 us at the pipe's rate on all SMs); at K = 8, 1100 tasks: 162 us
+// either way.
 template <int K>
-__global__ void __launch_bounds__(256) generate_kernel_t(DevBasis b, const GenTask *tasks, int n) {
-    constexpr int N2 = 2 * K, K3 = K * K * K, KK = K * K;
-    extern __shared__ double gsm[];
-    double *wt = gsm;                // W^T rows (c K + x) of length 2K, as b.WT
-    double *t1 = wt + N2 * N2;       // t1[Z][Y][x] (first step) or t1[z][y][x']
-    double *t2 = t1 + N2 * N2 * K;   // t2[Z][y][x] (first step) or t2[z][y'][x]
-    double *sc = t2 + N2 * KK;       // s[z][y][x]
-    __shared__ double s_red[8];
-    for (int i = threadIdx.x; i < N2 * N2; i += blockDim.x) wt[i] = b.WT[i];
+struct GenGeo {
+    static constexpr int N2 = 2 * K, KK = K * K, K3 = K * KK, NZ = 2, S = (K + 1) / 2, THREADS = 128;
+};
+
+// one step of a task for the output planes z0, z0 + 1 (z1 = z0 when there is one): `out` from the full block
+// `anc`, or from the scaling planes src[k] (two each) of the step before
+template <int K, bool FULL>
+__device__ __forceinline__ void gen_step(const double *anc, const double *const (&src)[GenGeo<K>::S], const double *wx,
+                                         const double *wy, const double *wz, int z0, double *t1, double *t2, double *out) {
+    using G = GenGeo<K>;
+    constexpr int N2 = G::N2, K3 = G::K3, KK = G::KK, NZ = G::NZ, NT = G::THREADS, M = FULL ? N2 : K;
+    const int tid = threadIdx.x, nz = min(NZ, K - z0), z1 = min(z0 + 1, K - 1);
+    for (int i = tid; i < M * M; i += NT) {
+        const int X = i % M, Y = i / M;
+        // components cx | cy << 1 | cz << 2
+        const double *col = FULL ? anc + ((X >= K ? 1 : 0) + (Y >= K ? 2 : 0)) * K3 + (Y % K) * K + X % K : nullptr;
+        double a0 = 0.0, a1 = 0.0;
+#pragma unroll
+        for (int Z = 0; Z < M; Z++) {
+            const double v = FULL ? col[(Z >= K ? 4 * K3 : 0) + (Z % K) * KK] : src[(Z % K) / NZ][(Z % NZ) * KK + i];
+            a0 += wz[z0 * N2 + Z] * v;
+            a1 += wz[z1 * N2 + Z] * v;
+        }
+        t1[i] = a0;
+        t1[M * M + i] = a1;
+    }
     __syncthreads();
-    for (int t = blockIdx.x; t < n; t += gridDim.x) {
+    for (int i = tid; i < nz * K * M; i += NT) {
+        const int X = i % M, y = (i / M) % K, z = i / (K * M);
+        double acc = 0.0;
+#pragma unroll
+        for (int Y = 0; Y < M; Y++) acc += wy[y * N2 + Y] * t1[(z * M + Y) * M + X];
+        t2[i] = acc;
+    }
+    __syncthreads();
+    for (int i = tid; i < nz * KK; i += NT) {
+        const int x = i % K, zy = i / K;
+        double acc = 0.0;
+#pragma unroll
+        for (int X = 0; X < M; X++) acc += wx[x * N2 + X] * t2[zy * M + X];
+        out[i] = acc;
+    }
+}
+
+// CL: a cluster per task, each CTA its two planes; else one CTA per task, the planes one pair after the other,
+// with the same operations in the same order
+template <int K, bool CL>
+__device__ __forceinline__ void generate_tasks(const DevBasis &b, const GenTask *tasks, int n) {
+    using G = GenGeo<K>;
+    constexpr int N2 = G::N2, K3 = G::K3, KK = G::KK, NZ = G::NZ, S = G::S, NT = G::THREADS, R = CL ? 1 : S;
+    __shared__ double wt[N2 * N2];          // W^T rows (c K + x) of length 2K, as b.WT
+    __shared__ double t1[NZ * N2 * N2];     // [z][Y][X]
+    __shared__ double t2[NZ * K * N2];      // [z][y][X]
+    __shared__ double sc[2][R * NZ * KK];   // the CTA's planes of s[z][y][x], of two steps in turn
+    __shared__ double s_w[NT / 32], s_part[S];
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int tid = threadIdx.x, r0 = CL ? (int)cluster.block_rank() : 0;
+    const int per = CL ? S : 1;
+    auto barrier = [&] {
+        if constexpr (CL)
+            cluster.sync();
+        else
+            __syncthreads();
+    };
+    for (int i = tid; i < N2 * N2; i += NT) wt[i] = b.WT[i];
+    __syncthreads();
+    for (int t = blockIdx.x / per; t < n; t += gridDim.x / per) {
         const GenTask task = tasks[t];
         const bool from_s = task.flags & GEN_FROM_S, only_s = task.flags & GEN_ONLY_S;
-        if (from_s) {
-            for (int i = threadIdx.x; i < K3; i += blockDim.x) sc[i] = task.anc[i];
-            __syncthreads();
-        }
         for (int s = 0; s < task.steps; s++) {
             const int c = (int)((task.path >> (3 * s)) & 7);
             const double *wx = wt + (c & 1) * K * N2, *wy = wt + ((c >> 1) & 1) * K * N2,
                          *wz = wt + ((c >> 2) & 1) * K * N2;
-            if (s == 0 && !from_s) {
-                for (int i = threadIdx.x; i < N2 * N2 * K; i += blockDim.x) {
-                    const int x = i % K, YZ = i / K, Y = YZ % N2, Z = YZ / N2;
-                    const int cyz = ((Y >= K) ? 2 : 0) | ((Z >= K) ? 4 : 0);
-                    const double *row = task.anc + (Z % K) * KK + (Y % K) * K;
-                    double acc = 0.0;
+            const double *src[S];
 #pragma unroll
-                    for (int X = 0; X < N2; X++) acc += wx[x * N2 + X] * row[(cyz | (X >= K ? 1 : 0)) * K3 + (X % K)];
-                    t1[i] = acc;
-                }
-                __syncthreads();
-                for (int i = threadIdx.x; i < N2 * KK; i += blockDim.x) {
-                    const int x = i % K, y = (i / K) % K, Z = i / KK;
-                    double acc = 0.0;
-#pragma unroll
-                    for (int Y = 0; Y < N2; Y++) acc += wy[y * N2 + Y] * t1[(Z * N2 + Y) * K + x];
-                    t2[i] = acc;
-                }
-                __syncthreads();
-                for (int i = threadIdx.x; i < K3; i += blockDim.x) {
-                    const int xy = i % KK, z = i / KK;
-                    double acc = 0.0;
-#pragma unroll
-                    for (int Z = 0; Z < N2; Z++) acc += wz[z * N2 + Z] * t2[Z * KK + xy];
-                    sc[i] = acc;
-                }
-            } else {
-                for (int i = threadIdx.x; i < K3; i += blockDim.x) {
-                    const int x = i % K, zy = i / K;
-                    double acc = 0.0;
-#pragma unroll
-                    for (int X = 0; X < K; X++) acc += wx[x * N2 + X] * sc[zy * K + X];
-                    t1[i] = acc;
-                }
-                __syncthreads();
-                for (int i = threadIdx.x; i < K3; i += blockDim.x) {
-                    const int x = i % K, y = (i / K) % K, z = i / KK;
-                    double acc = 0.0;
-#pragma unroll
-                    for (int Y = 0; Y < K; Y++) acc += wy[y * N2 + Y] * t1[(z * K + Y) * K + x];
-                    t2[i] = acc;
-                }
-                __syncthreads();
-                for (int i = threadIdx.x; i < K3; i += blockDim.x) {
-                    const int xy = i % KK, z = i / KK;
-                    double acc = 0.0;
-#pragma unroll
-                    for (int Z = 0; Z < K; Z++) acc += wz[z * N2 + Z] * t2[Z * KK + xy];
-                    sc[i] = acc;
-                }
+            for (int k = 0; k < S; k++) {
+                if (s == 0)
+                    src[k] = task.anc + k * NZ * KK;
+                else if constexpr (CL)
+                    src[k] = cluster.map_shared_rank(sc[(s - 1) & 1], k);
+                else
+                    src[k] = sc[(s - 1) & 1] + k * NZ * KK;
             }
+            for (int q = 0; q < R; q++) {
+                const int z0 = NZ * (r0 + q);
+                double *out = sc[s & 1] + q * NZ * KK;
+                if (s == 0 && !from_s)
+                    gen_step<K, true>(task.anc, src, wx, wy, wz, z0, t1, t2, out);
+                else
+                    gen_step<K, false>(nullptr, src, wx, wy, wz, z0, t1, t2, out);
+            }
+            barrier();  // every plane of this step is there
+        }
+        if (task.steps == 0) {
             __syncthreads();
+            for (int q = 0; q < R; q++)
+                for (int i = tid; i < min(NZ, K - NZ * (r0 + q)) * KK; i += NT)
+                    sc[1][q * NZ * KK + i] = task.anc[NZ * (r0 + q) * KK + i];
+            barrier();
         }
-        if (only_s) {
-            for (int i = threadIdx.x; i < K3; i += blockDim.x) task.out[i] = sc[i];
+        for (int q = 0; q < R; q++) {
+            const int z0 = NZ * (r0 + q), nz = min(NZ, K - z0);
+            const double *mine = sc[(task.steps + 1) & 1] + q * NZ * KK;
+            double ss = 0.0;
+            for (int i = tid; i < nz * KK; i += NT) {
+                const double v = mine[i];
+                task.out[z0 * KK + i] = v;
+                ss += v * v;
+            }
+            if (only_s) continue;  // the next task's first barrier comes before anything here is written again
+            // the block's other components and their norms are zero
+            for (int i = K3 + (r0 + q) * NT + tid; i < 8 * K3; i += S * NT) task.out[i] = 0.0;
+            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if ((tid & 31) == 0) s_w[tid >> 5] = ss;
             __syncthreads();
-            continue;
+            if (tid == 0) {
+                double tot = 0.0;
+                for (int w = 0; w < NT / 32; w++) tot += s_w[w];
+                if constexpr (CL)
+                    *cluster.map_shared_rank(&s_part[r0], 0) = tot;
+                else
+                    s_part[q] = tot;
+            }
+            barrier();
         }
-        double ss = 0.0;
-        for (int i = threadIdx.x; i < 8 * K3; i += blockDim.x) {
-            const double v = i < K3 ? sc[i] : 0.0;
-            task.out[i] = v;
-            ss += v * v;
-        }
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = ss;
-        __syncthreads();
-        if (threadIdx.x < 8) {
+        if (!only_s && r0 == 0 && tid < 8) {
             double tot = 0.0;
-            if (threadIdx.x == 0)
-                for (int w = 0; w < (int)(blockDim.x >> 5); w++) tot += s_red[w];
-            task.cn[threadIdx.x] = threadIdx.x == 0 ? sqrt(tot) : 0.0;
+            if (tid == 0)
+                for (int k = 0; k < S; k++) tot += s_part[k];
+            task.cn[tid] = tid == 0 ? sqrt(tot) : 0.0;
         }
-        __syncthreads();
     }
+    barrier();  // no CTA's shared memory goes before the others are done with it
+}
+
+template <int K>
+__global__ void __cluster_dims__(GenGeo<K>::S, 1, 1) __launch_bounds__(GenGeo<K>::THREADS)
+    generate_cluster_kernel(DevBasis b, const GenTask *tasks, int n) {
+    generate_tasks<K, true>(b, tasks, n);
+}
+
+template <int K>
+__global__ void __launch_bounds__(GenGeo<K>::THREADS, 4) generate_kernel_t(DevBasis b, const GenTask *tasks, int n) {
+    generate_tasks<K, false>(b, tasks, n);
 }
 
 template <int K>
 void launch_generate_t(const DevBasis &b, const GenTask *tasks, int n, int nsm, cudaStream_t s) {
-    constexpr int N2 = 2 * K;
-    constexpr size_t smem = sizeof(double) * ((size_t)N2 * N2 + (size_t)N2 * N2 * K + (size_t)N2 * K * K + (size_t)K * K * K);
-    kernel_smem((const void *)generate_kernel_t<K>, (int)smem);
-    const int grid = std::min(n, 4 * std::max(nsm, 1));
-    generate_kernel_t<K><<<grid, 256, smem, s>>>(b, tasks, n);
+    using G = GenGeo<K>;
+    nsm = std::max(nsm, 1);
+    if (n < 2 * nsm)  // too few tasks to fill the chip
+        generate_cluster_kernel<K><<<n * G::S, G::THREADS, 0, s>>>(b, tasks, n);
+    else
+        generate_kernel_t<K><<<std::min(n, 4 * nsm), G::THREADS, 0, s>>>(b, tasks, n);
     MWG_CUDA(cudaGetLastError());
 }
 
