@@ -301,7 +301,7 @@ int *launch_tier(Ctx &ctx, Arena &arena, LevelItems &li, bool root, bool set, in
     // writes a partial block; the CTA that ends a node's last chunk sums its partials in chunk
     // order (mw_chunks.cuh).
     // The split depends only on the tier and the node's own item count, so results do not depend
-    // on which nodes share the launch.  CHUNK (Ctx::Tuning; by default 8, 32, 96 and 8 items) is
+    // on which nodes share the launch.  CHUNK (Ctx::Tuning; by default 8 (12 from order 8 on), 32, 96 and 8 items) is
     // two to six tenths of a millisecond of one CTA's work at order 9: an item costs ~22 us (fixed point),
     // ~20 us (FP32) and ~3 us (TF32).
     const long long CHUNK = chunk > 0 ? chunk : 1;
@@ -1026,7 +1026,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         cudaEvent_t ev_prep = nullptr;   // ... reduced copies and screening tables written
     };
     // launch settings: the autotuner's for this (order, jobs, mode) if it ran, else the context's
-    Ctx::Tuning tune;
+    Ctx::Tuning tune(K);
     tune.groups = ctx.groups;
     {
         auto it = ctx.tuned.find(std::make_tuple(b.K, (int)jobs.size(), precision_mode));
@@ -2432,7 +2432,7 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
         st.items_fp64 += items;
         st.out_nodes += (long long)li.out.size();
         if (fixed_point && items > 0) fxops.make(ctx, st);
-        launch_tier(ctx, ar, li, root, true, 0, Ctx::Tuning().chunk[0], st, nullptr, false, fixed_point);
+        launch_tier(ctx, ar, li, root, true, 0, Ctx::Tuning(b.K).chunk[0], st, nullptr, false, fixed_point);
         MWG_CUDA(cudaEventRecord(done[turn].e, ctx.stream));
         turn ^= 1;
         st.levels++;

@@ -664,7 +664,7 @@ int mw_apply_batch_autotune(int n, const double *precs, mw_tree *outs, mw_op *op
             std::sort(v.begin(), v.end());
             return v[v.size() / 2];
         };
-        mwg::Ctx::Tuning best;
+        mwg::Ctx::Tuning best(ctx->basis.K);
         best.groups = ctx->groups;
         run(best, 1);  // warm-up: allocations, arenas, shadows
         double bt = run(best, repeats);

@@ -214,7 +214,13 @@ struct Ctx {
     // task takes per tier (FP64, FP32, TF32, double-FP32) before a node is split into chunks
     struct Tuning {
         int groups = DEFAULT_GROUPS;
+        // FP64: larger chunks save cut rows and partial blocks, smaller ones end sooner.  Chunks of 8 and 12: two
+        // applies of order 9 15.5 and 14.8 ms, the adjoint of order 8 17.5 and 17.1 ms, but the Poisson apply of
+        // order 7 3.83 and 3.92 ms and the Coulomb apply of order 5 2.19 and 2.45 ms.
         long long chunk[4] = {8, 32, 96, 8};
+        explicit Tuning(int K = 0) {
+            if (K > 8) chunk[0] = 12;
+        }
     };
     // settings picked by the autotuner (mw_apply_batch_autotune) per (order K, jobs, precision
     // mode); a batched apply with the same key uses them unless overlap is off (groups == 1)
