@@ -438,36 +438,39 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS) to_fx_kernel(__grid_constan
         const double *in = S.pairs ? (S.up ? S.pairs[b].child0 : S.pairs[b].parent)
                                    : S.in[k] + (size_t)(b - S.first[k]) * 8 * K3;
         uint32_t *o = S.out[k] + (size_t)(b - S.first[k]) * G::IN_WORDS;
-        int ef = 0;
-        auto at = [&](int X, int Y, int Z) -> long long {
-            if (X >= N2 || Y >= N2) return 0;
+        auto at = [&](int X, int Y, int Z) -> double {
+            if (X >= N2 || Y >= N2) return 0.0;
             const int cx = X >= K, cy = Y >= K, cz = Z >= K;
-            return fx_from_double(
-                in[(cx + 2 * cy + 4 * cz) * cs + (Z - cz * K) * K2 + (Y - cy * K) * K + (X - cx * K)], ef);
-        };
-        auto field = [&](int X, int Y, int Z) -> int {
-            if (X >= N2 || Y >= N2) return 0;
-            const int cx = X >= K, cy = Y >= K, cz = Z >= K;
-            return (__double2hiint(in[(cx + 2 * cy + 4 * cz) * cs + (Z - cz * K) * K2 + (Y - cy * K) * K + (X - cx * K)]) >> 20) & 0x7ff;
+            return in[(cx + 2 * cy + 4 * cz) * cs + (Z - cz * K) * K2 + (Y - cy * K) * K + (X - cx * K)];
         };
         for (int tile = warp; tile < G::NTIN; tile += G::WARPS) {
             int Y, Z;
             fx_in_column<K>(tile / G::TL, tile % G::TL, g, Y, Z);
-            ef = 0;
-            for (int X = t; X < N2; X += 4) ef = max(ef, field(X, Y, Z));
+            // this lane's X of the column, every X in one lane (those of the remainder in two)
+            constexpr int NX = G::BIG ? 6 : (N2 > 8 ? 4 : 2);
+            double x[NX];
+#pragma unroll
+            for (int j = 0; j < NX; j++) x[j] = at(j < 4 ? 2 * t + (j & 1) + 8 * (j >> 1) : 16 + 2 * (t & 1) + (j & 1), Y, Z);
+            int ef = 0;
+#pragma unroll
+            for (int j = 0; j < NX; j++) ef = max(ef, (__double2hiint(x[j]) >> 20) & 0x7ff);
             ef = __reduce_max_sync(0xffffffffu, ef);
             if (lane == 0) reinterpret_cast<short *>(o + G::IN_EXP)[tile] = (short)(ef == 0 ? FX_NONE : ef - 1022);
             uint32_t w[G::WB];
             uint32_t q[7];
-            fx_digits(at(2 * t, Y, Z), at(2 * t + 1, Y, Z), q);
+            fx_digits(fx_from_double(x[0], ef), fx_from_double(x[1], ef), q);
 #pragma unroll
-            for (int s = 0; s < 7; s++) w[2 * s] = q[s];
-            fx_digits(at(2 * t + 8, Y, Z), at(2 * t + 9, Y, Z), q);
+            for (int s = 0; s < 7; s++) {
+                w[2 * s] = q[s];
+                w[2 * s + 1] = 0u;
+            }
+            if constexpr (N2 > 8) {
+                fx_digits(fx_from_double(x[2], ef), fx_from_double(x[3], ef), q);
 #pragma unroll
-            for (int s = 0; s < 7; s++) w[2 * s + 1] = q[s];
+                for (int s = 0; s < 7; s++) w[2 * s + 1] = q[s];
+            }
             if constexpr (G::BIG) {
-                const int X = 16 + 2 * (t & 1);
-                fx_digits(at(X, Y, Z), at(X + 1, Y, Z), q);
+                fx_digits(fx_from_double(x[4], ef), fx_from_double(x[5], ef), q);
                 FxB B;
                 B.fold(q, t >= 2);
                 w[14] = B.s01;
