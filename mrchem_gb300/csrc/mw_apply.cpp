@@ -671,6 +671,7 @@ bool screen_setup(Ctx &ctx, std::vector<ApplyJob> &jobs, const std::vector<JobSt
 
 struct TierRule {  // the apply's precision mode, as the tier choice reads it
     bool mixed, near_fp64, df_only, dfp, tensor;
+    bool fp32() const { return mixed && !tensor && !df_only; }  // tier 1 on the CUDA cores
 };
 
 // the walk kernels' (t, lz) rows at a scale: the most over the group's operators
@@ -860,7 +861,7 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
     P.gcn = (double *)ar.alloc(sizeof(double) * 8 * ng);
     P.gcn32 = (float *)ar.alloc(sizeof(float) * 8 * ng);
     P.g64 = (double *)ar.alloc(sizeof(double) * (size_t)bs * ng);
-    P.g32 = rule.mixed ? (float *)ar.alloc(sizeof(float) * 2 * (size_t)bs * ng) : nullptr;
+    P.g32 = rule.fp32() ? (float *)ar.alloc(sizeof(float) * (size_t)bs * ng) : nullptr;
     P.gtc = rule.tensor ? (float *)ar.alloc(sizeof(float) * P.tx * ng) : nullptr;
     P.fx = fxops ? fx_words(K) : 0;
     P.gfx = fxops ? (uint32_t *)ar.alloc(sizeof(uint32_t) * P.fx * ng) : nullptr;
@@ -894,13 +895,13 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
             k_screen_gen_norms32(P, ngen, ctx.stream);
             st.launches += 3;
             st.generated += ngen;
-            if (rule.mixed) {
+            if (rule.fp32()) {
                 k_to_fp32_cube(P.g64, P.g32, (size_t)ngen, K, ctx.stream);
                 st.launches++;
-                if (rule.tensor) {
-                    k_to_tc_x(P.g32, P.gtc, (size_t)ngen, K, ctx.stream);
-                    st.launches++;
-                }
+            }
+            if (rule.tensor) {
+                k_to_tc_x(P.g64, P.gtc, (size_t)ngen, K, ctx.stream);
+                st.launches++;
             }
         }
         const auto tC = now();
@@ -982,6 +983,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
     const bool tensor = mixed && precision_mode != MW_PREC_MIXED_FP32 && precision_mode != MW_PREC_DF;
     const bool dfp = tensor;  // the double-FP32 tier comes with the tensor-core tier
     const bool df_only = precision_mode == MW_PREC_DF;
+    const bool fp32 = mixed && !tensor && !df_only;  // tier 1 on the CUDA cores
     auto t_start = std::chrono::steady_clock::now();
     const long long fetch0 = ctx.fetch_launches;
     Arena &arena = ctx.arena;
@@ -994,15 +996,14 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
     for (auto &e : ev_span) MWG_CUDA(cudaEventCreate(&e));
     MWG_CUDA(cudaEventRecord(ev_span[0], ctx.stream));
 
-    // the reduced tiers' copies of an input tree's blocks (FP32 cube-order shadows, and the TF32
-    // tier's x-pass operand), on the context's current stream
+    // the reduced tiers' copy of an input tree's blocks (the tensor-core tiers' x-pass operand, or where
+    // tier 1 runs on the CUDA cores an FP32 shadow in cube order), on the context's current stream
     auto convert_input = [&](Tree &in) {
-        k_to_fp32_cube(in.d_coefs, in.d_coefs32, (size_t)in.nn(), b.K, ctx.stream);
-        st.launches++;
-        if (tensor) {
-            k_to_tc_x(in.d_coefs32, in.d_coefs_tc, (size_t)in.nn(), b.K, ctx.stream);
-            st.launches++;
-        }
+        if (tensor)
+            k_to_tc_x(in.d_coefs, in.d_coefs_tc, (size_t)in.nn(), b.K, ctx.stream);
+        else if (fp32)
+            k_to_fp32_cube(in.d_coefs, in.d_coefs32, (size_t)in.nn(), b.K, ctx.stream);
+        st.launches += tensor || fp32;
     };
     // The jobs are split into up to four groups that take turns: while the GPU runs the other
     // groups' levels, the host enumerates, screens and builds the items of one group's level.
@@ -1095,9 +1096,9 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         tree_zero(*job.out, 0, job.out->nn());
         if (mixed) {
             Tree &in = *job.inp;
-            if (in.cap32 < (size_t)in.nn()) {
+            if (fp32 && in.cap32 < (size_t)in.nn()) {
                 if (in.d_coefs32) cudaFree(in.d_coefs32);
-                MWG_CUDA(cudaMalloc(&in.d_coefs32, sizeof(float) * 2 * (size_t)bs * in.cap));
+                MWG_CUDA(cudaMalloc(&in.d_coefs32, sizeof(float) * (size_t)bs * in.cap));
                 in.cap32 = in.cap;
             }
             if (tensor && in.cap_tc < (size_t)in.nn()) {
@@ -1331,15 +1332,15 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                 for (JobState *sp : jp)
                     if (sp->gens.base && !first) first = sp->gens.base;
                 float *first32 = nullptr, *firsttc = nullptr;
-                if (mixed && total > 0) {
-                    first32 = (float *)ar.alloc(sizeof(float) * 2 * (size_t)bs * total);
+                if (fp32 && total > 0) {
+                    first32 = (float *)ar.alloc(sizeof(float) * (size_t)bs * total);
                     k_to_fp32_cube(first, first32, total, b.K, ctx.stream);
                     st.launches++;
-                    if (tensor) {
-                        firsttc = (float *)ar.alloc(sizeof(float) * tc5_x_stride(b.K) * total);
-                        k_to_tc_x(first32, firsttc, total, b.K, ctx.stream);
-                        st.launches++;
-                    }
+                }
+                if (tensor && total > 0) {
+                    firsttc = (float *)ar.alloc(sizeof(float) * tc5_x_stride(b.K) * total);
+                    k_to_tc_x(first, firsttc, total, b.K, ctx.stream);
+                    st.launches++;
                 }
                 uint32_t *firstfx = nullptr;
                 if (fixed_point && total > 0) firstfx = (uint32_t *)ar.alloc(sizeof(uint32_t) * fxw * total);
@@ -1351,7 +1352,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                     s.gbase = s.gens.base;
                     s.gbase_fx = (firstfx && s.gbase) ? firstfx + fxw * (size_t)((s.gbase - first) / bs) : nullptr;
                     s.gcn.swap(s.gens.cn);
-                    s.gbase32 = (first32 && s.gbase) ? first32 + 2 * (s.gbase - first) : nullptr;
+                    s.gbase32 = (first32 && s.gbase) ? first32 + (s.gbase - first) : nullptr;
                     s.gbase_tc = (firsttc && s.gbase) ? firsttc + tc5_x_stride(b.K) * (size_t)((s.gbase - first) / bs) : nullptr;
                 }
             }
@@ -1471,13 +1472,12 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                         T.ay[pi] = bt + tb * (size_t)byi;
                         T.az[pi] = bt + tb * (size_t)bzi;
                     } else {
-                        // the reduced tiers read the FP32 cube-order shadows and the FP32 operator blocks
-                        // (high part first, low part after it)
-                        T.in[pi] = cd.gen ? (const void *)(s.gbase32 + 2 * (size_t)cd.src * bs)
-                                          : (const void *)(inp.d_coefs32 + 2 * (size_t)cd.src * bs);
-                        T.ax[pi] = op.d_blocks32 + 2 * (size_t)bxi * bsz;
-                        T.ay[pi] = op.d_blocks32 + 2 * (size_t)byi * bsz;
-                        T.az[pi] = op.d_blocks32 + 2 * (size_t)bzi * bsz;
+                        // the FP32 tier reads the FP32 cube-order shadows and the FP32 operator blocks
+                        T.in[pi] = cd.gen ? (const void *)(s.gbase32 + (size_t)cd.src * bs)
+                                          : (const void *)(inp.d_coefs32 + (size_t)cd.src * bs);
+                        T.ax[pi] = op.d_blocks32 + (size_t)bxi * bsz;
+                        T.ay[pi] = op.d_blocks32 + (size_t)byi * bsz;
+                        T.az[pi] = op.d_blocks32 + (size_t)bzi * bsz;
                     }
                     T.coef[pi] = op.c[cd.t];
                     pi++;

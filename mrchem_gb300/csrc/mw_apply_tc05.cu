@@ -525,28 +525,32 @@ void launch_tc05(const ApplyLaunch &L, cudaStream_t s) {
     MWG_CUDA(cudaGetLastError());
 }
 
-// FP32 cube-order shadow -> x-pass operand: float4 (g, r) = row r = Z * 2K + Y, X = 4g .. 4g+3, per
-// block the value rounded to TF32 (hi), then the remainder (the shadow's high cube minus hi, plus its
-// low cube) rounded to TF32 (lo)
-__global__ void to_tc_x_kernel(const float *cube32, float *out, size_t nblocks, int K) {
-    const int N2 = 2 * K, NN = N2 * N2, KG = tc5_kg(K), C = NN * N2;
-    const size_t per = (size_t)KG * NN, total = nblocks * per;
+// FP64 blocks -> x-pass operand: float4 (g, r) = row r = Z * 2K + Y, X = 4g .. 4g+3, per block the value rounded
+// to FP32 and then to TF32 (hi), then the remainder rounded to TF32 (lo).  Bound: HBM (8 bytes read and 8 written
+// per element; a thread's four X are 32 bytes of the block).  16-orbital batch: 0.61 ms of launches a step; 0.88 ms
+// with an FP32 shadow made first and read here, which nothing else read.  Splitting the values with integer
+// operations (mw_dfconv.cuh) changes little (0.58 ms).
+template <int K>
+__global__ void __launch_bounds__(256) to_tc_x_kernel(const double *blocks, float *out, size_t nblocks) {
+    constexpr int N2 = 2 * K, NN = N2 * N2, KG = tc5_kg(K), K3 = K * K * K, PER = KG * NN;
+    const size_t total = nblocks * PER;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t blk = i / per;
-        const int rem = (int)(i - blk * per), g = rem / NN, r = rem - g * NN;
-        const float *src = cube32 + blk * 2 * (size_t)C + (size_t)r * N2 + 4 * g;
-        const float *srl = src + C;  // the low cube
+        const size_t blk = i / PER;
+        const int rem = (int)(i - blk * PER), g = rem / NN, r = rem - g * NN, Y = r % N2, Z = r / N2;
+        // components cx | cy << 1 | cz << 2
+        const double *row = blocks + blk * 8 * K3 + ((Y >= K ? 2 : 0) + (Z >= K ? 4 : 0)) * K3 + (Z % K) * K * K + (Y % K) * K;
         float h[4], l[4];
 #pragma unroll
         for (int c = 0; c < 4; c++) {
-            const bool in = 4 * g + c < N2;
-            const float v = in ? src[c] : 0.0f;
+            const int X = 4 * g + c;
+            const double d = X < N2 ? row[X >= K ? K3 + X - K : X] : 0.0;
+            const float v = __double2float_rn(d);
             h[c] = tf32r(v);
-            l[c] = tf32r(in ? __fadd_rn(__fsub_rn(v, h[c]), srl[c]) : 0.0f);
+            l[c] = tf32r(__fadd_rn(__fsub_rn(v, h[c]), __double2float_rn(d - (double)v)));
         }
         float4 *o4 = reinterpret_cast<float4 *>(out);
-        o4[2 * blk * per + rem] = make_float4(h[0], h[1], h[2], h[3]);
-        o4[2 * blk * per + per + rem] = make_float4(l[0], l[1], l[2], l[3]);
+        o4[2 * blk * PER + rem] = make_float4(h[0], h[1], h[2], h[3]);
+        o4[2 * blk * PER + PER + rem] = make_float4(l[0], l[1], l[2], l[3]);
     }
 }
 
@@ -622,11 +626,20 @@ double probe_tc05_tflops(int n, int nsm, cudaStream_t s) {
     return flops / (best * 1e-3) / 1e12;
 }
 
-void k_to_tc_x(const float *cube32, float *out, size_t nblocks, int K, cudaStream_t s) {
+void k_to_tc_x(const double *blocks, float *out, size_t nblocks, int K, cudaStream_t s) {
     if (nblocks == 0) return;
     const size_t total = nblocks * (size_t)tc5_kg(K) * (size_t)(4 * K * K);
     const int grid = (int)std::min<size_t>((total + 255) / 256, 4096);
-    to_tc_x_kernel<<<grid, 256, 0, s>>>(cube32, out, nblocks, K);
+    switch (K) {
+        case 4: to_tc_x_kernel<4><<<grid, 256, 0, s>>>(blocks, out, nblocks); break;
+        case 5: to_tc_x_kernel<5><<<grid, 256, 0, s>>>(blocks, out, nblocks); break;
+        case 6: to_tc_x_kernel<6><<<grid, 256, 0, s>>>(blocks, out, nblocks); break;
+        case 7: to_tc_x_kernel<7><<<grid, 256, 0, s>>>(blocks, out, nblocks); break;
+        case 8: to_tc_x_kernel<8><<<grid, 256, 0, s>>>(blocks, out, nblocks); break;
+        case 9: to_tc_x_kernel<9><<<grid, 256, 0, s>>>(blocks, out, nblocks); break;
+        case 10: to_tc_x_kernel<10><<<grid, 256, 0, s>>>(blocks, out, nblocks); break;
+        default: throw Error(MW_ERR_ARG, "no tensor-core apply kernel for this order");
+    }
     MWG_CUDA(cudaGetLastError());
 }
 

@@ -472,12 +472,11 @@ void build_operators(const std::vector<Oper *> &ops, const Basis &b) {
         const OperScreenLayout ly(*ops[o]);
         MWG_CUDA(cudaMemcpyAsync(ops[o]->d_screen, stage[o], ly.ib + ly.db + ly.fb, cudaMemcpyHostToDevice, st));
     }
-    // device copies for the reduced tiers: FP32 high part then low part per block (FP32
-    // tier), and the tensor-core tier's B operand (mw_tc05_layout.h)
+    // device copies for the reduced tiers: FP32 (tier 1 on the CUDA cores), and the tensor-core tier's B operand (mw_tc05_layout.h)
     const bool tc = K >= 4 && K <= KMAX;
     for (Oper *op : ops) {
         const long nb = std::max<long>(op->nblocks, 1);
-        MWG_CUDA(cudaMallocAsync(&op->d_blocks32, sizeof(float) * 2 * (size_t)nb * bsz, st));
+        MWG_CUDA(cudaMallocAsync(&op->d_blocks32, sizeof(float) * (size_t)nb * bsz, st));
         if (tc) {
             MWG_CUDA(cudaMallocAsync(&op->d_blocks_tc, sizeof(float) * tc5_b_stride(K) * (size_t)nb, st));
             if (tc5_split_wide(K)) MWG_CUDA(cudaMallocAsync(&op->d_blocks_tc2, sizeof(float) * tc5_b_stride(K) * (size_t)nb, st));

@@ -97,7 +97,7 @@ struct Tree {
     std::vector<double> cn;       // 8 component norms per node (host copy)
     double *d_coefs = nullptr;    // cap * bs
     double *d_cn = nullptr;       // cap * 8
-    float *d_coefs32 = nullptr;   // FP32 shadow (mixed-precision applies): cap32 x (high cube, low cube)
+    float *d_coefs32 = nullptr;   // FP32 shadow in cube order (applies whose tier 1 runs on the CUDA cores), cap32 blocks
     float *d_coefs_tc = nullptr;  // TF32 x-pass operand of the tensor-core tier (mw_tc05_layout.h), cap_tc blocks
     size_t cap = 0, cap32 = 0, cap_tc = 0;
     int nroots = 0;
@@ -130,7 +130,7 @@ struct Oper {
     std::vector<double> amax, xmax;  // per (t,s)
     long nblocks = 0;
     double *d_blocks = nullptr;  // (2K)^2 per block, FP64
-    float *d_blocks32 = nullptr; // FP32 copy: per block the high part, then the low part (2 x (2K)^2)
+    float *d_blocks32 = nullptr; // FP32 copy
     float *d_blocks_tc = nullptr; // TF32 B operand of the tensor-core tier per block (mw_tc05_layout.h)
     float *d_blocks_tc2 = nullptr; // ... in the split-TF32 tier's wide layout (tc5_split_wide(K) only)
     // the operator blocks the split-TF32 tier reads: the wide layout where the kernel uses it
@@ -364,7 +364,7 @@ void k_apply(const DevBasis &b, const ApplyLaunch &L, int fp32, int nsm, cudaStr
 // FP32 tier.  Item pointers point at the hi copies of mw_tc05_layout.h's operand layouts.
 void k_apply_tc05(const DevBasis &b, const ApplyLaunch &L, bool split, cudaStream_t s);
 // FP32 cube-order shadows (high cube read) -> the tensor-core tier's x-pass operand layout
-void k_to_tc_x(const float *cube32, float *out, size_t nblocks, int K, cudaStream_t s);
+void k_to_tc_x(const double *blocks, float *out, size_t nblocks, int K, cudaStream_t s);
 // round to TF32: nearest, ties away from zero (as cvt.rna.tf32.f32)
 inline float tf32_round_host(float x) {
     uint32_t u;

@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(OB_THREADS) op_block_kernel(const double *W, c
     }
 }
 
-// FP32 high and low parts of every block, and the tensor-core tier's B operand (mw_tc05_layout.h)
+// FP32 copy of every block, and the tensor-core tier's B operand (mw_tc05_layout.h)
 // round to TF32: nearest, ties away from zero (infinities and NaNs unchanged)
 __device__ __forceinline__ float tf32_round(float v) {
     uint32_t u = __float_as_uint(v);
@@ -300,14 +300,8 @@ __global__ void op_convert_kernel(const double *blocks, float *b32, float *btc, 
                                   int NB, int groups) {
     const int N2 = 2 * K, bsz = N2 * N2;
     const size_t total = (size_t)nblocks * bsz;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t blk = i / bsz;
-        const int r = (int)(i - blk * bsz);
-        const double d = blocks[i];
-        const float h = __double2float_rn(d);
-        b32[2 * blk * bsz + r] = h;
-        b32[2 * blk * bsz + bsz + r] = __double2float_rn(d - (double)h);
-    }
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
+        b32[i] = __double2float_rn(blocks[i]);
     if (!btc) return;
     // per block: the B operand rounded to TF32 (hi), then the remainder rounded to TF32 (lo)
     const size_t per = (size_t)groups * NB * 4, ttot = (size_t)nblocks * per;

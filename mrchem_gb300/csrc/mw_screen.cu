@@ -702,10 +702,10 @@ __global__ void __launch_bounds__(FT) fill_kernel(ScreenLevel P) {
                 P.ay[dst] = bt + P.tb * by;
                 P.az[dst] = bt + P.tb * bz;
             } else {
-                P.in[dst] = cd.gen ? (const void *)(P.g32 + 2 * src * P.bs) : (const void *)(J.in32 + 2 * src * P.bs);
-                P.ax[dst] = op.b32 + 2 * bx * P.bsz;
-                P.ay[dst] = op.b32 + 2 * by * P.bsz;
-                P.az[dst] = op.b32 + 2 * bz * P.bsz;
+                P.in[dst] = cd.gen ? (const void *)(P.g32 + src * P.bs) : (const void *)(J.in32 + src * P.bs);
+                P.ax[dst] = op.b32 + bx * P.bsz;
+                P.ay[dst] = op.b32 + by * P.bsz;
+                P.az[dst] = op.b32 + bz * P.bsz;
             }
             P.coef[dst] = op.c[cd.t];
         }
