@@ -129,6 +129,7 @@ struct JobState {
     std::vector<double> fmax_lv;
     double fmax_at(int lv) const { return lv < (int)fmax_lv.size() ? fmax_lv[lv] : fmax; }
     bool fixed_point = true;  // every input norm is finite and far from overflow
+    int *fxneed = nullptr;    // per input node: its digits have been asked for (made on demand only)
     void set_fmax(const Tree &t, int n0) {
         fmax = 0.0;
         fixed_point = true;
@@ -287,6 +288,8 @@ struct DevItems {
     const void **in = nullptr, **ax = nullptr, **ay = nullptr, **az = nullptr;
     double *coef = nullptr;
     long long base[NTIER] = {0, 0, 0, 0};
+    FxBlock *fxlist = nullptr;  // the blocks whose digits the level asks for, where they are made on demand
+    int *fxcnt = nullptr;
     const double *g64 = nullptr;  // the level's generated blocks and the place of their digits
     uint32_t *gfx = nullptr;
     size_t ngen = 0;
@@ -622,6 +625,7 @@ void screen_setup_inputs(Ctx &ctx, std::vector<ApplyJob> &jobs, const std::vecto
         J.in32 = t.d_coefs32;
         J.intc = t.d_coefs_tc;
         J.infx = js[j].fx;
+        J.fxneed = js[j].fxneed;
     }
     // read by kernels from the pinned staging: with host inputs these tables go up while the later
     // job groups' input blocks still occupy the copy engines
@@ -868,6 +872,13 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
     dv.g64 = P.g64;
     dv.gfx = P.gfx;
     dv.ngen = fxops ? (size_t)ngen : 0;
+    if (fxops && jp[0]->fxneed) {
+        size_t most = ng;
+        for (JobState *sp : jp) most += (size_t)sp->job->inp->nn();
+        dv.fxlist = P.fxlist = (FxBlock *)ar.alloc(sizeof(FxBlock) * most);
+        dv.fxcnt = P.fxcnt = (int *)ar.alloc(sizeof(int) * (1 + ng));
+        P.gneed = P.fxcnt + 1;
+    }
     std::vector<const uint32_t *> fxop;  // per job of the apply its operator's digits
     if (fxops) {
         P.fxo = fxops->words;
@@ -882,6 +893,7 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
         pk.add(coff.data(), sizeof(long long) * NN);
         pk.add(fxop.data(), sizeof(uint32_t *) * fxop.size());
         pk.ship(ctx, ar);
+        if (P.fxlist) MWG_CUDA(cudaMemsetAsync(P.fxcnt, 0, sizeof(int) * (1 + ng), ctx.stream));
         P.cand_off = (const long long *)pk.ptr(0);
         P.fxop = (const uint32_t *const *)pk.ptr(1);
         if (ngen > 0) {
@@ -1112,6 +1124,10 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         if (fixed_grid) max_levels = std::max(max_levels, job.out->max_scale() - b.n0 + 1);
         s.R = 1.0;
     }
+    // Digits up front (inputs' once, operators' beside a level's screening) where most items need them; in the
+    // other modes a level that has such items makes those of the blocks that its items ask for (few of the
+    // 125 thousand input nodes of 528 exchange products: 70 ms on demand)
+    const bool ops_first = !mixed || near_fp64 || df_only;
     // The digits of every distinct input tree (the FP64 and double-FP32 tiers' fixed-point kernel), for the
     // length of the call.  They take 1.8 times the blocks' own space: trees that would not leave room for
     // them go to the kernel that reads the FP64 blocks.
@@ -1124,11 +1140,25 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         for (JobState &s : js)
             if (tree_fx.emplace(s.job->inp, nullptr).second) bytes += sizeof(uint32_t) * fxw * (size_t)s.job->inp->nn();
         digits = ctx.sarena.room_for(bytes);
+        uint32_t *next = digits ? (uint32_t *)ctx.sarena.alloc(bytes) : nullptr;
         for (JobState &s : js) {
             if (!digits) break;
             uint32_t *&d = tree_fx[s.job->inp];
-            if (!d) d = (uint32_t *)ctx.sarena.alloc(sizeof(uint32_t) * fxw * (size_t)s.job->inp->nn());
+            if (!d) {
+                d = next;
+                next += fxw * (size_t)s.job->inp->nn();
+            }
             s.fx = d;
+        }
+        if (digits && !ops_first) {
+            size_t total = 0;
+            for (JobState &s : js) total += (size_t)s.job->inp->nn();
+            int *need = (int *)ctx.sarena.alloc(sizeof(int) * total);
+            MWG_CUDA(cudaMemsetAsync(need, 0, sizeof(int) * total, ctx.stream));
+            for (JobState &s : js) {
+                s.fxneed = need;
+                need += s.job->inp->nn();
+            }
         }
     }
     auto to_digits = [&](const std::vector<int> &which) {  // of these jobs' trees, each once
@@ -1141,14 +1171,11 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         k_to_fx(sets.data(), sets.size(), K, ctx.stream);
         st.launches++;
     };
-    if (digits && !hin) {
+    if (digits && ops_first && !hin) {
         std::vector<int> all(js.size());
         for (size_t j = 0; j < js.size(); j++) all[j] = (int)j;
         to_digits(all);
     }
-    // the operators' digits of a level: beside its screening where most items need them, else once it is
-    // known that any does
-    const bool ops_first = !mixed || near_fp64 || df_only;
     // screening on the GPU (mw_screen.cu) when the context asks for it and the jobs fit its tables
     const TierRule rule{mixed, near_fp64, df_only, dfp, tensor};
     DevScreen ds;
@@ -1237,7 +1264,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                     js[j].set_fmax(in, b.n0);
                     if (mixed) convert_input(in);
                 }
-                if (digits) to_digits(G.jobs);
+                if (digits && ops_first) to_digits(G.jobs);
                 if (ds.on) screen_setup_inputs(ctx, jobs, js, G.jobs, ds);
                 MWG_CUDA(cudaEventCreateWithFlags(&G.ev_prep, cudaEventDisableTiming));
                 MWG_CUDA(cudaEventRecord(G.ev_prep, ctx.stream));
@@ -1502,7 +1529,29 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         G.status.clear();
         if (fixed_point && lt[0].items + lt[3].items > 0) {
             if (!ops_first) fxops.make(ctx, st);
-            if (dv.ngen > 0) {
+            if (!ops_first && !dscreen) {  // screened on the host: its items' input nodes
+                std::vector<FxBlock> list;
+                for (JobState *sp : jp) {
+                    std::vector<char> seen(sp->job->inp->nn(), 0);
+                    for (const auto &cv : sp->cand)
+                        for (const Cand &cd : cv)
+                            if ((cd.tier == 0 || cd.tier == 3) && !cd.gen && !seen[cd.src]) {
+                                seen[cd.src] = 1;
+                                list.push_back(FxBlock{sp->job->inp->block(cd.src), sp->fx + fxw * (size_t)cd.src});
+                            }
+                }
+                const int count = (int)list.size();
+                Packer pk;
+                pk.add(list.data(), list.size() * sizeof(FxBlock));
+                pk.add(&count, sizeof count);
+                pk.ship(ctx, ar);
+                if (count > 0) k_to_fx_list((const FxBlock *)pk.ptr(0), (const int *)pk.ptr(1), list.size(), K, ctx.stream);
+                st.launches += count > 0;
+            }
+            if (dv.fxlist) {
+                k_to_fx_list(dv.fxlist, dv.fxcnt, (size_t)(lt[0].items + lt[3].items), K, ctx.stream);
+                st.launches++;
+            } else if (dv.ngen > 0) {
                 const FxBlocks gen{dv.g64, dv.gfx, dv.ngen};
                 k_to_fx(&gen, 1, K, ctx.stream);
                 st.launches++;

@@ -682,6 +682,10 @@ __global__ void __launch_bounds__(FT) fill_kernel(ScreenLevel P) {
             const size_t src = (size_t)cd.src;
             if (tier == 0 || tier == 3) {  // the same kernel, or for both the FP64 one
                 if (P.fx) {
+                    if (P.fxlist && atomicExch(cd.gen ? P.gneed + src : J.fxneed + src, 1) == 0)
+                        P.fxlist[atomicAdd(P.fxcnt, 1)] =
+                            cd.gen ? FxBlock{P.g64 + src * P.bs, P.gfx + P.fx * src}
+                                   : FxBlock{J.in64 + src * P.bs, const_cast<uint32_t *>(J.infx) + P.fx * src};
                     const uint32_t *b = P.fxop[nd.job] + P.fxo * (size_t)(op.first[cd.t * S + s] + op.band[cd.t * S + s]);
                     const long o = (long)P.fxo;
                     P.in[dst] = cd.gen ? (const void *)(P.gfx + P.fx * src) : (const void *)(J.infx + P.fx * src);
