@@ -546,6 +546,19 @@ void fx_pairs(Ctx &ctx, Arena &ar, const std::vector<PairTask> &all, bool up, ui
     }
 }
 
+// room for `bytes` from the device's stream-ordered pool: what it holds unused and a quarter of what is free
+bool pool_room(int device, size_t bytes) {
+    size_t free_b = 0, total_b = 0;
+    uint64_t reserved = 0, used = 0;
+    cudaMemPool_t pool = nullptr;
+    MWG_CUDA(cudaDeviceGetDefaultMemPool(&pool, device));
+    MWG_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+    MWG_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+    if (bytes <= (size_t)(reserved - used)) return true;  // without the slow query below
+    MWG_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    return bytes <= (size_t)(reserved - used) + free_b / 4;
+}
+
 void ensure_fast(Ctx &ctx) {  // the generation's and screening's high-priority stream
     if (ctx.fast) return;
     int least = 0, greatest = 0;
@@ -1139,8 +1152,13 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         size_t bytes = 0;
         for (JobState &s : js)
             if (tree_fx.emplace(s.job->inp, nullptr).second) bytes += sizeof(uint32_t) * fxw * (size_t)s.job->inp->nn();
-        digits = ctx.sarena.room_for(bytes);
-        uint32_t *next = digits ? (uint32_t *)ctx.sarena.alloc(bytes) : nullptr;
+        digits = pool_room(ctx.device, bytes);
+        uint32_t *next = nullptr;
+        if (digits) {  // from the stream-ordered pool, to which it goes back when the call has ended
+            MWG_CUDA(cudaMallocAsync(&next, std::max<size_t>(bytes, 256), ctx.stream));
+            std::lock_guard<std::mutex> lock(ctx.retired_mu);
+            ctx.retired.push_back(next);
+        }
         for (JobState &s : js) {
             if (!digits) break;
             uint32_t *&d = tree_fx[s.job->inp];
