@@ -709,11 +709,11 @@ def run(args):
     fma_src = "probed FMA throughput of this GPU (mw_probe_fma_peak); MEASURED_PEAKS.json holds no FP64/FP32 figure"
     mma_src = ("probed dense tcgen05.mma TF32 throughput of this GPU at M128 N256 K8 (mw_probe_mma_peak kind 2); "
                "MEASURED_PEAKS.json holds no TF32 figure")
-    # the fixed-point kernel's multiply-add takes 48.6 products of mma.sync (per 8 columns two row tiles x 38
-    # products of 16 x 8 x 16, for 8 x 20 x 20 multiply-adds), which runs 960 of them per SM and cycle, 7.5
-    # times the FP32 pipe's 128
-    fx_tf = fp32_tf * (960.0 / 128.0) / 48.6
-    fx_src = fma_src + "; FP32 rate times 7.5 for mma.sync's FP16 products, divided by 48.6 products per multiply-add"
+    # the fixed-point kernel's multiply-add takes 39.5 products of mma.sync (per 8 columns of 20 x 20 multiply-adds
+    # 38 products of 16 x 8 x 16 for rows 0..15, 14 to 38 for the others, and the scaling columns' second
+    # operand), which runs 960 multiply-adds per SM and cycle, 7.5 times the FP32 pipe's 128
+    fx_tf = fp32_tf * (960.0 / 128.0) / 39.5
+    fx_src = fma_src + "; FP32 rate times 7.5 for mma.sync's FP16 products, divided by 39.5 products per multiply-add"
     roofs = {
         "fp64": roof("fp64", st_ser["kernel_ms_fp64"], fx_tf, "apply_fx_kernel<10>", "tensor (62-bit fixed point)", fx_src),
         # the FP32-accuracy tier of the mixed step runs on the tensor cores as split TF32: per tile
