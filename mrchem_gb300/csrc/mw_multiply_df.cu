@@ -17,7 +17,7 @@
 // with M_out, the last writing the FP64 block and its norms.
 //
 // Arithmetic: every value is an unevaluated FP32 pair (hi + lo) and every multiply-add is the
-// error-free double-FP32 update of the apply's double-FP32 tier, as in the post-processing
+// error-free double-FP32 update (Dekker / Knuth transformations), as in the post-processing
 // transforms (mw_post_df.cu): about (2K + 4) 2^-48 of sum |M| |x| per pass, 1e-14 relative, at
 // about 8x GB300's FP64 rate.  Blocks in global memory stay FP64; norms are summed in FP64.  The
 // FP64 blocks are split into FP32 pairs and joined back with integer operations (mw_dfconv.cuh),

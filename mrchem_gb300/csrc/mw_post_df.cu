@@ -10,7 +10,7 @@
 // Each node costs 3 (2K)^4 multiply-adds, which GB300's FP64 pipe (about
 // 1.7 FMA per clock per SM) turns into ~140 us per node and SM.  Here every
 // value is an unevaluated FP32 pair (hi + lo) and every multiply-add is the
-// error-free double-FP32 update of the double-FP32 apply tier, so a pass is
+// error-free double-FP32 update (Dekker / Knuth transformations), so a pass is
 // accurate to about (2K + 4) 2^-48 of sum |W| |x| -- 1e-14 relative, far below
 // any precision an apply is asked for -- at ~8x the FP64 rate.  The blocks in
 // global memory stay FP64; the norms are summed in FP64.  The FP64 values are split into FP32
