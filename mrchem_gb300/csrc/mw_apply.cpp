@@ -559,6 +559,29 @@ bool pool_room(int device, size_t bytes) {
     return bytes <= (size_t)(reserved - used) + free_b / 4;
 }
 
+// Memory of the stream-ordered pool for one apply's digits.  It goes back to the pool when the apply has ended
+// (one call of the library may run many applies); after an error, whose work may still be running, when the call
+// has (Ctx::release_retired).
+struct DigitsMemory {
+    Ctx &ctx;
+    void *p = nullptr;
+    explicit DigitsMemory(Ctx &c) : ctx(c) {}
+    DigitsMemory(const DigitsMemory &) = delete;
+    ~DigitsMemory() {
+        if (!p) return;
+        std::lock_guard<std::mutex> lock(ctx.retired_mu);
+        ctx.retired.push_back(p);
+    }
+    void *alloc(size_t bytes) {
+        MWG_CUDA(cudaMallocAsync(&p, std::max<size_t>(bytes, 256), ctx.stream));
+        return p;
+    }
+    void release() {  // the apply's work has ended on every stream
+        if (p) MWG_CUDA(cudaFreeAsync(p, ctx.stream));
+        p = nullptr;
+    }
+};
+
 void ensure_fast(Ctx &ctx) {  // the generation's and screening's high-priority stream
     if (ctx.fast) return;
     int least = 0, greatest = 0;
@@ -1147,6 +1170,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
     const size_t fxw = fx_words(K);
     ctx.sarena.reset();
     bool digits = true;
+    DigitsMemory digits_mem(ctx);
     std::unordered_map<const Tree *, uint32_t *> tree_fx;
     {
         size_t bytes = 0;
@@ -1154,11 +1178,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
             if (tree_fx.emplace(s.job->inp, nullptr).second) bytes += sizeof(uint32_t) * fxw * (size_t)s.job->inp->nn();
         digits = pool_room(ctx.device, bytes);
         uint32_t *next = nullptr;
-        if (digits) {  // from the stream-ordered pool, to which it goes back when the call has ended
-            MWG_CUDA(cudaMallocAsync(&next, std::max<size_t>(bytes, 256), ctx.stream));
-            std::lock_guard<std::mutex> lock(ctx.retired_mu);
-            ctx.retired.push_back(next);
-        }
+        if (digits) next = (uint32_t *)digits_mem.alloc(bytes);
         for (JobState &s : js) {
             if (!digits) break;
             uint32_t *&d = tree_fx[s.job->inp];
@@ -1815,6 +1835,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
     MWG_CUDA(cudaEventRecord(ev_span[1], ctx.stream));
     MWG_CUDA(cudaEventRecord(ev_span[2], ctx.stream));
     ctx.sync();
+    digits_mem.release();
     for (auto &p : cn_staging) std::copy(p.second, p.second + 8 * (size_t)p.first->nn(), p.first->cn.begin());
     arena.reset();
     for (int g = 1; g < ngroups; g++) ctx.xarena[g - 1].reset();
