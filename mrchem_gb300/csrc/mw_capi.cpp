@@ -41,6 +41,9 @@ int guard(mwg::Ctx *ctx, F &&f) {
         (ctx ? ctx->err : g_noctx_err) = e.what();
         rc = MW_ERR_STATE;
     }
+    // a call that failed half-way may have left work on any stream: it ends before the caller can free or reuse
+    // what that work reads and writes
+    if (ctx && rc != MW_OK) ctx->wait_idle();
     // device arrays that trees outgrew during the call, released once the call's work is done
     if (ctx) ctx->release_retired();
     return rc;
@@ -128,13 +131,7 @@ int mw_ctx_create(int device, int root_scale, const int corner[3], const int box
 static void ctx_free(mw_ctx c) {
     cudaSetDevice(c->ctx.device);
     c->ctx.release_retired();
-    cudaStreamSynchronize(c->ctx.stream);
-    for (auto &xs : c->ctx.xstream)
-        if (xs) cudaStreamSynchronize(xs);
-    if (c->ctx.fast) cudaStreamSynchronize(c->ctx.fast);
-    if (c->ctx.ustream) cudaStreamSynchronize(c->ctx.ustream);
-    for (auto &ps : c->ctx.pstream)
-        if (ps) cudaStreamSynchronize(ps);
+    c->ctx.wait_idle();
     c->ctx.arena.release();
     c->ctx.sarena.release();
     for (auto &xa : c->ctx.xarena) xa.release();

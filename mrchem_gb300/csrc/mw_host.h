@@ -250,6 +250,8 @@ struct Ctx {
     std::vector<void *> retired;
     std::mutex retired_mu;  // trees of one call may grow on several host threads
     void release_retired();
+    // waits for every stream of the context; no error is reported
+    void wait_idle();
 };
 
 // Packs host arrays into the context's pinned buffer and ships them to the

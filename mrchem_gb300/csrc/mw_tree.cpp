@@ -113,12 +113,19 @@ void *Ctx::pinned(size_t bytes) {
 
 void Ctx::sync() { MWG_CUDA(cudaStreamSynchronize(stream)); }
 
-void Ctx::release_retired() {
-    if (retired.empty()) return;
-    cudaStreamSynchronize(stream);
+void Ctx::wait_idle() {
+    if (stream) cudaStreamSynchronize(stream);
     for (auto &xs : xstream)
         if (xs) cudaStreamSynchronize(xs);
+    for (auto &ps : pstream)
+        if (ps) cudaStreamSynchronize(ps);
     if (fast) cudaStreamSynchronize(fast);
+    if (ustream) cudaStreamSynchronize(ustream);
+}
+
+void Ctx::release_retired() {
+    if (retired.empty()) return;
+    wait_idle();
     for (void *p : retired) cudaFreeAsync(p, stream);  // back to the pool, which keeps it for reuse
     retired.clear();
 }
