@@ -807,6 +807,7 @@ int mw_rotate(int nout, mw_tree *outs, int nin, const mw_tree *ins, const double
         std::vector<const mwg::Tree *> in;
         for (int i = 0; i < nout; i++) {
             if (!outs[i]) throw mwg::Error(MW_ERR_ARG, "rotate: null output");
+            check_same(outs[0]->tree, outs[i]->tree);  // one launch on one stream writes them all
             o.push_back(&outs[i]->tree);
         }
         for (int j = 0; j < nin; j++) {

@@ -57,3 +57,14 @@ def test_coefficients_that_are_not_finite_reach_every_value(engine, oracle, valu
     c = s.download()[1]
     # infinity times a zero coefficient is NaN, times any other infinite
     assert not np.isfinite(c).any()
+
+
+@pytest.mark.parametrize("other", [4, 6])
+def test_rotate_refuses_outputs_of_another_context(engine, oracle, other):
+    # one launch writes all outputs: of another context they have a stream, and here an order, of their own
+    mra, omra = engine.MultiResolutionAnalysis(6), oracle.MRA(6)
+    ins = [engine.FunctionTree(mra).upload(*t.export()[:2]) for t in trees(oracle, omra, 1e-3)[:2]]
+    a, b = engine.FunctionTree(mra), engine.FunctionTree(engine.MultiResolutionAnalysis(other))
+    for outs in ([a, b], [b, a]):
+        with pytest.raises(engine.MWError, match="different contexts"):
+            engine.rotate(outs, ins, np.eye(2))
