@@ -886,13 +886,17 @@ __global__ void add_kernel(DevBasis b, const AddTask *tasks, const double *const
 // every input again for each).  Bound: the FP64 pipe (1.6 multiply-adds per SM and cycle: NO per element
 // and input) for rotations of many inputs, HBM for sums of a few; the zero wavelet parts of generated
 // blocks are neither stored nor multiplied.  The sums run in input order, as add_kernel's.
+constexpr int COMBINE_SHARED = 16384;  // coefficients that fit in shared memory (128 KB)
+
 template <int NO>
 __global__ void __launch_bounds__(256) combine_kernel(CombineArgs A) {
     __shared__ double s_red[8][NO];
-    extern __shared__ double s_u[];  // [input][NO]
+    extern __shared__ double s_u[];  // [input][NO]; more inputs than it holds: NO = 1, read from A.U
     const int K3 = A.K * A.K * A.K, bs = 8 * K3, o0 = blockIdx.y * NO, no = min(NO, A.nout - o0);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < A.nin * NO; i += blockDim.x) {
+    const bool wide = NO == 1 && A.nin > COMBINE_SHARED;
+    const double *coef = wide ? A.U + (size_t)o0 * A.nin : s_u;
+    for (int i = threadIdx.x; i < A.nin * NO && !wide; i += blockDim.x) {
         const int k = i / NO, o = i % NO;
         s_u[i] = o < no ? A.U[(size_t)(o0 + o) * A.nin + k] : 0.0;
     }
@@ -911,7 +915,7 @@ __global__ void __launch_bounds__(256) combine_kernel(CombineArgs A) {
                     const unsigned tr = __ldg(A.tree + f + k);
                     if (c > 0 && (tr >> 31)) continue;
                     const double x = __ldg(A.src[f + k] + (size_t)c * K3 + i);
-                    const double *u = s_u + (tr & 0x7fffffffu) * NO;
+                    const double *u = coef + (tr & 0x7fffffffu) * NO;
 #pragma unroll
                     for (int o = 0; o < NO; o++) acc[o] += u[o] * x;
                 }
@@ -941,7 +945,7 @@ __global__ void __launch_bounds__(256) combine_kernel(CombineArgs A) {
 
 template <int NO>
 void launch_combine(const CombineArgs &A, cudaStream_t s) {
-    const size_t smem = sizeof(double) * (size_t)A.nin * NO;
+    const size_t smem = NO == 1 && A.nin > COMBINE_SHARED ? 0 : sizeof(double) * (size_t)A.nin * NO;
     if (smem > 40 * 1024) kernel_smem((const void *)combine_kernel<NO>, (int)smem);
     combine_kernel<NO><<<dim3(std::min(A.n, 65535), (A.nout + NO - 1) / NO), 256, smem, s>>>(A);
     MWG_CUDA(cudaGetLastError());

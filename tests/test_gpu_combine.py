@@ -68,3 +68,23 @@ def test_rotate_refuses_outputs_of_another_context(engine, oracle, other):
     for outs in ([a, b], [b, a]):
         with pytest.raises(engine.MWError, match="different contexts"):
             engine.rotate(outs, ins, np.eye(2))
+
+
+@pytest.mark.parametrize("n,nout", [(16385, 1), (30001, 1), (16384, 2)])
+def test_sums_of_more_trees_than_shared_memory_has_coefficients_for(engine, oracle, n, nout):
+    # the same few trees many times over; against their sum with the added coefficients, whose rounding differs by
+    # at most n roundings of the sum of absolute values
+    mra, omra = engine.MultiResolutionAnalysis(3), oracle.MRA(3)
+    ins = [engine.FunctionTree(mra).upload(*t.export()[:2]) for t in trees(oracle, omra, 1e-1)[:3]]
+    U = np.random.default_rng(n).standard_normal((nout, n))
+    outs = [engine.FunctionTree(mra) for _ in range(nout)]
+    many = [ins[k % 3] for k in range(n)]
+    if nout == 1:
+        engine.add(1e-1, outs[0], list(zip(U[0], many)))
+    else:
+        engine.rotate(outs, many, U)
+    for o, row in zip(outs, U):
+        s = engine.FunctionTree(mra)
+        engine.add(1e-1, s, [(float(np.sum(row[k::3])), ins[k]) for k in range(3)])
+        d = o.download()[1] - s.download()[1]
+        assert np.linalg.norm(d) <= n * 2.3e-16 * np.abs(row).sum() * max(t.norm() for t in ins)
