@@ -129,7 +129,7 @@ struct JobState {
     std::vector<double> fmax_lv;
     double fmax_at(int lv) const { return lv < (int)fmax_lv.size() ? fmax_lv[lv] : fmax; }
     bool fixed_point = true;  // every input norm is finite and far from overflow
-    int *fxneed = nullptr;    // per input node: its digits have been asked for (made on demand only)
+    int *fxslot = nullptr;    // digits on demand: per input node 1 + their place in its level's list, 0: not asked for
     void set_fmax(const Tree &t, int n0) {
         fmax = 0.0;
         fixed_point = true;
@@ -288,8 +288,6 @@ struct DevItems {
     const void **in = nullptr, **ax = nullptr, **ay = nullptr, **az = nullptr;
     double *coef = nullptr;
     long long base[NTIER] = {0, 0, 0, 0};
-    FxBlock *fxlist = nullptr;  // the blocks whose digits the level asks for, where they are made on demand
-    int *fxcnt = nullptr;
     const double *g64 = nullptr;  // the level's generated blocks and the place of their digits
     uint32_t *gfx = nullptr;
     size_t ngen = 0;
@@ -476,14 +474,12 @@ struct FxLevelOps {
     std::vector<FxOpJob> jobs;
     size_t words = 0, zoff = 0;
     int s = 0;
-    bool add(Oper &op, Arena &ar) {
-        if (base.count(&op)) return true;
-        if (!op.d_screen) return false;
+    void add(Oper &op, Arena &ar) {
+        if (base.count(&op)) return;
         const int n = op.fx_count[s];
         uint32_t *b = (uint32_t *)ar.alloc(sizeof(uint32_t) * words * (size_t)std::max(n, 1));
         base.emplace(&op, b);
         jobs.push_back(FxOpJob{oper_screen_view(op), b, s, n});
-        return true;
     }
     const uint32_t *block(const Oper &op, int t, int l) const {
         return base.at(&op) + words * (size_t)(op.fx_first[t * op.S + s] + op.band[t * op.S + s] + l);
@@ -661,7 +657,7 @@ void screen_setup_inputs(Ctx &ctx, std::vector<ApplyJob> &jobs, const std::vecto
         J.in32 = t.d_coefs32;
         J.intc = t.d_coefs_tc;
         J.infx = js[j].fx;
-        J.fxneed = js[j].fxneed;
+        J.fxslot = js[j].fxslot;
     }
     // read by kernels from the pinned staging: with host inputs these tables go up while the later
     // job groups' input blocks still occupy the copy engines
@@ -737,7 +733,7 @@ constexpr size_t SCREEN_SMEM_MAX = 136 * 1024;  // larger walks (very wide bands
 // screening does.  The group's stream waits for the item arrays with an event.
 void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobState *> &jp,
                       const std::vector<int> &jglob, int level, int zmax, const TierRule &rule, LevelItems *lt,
-                      const FxLevelOps *fxops, DevItems &dv, mw_stats &st, double &t_enum, double &t_gen, double &t_items) {
+                      FxLevelOps *fxops, bool on_demand, DevItems &dv, mw_stats &st, double &t_enum, double &t_gen, double &t_items) {
     const Basis &b = ctx.basis;
     const int K = b.K, bs = b.bs, bsz = 4 * K * K;
     const double K4 = (double)K * K * K * K;
@@ -903,33 +899,38 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
     P.g64 = (double *)ar.alloc(sizeof(double) * (size_t)bs * ng);
     P.g32 = rule.fp32() ? (float *)ar.alloc(sizeof(float) * (size_t)bs * ng) : nullptr;
     P.gtc = rule.tensor ? (float *)ar.alloc(sizeof(float) * P.tx * ng) : nullptr;
-    P.fx = fxops ? fx_words(K) : 0;
-    P.gfx = fxops ? (uint32_t *)ar.alloc(sizeof(uint32_t) * P.fx * ng) : nullptr;
-    dv.g64 = P.g64;
-    dv.gfx = P.gfx;
-    dv.ngen = fxops ? (size_t)ngen : 0;
-    if (fxops && jp[0]->fxneed) {
+    P.part = on_demand ? 1 : 3;
+    if (on_demand) {
         size_t most = ng;
         for (JobState *sp : jp) most += (size_t)sp->job->inp->nn();
-        dv.fxlist = P.fxlist = (FxBlock *)ar.alloc(sizeof(FxBlock) * most);
-        dv.fxcnt = P.fxcnt = (int *)ar.alloc(sizeof(int) * (1 + ng));
-        P.gneed = P.fxcnt + 1;
+        P.fxlist = (const double **)ar.alloc(sizeof(double *) * most);
+        P.fxcnt = (int *)ar.alloc(sizeof(int) * (1 + ng));
+        P.gslot = P.fxcnt + 1;
+    } else if (fxops) {
+        P.fx = fx_words(K);
+        P.gfx = (uint32_t *)ar.alloc(sizeof(uint32_t) * P.fx * ng);
+        dv.g64 = P.g64;
+        dv.gfx = P.gfx;
+        dv.ngen = (size_t)ngen;
     }
-    std::vector<const uint32_t *> fxop;  // per job of the apply its operator's digits
-    if (fxops) {
+    auto op_digits = [&] {  // per job of the apply its operator's digits
         P.fxo = fxops->words;
         P.fxz = fxops->zoff;
-        fxop.resize(*std::max_element(jglob.begin(), jglob.end()) + 1, nullptr);
+        std::vector<const uint32_t *> fxop(*std::max_element(jglob.begin(), jglob.end()) + 1, nullptr);
         for (size_t j = 0; j < jp.size(); j++) fxop[jglob[j]] = fxops->base.at(jp[j]->job->op);
-    }
-    int *hs = (int *)ar.halloc(sizeof(int) * (8 * (size_t)NN + 1));
+        return fxop;
+    };
+    int *hs = (int *)ar.halloc(sizeof(int) * (8 * (size_t)NN + 2));
+    hs[8 * NN + 1] = 0;
     {
         StreamSwap fast(ctx, ctx.fast);
+        std::vector<const uint32_t *> fxop;
+        if (fxops && !on_demand) fxop = op_digits();
         Packer pk;
         pk.add(coff.data(), sizeof(long long) * NN);
         pk.add(fxop.data(), sizeof(uint32_t *) * fxop.size());
         pk.ship(ctx, ar);
-        if (P.fxlist) MWG_CUDA(cudaMemsetAsync(P.fxcnt, 0, sizeof(int) * (1 + ng), ctx.stream));
+        if (on_demand) MWG_CUDA(cudaMemsetAsync(P.fxcnt, 0, sizeof(int) * (1 + ng), ctx.stream));
         P.cand_off = (const long long *)pk.ptr(0);
         P.fxop = (const uint32_t *const *)pk.ptr(1);
         if (ngen > 0) {
@@ -959,6 +960,8 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
         st.launches += 2;
         MWG_CUDA(cudaMemcpyAsync(hs, P.tcnt, sizeof(int) * 8 * NN, cudaMemcpyDeviceToHost, ctx.stream));
         MWG_CUDA(cudaMemcpyAsync(hs + 8 * NN, P.overflow, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
+        if (on_demand)
+            MWG_CUDA(cudaMemcpyAsync(hs + 8 * NN + 1, P.fxcnt, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
         MWG_CUDA(cudaEventRecord(ds.ev_counts, ctx.stream));
         k_screen_fill(P, ctx.stream);
         st.launches++;
@@ -1009,6 +1012,28 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
     st.flops_tf32 += 6.0 * K4 * (double)pairs[2];
     st.flops_df += 6.0 * K4 * (double)pairs[3];
     t_items += ms(tD, now());
+    // the items of tiers 0 and 3, and the digits of what they read: room for the blocks that they ask for
+    if (on_demand && tot[0] + tot[3] > 0) {
+        const size_t n = (size_t)hs[8 * NN + 1];
+        std::vector<const uint32_t *> fxop;
+        if (fxops) {
+            for (JobState *sp : jp) fxops->add(*sp->job->op, ar);
+            fxops->make(ctx, st);
+            fxop = op_digits();
+            P.fx = fx_words(K);
+            uint32_t *base = (uint32_t *)ar.alloc(sizeof(uint32_t) * P.fx * n);
+            P.fxbase = base;
+            k_to_fx_list(P.fxlist, base, n, K, ctx.stream);
+            st.launches++;
+        }
+        Packer pk;
+        pk.add(fxop.data(), sizeof(uint32_t *) * fxop.size());
+        pk.ship(ctx, ar);
+        P.fxop = (const uint32_t *const *)pk.ptr(0);
+        P.part = 2;
+        k_screen_fill(P, ctx.stream);
+        st.launches++;
+    }
 }
 
 void check_status(const int *hs) {
@@ -1161,18 +1186,17 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         s.R = 1.0;
     }
     // Digits up front (inputs' once, operators' beside a level's screening) where most items need them; in the
-    // other modes a level that has such items makes those of the blocks that its items ask for (few of the
-    // 125 thousand input nodes of 528 exchange products: 70 ms on demand)
+    // other modes a level that has such items makes those of the blocks that its items ask for, in the group's
+    // arena (few of the 125 thousand input nodes of 528 exchange products, whose digits would take 7 GB)
     const bool ops_first = !mixed || near_fp64 || df_only;
-    // The digits of every distinct input tree (the FP64 and double-FP32 tiers' fixed-point kernel), for the
-    // length of the call.  They take 1.8 times the blocks' own space: trees that would not leave room for
-    // them go to the kernel that reads the FP64 blocks.
+    // Up front, the digits of every distinct input tree are held for the length of the apply.  They take 1.8 times
+    // the blocks' own space: trees that would not leave room for them go to the kernel that reads the FP64 blocks.
     const size_t fxw = fx_words(K);
     ctx.sarena.reset();
     bool digits = true;
     DigitsMemory digits_mem(ctx);
     std::unordered_map<const Tree *, uint32_t *> tree_fx;
-    {
+    if (ops_first) {
         size_t bytes = 0;
         for (JobState &s : js)
             if (tree_fx.emplace(s.job->inp, nullptr).second) bytes += sizeof(uint32_t) * fxw * (size_t)s.job->inp->nn();
@@ -1188,15 +1212,14 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
             }
             s.fx = d;
         }
-        if (digits && !ops_first) {
-            size_t total = 0;
-            for (JobState &s : js) total += (size_t)s.job->inp->nn();
-            int *need = (int *)ctx.sarena.alloc(sizeof(int) * total);
-            MWG_CUDA(cudaMemsetAsync(need, 0, sizeof(int) * total, ctx.stream));
-            for (JobState &s : js) {
-                s.fxneed = need;
-                need += s.job->inp->nn();
-            }
+    } else {
+        size_t total = 0;
+        for (JobState &s : js) total += (size_t)s.job->inp->nn();
+        int *slot = (int *)ctx.sarena.alloc(sizeof(int) * total);
+        MWG_CUDA(cudaMemsetAsync(slot, 0, sizeof(int) * total, ctx.stream));
+        for (JobState &s : js) {
+            s.fxslot = slot;
+            slot += s.job->inp->nn();
         }
     }
     auto to_digits = [&](const std::vector<int> &which) {  // of these jobs' trees, each once
@@ -1321,8 +1344,11 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         fxops.words = fx_op_words(K);
         fxops.zoff = fx_op_z(K);
         fxops.s = sidx;
-        for (JobState *sp : jp) fixed_point = fixed_point && fxops.add(*sp->job->op, ar);
-        if (fixed_point && ops_first) fxops.make(ctx, st);
+        for (JobState *sp : jp) fixed_point = fixed_point && sp->job->op->d_screen;
+        if (fixed_point && ops_first) {
+            for (JobState *sp : jp) fxops.add(*sp->job->op, ar);
+            fxops.make(ctx, st);
+        }
         // thresholds and precision-steering weights
         for (JobState *sp : jp) {
             JobState &s = *sp;
@@ -1337,8 +1363,8 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         const int zmax = ds.on ? level_zrows(jp, sidx) : 0;
         const bool dscreen = ds.on && level < ds.levels && screen_smem(ds.maxT, zmax) <= SCREEN_SMEM_MAX;
         if (dscreen) {
-            screen_level_gpu(ctx, ar, ds, jp, G.jobs, level, zmax, rule, G.lt, fixed_point ? &fxops : nullptr, dv, st, st.host_enum_ms,
-                             st.host_gen_ms, st.host_items_ms);
+            screen_level_gpu(ctx, ar, ds, jp, G.jobs, level, zmax, rule, G.lt, fixed_point ? &fxops : nullptr, !ops_first, dv, st,
+                             st.host_enum_ms, st.host_gen_ms, st.host_items_ms);
         } else {
             // phase A: candidate enumeration (host, all the group's nodes in parallel)
             auto tA = std::chrono::steady_clock::now();
@@ -1408,10 +1434,10 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                     st.launches++;
                 }
                 uint32_t *firstfx = nullptr;
-                if (fixed_point && total > 0) firstfx = (uint32_t *)ar.alloc(sizeof(uint32_t) * fxw * total);
+                if (fixed_point && ops_first && total > 0) firstfx = (uint32_t *)ar.alloc(sizeof(uint32_t) * fxw * total);
                 dv.g64 = first;
                 dv.gfx = firstfx;
-                dv.ngen = total;
+                dv.ngen = firstfx ? total : 0;
                 for (JobState *sp : jp) {
                     JobState &s = *sp;
                     s.gbase = s.gens.base;
@@ -1494,6 +1520,34 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                 ntot[k] = cnt[k][NN];
                 lt[k].resize(nnt[k], ntot[k]);
             }
+            // digits on demand: those of the blocks that the items of tiers 0 and 3 ask for, one after the other
+            std::vector<std::vector<uint32_t>> in_slot(jp.size()), gen_slot(jp.size());  // 1 + place, 0: not asked for
+            const uint32_t *fxbase = nullptr;
+            if (fixed_point && !ops_first && ntot[0] + ntot[3] > 0) {
+                std::vector<const double *> list;
+                for (size_t j = 0; j < jp.size(); j++) {
+                    JobState &s = *jp[j];
+                    in_slot[j].assign(s.job->inp->nn(), 0);
+                    gen_slot[j].assign(s.gens.keys.size(), 0);
+                    for (const auto &cv : s.cand)
+                        for (const Cand &cd : cv) {
+                            if (cd.tier != 0 && cd.tier != 3) continue;
+                            uint32_t &at = cd.gen ? gen_slot[j][cd.src] : in_slot[j][cd.src];
+                            if (at) continue;
+                            list.push_back(cd.gen ? s.gbase + (size_t)cd.src * bs : s.job->inp->block(cd.src));
+                            at = (uint32_t)list.size();
+                        }
+                }
+                for (JobState *sp : jp) fxops.add(*sp->job->op, ar);
+                fxops.make(ctx, st);
+                uint32_t *base = (uint32_t *)ar.alloc(sizeof(uint32_t) * fxw * list.size());
+                fxbase = base;
+                Packer pk;
+                pk.add(list.data(), list.size() * sizeof(double *));
+                pk.ship(ctx, ar);
+                k_to_fx_list((const double *const *)pk.ptr(0), base, list.size(), K, ctx.stream);
+                st.launches++;
+            }
     #pragma omp parallel for schedule(dynamic, 4)
             for (long q = 0; q < NN; q++) {
                 JobState &s = *jp[nodes_flat[q].first];
@@ -1517,7 +1571,10 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                     long long &pi = p[cd.tier];
                     if (cd.tier == 0 || cd.tier == 3) {
                         if (fixed_point) {
-                            T.in[pi] = cd.gen ? s.gbase_fx + fxw * (size_t)cd.src : s.fx + fxw * (size_t)cd.src;
+                            if (fxbase)
+                                T.in[pi] = fxbase + fxw * (size_t)((cd.gen ? gen_slot : in_slot)[nodes_flat[q].first][cd.src] - 1);
+                            else
+                                T.in[pi] = cd.gen ? s.gbase_fx + fxw * (size_t)cd.src : s.fx + fxw * (size_t)cd.src;
                             T.ax[pi] = fxops.block(op, cd.t, cd.lx);
                             T.ay[pi] = fxops.block(op, cd.t, cd.ly);
                             T.az[pi] = fxops.block(op, cd.t, cd.lz) + fxops.zoff;
@@ -1565,35 +1622,10 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         const auto tD = std::chrono::steady_clock::now();
         MWG_CUDA(cudaEventRecord(G.ev[0], ctx.stream));
         G.status.clear();
-        if (fixed_point && lt[0].items + lt[3].items > 0) {
-            if (!ops_first) fxops.make(ctx, st);
-            if (!ops_first && !dscreen) {  // screened on the host: its items' input nodes
-                std::vector<FxBlock> list;
-                for (JobState *sp : jp) {
-                    std::vector<char> seen(sp->job->inp->nn(), 0);
-                    for (const auto &cv : sp->cand)
-                        for (const Cand &cd : cv)
-                            if ((cd.tier == 0 || cd.tier == 3) && !cd.gen && !seen[cd.src]) {
-                                seen[cd.src] = 1;
-                                list.push_back(FxBlock{sp->job->inp->block(cd.src), sp->fx + fxw * (size_t)cd.src});
-                            }
-                }
-                const int count = (int)list.size();
-                Packer pk;
-                pk.add(list.data(), list.size() * sizeof(FxBlock));
-                pk.add(&count, sizeof count);
-                pk.ship(ctx, ar);
-                if (count > 0) k_to_fx_list((const FxBlock *)pk.ptr(0), (const int *)pk.ptr(1), list.size(), K, ctx.stream);
-                st.launches += count > 0;
-            }
-            if (dv.fxlist) {
-                k_to_fx_list(dv.fxlist, dv.fxcnt, (size_t)(lt[0].items + lt[3].items), K, ctx.stream);
-                st.launches++;
-            } else if (dv.ngen > 0) {
-                const FxBlocks gen{dv.g64, dv.gfx, dv.ngen};
-                k_to_fx(&gen, 1, K, ctx.stream);
-                st.launches++;
-            }
+        if (dv.ngen > 0 && lt[0].items + lt[3].items > 0) {
+            const FxBlocks gen{dv.g64, dv.gfx, dv.ngen};
+            k_to_fx(&gen, 1, K, ctx.stream);
+            st.launches++;
         }
         for (int k = 0; k < NTIER; k++) {
             int *hs = launch_tier(ctx, ar, lt[k], root, false, k, tune.chunk[k], st, dscreen ? &dv : nullptr,

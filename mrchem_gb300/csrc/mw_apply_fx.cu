@@ -367,8 +367,7 @@ struct FxSets {
     uint32_t *out[MAX];
     long long first[MAX + 1];  // blocks of the sets before
     int n;
-    const FxBlock *list;    // or these *count blocks, at most first[1] (n = 1)
-    const int *count;
+    const double *const *list;  // or (n = 1): these blocks
     const PairTask *pairs;  // or (n = 1): pairs' parents, or the cubes of their children's scaling parts (up)
     int up;
 };
@@ -434,19 +433,14 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS) to_fx_kernel(__grid_constan
     constexpr int N2 = G::N2, K2 = G::K2, K3 = G::K3;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const size_t cs = (size_t)(S.pairs && S.up ? 8 : 1) * K3;  // distance of a block's components
-    const long long nb = S.list ? *S.count : S.first[S.n];
+    const long long nb = S.first[S.n];
     for (long long b = blockIdx.x; b < nb; b += gridDim.x) {
-        const double *in;
-        uint32_t *o;
-        if (S.list) {
-            in = S.list[b].in;
-            o = S.list[b].out;
-        } else {
-            int k = 0;
-            while (b >= S.first[k + 1]) k++;
-            in = S.pairs ? (S.up ? S.pairs[b].child0 : S.pairs[b].parent) : S.in[k] + (size_t)(b - S.first[k]) * 8 * K3;
-            o = S.out[k] + (size_t)(b - S.first[k]) * G::IN_WORDS;
-        }
+        int k = 0;
+        while (b >= S.first[k + 1]) k++;
+        const double *in = S.list    ? S.list[b]
+                           : S.pairs ? (S.up ? S.pairs[b].child0 : S.pairs[b].parent)
+                                     : S.in[k] + (size_t)(b - S.first[k]) * 8 * K3;
+        uint32_t *o = S.out[k] + (size_t)(b - S.first[k]) * G::IN_WORDS;
         auto at = [&](int X, int Y, int Z) -> double {
             if (X >= N2 || Y >= N2) return 0.0;
             const int cx = X >= K, cy = Y >= K, cz = Z >= K;
@@ -988,12 +982,12 @@ void k_to_fx(const FxBlocks *sets, size_t n, int K, cudaStream_t s) {
     }
 }
 
-void k_to_fx_list(const FxBlock *list, const int *n, size_t most, int K, cudaStream_t s) {
+void k_to_fx_list(const double *const *list, uint32_t *out, size_t n, int K, cudaStream_t s) {
     FxSets S{};
     S.n = 1;
-    S.first[1] = (long long)std::min<size_t>(most, 2048);  // the launch's CTAs; they go through the list
+    S.out[0] = out;
+    S.first[1] = (long long)n;
     S.list = list;
-    S.count = n;
     to_fx(S, K, s);
 }
 

@@ -387,12 +387,8 @@ struct FxBlocks {  // n consecutive blocks
     size_t n;
 };
 void k_to_fx(const FxBlocks *sets, size_t n, int K, cudaStream_t s);
-// digits of *n listed blocks (both in device memory), at most `most`
-struct FxBlock {
-    const double *in;
-    uint32_t *out;
-};
-void k_to_fx_list(const FxBlock *list, const int *n, size_t most, int K, cudaStream_t s);
+// digits of n listed blocks (the list in device memory), one after the other from `out` on
+void k_to_fx_list(const double *const *list, uint32_t *out, size_t n, int K, cudaStream_t s);
 // digits of n pairs' parent blocks, or (up) of the cubes of their children's scaling parts
 void k_pairs_to_fx(const PairTask *pairs, bool up, uint32_t *out, size_t n, int K, cudaStream_t s);
 void k_norms(const DevBasis &b, double *const *blocks, double *const *cn, int n, cudaStream_t s);
@@ -513,7 +509,7 @@ struct ScreenJob {  // one job of the apply (device)
     const double *in64;  // the input's blocks and shadows
     const float *in32, *intc;
     const uint32_t *infx;  // digits of the fixed-point FP64 tier (fx words per block), or null: FP64 blocks
-    int *fxneed;           // per block: an item of the fixed-point tiers has asked for its digits (ScreenLevel::fxlist)
+    int *fxslot;           // digits on demand, per block: 1 + its place in the level's list, 0: not asked for
 };
 struct ScreenNode {  // one output node of the level (device)
     double thr, thr2;      // screening threshold of the walk, and of the items after generation
@@ -558,10 +554,13 @@ struct ScreenLevel {
     double *g64;                // generated blocks and their shadows
     float *g32, *gtc;
     uint32_t *gfx;
-    // where the digits are made on demand: the blocks that a level's items ask for first, their number and the
-    // generated blocks' flags; else null
-    FxBlock *fxlist;
-    int *fxcnt, *gneed;
+    // where the digits are made on demand: the blocks that the level's items ask for, in the order of their places,
+    // their number, the generated blocks' places (as ScreenJob::fxslot) and, for k_screen_fill's tiers 0 and 3, the
+    // first one's digits; else null
+    const double **fxlist;
+    int *fxcnt, *gslot;
+    const uint32_t *fxbase;
+    int part;                   // k_screen_fill writes the items of tiers 1, 2 (bit 0) and of tiers 0, 3 (bit 1)
     const uint32_t *const *fxop;  // per job its operator's digits at this scale
     size_t fxo, fxz;            // words per operator block, and the place of the z pass's operand in it
     size_t fx;                  // words per block of the fixed-point digits; 0: the FP64 tier reads FP64 blocks

@@ -569,6 +569,14 @@ __global__ void __launch_bounds__(ST) screen_kernel(ScreenLevel P, int maxT, int
                     cd.tier = (unsigned char)it.tier;
                     cd.gen = (unsigned char)it.gen;
                     cd.t = t;
+                    if (P.fxlist && (it.tier == 0 || it.tier == 3)) {
+                        int *place = it.gen ? P.gslot + it.src : J.fxslot + it.src;
+                        if (atomicCAS(place, 0, -1) == 0) {  // the first to ask
+                            const int at = atomicAdd(P.fxcnt, 1);
+                            P.fxlist[at] = (it.gen ? P.g64 : J.in64) + (size_t)it.src * P.bs;
+                            *place = at + 1;
+                        }
+                    }
                 }
                 written += total;
             }
@@ -675,20 +683,20 @@ __global__ void __launch_bounds__(FT) fill_kernel(ScreenLevel P) {
         }
         unsigned total;
         const unsigned pre = block_scan<unsigned, FT>(onehot, wsum, &total);
-        if (i < m) {
+        const bool fixed = tier == 0 || tier == 3;  // the same kernel, or for both the FP64 one
+        if (i < m && ((P.part >> (fixed ? 1 : 0)) & 1)) {
             const long long dst = s_run[tier] + ((pre >> (8 * tier)) & 255);
             const long ob = (long)op.off[cd.t * S + s] + op.band[cd.t * S + s];
             const size_t bx = (size_t)(ob + cd.lx), by = (size_t)(ob + cd.ly), bz = (size_t)(ob + cd.lz);
             const size_t src = (size_t)cd.src;
-            if (tier == 0 || tier == 3) {  // the same kernel, or for both the FP64 one
+            if (fixed) {
                 if (P.fx) {
-                    if (P.fxlist && atomicExch(cd.gen ? P.gneed + src : J.fxneed + src, 1) == 0)
-                        P.fxlist[atomicAdd(P.fxcnt, 1)] =
-                            cd.gen ? FxBlock{P.g64 + src * P.bs, P.gfx + P.fx * src}
-                                   : FxBlock{J.in64 + src * P.bs, const_cast<uint32_t *>(J.infx) + P.fx * src};
                     const uint32_t *b = P.fxop[nd.job] + P.fxo * (size_t)(op.first[cd.t * S + s] + op.band[cd.t * S + s]);
                     const long o = (long)P.fxo;
-                    P.in[dst] = cd.gen ? (const void *)(P.gfx + P.fx * src) : (const void *)(J.infx + P.fx * src);
+                    if (P.fxlist)
+                        P.in[dst] = P.fxbase + P.fx * (size_t)((cd.gen ? P.gslot[src] : J.fxslot[src]) - 1);
+                    else
+                        P.in[dst] = cd.gen ? (const void *)(P.gfx + P.fx * src) : (const void *)(J.infx + P.fx * src);
                     P.ax[dst] = b + o * cd.lx;
                     P.ay[dst] = b + o * cd.ly;
                     P.az[dst] = b + o * cd.lz + P.fxz;

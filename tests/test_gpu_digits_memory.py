@@ -53,3 +53,41 @@ def test_autotuner_holds_the_digits_of_one_apply(engine, precision):
     tuned = pool.most(lambda: engine.autotune_batch([prec] * n, outs, Hs, fs, precision=precision, repeats=2))
     # the digits' 1.8 times the inputs of some 40 applies, were they held, against the same for one
     assert tuned <= 1.25 * single, (tuned, single)
+
+
+def test_digits_on_demand_take_no_room_for_every_input_node(engine):
+    # the norm-tiered mode converts what the items of its large tiers read, a few of the inputs' nodes
+    n, prec = 3, 1e-4
+    mra, fs, Hs, outs = batch(engine, 5, n, prec)
+    blocks = sum(8 * f.download()[1].size for f in fs)
+    pool = Pool()
+
+    def one():
+        for o in outs:
+            o.clear()
+        return engine.apply_batch([prec] * n, outs, Hs, fs, precision="mixed")
+
+    st = one()  # grows the outputs' trees to their final size
+    assert st["items_df"] + st["items_fp64"] > 0
+    used = pool.most(lambda: None)
+    assert pool.most(one) - used <= 0.1 * blocks
+
+
+@pytest.mark.parametrize("screening", ["gpu", "host"])
+@pytest.mark.parametrize("precision", ["mixed", "mixed-fp32", "df", "fp64"])
+def test_operators_on_one_input_tree_in_several_groups(engine, precision, screening):
+    # jobs that share an input run in different groups, on streams of their own; each as alone, where only the
+    # order of sums may differ (the mixed modes' FP32 sums: 1e-3 of prec, as the autotuner's test has it)
+    prec, n = 1e-5, 6
+    mra = engine.MultiResolutionAnalysis(7)
+    mra.set_screening(screening)
+    f = engine.project(prec, engine.FunctionTree(mra), [(1.0, 40.0, (0.1, -0.2, 0.3), (1, 0, 0))], abs_prec=True)
+    Hs = [engine.HelmholtzOperator(mra, 0.5 + 0.1 * i, prec) for i in range(n)]
+    outs = [engine.FunctionTree(mra) for _ in Hs]
+    st = engine.apply_batch([prec] * n, outs, Hs, [f] * n, abs_prec=True, precision=precision)
+    assert st["items_df"] + st["items_fp64"] > 0
+    for H, o in zip(Hs, outs):
+        one, d = engine.FunctionTree(mra), engine.FunctionTree(mra)
+        engine.apply(prec, one, H, f, abs_prec=True, precision=precision)
+        engine.add(-1.0, d, [(1.0, o), (-1.0, one)])
+        assert d.norm() <= (2e-2 * prec if precision.startswith("mixed") else 2e-14 * one.norm())
