@@ -474,6 +474,14 @@ struct FxLevelOps {
     std::vector<FxOpJob> jobs;
     size_t words = 0, zoff = 0;
     int s = 0;
+    size_t bytes(const std::vector<const Oper *> &ops) const {  // room that these operators' digits take
+        std::vector<const Oper *> v(ops);
+        std::sort(v.begin(), v.end());
+        size_t b = 0;
+        for (size_t i = 0; i < v.size(); i++)
+            if (i == 0 || v[i] != v[i - 1]) b += ((sizeof(uint32_t) * words * (size_t)std::max(v[i]->fx_count[s], 1)) | 255) + 1;
+        return b;
+    }
     void add(Oper &op, Arena &ar) {
         if (base.count(&op)) return;
         const int n = op.fx_count[s];
@@ -542,8 +550,13 @@ void fx_pairs(Ctx &ctx, Arena &ar, const std::vector<PairTask> &all, bool up, ui
     }
 }
 
-// room for `bytes` from the device's stream-ordered pool: what it holds unused and a quarter of what is free
-bool pool_room(int device, size_t bytes) {
+// room for `bytes` of digits in an arena
+bool arena_room(const Ctx &ctx, const Arena &ar, size_t bytes) { return bytes <= ctx.digits_room && ar.room_for(bytes); }
+
+// ... from the device's stream-ordered pool: what it holds unused and a quarter of what is free
+bool pool_room(const Ctx &ctx, size_t bytes) {
+    if (bytes > ctx.digits_room) return false;
+    const int device = ctx.device;
     size_t free_b = 0, total_b = 0;
     uint64_t reserved = 0, used = 0;
     cudaMemPool_t pool = nullptr;
@@ -733,7 +746,7 @@ constexpr size_t SCREEN_SMEM_MAX = 136 * 1024;  // larger walks (very wide bands
 // screening does.  The group's stream waits for the item arrays with an event.
 void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobState *> &jp,
                       const std::vector<int> &jglob, int level, int zmax, const TierRule &rule, LevelItems *lt,
-                      FxLevelOps *fxops, bool on_demand, DevItems &dv, mw_stats &st, double &t_enum, double &t_gen, double &t_items) {
+                      FxLevelOps &fxops, bool &fixed_point, bool on_demand, DevItems &dv, mw_stats &st, double &t_enum, double &t_gen, double &t_items) {
     const Basis &b = ctx.basis;
     const int K = b.K, bs = b.bs, bsz = 4 * K * K;
     const double K4 = (double)K * K * K * K;
@@ -906,7 +919,10 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
         P.fxlist = (const double **)ar.alloc(sizeof(double *) * most);
         P.fxcnt = (int *)ar.alloc(sizeof(int) * (1 + ng));
         P.gslot = P.fxcnt + 1;
-    } else if (fxops) {
+    } else {
+        fixed_point = fixed_point && arena_room(ctx, ar, sizeof(uint32_t) * fx_words(K) * ng);
+    }
+    if (!on_demand && fixed_point) {
         P.fx = fx_words(K);
         P.gfx = (uint32_t *)ar.alloc(sizeof(uint32_t) * P.fx * ng);
         dv.g64 = P.g64;
@@ -914,10 +930,10 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
         dv.ngen = (size_t)ngen;
     }
     auto op_digits = [&] {  // per job of the apply its operator's digits
-        P.fxo = fxops->words;
-        P.fxz = fxops->zoff;
+        P.fxo = fxops.words;
+        P.fxz = fxops.zoff;
         std::vector<const uint32_t *> fxop(*std::max_element(jglob.begin(), jglob.end()) + 1, nullptr);
-        for (size_t j = 0; j < jp.size(); j++) fxop[jglob[j]] = fxops->base.at(jp[j]->job->op);
+        for (size_t j = 0; j < jp.size(); j++) fxop[jglob[j]] = fxops.base.at(jp[j]->job->op);
         return fxop;
     };
     int *hs = (int *)ar.halloc(sizeof(int) * (8 * (size_t)NN + 2));
@@ -925,7 +941,7 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
     {
         StreamSwap fast(ctx, ctx.fast);
         std::vector<const uint32_t *> fxop;
-        if (fxops && !on_demand) fxop = op_digits();
+        if (fixed_point && !on_demand) fxop = op_digits();
         Packer pk;
         pk.add(coff.data(), sizeof(long long) * NN);
         pk.add(fxop.data(), sizeof(uint32_t *) * fxop.size());
@@ -1016,9 +1032,12 @@ void screen_level_gpu(Ctx &ctx, Arena &ar, DevScreen &ds, const std::vector<JobS
     if (on_demand && tot[0] + tot[3] > 0) {
         const size_t n = (size_t)hs[8 * NN + 1];
         std::vector<const uint32_t *> fxop;
-        if (fxops) {
-            for (JobState *sp : jp) fxops->add(*sp->job->op, ar);
-            fxops->make(ctx, st);
+        std::vector<const Oper *> ops;
+        for (JobState *sp : jp) ops.push_back(sp->job->op);
+        fixed_point = fixed_point && arena_room(ctx, ar, sizeof(uint32_t) * fx_words(K) * n + fxops.bytes(ops));
+        if (fixed_point) {
+            for (JobState *sp : jp) fxops.add(*sp->job->op, ar);
+            fxops.make(ctx, st);
             fxop = op_digits();
             P.fx = fx_words(K);
             uint32_t *base = (uint32_t *)ar.alloc(sizeof(uint32_t) * P.fx * n);
@@ -1200,7 +1219,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         size_t bytes = 0;
         for (JobState &s : js)
             if (tree_fx.emplace(s.job->inp, nullptr).second) bytes += sizeof(uint32_t) * fxw * (size_t)s.job->inp->nn();
-        digits = pool_room(ctx.device, bytes);
+        digits = pool_room(ctx, bytes);
         uint32_t *next = nullptr;
         if (digits) next = (uint32_t *)digits_mem.alloc(bytes);
         for (JobState &s : js) {
@@ -1345,6 +1364,9 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         fxops.zoff = fx_op_z(K);
         fxops.s = sidx;
         for (JobState *sp : jp) fixed_point = fixed_point && sp->job->op->d_screen;
+        std::vector<const Oper *> level_ops;
+        for (JobState *sp : jp) level_ops.push_back(sp->job->op);
+        if (ops_first) fixed_point = fixed_point && arena_room(ctx, ar, fxops.bytes(level_ops));
         if (fixed_point && ops_first) {
             for (JobState *sp : jp) fxops.add(*sp->job->op, ar);
             fxops.make(ctx, st);
@@ -1363,7 +1385,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
         const int zmax = ds.on ? level_zrows(jp, sidx) : 0;
         const bool dscreen = ds.on && level < ds.levels && screen_smem(ds.maxT, zmax) <= SCREEN_SMEM_MAX;
         if (dscreen) {
-            screen_level_gpu(ctx, ar, ds, jp, G.jobs, level, zmax, rule, G.lt, fixed_point ? &fxops : nullptr, !ops_first, dv, st,
+            screen_level_gpu(ctx, ar, ds, jp, G.jobs, level, zmax, rule, G.lt, fxops, fixed_point, !ops_first, dv, st,
                              st.host_enum_ms, st.host_gen_ms, st.host_items_ms);
         } else {
             // phase A: candidate enumeration (host, all the group's nodes in parallel)
@@ -1434,6 +1456,7 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                     st.launches++;
                 }
                 uint32_t *firstfx = nullptr;
+                if (ops_first) fixed_point = fixed_point && arena_room(ctx, ar, sizeof(uint32_t) * fxw * total);
                 if (fixed_point && ops_first && total > 0) firstfx = (uint32_t *)ar.alloc(sizeof(uint32_t) * fxw * total);
                 dv.g64 = first;
                 dv.gfx = firstfx;
@@ -1538,15 +1561,18 @@ void apply_batch(std::vector<ApplyJob> &jobs, int precision_mode, bool fixed_gri
                             at = (uint32_t)list.size();
                         }
                 }
-                for (JobState *sp : jp) fxops.add(*sp->job->op, ar);
-                fxops.make(ctx, st);
-                uint32_t *base = (uint32_t *)ar.alloc(sizeof(uint32_t) * fxw * list.size());
-                fxbase = base;
-                Packer pk;
-                pk.add(list.data(), list.size() * sizeof(double *));
-                pk.ship(ctx, ar);
-                k_to_fx_list((const double *const *)pk.ptr(0), base, list.size(), K, ctx.stream);
-                st.launches++;
+                fixed_point = arena_room(ctx, ar, sizeof(uint32_t) * fxw * list.size() + fxops.bytes(level_ops));
+                if (fixed_point) {
+                    for (JobState *sp : jp) fxops.add(*sp->job->op, ar);
+                    fxops.make(ctx, st);
+                    uint32_t *base = (uint32_t *)ar.alloc(sizeof(uint32_t) * fxw * list.size());
+                    fxbase = base;
+                    Packer pk;
+                    pk.add(list.data(), list.size() * sizeof(double *));
+                    pk.ship(ctx, ar);
+                    k_to_fx_list((const double *const *)pk.ptr(0), base, list.size(), K, ctx.stream);
+                    st.launches++;
+                }
             }
     #pragma omp parallel for schedule(dynamic, 4)
             for (long q = 0; q < NN; q++) {
@@ -2397,7 +2423,7 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
     const size_t fxw = fx_words(b.K);
     uint32_t *yfx = nullptr;
     ctx.sarena.reset();
-    fixed_point = fixed_point && op.d_screen && ctx.sarena.room_for(sizeof(uint32_t) * fxw * (size_t)y.nn());
+    fixed_point = fixed_point && op.d_screen && arena_room(ctx, ctx.sarena, sizeof(uint32_t) * fxw * (size_t)y.nn());
     if (fixed_point) {
         yfx = (uint32_t *)ctx.sarena.alloc(sizeof(uint32_t) * fxw * (size_t)y.nn());
         const FxBlocks ys{y.d_coefs, yfx, (size_t)y.nn()};
@@ -2519,7 +2545,8 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
         fxops.words = fx_op_words(b.K);
         fxops.zoff = fx_op_z(b.K);
         fxops.s = sidx;
-        if (fixed_point) fxops.add(op, ar);
+        const bool fx = fixed_point && arena_room(ctx, ar, fxops.bytes({&op}));
+        if (fx) fxops.add(op, ar);
         li.in.resize(items);
         li.ax.resize(items);
         li.ay.resize(items);
@@ -2537,9 +2564,9 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
                 const int l[3] = {-c.lx, -c.ly, -c.lz};
                 const void *a[3];
                 for (int d = 0; d < 3; d++)
-                    a[d] = fixed_point ? (const void *)(fxops.block(op, c.t, l[d]) + (d == 2 ? fxops.zoff : 0))
+                    a[d] = fx ? (const void *)(fxops.block(op, c.t, l[d]) + (d == 2 ? fxops.zoff : 0))
                                        : (const void *)(op.d_blocks + (size_t)op.block_index(c.t, sidx, l[d]) * bsz);
-                li.in[q] = fixed_point ? (const void *)(yfx + fxw * (size_t)s.work[w]) : (const void *)y.block(s.work[w]);
+                li.in[q] = fx ? (const void *)(yfx + fxw * (size_t)s.work[w]) : (const void *)y.block(s.work[w]);
                 li.ax[q] = a[0];
                 li.ay[q] = a[1];
                 li.az[q] = a[2];
@@ -2551,8 +2578,8 @@ void apply_adjoint(double prec, Tree &res, Oper &op, Tree &x, Tree &y, mw_stats 
         st.items += items;
         st.items_fp64 += items;
         st.out_nodes += (long long)li.out.size();
-        if (fixed_point && items > 0) fxops.make(ctx, st);
-        launch_tier(ctx, ar, li, root, true, 0, Ctx::Tuning(b.K).chunk[0], st, nullptr, false, fixed_point);
+        if (fx && items > 0) fxops.make(ctx, st);
+        launch_tier(ctx, ar, li, root, true, 0, Ctx::Tuning(b.K).chunk[0], st, nullptr, false, fx);
         MWG_CUDA(cudaEventRecord(done[turn].e, ctx.stream));
         turn ^= 1;
         st.levels++;

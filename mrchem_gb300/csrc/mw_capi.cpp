@@ -122,6 +122,7 @@ int mw_ctx_create(int device, int root_scale, const int corner[3], const int box
     }
     c->ctx.owner = c;
     if (const char *e = std::getenv("MW_SCREEN_GEN_SLOTS")) c->ctx.screen_gen_slots = std::max(0L, std::atol(e));
+    if (const char *e = std::getenv("MW_DIGITS_ROOM")) c->ctx.digits_room = (size_t)std::max(0LL, std::atoll(e));
     *out = c;
     return MW_OK;
 }

@@ -175,7 +175,7 @@ struct Arena {
     void *halloc(size_t bytes);
     // call only when the GPU no longer reads anything allocated since the last reset
     void reset();
-    bool room_for(size_t bytes) const;  // held already, or a quarter of the device's free memory
+    bool room_for(size_t bytes) const;  // held already, or at most a quarter of the device's free memory
     void release();
 };
 
@@ -209,6 +209,10 @@ struct Ctx {
     // walk repeated.  MW_SCREEN_GEN_SLOTS in the environment at context creation sets it, which
     // the tests use to run the growth path.
     long screen_gen_slots = 0;
+    // the most bytes of fixed-point digits that are made at a time; where they would take more, or more than the
+    // device has room for, the kernels that read the FP64 blocks run.  MW_DIGITS_ROOM in the environment at
+    // context creation sets it, which the tests use to run that path.
+    size_t digits_room = SIZE_MAX;
     Arena sarena;  // per-apply tables of the GPU screening (input hash tables and norms)
     // launch settings of a batched apply: job groups, and the largest number of items one CTA
     // task takes per tier (FP64, FP32, TF32, double-FP32) before a node is split into chunks

@@ -85,11 +85,12 @@ void Arena::reset() {
 }
 
 bool Arena::room_for(size_t bytes) const {
-    size_t held = 0, free_b = 0, total_b = 0;
-    for (const auto &c : chunks) held += c.size - c.used;
-    if (bytes <= held) return true;
+    size_t free_b = 0, total_b = 0;
+    if (!chunks.empty() && bytes + 256 <= chunks.back().size - chunks.back().used) return true;
     MWG_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    return bytes <= held + free_b / 4;
+    // the chunk that alloc() would add
+    const size_t add = std::max(bytes, chunks.empty() ? (size_t)64 << 20 : chunks.back().size * 2);
+    return bytes <= free_b / 4 && add <= free_b / 2;
 }
 
 void Arena::release() {
