@@ -44,6 +44,7 @@
 // 2^22.  Accumulators start at 1.5 x 2^23, so every partial sum is an integer in [2^23, 2^24): exact in
 // FP32, and the result's bits minus the start's are the integer.
 #include "mw_chunks.cuh"
+#include "mw_fx_round.h"
 #include "mw_host.h"
 
 #include <cuda_fp16.h>
@@ -219,17 +220,11 @@ __device__ __forceinline__ void fx_digits(long long a, long long b, uint32_t (&w
     }
 }
 
-// v 2^-right, rounded to nearest: a truncation here would be a bias that adds up over the items
-__device__ __forceinline__ long long fx_shift(long long v, int right) {
-    if (right <= 0) return (long long)((unsigned long long)v << min(-right, 63));
-    return ((v >> min(right - 1, 62)) + 1) >> 1;
-}
-
-// the same with the two directions' counts and the rounding term prepared
+// v 2^-d rounded to nearest, with the two directions' counts and the rounding term of fx_round prepared
 struct FxShift {
     int left, right;
     long long half;
-    __device__ __forceinline__ explicit FxShift(int d) : left(min(max(-d, 0), 63)), right(min(max(d, 0), 63)), half((1ll << right) >> 1) {}
+    __device__ __forceinline__ explicit FxShift(int d) : left(min(max(-d, 0), 63)), right(min(max(d, 0), 62)), half((1ll << right) >> 1) {}
     __device__ __forceinline__ long long operator()(long long v) const {
         return ((long long)((unsigned long long)v << left) + half) >> right;
     }
@@ -839,15 +834,14 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
                     int over = 0;
 #pragma unroll
                     for (int r = 0; r < RA; r++) {
-                        const int sh = min(eq - e[r], 63);
-                        s[r] = (up ? fx_shift(acc[q][r], up) : acc[q][r]) + ((v[r] + ((1ll << sh) >> 1)) >> sh);
+                        s[r] = (up ? fx_round(acc[q][r], up) : acc[q][r]) + fx_round(v[r], eq - e[r]);
                         const int hi = (int)(s[r] >> 32);
                         over |= hi ^ (hi >> 31);
                     }
                     const int room = (over >> 29) ? 2 : 0;  // |sum| >= 2^61: make room for the next row's 2^62
                     ea[q] = eq + room;
 #pragma unroll
-                    for (int r = 0; r < RA; r++) acc[q][r] = s[r] >> room;
+                    for (int r = 0; r < RA; r++) acc[q][r] = fx_round(s[r], room);
                 }
                 nrows++;
                 par ^= 1;
