@@ -3,10 +3,22 @@
 // GB300's FP64 pipe runs 1.6 multiply-adds per SM and cycle, which bounds apply_kernel.  Here every
 // operand of the three passes is a 62-bit fixed-point number with a power-of-two scale per row of an
 // operator block and per column of the data, cut into seven signed 9-bit digits held as FP16
-// integers.  A pass is a sum of 28 FP16 products (digit pairs i + j <= 6) on mma.sync.m16n8k16 with
-// FP32 accumulation, and every sum is exact: see "ranges" below.  The dropped pairs (i + j >= 7) and
-// the rounding of a pass's result to 62 bits are below 2^-58 of (row 1-norm) x (column maximum), less
-// than FP64's own rounding of the same sums.
+// integers: the error-free splitting of matrix products into low-precision ones that Ozaki et al. (Numer.
+// Algorithms 59, 2012) describe.  A pass is a sum of 28 FP16 products (digit pairs i + j <= 6) on
+// mma.sync.m16n8k16 with FP32 accumulation, and every sum is exact: see "ranges" below.
+//
+// Accuracy.  A column is brought to its own largest number before it is cut, in every pass: the dropped pairs
+// (i + j >= 7) and the rounding of a result to 62 bits are below 2^-58 of (row 1-norm) x (column maximum).  Between
+// the passes a number is held as 54 significant bits with its own exponent (fx_pack), so that no element loses bits
+// to a larger one elsewhere in the block.  A node's sum has an exponent per row Z' and pair of columns.  What is
+// left of the fixed scale is the column itself: a wavelet row of a narrow Gaussian takes little from the scaling half
+// of a column and much from the small wavelet half.  The wavelet half of the data therefore counts 2^FX_UP times in a
+// column's scale, and the operators' wavelet columns 2^-FX_UP: with 4 the small components of such items gain four
+// bits and the scaling rows, nine bits better than FP64, lose none that FP64 has; with 7 and 9 they do.  In the
+// results every component, the pure wavelet ones of far nodes too, is as close to the exact sums as apply_kernel's
+// (at most 1.7 times its error, mostly less: tests/test_gpu_components.py).  With one exponent per X' for a whole
+// block's intermediate and one per column tile for the node's sum, components that vanish beside the scaling part of
+// a far node were off by 1e-6 of themselves.
 //
 // Why mma.sync and not tcgen05: an item needs ten accumulators (one per weight, two for the widest)
 // and its digits cut anew before each pass, and that integer work takes about as long as the tensor
@@ -20,8 +32,8 @@
 //   x pass  T[Z][Y][X'] = sum_X Ax[X'][X] in[X][Y, Z]    input digits read as they lie in memory
 //   y pass  T[Z][Y'][X'] = sum_Y Ay[Y'][Y] T[Z][Y][X']   in place: a warp owns its columns (X', Z)
 //   z pass  out[Z'][Y', X'] += sum_Z c Az[Z'][Z] T[Z]    columns (Y', X')
-// T is int64 in shared memory (64 KB at 2K = 20), its row pitches 2 modulo 4 so that the rows 2t apart of
-// one operand fall into distinct banks.  Digits are made where they serve many times: an input block's
+// T is in shared memory, a 64-bit word per number (64 KB at 2K = 20), its row pitches 2 modulo 4 so that the rows 2t
+// apart of one operand fall into distinct banks.  Digits are made where they serve many times: an input block's
 // once per call, an operator block's once per level (op_to_fx_kernel; the z pass's with its term's
 // coefficient), both laid out as mma.sync operands, the operators' copied to shared memory by cp.async one
 // pass ahead.  Rows of items as in apply_kernel: a row's x passes add up, its y and z passes run once.
@@ -74,8 +86,9 @@ struct FxGeo {
     static constexpr int MINB = K == 8 || K <= 6 ? 2 : 1;  // CTAs per SM that the registers are cut for
     // column tiles of the x pass: Y = 0..7, 8..15 of every plane Z; K > 8: Y >= 16 of two planes together
     static constexpr int CT = N2 > 8 ? 2 : 1, GRP = BIG ? K : N2, TL = BIG ? 5 : CT, NTIN = GRP * TL;
-    static constexpr int NT = (NC + 7) / 8;           // column tiles of the y and z passes
-    static constexpr int NTX = (K2 + 7) / 8;          // ... of which take the second operand
+    // columns of the y and z passes: a component's K^2 and for odd K an empty one, so that the two columns of
+    // a thread's results are of one component; their tiles, and those of them that take the second operand
+    static constexpr int KE = K2 + (K2 & 1), NCE = 4 * KE, NT = (NCE + 7) / 8, NTX = (KE + 7) / 8;
     static constexpr int TPW = (NT + WARPS - 1) / WARPS;
     // T[Z][Y][X'] and u[Z][Y][X'] (Z, Y, X' < K), 62-bit numbers
     static constexpr int PX = fx_pitch(N2), PZ = fx_pitch(N2 * PX), UX = fx_pitch(K), UZ = fx_pitch(K * UX);
@@ -88,10 +101,10 @@ struct FxGeo {
                          O_Z = O_Y + YW, WORDS = O_Z + YW;
     static constexpr size_t SMEM = 4 * (size_t)WORDS;
     // input digits of a block: per column tile the lanes' operands as 16-byte groups and one 8-byte group, then
-    // the tiles' exponents
-    static constexpr int WB = BIG ? 18 : 14, IN_EXP = NTIN * WB * 32, IN_WORDS = IN_EXP + (NTIN + 7) / 8 * 4;
-    // operator digits of a block: the x pass's (the y pass's from X_Y on) and the rows' exponents; then those
-    // of the block times its term's coefficient (the z pass's)
+    // the columns' exponents (16 bits) and the largest of them
+    static constexpr int WB = BIG ? 18 : 14, IN_EXP = NTIN * WB * 32, IN_MAX = IN_EXP + 4 * NTIN, IN_WORDS = IN_MAX + 4;
+    // operator digits of a block: the x pass's (the y pass's from X_Y on) and the rows' exponents, the largest of
+    // them in place EMAX; then those of the block times its term's coefficient (the z pass's)
     static constexpr int X_Y = TILEW, X_EXP = XW, Z_OFF = X_EXP + 16, Z_EXP = YW, OP_WORDS = Z_OFF + Z_EXP + 16;
     static_assert(Z_OFF == (BIG ? 2 * (7 + 10) + 14 : 2 * 7) * 128 + 16, "the same for all K of a kind");
     static_assert(O_U % 4 == 0 && O_X % 4 == 0 && TILEW % 4 == 0 && IN_WORDS % 4 == 0, "16-byte aligned copies");
@@ -100,7 +113,9 @@ struct FxGeo {
 constexpr float FX_MAGIC = 12582912.0f;  // 1.5 * 2^23
 constexpr int FX_MAGIC_BITS = 0x4B400000;
 constexpr int FX_SEG = 32;           // items whose pointers and exponents a CTA holds at a time
-constexpr int FX_NONE = -20000;      // exponent of a zero row or block
+constexpr int FX_NONE = -20000;      // exponent of a zero row, column or block
+constexpr int FX_EMAX = 31;          // place of a block's largest row exponent
+constexpr int FX_UP = 4;             // data of the wavelet half count 2^FX_UP times, operators' wavelet columns 2^-FX_UP
 
 // accumulator of digit pair (i, d - i): weights 0..3 have one, 4..6 two
 __device__ constexpr int fx_slot(int d, int i) { return d < 4 ? d : 4 + 2 * (d - 4) + ((i >= 2 && i <= 4) ? 1 : 0); }
@@ -125,6 +140,7 @@ __device__ __forceinline__ void fx_mma(float (&d)[4], const uint4 &a, uint32_t b
 struct FxB {
     uint32_t m[7][2];
     uint32_t s01, s23, s56, s4;
+    uint32_t ec;  // x pass: the exponents of the columns 2t and 2t + 1 of the results
     // from this lane's pair of remainder elements (k = 16 + 2 (t & 1), + 1), up: t >= 2
     __device__ __forceinline__ void fold(const uint32_t (&q)[7], bool up) {
         s01 = up ? q[1] : q[0];
@@ -220,15 +236,15 @@ __device__ __forceinline__ void fx_digits(long long a, long long b, uint32_t (&w
     }
 }
 
-// v 2^-d rounded to nearest, with the two directions' counts and the rounding term of fx_round prepared
-struct FxShift {
-    int left, right;
-    long long half;
-    __device__ __forceinline__ explicit FxShift(int d) : left(min(max(-d, 0), 63)), right(min(max(d, 0), 62)), half((1ll << right) >> 1) {}
-    __device__ __forceinline__ long long operator()(long long v) const {
-        return ((long long)((unsigned long long)v << left) + half) >> right;
-    }
-};
+// A number of the T arrays: 54 significant bits and in the low byte its binary places below the array's base B (a
+// power of two that no number's unit exceeds).  v 2^(B - d - 62), |v| <= 2^62, d >= 0, to such a word; zero, and what
+// lies 255 places and more below the base, becomes FX_ZERO.
+constexpr int FX_ZERO = 255;
+__device__ __forceinline__ long long fx_pack(long long v, int d) {
+    const int n = max(__clzll(v ^ (v >> 63)) - 2, 0), f = d + n;
+    const long long w = (((v << n) + 128) & ~255ll) | f;
+    return v == 0 || f > 255 ? FX_ZERO : w;
+}
 
 // f 2^e, rounded to nearest, without the FP64 pipe in the normal range
 __device__ __forceinline__ double fx_to_double(long long f, int e) {
@@ -283,7 +299,7 @@ __device__ __forceinline__ void fx_put(const double (&rows)[FxRows<K>::N], doubl
 #pragma unroll
     for (int it = 0; it < FxRows<K>::N; it++) {
         const int r = G::BIG ? unit + it * K : 2 * unit + lane / LW;
-        const double a = rows[it] * cf;
+        const double a = rows[it] * cf * (k >= K ? 1.0 / (1 << FX_UP) : 1.0);
         const int hi = __double2hiint(a), lo = __double2loint(a);
         const int ef = (hi >> 20) & 0x7ff;
         const int em = __reduce_max_sync(mask, ef);
@@ -400,6 +416,12 @@ __global__ void __launch_bounds__(32 * K) op_to_fx_kernel(__grid_constant__ cons
         uint32_t *z = fsm + G::Z_OFF;
         fx_put<K, false>(rows, J.op.c[t], warp, lane, z, nullptr, z + G::TILEW, reinterpret_cast<short *>(z + G::Z_EXP));
         __syncthreads();
+        if (warp == 0) {
+            short *exps = reinterpret_cast<short *>(fsm + G::X_EXP);
+            const int e = __reduce_max_sync(0xffffffffu, lane < G::N2 ? (int)exps[lane] : FX_NONE);
+            if (lane == 0) exps[FX_EMAX] = (short)e;
+        }
+        __syncthreads();
         for (int i = threadIdx.x; i < G::OP_WORDS / 4; i += 32 * K)
             reinterpret_cast<uint4 *>(out)[i] = reinterpret_cast<const uint4 *>(fsm)[i];
         __syncthreads();
@@ -420,8 +442,7 @@ __device__ __forceinline__ void fx_in_column(int gr, int ti, int n, int &Y, int 
 }
 
 // The digits of input blocks as the x pass's column operands (FxGeo::IN_WORDS words per block), one scale
-// per column tile (16-bit exponents), for the blocks of several trees at once.  One CTA per block, a warp
-// per tile.
+// per column, for the blocks of several trees at once.  One CTA per block, a warp per tile.
 template <int K>
 __global__ void __launch_bounds__(FxGeo<K>::THREADS) to_fx_kernel(__grid_constant__ const FxSets S) {
     using G = FxGeo<K>;
@@ -429,6 +450,7 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS) to_fx_kernel(__grid_constan
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const size_t cs = (size_t)(S.pairs && S.up ? 8 : 1) * K3;  // distance of a block's components
     const long long nb = S.first[S.n];
+    __shared__ int s_most;
     for (long long b = blockIdx.x; b < nb; b += gridDim.x) {
         int k = 0;
         while (b >= S.first[k + 1]) k++;
@@ -441,34 +463,44 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS) to_fx_kernel(__grid_constan
             const int cx = X >= K, cy = Y >= K, cz = Z >= K;
             return in[(cx + 2 * cy + 4 * cz) * cs + (Z - cz * K) * K2 + (Y - cy * K) * K + (X - cx * K)];
         };
+        if (threadIdx.x == 0) s_most = FX_NONE;
+        __syncthreads();
+        int most = FX_NONE;
         for (int tile = warp; tile < G::NTIN; tile += G::WARPS) {
             int Y, Z;
             fx_in_column<K>(tile / G::TL, tile % G::TL, g, Y, Z);
             // this lane's X of the column, every X in one lane (those of the remainder in two)
             constexpr int NX = G::BIG ? 6 : (N2 > 8 ? 4 : 2);
             double x[NX];
-#pragma unroll
-            for (int j = 0; j < NX; j++) x[j] = at(j < 4 ? 2 * t + (j & 1) + 8 * (j >> 1) : 16 + 2 * (t & 1) + (j & 1), Y, Z);
+            auto col = [&](int j) { return j < 4 ? 2 * t + (j & 1) + 8 * (j >> 1) : 16 + 2 * (t & 1) + (j & 1); };
             int ef = 0;
 #pragma unroll
-            for (int j = 0; j < NX; j++) ef = max(ef, (__double2hiint(x[j]) >> 20) & 0x7ff);
-            ef = __reduce_max_sync(0xffffffffu, ef);
-            if (lane == 0) reinterpret_cast<short *>(o + G::IN_EXP)[tile] = (short)(ef == 0 ? FX_NONE : ef - 1022);
+            for (int j = 0; j < NX; j++) {
+                x[j] = at(col(j), Y, Z);
+                const int e = (__double2hiint(x[j]) >> 20) & 0x7ff;
+                ef = max(ef, e == 0 ? 0 : e + (col(j) >= K ? FX_UP : 0));
+            }
+            ef = max(ef, __shfl_xor_sync(0xffffffffu, ef, 1));
+            ef = max(ef, __shfl_xor_sync(0xffffffffu, ef, 2));
+            const int ec = ef == 0 ? FX_NONE : ef - 1022;
+            most = max(most, ec);
+            if (t == 0) reinterpret_cast<short *>(o + G::IN_EXP)[8 * tile + g] = (short)ec;
+            auto fixed = [&](int j) { return fx_from_double(x[j], ef - (col(j) >= K ? FX_UP : 0)); };
             uint32_t w[G::WB];
             uint32_t q[7];
-            fx_digits(fx_from_double(x[0], ef), fx_from_double(x[1], ef), q);
+            fx_digits(fixed(0), fixed(1), q);
 #pragma unroll
             for (int s = 0; s < 7; s++) {
                 w[2 * s] = q[s];
                 w[2 * s + 1] = 0u;
             }
             if constexpr (N2 > 8) {
-                fx_digits(fx_from_double(x[2], ef), fx_from_double(x[3], ef), q);
+                fx_digits(fixed(2), fixed(3), q);
 #pragma unroll
                 for (int s = 0; s < 7; s++) w[2 * s + 1] = q[s];
             }
             if constexpr (G::BIG) {
-                fx_digits(fx_from_double(x[4], ef), fx_from_double(x[5], ef), q);
+                fx_digits(fixed(4), fixed(5), q);
                 FxB B;
                 B.fold(q, t >= 2);
                 w[14] = B.s01;
@@ -482,6 +514,11 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS) to_fx_kernel(__grid_constan
                 reinterpret_cast<uint4 *>(d)[v * 32 + lane] = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
             reinterpret_cast<uint2 *>(d + (G::WB / 4) * 128)[lane] = make_uint2(w[G::WB - 2], w[G::WB - 1]);
         }
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (lane == 0) atomicMax(&s_most, most);
+        __syncthreads();
+        if (threadIdx.x == 0) o[G::IN_MAX] = (uint32_t)s_most;
+        __syncthreads();
     }
 }
 
@@ -500,6 +537,7 @@ __device__ __forceinline__ void fx_load(FxB &B, const uint32_t *blk, int tile, i
     asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];"
                  : "=r"(w[G::WB - 2]), "=r"(w[G::WB - 1])
                  : "l"(reinterpret_cast<const uint2 *>(d + (G::WB / 4) * 128) + lane));
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(B.ec) : "l"(blk + G::IN_EXP + 4 * tile + (lane & 3)));
 #pragma unroll
     for (int s = 0; s < 7; s++) {
         B.m[s][0] = w[2 * s];
@@ -513,36 +551,51 @@ __device__ __forceinline__ void fx_load(FxB &B, const uint32_t *blk, int tile, i
     }
 }
 
-// One lane's operand of a y- or z-pass tile: p(k) is the column's k-th value, zero for k >= 2K.
+// One lane's operand of a y- or z-pass tile: word(k) is the column's k-th number (fx_pack), FX_ZERO for k >= 2K.
+// The column's numbers are brought to the largest one's places: returned, for the digits' scale 2^(B - places).
 template <int K, typename F>
-__device__ __forceinline__ void fx_operand(FxB &B, int t, F p) {
+__device__ __forceinline__ int fx_operand(FxB &B, int t, F word) {
     using G = FxGeo<K>;
+    constexpr int NE = G::BIG ? 6 : (G::N2 > 8 ? 4 : 2);
+    long long m[NE];
+    int f[NE], places = 1000;
+#pragma unroll
+    for (int j = 0; j < NE; j++) {
+        const int k = j < 4 ? 2 * t + (j & 1) + 8 * (j >> 1) : 16 + 2 * (t & 1) + (j & 1);
+        const long long w = word(k);
+        f[j] = (int)(w & 255) - (k >= K ? FX_UP : 0);
+        m[j] = w & ~255ll;
+        places = min(places, f[j]);
+    }
+    places = min(places, __shfl_xor_sync(0xffffffffu, places, 1));
+    places = min(places, __shfl_xor_sync(0xffffffffu, places, 2));
     uint32_t q[7];
-    fx_digits(p(2 * t), p(2 * t + 1), q);
+    fx_digits(fx_round(m[0], f[0] - places), fx_round(m[1], f[1] - places), q);
 #pragma unroll
     for (int s = 0; s < 7; s++) B.m[s][0] = q[s];
-    if constexpr (G::N2 > 8) {
-        fx_digits(p(2 * t + 8), p(2 * t + 9), q);
+    if constexpr (NE > 2) {
+        fx_digits(fx_round(m[2], f[2] - places), fx_round(m[3], f[3] - places), q);
 #pragma unroll
         for (int s = 0; s < 7; s++) B.m[s][1] = q[s];
     } else {
 #pragma unroll
         for (int s = 0; s < 7; s++) B.m[s][1] = 0u;
     }
-    if constexpr (G::BIG) {
-        const int k = 16 + 2 * (t & 1);
-        fx_digits(p(k), p(k + 1), q);
+    if constexpr (NE > 4) {
+        fx_digits(fx_round(m[4], f[4] - places), fx_round(m[5], f[5] - places), q);
         B.fold(q, t >= 2);
     }
+    return places;
 }
 
-// column c of the y pass (a = Z) or z pass (a = Y'): the scaling columns (a < K, X' < K) first
+// column c of the y pass (a = Z) or z pass (a = Y'): the scaling columns (a < K, X' < K) first; false for an empty one
 template <int K>
-__device__ __forceinline__ void fx_column(int c, int &a, int &x) {
-    constexpr int K2 = K * K;
-    const int q = c / K2, r = c - q * K2, i = r / K;
+__device__ __forceinline__ bool fx_column(int c, int &a, int &x) {
+    using G = FxGeo<K>;
+    const int q = min(c / G::KE, 3), r = min(c - q * G::KE, G::K2 - 1), i = r / K;
     a = (q >> 1) * K + i;
     x = (q & 1) * K + r - i * K;
+    return c < G::NCE && c - q * G::KE < G::K2;
 }
 
 __device__ __forceinline__ void fx_copy(uint32_t *dst, const uint32_t *src, int words) {
@@ -566,9 +619,8 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
     constexpr int RA = BIG ? 6 : 4;  // results of a thread per column tile
     extern __shared__ __align__(16) uint32_t fsm[];
     long long *s_t = reinterpret_cast<long long *>(fsm), *s_u = reinterpret_cast<long long *>(fsm + G::O_U);
-    __shared__ int s_node, s_redf, s_e1[2][32];  // s_e1: T1's column exponents
+    __shared__ int s_node, s_redf, s_most[FX_SEG];  // s_most: the input blocks' largest exponents
     __shared__ const uint32_t *s_pi[FX_SEG], *s_px[FX_SEG], *s_py[FX_SEG], *s_pz[FX_SEG];
-    __shared__ short s_ein[FX_SEG][(G::NTIN + 7) / 8 * 8];  // column exponents, per x-pass tile
     __shared__ short s_exx[FX_SEG][32], s_exy[FX_SEG][32], s_exz[FX_SEG][32];  // row exponents
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const bool root = L.root != 0;
@@ -578,22 +630,22 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
     while (true) {
         __syncthreads();
         if (tid == 0) s_node = atomicAdd(L.counter, 1);
-        if (tid < 64) (&s_e1[0][0])[tid] = FX_NONE;
         __syncthreads();
         const int w = s_node;
         if (w >= L.nnodes) break;
         const long long b0 = L.begin[w], b1 = L.end[w];
         // node accumulator: per column tile of this warp (columns 8 nt + 2t, + 1) rows Z' = g, 8 + g, 12 + g
-        // (g >= 4), each tile of a thread in units of 2^(ea - 62).  Indexed in a rolled loop, so it lives in
+        // (g >= 4), each row of a thread in units of 2^(ea - 62).  Indexed in a rolled loop, so it lives in
         // local memory between the z passes.
         long long acc[G::TPW][RA];
-        int ea[G::TPW];
+        int ea[G::TPW][RA / 2];
 #pragma unroll 1
-        for (int q = 0; q < G::TPW; q++) {
-            ea[q] = -1000000;
-            for (int r = 0; r < RA; r++) acc[q][r] = 0;
-        }
-        int nrows = 0, par = 0;
+        for (int q = 0; q < G::TPW; q++)
+            for (int r = 0; r < RA; r++) {
+                ea[q][r / 2] = -1000000;
+                acc[q][r] = 0;
+            }
+        int nrows = 0;
         for (long long sb = b0; sb < b1; sb += FX_SEG) {
             const int ni = (int)min((long long)FX_SEG, b1 - sb);
             if (sb != b0) __syncthreads();
@@ -602,6 +654,7 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
                 s_px[i] = reinterpret_cast<const uint32_t *>(L.ax[sb + i]);
                 s_py[i] = reinterpret_cast<const uint32_t *>(L.ay[sb + i]);
                 s_pz[i] = reinterpret_cast<const uint32_t *>(L.az[sb + i]);
+                s_most[i] = (int)s_pi[i][G::IN_MAX];
             }
             __syncthreads();
             fx_copy(fsm + G::O_X, s_px[0], G::XW);
@@ -612,19 +665,13 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
                 s_exy[j][r] = reinterpret_cast<const short *>(s_py[j] + G::X_EXP)[r];
                 s_exz[j][r] = reinterpret_cast<const short *>(s_pz[j] + G::Z_EXP)[r];
             }
-            for (int i = tid; i < ni * G::NTIN; i += G::THREADS) {
-                const int j = i / G::NTIN, r = i - j * G::NTIN;
-                s_ein[j][r] = reinterpret_cast<const short *>(s_pi[j] + G::IN_EXP)[r];
-            }
             const uint32_t *lastz = nullptr;
             for (int j0 = 0; j0 < ni;) {
                 int j1 = j0 + 1;  // the row: items of one term, ly and lz
                 while (j1 < ni && s_py[j1] == s_py[j0] && s_pz[j1] == s_pz[j0]) j1++;
-                const int hb = 32 - __clz(j1 - j0 - 1);  // head room of the row's sum, bits
-                const bool single = j1 == j0 + 1;
-                int h0 = 5 * FX_NONE, h1 = h0, h2 = h0;  // largest exponents of T1's rows X' = g, 8 + g, x2
+                int base = 0;  // of T1 and u: no item's units nor their sums' exceed it
                 for (int j = j0; j < j1; j++) {
-                    const bool first = j == j0, last = j + 1 == j1;
+                    const bool first = j == j0;
                     const uint32_t *in = s_pi[j];
                     FxB B, Bn;
                     if (warp < G::NTIN) fx_load<K>(Bn, in, warp, lane);
@@ -634,8 +681,12 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
                             lastz = s_pz[j0];
                             fx_copy(fsm + G::O_Z, lastz, G::YW);
                         }
+                        base = s_most[j0] + s_exx[j0][FX_EMAX];
+                        for (int i = j0 + 1; i < j1; i++) base = max(base, s_most[i] + s_exx[i][FX_EMAX]);
+                        if (j1 - j0 > 1) base += 34 - __clz(j1 - j0 - 1);  // the sums' bits, and one for each addition's room
                     }
-                    const int exg = s_exx[j][g], exh = s_exx[j][8 + g], exq = s_exx[j][x2];
+                    // places of the rows' units below the base, less the column's exponent
+                    const int dg = base - s_exx[j][g], dh = base - s_exx[j][8 + g], dq = base - s_exx[j][x2];
                     const uint32_t *fx1 = fsm + G::O_X + (j & 1) * G::XW, *fx0 = fx1 + G::X_Y, *fxs = fx0 + G::TILEW;
                     if (j + 1 < ni) fx_copy(fsm + G::O_X + ((j + 1) & 1) * G::XW, s_px[j + 1], G::XW);
 #pragma unroll 1
@@ -643,31 +694,16 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
                         B = Bn;  // the next tile's operand comes from L2 behind this one's products
                         if (tile + G::WARPS < G::NTIN) fx_load<K>(Bn, in, tile + G::WARPS, lane);
                         const int gr = tile / G::TL, ti = tile - gr * G::TL;
-                        // the row's sums at the tile's largest exponents, with head room; of several items every
-                        // result moves right by at least that, rounded
-                        const int ej = s_ein[j][tile];
-                        int et0 = ej + exg, et1 = ej + exh, et2 = ej + exq, m0 = 0, m1 = 0, m2 = 0;
-                        if (!single) {
-                            const int f0 = et0, f1 = et1, f2 = et2;
-                            for (int i = j0; i < j1; i++) {
-                                const int e = s_ein[i][tile];
-                                et0 = max(et0, e + s_exx[i][g]);
-                                et1 = max(et1, e + s_exx[i][8 + g]);
-                                if (BIG) et2 = max(et2, e + s_exx[i][x2]);
+                        const int ec[2] = {(int)(short)(B.ec & 0xffffu), (int)B.ec >> 16};
+                        // the row's sum so far and this item's result, in the coarser unit with one bit of room
+                        auto add = [&](long long *s, long long v, int d) {
+                            if (!first) {
+                                const long long o = *s;
+                                const int f = (int)(o & 255), to = min(d, f) - 1;
+                                v = fx_round(v, d - to) + fx_round(o & ~255ll, f - to);
+                                d = to;
                             }
-                            et0 += hb;
-                            et1 += hb;
-                            et2 += hb;
-                            m0 = min(et0 - f0 - 1, 62), m1 = min(et1 - f1 - 1, 62), m2 = min(et2 - f2 - 1, 62);
-                        }
-                        unsigned long long o0 = 0, o1 = 0, o2 = 0;
-                        auto add = [&](long long *s, long long v, int m, unsigned long long &o) {
-                            if (!single) {
-                                v = ((v >> m) + 1) >> 1;
-                                if (!first) v += *s;
-                            }
-                            *s = v;
-                            o |= (unsigned long long)(v ^ (v >> 63));
+                            *s = fx_pack(v, d);
                         };
                         int Y, Z;  // of column 2t; column 2t + 1 is Y + 1
                         fx_in_column<K>(gr, ti, 2 * t, Y, Z);
@@ -677,7 +713,7 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
 #pragma unroll
                         for (int r = 0; r < 4; r++)
                             if (g + 8 * (r >> 1) < N2 && Y + (r & 1) < N2)
-                                add(T + (r & 1) * PX + g + 8 * (r >> 1), fx_value(D, r), r < 2 ? m0 : m1, r < 2 ? o0 : o1);
+                                add(T + (r & 1) * PX + g + 8 * (r >> 1), fx_value(D, r), (r < 2 ? dg : dh) - ec[r & 1]);
                         const bool has_u = !root && Z < K && Y < K;
                         if (BIG && (root || ti == 4 || 2 * gr + ti / 2 >= K)) {  // no column with u (the warp's tile as a whole)
                             float E[3][4];
@@ -685,88 +721,67 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
 #pragma unroll
                             for (int r = 0; r < 2; r++) {
                                 const long long v = fx_stack_value(E, r, g);
-                                if (g >= 4 && 12 + g < N2 && Y + r < N2) add(T + r * PX + 12 + g, v, m2, o2);
+                                if (g >= 4 && 12 + g < N2 && Y + r < N2) add(T + r * PX + 12 + g, v, dq - ec[r]);
                             }
                         } else if constexpr (BIG) {
                             fx_tile<BIG>(D, fx1, B, lane);
 #pragma unroll
                             for (int r = 0; r < 2; r++) {
-                                if (g >= 4 && 12 + g < N2 && Y + r < N2) add(T + r * PX + 12 + g, fx_value(D, r), m2, o2);
-                                if (g < 2 && 8 + g < K && has_u && Y + r < K) add(u + r * UX + 8 + g, fx_value(D, r), m2, o2);
-                                if (has_u && Y + r < K) add(u + r * UX + g, fx_value(D, 2 + r), m0, o0);
+                                if (g >= 4 && 12 + g < N2 && Y + r < N2) add(T + r * PX + 12 + g, fx_value(D, r), dq - ec[r]);
+                                if (g < 2 && 8 + g < K && has_u && Y + r < K) add(u + r * UX + 8 + g, fx_value(D, r), dq - ec[r]);
+                                if (has_u && Y + r < K) add(u + r * UX + g, fx_value(D, 2 + r), dg - ec[r]);
                             }
                         } else if (!root && ti == 0 && gr < K) {
                             fx_tile<BIG>(D, fx1, B, lane);
 #pragma unroll
                             for (int r = 0; r < 2; r++)
-                                if (g < K && Y + r < K) add(u + r * UX + g, fx_value(D, r), m0, o0);
-                        }
-                        if (last) {  // |v| < 2^(64 - clz)
-                            if (o0) h0 = max(h0, et0 + 2 - __clzll(o0));
-                            if (o1) h1 = max(h1, et1 + 2 - __clzll(o1));
-                            if (o2) h2 = max(h2, et2 + 2 - __clzll(o2));
+                                if (g < K && Y + r < K) add(u + r * UX + g, fx_value(D, r), dg - ec[r]);
                         }
                     }
                 }
-                // T1's columns X' to their largest magnitude
-                {
-                    auto post = [&](int e, int X) {
-                        e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
-                        e = max(e, __shfl_xor_sync(0xffffffffu, e, 2));
-                        if (t == 0 && e > FX_NONE) atomicMax(&s_e1[par][X], e);
-                    };
-                    post(h0, g);
-                    if (N2 > 8) post(h1, 8 + g);
-                    if constexpr (BIG) post(h2, x2);
-                }
                 fx_landed();
-                if (tid < 32) s_e1[par ^ 1][tid] = FX_NONE;
                 // y pass in place: a warp reads its 8 columns (Z, X') whole before it writes them
+                const int base2 = base + FX_UP + s_exy[j0][FX_EMAX];  // of T2
+                const int yg = base2 - base - s_exy[j0][g], yh = base2 - base - s_exy[j0][8 + g],
+                          yq = base2 - base - s_exy[j0][x2];
                 const uint32_t *fy0 = fsm + G::O_Y, *fys = fy0 + G::TILEW;
 #pragma unroll 1
                 for (int tile = warp; tile < G::NT; tile += G::WARPS) {
-                    const int c = 8 * tile + g;
                     int Z, X;
-                    fx_column<K>(min(c, G::NC - 1), Z, X);
-                    // T1's exponents by the x-pass tiles that Y = 0..7, 8..15 and 16.. came from
-                    const int gr = BIG ? Z >> 1 : Z, it = gr * G::TL + (BIG ? (Z & 1) * G::CT : 0);
-                    int e0 = 5 * FX_NONE, e1 = e0, e2 = e0;
-                    for (int i = j0; i < j1; i++) {
-                        const int ex = s_exx[i][X] + hb;
-                        e0 = max(e0, s_ein[i][it] + ex);
-                        if (N2 > 8) e1 = max(e1, s_ein[i][it + 1] + ex);
-                        if (BIG) e2 = max(e2, s_ein[i][gr * G::TL + 4] + ex);
-                    }
-                    const int ee = s_e1[par][X];
-                    const FxShift sh0(ee - e0), sh1(ee - e1), sh2(ee - e2);
-                    auto sh = [&](long long v, int Y) { return Y < 8 ? sh0(v) : (Y < 16 ? sh1(v) : sh2(v)); };
+                    const bool in = fx_column<K>(8 * tile + g, Z, X);
                     const long long *T = s_t + Z * PZ + X, *u = s_u + Z * UZ + X;
-                    int Zr[2], Xr[2];  // of the results' columns 2t, 2t + 1
+                    int Zr[2], Xr[2], at[2];  // of the results' columns 2t, 2t + 1, and the places of their scales
+                    bool inr[2];
 #pragma unroll
-                    for (int b = 0; b < 2; b++) fx_column<K>(min(8 * tile + 2 * t + b, G::NC - 1), Zr[b], Xr[b]);
+                    for (int b = 0; b < 2; b++) inr[b] = fx_column<K>(8 * tile + 2 * t + b, Zr[b], Xr[b]);
                     FxB B;
                     float D[10][4];
                     if (!root && tile < G::NTX) {  // scaling columns: u where Y < K
-                        const bool in = c < K2;
-                        fx_operand<K>(B, t, [&](int Y) -> long long {
-                            return !in || Y >= N2 ? 0 : sh(Y < K ? u[Y * UX] : T[Y * PX], Y);
+                        const bool s = in && Z < K && X < K;
+                        const int p = fx_operand<K>(B, t, [&](int Y) -> long long {
+                            return !s || Y >= N2 ? FX_ZERO : Y < K ? u[Y * UX] : T[Y * PX];
                         });
+#pragma unroll
+                        for (int b = 0; b < 2; b++) at[b] = __shfl_sync(0xffffffffu, p, 4 * (2 * t + b));
                         fx_tile<BIG>(D, fy0, B, lane);
                         __syncwarp();
 #pragma unroll
                         for (int r = 0; r < 4; r++) {
                             const int Yq = g + 8 * (r >> 1), b = r & 1;
-                            if (Yq < K && 8 * tile + 2 * t + b < K2) s_u[Zr[b] * UZ + Yq * UX + Xr[b]] = fx_value(D, r);
+                            if (Yq < K && inr[b] && Zr[b] < K && Xr[b] < K)
+                                s_u[Zr[b] * UZ + Yq * UX + Xr[b]] = fx_pack(fx_value(D, r), (r < 2 ? yg : yh) + at[b]);
                         }
                     }
-                    const bool in = c < G::NC;
-                    fx_operand<K>(B, t, [&](int Y) -> long long { return !in || Y >= N2 ? 0 : sh(T[Y * PX], Y); });
+                    const int p = fx_operand<K>(B, t, [&](int Y) -> long long { return !in || Y >= N2 ? FX_ZERO : T[Y * PX]; });
+#pragma unroll
+                    for (int b = 0; b < 2; b++) at[b] = __shfl_sync(0xffffffffu, p, 4 * (2 * t + b));
                     fx_tile<BIG>(D, fy0, B, lane);
                     __syncwarp();
 #pragma unroll
                     for (int r = 0; r < 4; r++) {
                         const int Yq = g + 8 * (r >> 1), b = r & 1;
-                        if (Yq < N2 && 8 * tile + 2 * t + b < G::NC) s_t[Zr[b] * PZ + Yq * PX + Xr[b]] = fx_value(D, r);
+                        if (Yq < N2 && inr[b])
+                            s_t[Zr[b] * PZ + Yq * PX + Xr[b]] = fx_pack(fx_value(D, r), (r < 2 ? yg : yh) + at[b]);
                     }
                     if constexpr (BIG) {
                         float E[3][4];
@@ -774,8 +789,7 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
 #pragma unroll
                         for (int b = 0; b < 2; b++) {
                             const long long v = fx_stack_value(E, b, g);
-                            if (g >= 4 && 12 + g < N2 && 8 * tile + 2 * t + b < G::NC)
-                                s_t[Zr[b] * PZ + (12 + g) * PX + Xr[b]] = v;
+                            if (g >= 4 && 12 + g < N2 && inr[b]) s_t[Zr[b] * PZ + (12 + g) * PX + Xr[b]] = fx_pack(v, yq + at[b]);
                         }
                     }
                 }
@@ -783,20 +797,20 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
                 if (j1 < ni) fx_copy(fsm + G::O_Y, s_py[j1] + G::X_Y, G::YW);
                 // z pass over this warp's column tiles
                 const uint32_t *fz0 = fsm + G::O_Z, *fzs = fz0 + G::TILEW;
-                const int ez0 = s_exz[j0][g], ez1 = s_exz[j0][8 + g], ez2 = g >= 4 && BIG ? s_exz[j0][12 + g] : FX_NONE;
+                const int ez[3] = {base2 + s_exz[j0][g], base2 + s_exz[j0][8 + g],
+                                   g >= 4 && BIG ? base2 + s_exz[j0][12 + g] : 2 * FX_NONE};
 #pragma unroll 1
                 for (int q = 0; q < G::TPW; q++) {
                     const int nt = warp + q * G::WARPS;
                     if (nt >= G::NT) continue;
-                    const int c = 8 * nt + g;
                     int Yc, X;
-                    fx_column<K>(min(c, G::NC - 1), Yc, X);
+                    const bool in = fx_column<K>(8 * nt + g, Yc, X);
                     const long long *T = s_t + Yc * PX + X, *u = s_u + Yc * UX + X;
                     FxB B;
                     float D[10][4];
                     long long v[RA];
-                    const bool in = c < G::NC;
-                    fx_operand<K>(B, t, [&](int Z) -> long long { return !in || Z >= N2 ? 0 : T[Z * PZ]; });
+                    int e[RA];
+                    int p = fx_operand<K>(B, t, [&](int Z) -> long long { return !in || Z >= N2 ? FX_ZERO : T[Z * PZ]; });
                     fx_tile<BIG>(D, fz0, B, lane);
 #pragma unroll
                     for (int r = 0; r < 4; r++) v[r] = fx_value(D, r);
@@ -806,45 +820,48 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
 #pragma unroll
                         for (int r = 0; r < 2; r++) v[4 + r] = fx_stack_value(E, r, g);
                     }
-                    if (!root && nt < G::NTX) {  // scaling columns: the path without scaling-scaling where Z < K
-                        const bool ins = c < K2;
-                        fx_operand<K>(B, t, [&](int Z) -> long long { return !ins || Z >= N2 ? 0 : Z < K ? u[Z * UZ] : T[Z * PZ]; });
-                        fx_tile<BIG>(D, fz0, B, lane);
-#pragma unroll
-                        for (int r = 0; r < 4; r++)
-                            if (8 * nt + 2 * t + (r & 1) < K2 && g + 8 * (r >> 1) < K) v[r] = fx_value(D, r);
-                    }
-                    int ec[2];
 #pragma unroll
                     for (int b = 0; b < 2; b++) {
-                        int Yr, Xr;
-                        fx_column<K>(min(8 * nt + 2 * t + b, G::NC - 1), Yr, Xr);
-                        ec[b] = s_e1[par][Xr] + s_exy[j0][Yr];
+                        const int at = __shfl_sync(0xffffffffu, p, 4 * (2 * t + b));
+#pragma unroll
+                        for (int r = b; r < RA; r += 2) e[r] = ez[r >> 1] - at;
                     }
-                    int e[RA];
+                    if (!root && nt < G::NTX) {  // scaling columns: the path without scaling-scaling where Z < K
+                        const bool s = in && Yc < K && X < K;
+                        p = fx_operand<K>(B, t, [&](int Z) -> long long { return !s || Z >= N2 ? FX_ZERO : Z < K ? u[Z * UZ] : T[Z * PZ]; });
+                        fx_tile<BIG>(D, fz0, B, lane);
 #pragma unroll
-                    for (int r = 0; r < RA; r++) e[r] = ec[r & 1] + (r < 2 ? ez0 : (r < 4 ? ez1 : ez2));
-                    int em = e[0];
+                        for (int b = 0; b < 2; b++) {
+                            const int at = __shfl_sync(0xffffffffu, p, 4 * (2 * t + b));
+                            int Yr, Xr;
+                            if (!fx_column<K>(8 * nt + 2 * t + b, Yr, Xr) || Yr >= K || Xr >= K) continue;
 #pragma unroll
-                    for (int r = 1; r < RA; r++) em = max(em, e[r]);
-                    long long s[RA];
-                    int eq = ea[q];
-                    const int up = max(em - eq, 0);
-                    eq += up;
-                    int over = 0;
-#pragma unroll
-                    for (int r = 0; r < RA; r++) {
-                        s[r] = (up ? fx_round(acc[q][r], up) : acc[q][r]) + fx_round(v[r], eq - e[r]);
-                        const int hi = (int)(s[r] >> 32);
-                        over |= hi ^ (hi >> 31);
+                            for (int r = b; r < 4; r += 2)
+                                if (g + 8 * (r >> 1) < K) {
+                                    v[r] = fx_value(D, r);
+                                    e[r] = ez[r >> 1] - at;
+                                }
+                        }
                     }
-                    const int room = (over >> 29) ? 2 : 0;  // |sum| >= 2^61: make room for the next row's 2^62
-                    ea[q] = eq + room;
 #pragma unroll
-                    for (int r = 0; r < RA; r++) acc[q][r] = fx_round(s[r], room);
+                    for (int r = 0; r < RA; r += 2) {
+                        const int eq = max(ea[q][r / 2], max(e[r], e[r + 1])), up = eq - ea[q][r / 2];
+                        long long s0 = acc[q][r], s1 = acc[q][r + 1];
+                        if (up) {
+                            s0 = fx_round(s0, up);
+                            s1 = fx_round(s1, up);
+                        }
+                        s0 += fx_round(v[r], eq - e[r]);
+                        s1 += fx_round(v[r + 1], eq - e[r + 1]);
+                        const int h0 = (int)(s0 >> 32), h1 = (int)(s1 >> 32);
+                        // |sum| >= 2^61: make room for the next row's 2^62
+                        const int room = (((h0 ^ (h0 >> 31)) | (h1 ^ (h1 >> 31))) >> 29) ? 2 : 0;
+                        ea[q][r / 2] = eq + room;
+                        acc[q][r] = fx_round(s0, room);
+                        acc[q][r + 1] = fx_round(s1, room);
+                    }
                 }
                 nrows++;
-                par ^= 1;
                 j0 = j1;
             }
         }
@@ -859,10 +876,10 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
 #pragma unroll
             for (int r = 0; r < RA; r++) {
                 const int c = 8 * nt + 2 * t + (r & 1), Zq = r < 2 ? g : (r < 4 ? 8 + g : (g >= 4 ? 12 + g : N2));
-                if (c >= G::NC || Zq >= N2) continue;
-                const int hq = c / K2, hz = Zq >= K;
-                const double v = fx_to_double(acc[q][r], ea[q] - 62);
-                double *o = out + (hq + 4 * hz) * cs + (Zq - hz * K) * K2 + (c - hq * K2);
+                const int hq = c / G::KE, hz = Zq >= K;
+                if (c >= G::NCE || c - hq * G::KE >= K2 || Zq >= N2) continue;
+                const double v = fx_to_double(acc[q][r], ea[q][r / 2] - 62);
+                double *o = out + (hq + 4 * hz) * cs + (Zq - hz * K) * K2 + (c - hq * G::KE);
                 *o = set ? v : *o + v;
             }
         }
