@@ -237,13 +237,14 @@ __device__ __forceinline__ void fx_digits(long long a, long long b, uint32_t (&w
 }
 
 // A number of the T arrays: 54 significant bits and in the low byte its binary places below the array's base B (a
-// power of two that no number's unit exceeds).  v 2^(B - d - 62), |v| <= 2^62, d >= 0, to such a word; zero, and what
-// lies 255 places and more below the base, becomes FX_ZERO.
+// power of two that no number's unit exceeds).  v 2^(B - d - 62), |v| <= 2^62, d >= 0, to such a word; of what lies
+// more than 255 places below the base, nothing is left that counts beside it.  The shift goes up to 30 places: a
+// smaller v has no more than 32 bits that mean anything, and they all stay.
 constexpr int FX_ZERO = 255;
 __device__ __forceinline__ long long fx_pack(long long v, int d) {
-    const int n = max(__clzll(v ^ (v >> 63)) - 2, 0), f = d + n;
-    const long long w = (((v << n) + 128) & ~255ll) | f;
-    return v == 0 || f > 255 ? FX_ZERO : w;
+    const int hi = (int)(v >> 32);
+    const int n = max(__clz(hi ^ (hi >> 31)) - 2, 0), f = v ? min(d + n, 255) : FX_ZERO;
+    return (((v << n) + 128) & ~255ll) | f;
 }
 
 // f 2^e, rounded to nearest, without the FP64 pipe in the normal range
