@@ -41,11 +41,11 @@
 // operator rows in the x pass's second row tile, and the (Y' < K, X' < K) columns of the z pass take a
 // second operand whose Z < K part avoids that path.
 //
-// Measured on a full chip, ns per item, apply_kernel's FP64 pipe first and then this kernel:
-// 2K = 20: 653, 134;  2K = 18: 444, 119;  2K = 16: 256, 40;  2K = 12: 91, 33.  With T in registers and the
-// operators' digits made per item 2K = 20 took 172 and 2K = 12 36; with a row tile of their own for rows
-// 16.. 2K = 20 took 147 and 2K = 18 133.  Tier 3 of the 16-orbital Helmholtz batch (22 thousand items, alone
-// on the chip): 5.3 ms with their digits, 6.9 ms with the double-FP32 kernel it had.
+// Measured over 16 Helmholtz applies at once (all of their levels, the nearly empty ones included), ns per item at
+// 2K = 8, 10, .. 20: apply_kernel's FP64 pipe 30.9, 70.7, 116, 215, 308, 539, 797; this kernel 17.6, 36.7, 44.0, 67.0,
+// 54.4, 156, 174.  Of that the numbers' own exponents between the passes take 0 to 11% (17.7, 35.5, 42.6, 67.3, 50.6,
+// 140, 160 with common ones, which lost the small components).  Forms before, on a full chip at 2K = 20: T in
+// registers and the operators' digits made per item 172, a row tile of their own for rows 16.. 147, then 134.
 //
 // K > 8: the contraction index is 16 + (2K - 16).  The remainder's digit pairs are folded: one MMA
 // carries four digit pairs of the same weight in its 16 k slots, 10 MMAs instead of 28.
@@ -72,10 +72,16 @@ constexpr int fx_pitch(int n) {  // n or a little more, 2 modulo 4: int64 rows 2
     while (n % 4 != 2) n++;
     return n;
 }
-// warps of a CTA: a divisor of the column tiles' number (50, 41, 32, 25, 18, 13, 8) with little left over, at
-// most 16 (128 registers).  Two CTAs of 8 at 2K = 16: one's products run during the other's barriers (40 ns per item on a
-// full chip against 46 with one of 16; the FP64 Poisson apply alike).  Not at 2K = 18, 20, where shared memory
-// holds one CTA; 17 warps at 2K = 20 (no nearly empty last round) spill: 146 ns against 134.
+// Warps of a CTA: a divisor of the column tiles' number (50, 41, 32, 25, 18, 13, 8) with little left over, at
+// most 16 (128 registers).  ns per item as above, this choice first:
+//   K = 4: 8 warps, 2 CTAs per SM 17.6; 4, 4 CTAs 16.2; 8, 3 CTAs 16.3; 16, 1 CTA 25.8
+//   K = 5: 7, 2 CTAs 36.7; 5, 3 CTAs 32.9; 7, 3 CTAs 37.4; 13, 1 CTA 46.6
+//   K = 6: 9, 2 CTAs 44.0; 5, 3 CTAs 39.9; 9, 1 CTA 60.7
+//   K = 7: 13, 1 CTA 67.0; 7, 2 CTAs 54.9; 9, 2 CTAs 56.5; 9, 1 CTA 75.8
+//   K = 8: 8, 2 CTAs 54.4; 16, 1 CTA 63.5
+// Fewer warps and more CTAs fill a loaded chip better, but a task then takes longer, which is what levels of few
+// tasks wait for (K = 6 with 5 warps: 84 us a task against 70).  At 2K = 18, 20 shared memory holds one CTA; 17 warps
+// at 2K = 20 (no nearly empty last round) spill: 146 ns against 134 in an earlier form.
 constexpr int fx_warps(int K) { return K == 10 ? 16 : K == 9 ? 14 : K == 8 ? 8 : K == 7 ? 13 : K == 6 ? 9 : K == 5 ? 7 : 8; }
 
 template <int K>
@@ -90,7 +96,7 @@ struct FxGeo {
     // a thread's results are of one component; their tiles, and those of them that take the second operand
     static constexpr int KE = K2 + (K2 & 1), NCE = 4 * KE, NT = (NCE + 7) / 8, NTX = (KE + 7) / 8;
     static constexpr int TPW = (NT + WARPS - 1) / WARPS;
-    // T[Z][Y][X'] and u[Z][Y][X'] (Z, Y, X' < K), 62-bit numbers
+    // T[Z][Y][X'] and u[Z][Y][X'] (Z, Y, X' < K), numbers as fx_pack has them
     static constexpr int PX = fx_pitch(N2), PZ = fx_pitch(N2 * PX), UX = fx_pitch(K), UZ = fx_pitch(K * UX);
     static constexpr int MAINW = 7 * 128;             // words of a row tile's digits (512 B per digit)
     static constexpr int TILEW = MAINW + (BIG ? 10 * 128 : 0);
