@@ -135,8 +135,9 @@ struct Oper {
     float *d_blocks_tc2 = nullptr; // ... in the split-TF32 tier's wide layout (tc5_split_wide(K) only)
     // the operator blocks the split-TF32 tier reads: the wide layout where the kernel uses it
     const float *split_blocks() const { return d_blocks_tc2 ? d_blocks_tc2 : d_blocks_tc; }
-    // the screening tables on the device (bands, block offsets, sub-block norms, amax, xmax, term
-    // coefficients), uploaded by the first apply that screens on the GPU (mw_screen.cu)
+    // the screening tables on the device (bands, block offsets, sub-block norms, amax, xmax, term coefficients),
+    // made with the operator.  Null where a band or block number is beyond their fields: such an operator's applies
+    // are screened on the host, and their FP64 and tier 3 items go to apply_kernel (FxLevelOps reads these tables)
     void *d_screen = nullptr;
     std::vector<int> fx_first, fx_count;  // per (term, scale) the blocks of the terms before; per scale all blocks
     void free_device();
@@ -356,12 +357,7 @@ void kernel_smem(const void *fn, int bytes);
 int kernel_ctas_per_sm(const void *fn, int threads, int bytes);
 
 void k_project(const DevBasis &b, const ProjFunc &f, const ProjTask *tasks, int n, cudaStream_t s);
-// K = 4 .. 10: generate_kernel_t<K> (shared memory, scratch unused); other K: scratch holds
-// grid x generate_scratch_doubles(K) doubles (one slice per CTA)
-void k_generate(const DevBasis &b, const GenTask *tasks, int n, double *scratch, int grid, int nsm, cudaStream_t s);
-inline size_t generate_scratch_doubles(int K) {
-    return (size_t)4 * K * K * K + (size_t)2 * K * K * K + (size_t)K * K * K;
-}
+void k_generate(const DevBasis &b, const GenTask *tasks, int n, int nsm, cudaStream_t s);
 void k_apply(const DevBasis &b, const ApplyLaunch &L, int fp32, int nsm, cudaStream_t s);
 // TF32 tensor-core tier on the 5th-generation tensor cores (tcgen05.mma, accumulators in tensor
 // memory); items point at the operand layouts of mw_tc05_layout.h
@@ -369,7 +365,7 @@ void k_apply(const DevBasis &b, const ApplyLaunch &L, int fp32, int nsm, cudaStr
 // the TF32-rounded operands and their remainders, FP32 accumulation), the tensor-core form of the
 // FP32 tier.  Item pointers point at the hi copies of mw_tc05_layout.h's operand layouts.
 void k_apply_tc05(const DevBasis &b, const ApplyLaunch &L, bool split, cudaStream_t s);
-// FP32 cube-order shadows (high cube read) -> the tensor-core tier's x-pass operand layout
+// FP64 blocks -> the tensor-core tiers' x-pass operand layout
 void k_to_tc_x(const double *blocks, float *out, size_t nblocks, int K, cudaStream_t s);
 // round to TF32: nearest, ties away from zero (as cvt.rna.tf32.f32)
 inline float tf32_round_host(float x) {
@@ -453,8 +449,7 @@ void k_op_blocks(int K, const double *W, const double *cc, const double *gx, con
                  const OpBlockJob *jobs, int njob, const double *keep, cudaStream_t s);
 void k_op_convert(const double *blocks, float *b32, float *btc, float *btc2, long nblocks, int K, int NB, int groups,
                   cudaStream_t s);
-// FP32 shadow of whole blocks in cube order cube[Z][Y][X] (X = cx*K + ix): per block a high cube
-// and a low cube (2 * 8K^3 floats, the low one holds the rounded remainder)
+// FP32 shadow of whole blocks in cube order cube[Z][Y][X] (X = cx*K + ix): 8K^3 floats per block
 void k_to_fp32_cube(const double *in, float *out, size_t nblocks, int K, cudaStream_t s);
 void k_dot(const double *const *a, const double *const *b, const int *start, int n, int bs, double *partial,
            cudaStream_t s);

@@ -437,11 +437,7 @@ void generate_all(const std::vector<std::pair<GenSet *, const Tree *>> &sets, Ar
     Packer pk;
     pk.add(tasks.data(), tasks.size() * sizeof(GenTask));
     pk.ship(ctx, arena);
-    const int ggrid = (int)std::min<long>(total, 4L * std::max(ctx.nsm, 1));
-    const int K = ctx.basis.K;
-    double *gscratch =
-        (K >= 4 && K <= KMAX) ? nullptr : (double *)arena.alloc(sizeof(double) * generate_scratch_doubles(K) * ggrid);
-    k_generate(ctx.dbasis, (const GenTask *)pk.ptr(0), (int)total, gscratch, ggrid, ctx.nsm, ctx.stream);
+    k_generate(ctx.dbasis, (const GenTask *)pk.ptr(0), (int)total, ctx.nsm, ctx.stream);
     if (st) {
         st->launches++;
         st->generated += total;
@@ -1102,12 +1098,8 @@ void combine_on_grid(const std::vector<Tree *> &outs, const std::vector<const Tr
     const int fixed = 6;
     for (auto &s : steps) pk.add(s.data(), s.size() * sizeof(GenTask));
     pk.ship(ctx, arena);
-    const bool scratch = !(K >= 4 && K <= KMAX);
-    for (size_t d = 0; d < steps.size(); d++) {
-        const int n = (int)steps[d].size(), gg = std::min(n, 4 * std::max(ctx.nsm, 1));
-        double *gscr = scratch ? (double *)arena.alloc(sizeof(double) * generate_scratch_doubles(K) * gg) : nullptr;
-        k_generate(ctx.dbasis, (const GenTask *)pk.ptr(fixed + (int)d), n, gscr, gg, ctx.nsm, ctx.stream);
-    }
+    for (size_t d = 0; d < steps.size(); d++)
+        k_generate(ctx.dbasis, (const GenTask *)pk.ptr(fixed + (int)d), (int)steps[d].size(), ctx.nsm, ctx.stream);
     CombineArgs A;
     A.src = (const double *const *)pk.ptr(0);
     A.tree = (const unsigned *)pk.ptr(1);
