@@ -300,7 +300,7 @@ def other_configs(mw, device, world, sync, steps):
         e_64, same_64 = rel_vs_oracle(mra, o64[0], oout)
         out["helmholtz_prec%g" % prec] = {
             "value": stmx["out_nodes"] * world / (msmx / 1e3), "unit": "nodes/s", "ms_per_step": msmx,
-            "dtype": "f64+df32+f32+tf32", "fp64": {"value": st64["out_nodes"] * world / (ms64 / 1e3),
+            "dtype": "f64+fx62+df32+f32+tf32", "fp64": {"value": st64["out_nodes"] * world / (ms64 / 1e3),
                                                   "ms_per_step": ms64},
             "speedup_mixed_vs_fp64": ms64 / msmx,
             "input_nodes_total": int(sum(p.nnodes for p in phis)), "output_nodes": stmx["out_nodes"],
@@ -733,7 +733,7 @@ def run(args):
     line = {
         "metric": METRIC, "value": value, "unit": "nodes/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": None, "dtype": "f64+df32+f32+tf32", "data": "synthetic",
+        "vs_baseline": None, "dtype": "f64+fx62+df32+f32+tf32", "data": "synthetic",
         "config": workload_config(),
         "workload_detail": {"tuned": tuned, "input_nodes": in_nodes, "input_nodes_total": int(sum(in_nodes)),
                             "output_nodes": nodes,

@@ -39,16 +39,17 @@ extern "C" {
 #define MW_BASIS_INTERPOLATING 1
 
 /* precision modes of mw_apply / mw_apply_batch */
-#define MW_PREC_FP64 0   /* every contraction in FP64 */
-/* norm-tiered by the item's bound b against the screening threshold tau: double-FP32 or
- * better (62-bit fixed point, ~1e-15 b) when 2e6 tau < b <= 1e11 tau, FP64 above that, TF32 tensor cores (FP32
+#define MW_PREC_FP64 0   /* every contraction to FP64's accuracy, component by component (62-bit fixed point; on the
+                          * FP64 pipe for inputs that are not finite or of norm 1e150 and more) */
+/* norm-tiered by the item's bound b against the screening threshold tau: tier 3 (as FP64, ~1e-15 b;
+ * double-FP32 pairs once) when 2e6 tau < b <= 1e11 tau, FP64 above that, TF32 tensor cores (FP32
  * accumulation) when b <= 2e3 tau below the root scale, FP32 CUDA cores otherwise; root-scale
  * items under relative precision run in FP64 */
 #define MW_PREC_MIXED 1
 #define MW_PREC_MIXED_NEARFP64 2  /* as MW_PREC_MIXED, and every item with |l|_inf <= 1 in FP64 */
-#define MW_PREC_MIXED_FP32 3      /* FP64 or FP32 only: no tensor-core and no double-FP32 tier */
-#define MW_PREC_DF 4              /* double-FP32 for every item with b <= 1e11 tau, FP64 above that and for
-                                   * root-scale items under relative precision (the same kernel: error ~1e-15 b per item) */
+#define MW_PREC_MIXED_FP32 3      /* FP64 or FP32 only: no tensor-core tier and no tier 3 */
+#define MW_PREC_DF 4              /* tier 3 for every item with b <= 1e11 tau, FP64 above that and for root-scale items
+                                   * under relative precision: the same kernel for both, transforms in double-FP32 */
 
 typedef struct mw_ctx_s *mw_ctx;
 typedef struct mw_tree_s *mw_tree;
@@ -88,9 +89,10 @@ typedef struct {
     double host_wait_ms;     /* host: waiting for the level's kernels and norm downloads */
     double flops_tf32;       /* algorithmic flops of the TF32 tier */
     double kernel_ms_tf32;   /* CUDA-event time of the TF32 contraction launches */
-    long long items_df;      /* contractions of the double-FP32 tier (run in 62-bit fixed point) */
-    double flops_df;         /* algorithmic flops of the double-FP32 tier */
-    double kernel_ms_df;     /* CUDA-event time of the double-FP32 contraction launches */
+    long long items_df;      /* contractions of tier 3, which runs in 62-bit fixed point ("df" in these names is from the
+                              * double-FP32 pairs that it ran in first) */
+    double flops_df;         /* algorithmic flops of tier 3 */
+    double kernel_ms_df;     /* CUDA-event time of that tier's contraction launches */
     double host_gen_ms;      /* host: generation requests and the generation of missing input nodes */
     double host_launch_ms;   /* host: ordering, chunking and packing the item lists, launches */
     double host_refine_ms;   /* host: refinement decisions after each level */
@@ -103,7 +105,7 @@ typedef struct {
                                  z pass */
     long long rows_fp32;      /* ... of the FP32-accuracy tier */
     long long rows_tf32;      /* ... of the TF32 tier */
-    long long rows_df;        /* ... of the double-FP32 tier */
+    long long rows_df;        /* ... of tier 3 */
     double host_io_ms;        /* mw_apply_batch_host: host time building the input trees' structures,
                                  waiting for each job group's uploaded inputs and preparing them, and
                                  queueing the outputs' downloads */
@@ -233,10 +235,10 @@ int mw_apply_batch_host(int n, const double *precs, mw_tree *outs, mw_op *ops, m
                         unsigned char *const *out_leaf, int *out_nnodes);
 /* Autotuner of the batched apply's launch settings (no counterpart in the reference): runs the
  * batch (as mw_apply_batch with no precision trees and max_iter = -1) `repeats` times for each
- * candidate -- job groups 2..6, then the chunk size of the TF32, FP32 and double-FP32 tiers, one
+ * candidate -- job groups 2..6, then the chunk size of the TF32 and FP32 tiers and of tier 3, one
  * at a time -- and keeps the fastest (a candidate must beat the kept settings by 2%) in the context for this (order, n, precision_mode); later
  * batched applies with the same key use it.  The outputs hold the result of a last run with the
- * settings kept.  Returns the settings (groups, chunks[4] for FP64, FP32, TF32, double-FP32) and
+ * settings kept.  Returns the settings (groups, chunks[4] for FP64, FP32, TF32, tier 3) and
  * their median wall time in ms.  Needs job-group overlap on (mw_ctx_set_overlap). */
 int mw_apply_batch_autotune(int n, const double *precs, mw_tree *outs, mw_op *ops, mw_tree *inps, int abs_prec,
                             int precision_mode, int repeats, int *groups, long long *chunks, double *ms);
