@@ -429,7 +429,6 @@ struct CombineArgs {
 void k_combine(const CombineArgs &A, cudaStream_t s);
 void k_add(const DevBasis &b, const AddTask *tasks, const double *const *src, const double *coefs, int n, int bs,
            cudaStream_t s);
-void k_to_fp32(const double *in, float *out, size_t n, cudaStream_t s);
 // operator construction on the GPU (mw_opbuild.cu)
 struct OpBuildTask {  // one (term, scale): tau(m) = pref * (Legendre expansion . Gaussian moments of beta)
     double beta, pref;

@@ -858,11 +858,6 @@ void launch_combine(const CombineArgs &A, cudaStream_t s) {
     MWG_CUDA(cudaGetLastError());
 }
 
-__global__ void to_fp32_kernel(const double *in, float *out, size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        out[i] = (float)in[i];
-}
-
 // FP32 shadow of nblocks blocks, each written in cube order cube[Z][Y][X]
 __global__ void to_fp32_cube_kernel(const double *in, float *out, size_t nblocks, int K) {
     const size_t bs = 8 * (size_t)K * K * K, n = nblocks * bs;
@@ -1049,12 +1044,6 @@ void k_combine(const CombineArgs &A, cudaStream_t s) {
         launch_combine<4>(A, s);
     else
         launch_combine<1>(A, s);
-}
-
-void k_to_fp32(const double *in, float *out, size_t n, cudaStream_t s) {
-    if (n == 0) return;
-    to_fp32_kernel<<<4096, 256, 0, s>>>(in, out, n);
-    MWG_CUDA(cudaGetLastError());
 }
 
 void k_to_fp32_cube(const double *in, float *out, size_t nblocks, int K, cudaStream_t s) {
