@@ -42,8 +42,8 @@
 // second operand whose Z < K part avoids that path.
 //
 // Measured over 16 Helmholtz applies at once (all of their levels, the nearly empty ones included), ns per item at
-// 2K = 8, 10, .. 20: apply_kernel's FP64 pipe 30.9, 70.7, 116, 215, 308, 539, 797; this kernel 17.6, 36.7, 44.0, 67.0,
-// 54.4, 156, 174.  Of that the numbers' own exponents between the passes take 0 to 11% (17.7, 35.5, 42.6, 67.3, 50.6,
+// 2K = 8, 10, .. 20: apply_kernel's FP64 pipe 30.9, 70.7, 116, 215, 308, 539, 797; this kernel 17.7, 35.8, 44.4, 65.3,
+// 53.0, 150, 170.  Of that the numbers' own exponents between the passes take 0 to 7% (17.7, 35.5, 42.6, 67.3, 50.6,
 // 140, 160 with common ones, which lost the small components).  Forms before, on a full chip at 2K = 20: T in
 // registers and the operators' digits made per item 172, a row tile of their own for rows 16.. 147, then 134.
 //
@@ -74,11 +74,11 @@ constexpr int fx_pitch(int n) {  // n or a little more, 2 modulo 4: int64 rows 2
 }
 // Warps of a CTA: a divisor of the column tiles' number (50, 41, 32, 25, 18, 13, 8) with little left over, at
 // most 16 (128 registers).  ns per item as above, this choice first:
-//   K = 4: 8 warps, 2 CTAs per SM 17.6; 4, 4 CTAs 16.2; 8, 3 CTAs 16.3; 16, 1 CTA 25.8
-//   K = 5: 7, 2 CTAs 36.7; 5, 3 CTAs 32.9; 7, 3 CTAs 37.4; 13, 1 CTA 46.6
-//   K = 6: 9, 2 CTAs 44.0; 5, 3 CTAs 39.9; 9, 1 CTA 60.7
-//   K = 7: 13, 1 CTA 67.0; 7, 2 CTAs 54.9; 9, 2 CTAs 56.5; 9, 1 CTA 75.8
-//   K = 8: 8, 2 CTAs 54.4; 16, 1 CTA 63.5
+//   K = 4: 8 warps, 2 CTAs per SM 17.7; 4, 4 CTAs 16.3; 8, 3 CTAs 16.3; 16, 1 CTA 24.8
+//   K = 5: 7, 2 CTAs 35.8; 5, 3 CTAs 32.9; 7, 3 CTAs 37.1; 13, 1 CTA 46.4
+//   K = 6: 9, 2 CTAs 44.4; 5, 3 CTAs 40.0; 9, 1 CTA 57.8
+//   K = 7: 13, 1 CTA 65.3; 7, 2 CTAs 54.4; 9, 2 CTAs 55.2; 9, 1 CTA 71.8
+//   K = 8: 8, 2 CTAs 53.0; 16, 1 CTA 61.9
 // Fewer warps and more CTAs fill a loaded chip better, but a task then takes longer, which is what levels of few
 // tasks wait for (K = 6 with 5 warps: 84 us a task against 70).  At 2K = 18, 20 shared memory holds one CTA; 17 warps
 // at 2K = 20 (no nearly empty last round) spill: 146 ns against 134 in an earlier form.
@@ -696,55 +696,64 @@ __global__ void __launch_bounds__(FxGeo<K>::THREADS, FxGeo<K>::MINB) apply_fx_ke
                     const int dg = base - s_exx[j][g], dh = base - s_exx[j][8 + g], dq = base - s_exx[j][x2];
                     const uint32_t *fx1 = fsm + G::O_X + (j & 1) * G::XW, *fx0 = fx1 + G::X_Y, *fxs = fx0 + G::TILEW;
                     if (j + 1 < ni) fx_copy(fsm + G::O_X + ((j + 1) & 1) * G::XW, s_px[j + 1], G::XW);
+                    // the row's first item, which stores, has code of its own: with the additions in the same loop an
+                    // item took 2 to 4% longer (170 and 174 ns at 2K = 20)
+                    auto x_pass = [&](auto one) {
+                        constexpr bool ONE = decltype(one)::value;
 #pragma unroll 1
-                    for (int tile = warp; tile < G::NTIN; tile += G::WARPS) {
-                        B = Bn;  // the next tile's operand comes from L2 behind this one's products
-                        if (tile + G::WARPS < G::NTIN) fx_load<K>(Bn, in, tile + G::WARPS, lane);
-                        const int gr = tile / G::TL, ti = tile - gr * G::TL;
-                        const int ec[2] = {(int)(short)(B.ec & 0xffffu), (int)B.ec >> 16};
-                        // the row's sum so far and this item's result, in the coarser unit with one bit of room
-                        auto add = [&](long long *s, long long v, int d) {
-                            if (!first) {
-                                const long long o = *s;
-                                const int f = (int)(o & 255), to = min(d, f) - 1;
-                                v = fx_round(v, d - to) + fx_round(o & ~255ll, f - to);
-                                d = to;
+                        for (int tile = warp; tile < G::NTIN; tile += G::WARPS) {
+                            B = Bn;  // the next tile's operand comes from L2 behind this one's products
+                            if (tile + G::WARPS < G::NTIN) fx_load<K>(Bn, in, tile + G::WARPS, lane);
+                            const int gr = tile / G::TL, ti = tile - gr * G::TL;
+                            const int ec[2] = {(int)(short)(B.ec & 0xffffu), (int)B.ec >> 16};
+                            // the row's sum so far and this item's result, in the coarser unit with one bit of room
+                            auto add = [&](long long *s, long long v, int d) {
+                                if constexpr (!ONE) {
+                                    const long long o = *s;
+                                    const int f = (int)(o & 255), to = min(d, f) - 1;
+                                    v = fx_round(v, d - to) + fx_round(o & ~255ll, f - to);
+                                    d = to;
+                                }
+                                *s = fx_pack(v, d);
+                            };
+                            int Y, Z;  // of column 2t; column 2t + 1 is Y + 1
+                            fx_in_column<K>(gr, ti, 2 * t, Y, Z);
+                            long long *T = s_t + Z * PZ + Y * PX, *u = s_u + Z * UZ + Y * UX;
+                            float D[10][4];
+                            fx_tile<BIG>(D, fx0, B, lane);
+#pragma unroll
+                            for (int r = 0; r < 4; r++)
+                                if (g + 8 * (r >> 1) < N2 && Y + (r & 1) < N2)
+                                    add(T + (r & 1) * PX + g + 8 * (r >> 1), fx_value(D, r), (r < 2 ? dg : dh) - ec[r & 1]);
+                            const bool has_u = !root && Z < K && Y < K;
+                            if (BIG && (root || ti == 4 || 2 * gr + ti / 2 >= K)) {  // no column with u (the warp's tile as a whole)
+                                float E[3][4];
+                                fx_stack(E, fxs, B, lane);
+#pragma unroll
+                                for (int r = 0; r < 2; r++) {
+                                    const long long v = fx_stack_value(E, r, g);
+                                    if (g >= 4 && 12 + g < N2 && Y + r < N2) add(T + r * PX + 12 + g, v, dq - ec[r]);
+                                }
+                            } else if constexpr (BIG) {
+                                fx_tile<BIG>(D, fx1, B, lane);
+#pragma unroll
+                                for (int r = 0; r < 2; r++) {
+                                    if (g >= 4 && 12 + g < N2 && Y + r < N2) add(T + r * PX + 12 + g, fx_value(D, r), dq - ec[r]);
+                                    if (g < 2 && 8 + g < K && has_u && Y + r < K) add(u + r * UX + 8 + g, fx_value(D, r), dq - ec[r]);
+                                    if (has_u && Y + r < K) add(u + r * UX + g, fx_value(D, 2 + r), dg - ec[r]);
+                                }
+                            } else if (!root && ti == 0 && gr < K) {
+                                fx_tile<BIG>(D, fx1, B, lane);
+#pragma unroll
+                                for (int r = 0; r < 2; r++)
+                                    if (g < K && Y + r < K) add(u + r * UX + g, fx_value(D, r), dg - ec[r]);
                             }
-                            *s = fx_pack(v, d);
-                        };
-                        int Y, Z;  // of column 2t; column 2t + 1 is Y + 1
-                        fx_in_column<K>(gr, ti, 2 * t, Y, Z);
-                        long long *T = s_t + Z * PZ + Y * PX, *u = s_u + Z * UZ + Y * UX;
-                        float D[10][4];
-                        fx_tile<BIG>(D, fx0, B, lane);
-#pragma unroll
-                        for (int r = 0; r < 4; r++)
-                            if (g + 8 * (r >> 1) < N2 && Y + (r & 1) < N2)
-                                add(T + (r & 1) * PX + g + 8 * (r >> 1), fx_value(D, r), (r < 2 ? dg : dh) - ec[r & 1]);
-                        const bool has_u = !root && Z < K && Y < K;
-                        if (BIG && (root || ti == 4 || 2 * gr + ti / 2 >= K)) {  // no column with u (the warp's tile as a whole)
-                            float E[3][4];
-                            fx_stack(E, fxs, B, lane);
-#pragma unroll
-                            for (int r = 0; r < 2; r++) {
-                                const long long v = fx_stack_value(E, r, g);
-                                if (g >= 4 && 12 + g < N2 && Y + r < N2) add(T + r * PX + 12 + g, v, dq - ec[r]);
-                            }
-                        } else if constexpr (BIG) {
-                            fx_tile<BIG>(D, fx1, B, lane);
-#pragma unroll
-                            for (int r = 0; r < 2; r++) {
-                                if (g >= 4 && 12 + g < N2 && Y + r < N2) add(T + r * PX + 12 + g, fx_value(D, r), dq - ec[r]);
-                                if (g < 2 && 8 + g < K && has_u && Y + r < K) add(u + r * UX + 8 + g, fx_value(D, r), dq - ec[r]);
-                                if (has_u && Y + r < K) add(u + r * UX + g, fx_value(D, 2 + r), dg - ec[r]);
-                            }
-                        } else if (!root && ti == 0 && gr < K) {
-                            fx_tile<BIG>(D, fx1, B, lane);
-#pragma unroll
-                            for (int r = 0; r < 2; r++)
-                                if (g < K && Y + r < K) add(u + r * UX + g, fx_value(D, r), dg - ec[r]);
                         }
-                    }
+                    };
+                    if (first)
+                        x_pass(std::true_type());
+                    else
+                        x_pass(std::false_type());
                 }
                 fx_landed();
                 // y pass in place: a warp reads its 8 columns (Z, X') whole before it writes them
